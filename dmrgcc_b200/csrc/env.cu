@@ -13,6 +13,7 @@
 // :974-1060): per output bond index, blocks in row-major (first, second) sector
 // order, present wherever some contribution has a nonzero W.
 #include <algorithm>
+#include <map>
 
 #include "blocksparse.h"
 #include "gemm.cuh"
@@ -26,7 +27,11 @@ struct dmrg_env_s {
     int precision = DMRG_PREC_FP64;
     SiteDesc site;
     EnvDesc in, out;
-    GemmSchedule s1, s2;
+    GemmSchedule s1, s2;  // host description of both stages
+    // FP64: images of the ket and of the input environment, stage 1 into images, stage 2 into blocks
+    ImgPack img;
+    ImgSchedule i1, i2;
+    DeviceBuffer d_img, d_mid;
     SplitPlan p1, p2;  // split precisions: the same two stages on the tcgen05 path
     // the complex path (dmrg_zenv_create): the same stages on complex blocks
     bool cplx = false;
@@ -279,10 +284,64 @@ int build_right(dmrg_env_s& e) {
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-int dmrg_env_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg_blocks_t* ket, int d,
-                    int lb, int rb, const double* W, const dmrg_blocks_t* env_in, int precision, dmrg_env_t* out) {
+// The FP64 execution of s1 and s2 on packed operands (gemm_image.cu).  The ket's
+// images serve stage 1 (its A operand) and stage 2 (its B operand): left, both read
+// K^T; right, both read K.
+int build_images(dmrg_env_s& e, cudaStream_t st) {
+    const BlockListDesc& ket = e.site.ket;
+    std::map<int64_t, int64_t> ket_img, env_img, mid_img;  // by offset
+    for (int k = 0; k < ket.count(); ++k) {
+        if (ket.rows[k] == 0 || ket.cols[k] == 0) continue;
+        ket_img[ket.off[k]] = e.side == 0 ? e.img.add(0, ket.off[k], ket.cols[k], ket.rows[k], ket.cols[k], true)
+                                          : e.img.add(0, ket.off[k], ket.rows[k], ket.cols[k], ket.cols[k], false);
+    }
+    e.i1.panel = e.i2.panel = ImgSchedule::panel_for(e.s1.flops + e.s2.flops);
+    e.i1.out = kImgOutA;
+    int64_t mid = 0;
+    for (const GemmGroup& g : e.s1.groups) {
+        if (g.m <= 0 || g.n <= 0) continue;
+        mid_img[g.c_off] = mid;
+        e.i1.add_group(mid, 0, g.m, g.n);
+        mid += img_blocks(g.m, g.n);
+        for (int t = g.t0; t < g.t1; ++t) {
+            const GemmTerm& x = e.s1.terms[t];
+            if (x.k <= 0) continue;
+            auto it = env_img.find(x.b_off);
+            if (it == env_img.end()) it = env_img.emplace(x.b_off, e.img.add(1, x.b_off, g.n, x.k, x.ldb, true)).first;
+            e.i1.add_term(ket_img.at(x.a_off), it->second, x.k, x.scale);
+        }
+    }
+    for (const GemmGroup& g : e.s2.groups) {
+        e.i2.add_group(g.c_off, g.ldc, g.m, g.n);
+        for (int t = g.t0; t < g.t1; ++t) {
+            const GemmTerm& x = e.s2.terms[t];
+            if (x.k > 0 && g.m > 0 && g.n > 0) e.i2.add_term(mid_img.at(x.a_off), ket_img.at(x.b_off), x.k, x.scale);
+        }
+    }
+    // output blocks that no term reaches are groups too, so that stage 2 overwrites everything
+    std::map<int64_t, int> grouped;
+    for (const GemmGroup& g : e.s2.groups) grouped[g.c_off] = 1;
+    for (size_t o = 0; o < e.out.o.size(); ++o)
+        for (int q = 0; q < e.out.o[o].count(); ++q) {
+            const int64_t off = e.out.base[o] + e.out.o[o].off[q];
+            const int m = e.out.o[o].rows[q], n = e.out.o[o].cols[q];
+            if (m > 0 && n > 0 && !grouped.count(off)) e.i2.add_group(off, n, m, n);
+        }
+    DMRG_TRY(e.img.check_bounds(ket.size, e.in.size, 0));
+    DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, mid));
+    DMRG_TRY(e.i2.check_bounds(mid, e.img.blocks, e.out.size));
+    DMRG_TRY(e.img.finalize(e.i1.panel, st));
+    DMRG_TRY(e.i1.finalize(st, e.ctx->num_sms));
+    DMRG_TRY(e.i2.finalize(st, e.ctx->num_sms));
+    DMRG_TRY(e.d_img.alloc((size_t)std::max<int64_t>(e.img.blocks, 1) * kImgBlock * sizeof(double)));
+    return e.d_mid.alloc((size_t)std::max<int64_t>(mid, 1) * kImgBlock * sizeof(double));
+}
+
+// The common part of both creators: the structure, and for a real update its execution.
+int create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg_blocks_t* ket, int d, int lb, int rb,
+           const double* W, const dmrg_blocks_t* env_in, int precision, bool cplx, dmrg_env_t* out) {
     if (!ctx || !out || !env_in) return set_error(DMRG_E_ARG, "null argument");
     if (side != 0 && side != 1) return set_error(DMRG_E_ARG, "side must be 0 (left) or 1 (right)");
     if (precision != DMRG_PREC_FP64 && precision != DMRG_PREC_TF32X3 && precision != DMRG_PREC_BF16X3)
@@ -300,12 +359,11 @@ int dmrg_env_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, c
     cudaStream_t st = ctx->stream;
     if (rc == DMRG_OK) rc = e->s1.check_bounds(e->site.ket.size, e->in.size, e->scratch_size);
     if (rc == DMRG_OK) rc = e->s2.check_bounds(e->scratch_size, e->site.ket.size, e->out.size);
-    if (rc == DMRG_OK) rc = e->s1.finalize(64, 64, 16, st);
-    if (rc == DMRG_OK) rc = e->s2.finalize(64, 64, 16, st, ctx->num_sms);
-    if (rc == DMRG_OK) rc = e->scratch.alloc((size_t)std::max<int64_t>(e->scratch_size, 1) * sizeof(double));
+    if (rc == DMRG_OK && !cplx && precision == DMRG_PREC_FP64) rc = build_images(*e, st);
     if (rc == DMRG_OK && precision != DMRG_PREC_FP64) {
         const int fmt = precision == DMRG_PREC_BF16X3 ? kFmtBF16 : kFmtTF32;
-        rc = e->p1.build(e->s1, fmt, e->site.ket.size, e->in.size, e->scratch_size, st, ctx->num_sms);
+        rc = e->scratch.alloc((size_t)std::max<int64_t>(e->scratch_size, 1) * sizeof(double));
+        if (rc == DMRG_OK) rc = e->p1.build(e->s1, fmt, e->site.ket.size, e->in.size, e->scratch_size, st, ctx->num_sms);
         if (rc == DMRG_OK) rc = e->p2.build(e->s2, fmt, e->scratch_size, e->site.ket.size, e->out.size, st, ctx->num_sms);
     }
     if (rc != DMRG_OK) {
@@ -314,6 +372,15 @@ int dmrg_env_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, c
     }
     *out = e;
     return DMRG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int dmrg_env_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg_blocks_t* ket, int d,
+                    int lb, int rb, const double* W, const dmrg_blocks_t* env_in, int precision, dmrg_env_t* out) {
+    return create(ctx, side, nl, nr, phys, ket, d, lb, rb, W, env_in, precision, false, out);
 }
 
 int dmrg_env_destroy(dmrg_env_t e) {
@@ -353,18 +420,19 @@ int dmrg_env_flops(dmrg_env_t e, double* alg, double* exec) {
 int dmrg_env_apply(dmrg_env_t e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
     if (!e) return set_error(DMRG_E_ARG, "null env");
     cudaStream_t st = e->ctx->stream;
-    if (e->out.size) DMRG_CUDA_TRY(cudaMemsetAsync(env_out_dev, 0, (size_t)e->out.size * sizeof(double), st));
-    // Both sides: stage 1 reads (ket, env_in) into scratch, stage 2 reads
-    // (scratch, ket) into the output; the transposes live in the schedules.
+    // Both sides: stage 1 reads (ket, env_in), stage 2 its products and the ket.
     if (e->cplx) return set_error(DMRG_E_STATE, "a complex environment update runs through dmrg_zenv_apply");
     if (e->precision != DMRG_PREC_FP64) {  // tcgen05 split products, FP64 sums and FP64 storage
+        if (e->out.size) DMRG_CUDA_TRY(cudaMemsetAsync(env_out_dev, 0, (size_t)e->out.size * sizeof(double), st));
         DMRG_TRY(e->p1.run(ket_dev, env_in_dev, e->scratch.as<double>(), false, e->ctx->d_status, st));
         DMRG_TRY(e->p2.run(e->scratch.as<double>(), ket_dev, env_out_dev, true, e->ctx->d_status, st));
         return DMRG_OK;
     }
-    DMRG_TRY(launch_gemm_f64(e->s1, ket_dev, env_in_dev, e->scratch.as<double>(), false, st));
-    DMRG_TRY(launch_gemm_f64(e->s2, e->scratch.as<double>(), ket_dev, env_out_dev, true, st));
-    return DMRG_OK;
+    DMRG_TRY(launch_img_pack(e->img, e->i1.panel, 0, (int)e->img.chunks.size(), ket_dev, env_in_dev, nullptr,
+                             e->d_img.as<double>(), st));
+    DMRG_TRY(launch_img_gemm(e->i1, e->d_img.as<double>(), e->d_img.as<double>(), e->d_mid.as<double>(), false,
+                             e->ctx->d_status, st));
+    return launch_img_gemm(e->i2, e->d_mid.as<double>(), e->d_img.as<double>(), env_out_dev, false, e->ctx->d_status, st);
 }
 
 }  // extern "C"
@@ -389,7 +457,7 @@ int dmrg_zenv_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, 
     std::vector<double> ids(nw, 0.0);
     for (size_t i = 0; i < nw; ++i)
         if (W[2 * i] != 0.0 || W[2 * i + 1] != 0.0) ids[i] = (double)(i + 1);
-    DMRG_TRY(dmrg_env_create(ctx, side, nl, nr, phys, ket, d, lb, rb, ids.data(), env_in, DMRG_PREC_FP64, out));
+    DMRG_TRY(create(ctx, side, nl, nr, phys, ket, d, lb, rb, ids.data(), env_in, DMRG_PREC_FP64, true, out));
     dmrg_env_s* e = *out;
     auto convert = [&](const GemmSchedule& s, ZGemmSchedule& z, bool stage2, int conj) {
         z.reset();

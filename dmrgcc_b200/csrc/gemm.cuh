@@ -45,6 +45,8 @@ struct GemmSplit {
     int m;
     int n;
     int chunks;
+    int ticket;  // packed FP64 path: the tile's arrival counter
+    int pad_;
 };
 
 struct GemmTile {
@@ -104,6 +106,118 @@ struct GemmSchedule {
 // C (+)= sum of terms for every tile of `s`.  A, B, C are the base pointers.
 int launch_gemm_f64(const GemmSchedule& s, const double* A, const double* B, double* C,
                     bool accumulate, cudaStream_t stream);
+
+// ---------------------------------------------------------------------------
+// The same products on packed operands (gemm_image.cu): the form behind H_eff*psi
+// and the environment updates, whose operand tiles are read many times.
+//
+// An operand block X (rows x k; rows = output rows of an A operand, output columns
+// of a B operand, so both roles share one format) is packed once per application
+// into an image of 512-byte blocks.  Block (u, q) holds rows 8u .. 8u+7 and k
+// indices 8q .. 8q+7 in the order in which a warp's lanes hold DMMA fragments: lane
+// 4 (r mod 8) + (c mod 4) owns elements (r, c) and (r, c + 4), zero outside X.
+// Blocks are ordered by panel of `panel` rows (a schedule's tile extent), then by
+// slice of 32 k indices, then by u, then by q: the operand of one k-step of one
+// tile is one contiguous run of blocks.
+constexpr int kImgBlock = 64;  // doubles per block
+constexpr int kImgSlice = 4;   // blocks of k (of 8) per slice
+inline int64_t img_units(int extent) { return (extent + 7) / 8; }
+inline int64_t img_blocks(int rows, int k) { return img_units(rows) * img_units(k); }
+
+struct ImgJob {        // one operand block to pack
+    int64_t src_off;   // doubles, into its source
+    int64_t img;       // first block of its image
+    int rows, k, ld;   // X(r, c) = src[src_off + (trans ? c * ld + r : r * ld + c)]
+    int trans;
+    int src;           // which of the launch's sources
+    int pad_;
+};
+struct ImgChunk {      // one (panel, slice) of a job
+    int job, panel, slice, pad_;
+};
+struct ImgPack {
+    std::vector<ImgJob> jobs;
+    std::vector<ImgChunk> chunks;
+    int64_t blocks = 0;
+    DeviceBuffer d_jobs, d_chunks;
+    // Appends an operand block; returns its image (first block).
+    int64_t add(int src, int64_t src_off, int rows, int k, int ld, bool trans);
+    // Every read inside sources of the given sizes (doubles); DMRG_E_ARG otherwise.
+    int check_bounds(int64_t n0, int64_t n1, int64_t n2) const;
+    // Builds the chunk list for panels of `panel` rows and uploads.
+    int finalize(int panel, cudaStream_t stream);
+    std::vector<int> first_chunk;  // chunks before each job, and in all
+};
+// Packs the jobs of chunks [c0, c1) from the three sources into img.
+int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
+                    double* img, cudaStream_t stream);
+
+struct ImgTerm {
+    int64_t a, b;  // images (first blocks) of the two operands
+    int k;
+    int kb;        // blocks of k: ceil(k / 8)
+    double scale;
+};
+struct ImgGroup {
+    int64_t c_off;  // FP64 output: its offset; image output: the image's first block
+    int ldc;
+    int m, n;
+    int t0, t1;
+    int pad_;
+};
+// `steps` k-steps (slices) of one output tile, from slice k0 of term t0 on,
+// executed by one CTA.
+struct ImgSegment {
+    int64_t c_off;
+    int64_t aux_off; // its place in the aux buffer, if it is a part
+    int ldc;
+    int rows, cols;
+    int pm, pn;      // tile (panel) indices
+    int t0, t1;      // its first term; the end of the group's
+    int k0, steps;
+    int split;       // -1: the whole tile; else its GemmSplit: a part
+    int out_kb;      // image output: blocks of k of the output image
+    int pad_;
+};
+enum ImgOut {
+    kImgOutBlock = 0,   // row-major FP64 blocks
+    kImgOutB = 1,       // images of the transposed output: rows = columns n, k = rows m (a B operand)
+    kImgOutA = 2        // images of the output: rows = rows m, k = columns n (an A operand)
+};
+struct ImgSchedule {
+    std::vector<ImgTerm> terms;
+    std::vector<ImgGroup> groups;
+    int out = kImgOutBlock;
+    int panel = 64;         // tile extent: 64 or 32
+    bool scaled = false;    // some term's scale is not 1
+    std::vector<ImgSegment> segments;  // the queue: largest first
+    int ctas = 0;
+    std::vector<GemmSplit> splits;
+    int64_t aux_size = 0;
+    // tickets: the queue's two counters, then one per split tile; zero between launches
+    DeviceBuffer d_terms, d_segments, d_splits, tickets, aux;
+
+    void add_group(int64_t c_off, int ldc, int m, int n) {
+        groups.push_back(ImgGroup{c_off, ldc, m, n, (int)terms.size(), (int)terms.size(), 0});
+    }
+    void add_term(int64_t a, int64_t b, int k, double scale) {
+        terms.push_back(ImgTerm{a, b, k, (int)img_units(k), scale});
+        groups.back().t1 = (int)terms.size();
+    }
+    // The tile extent for a product of `flops`.
+    static int panel_for(double flops);
+    // Every image read and output write inside buffers of the given sizes (blocks;
+    // doubles for a block output); DMRG_E_ARG otherwise.
+    int check_bounds(int64_t a_blocks, int64_t b_blocks, int64_t out_size) const;
+    // Cuts the groups into tiles and long tiles into parts, orders the queue and
+    // uploads.  Groups without terms are part of it: a launch that does not
+    // accumulate writes zeros.
+    int finalize(cudaStream_t stream, int num_sms);
+};
+// C (+)= the products (block output), or the images of them into C (accumulate
+// is then ignored).  A wait that gives up sets *status = DMRG_E_NUMERIC.
+int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
+                    cudaStream_t stream);
 
 // ---------------------------------------------------------------------------
 // Split-precision paths on the tcgen05 tensor cores (gemm_split.cu).

@@ -1,0 +1,702 @@
+// FP64 grouped multi-term block GEMM on packed operand images (gemm.cuh), on the
+// FP64 tensor path (DMMA, mma.sync.m8n8k4.f64; tcgen05 has no f64 kind).
+//
+// Why packed.  The raw blocks are ragged (1 to ~200 rows) with offsets and leading
+// dimensions of any parity, so neither TMA tensor maps nor 16-byte loads fit them,
+// and 8-byte cp.async, with their addresses, cost as much time as they leave for
+// DMMAs (gemm_f64.cu: 77% DMMA pipe, but 1.5 times the algorithmic FLOPs in
+// padding; with the padding trimmed the same loads hold the pipe at 64%).  Every
+// operand tile is read by several tiles and terms, so the blocks are packed once
+// per application, in the order in which a warp's lanes hold DMMA fragments: a
+// k-step's operands are then two bulk copies (cp.async.bulk, up to 16 KB each), a
+// fragment pair is one conflict-free 16-byte shared load, k needs no masks, and
+// the first product of a chain leaves its result as the next one's image with
+// fully coalesced 512-byte stores.
+//
+// GEMM CTA: four consumer warps (2 x 2 quarters of the tile, MI x NJ units of 8x8
+// each) and a producer warp that issues the copies; steps are handed over by
+// mbarriers, so warps and tiles overlap.  All waits are bounded.
+//
+// Split of the work: two persistent CTAs per SM take tiles, largest first, from a
+// queue (equal shares dealt out beforehand left SMs idle for a fifth of a D=1024
+// launch: the time of a step depends on what the SM's other CTA runs).  A long tile
+// is cut into parts, summed in order by the last CTA to finish one.
+//
+// Measured, one H_eff*psi of the 8x4 cylinder's middle site: D=1024 216 -> 184 us
+// (pack 10, first stage 70, second 105; its DMMAs alone 104 us at the 37 TFLOP/s of
+// a register-only loop), D=300 59 -> 22.5 us, 16-site chain at D=64 21.5 -> 15.5 us.
+// What bounds it now: at D=1024 the DMMA pipe (75% busy; the rest is the tiles'
+// epilogues with one other CTA to cover them, and the last tiles); below D~300 three
+// launches' latency and the k-step chain of one tile.
+#include <algorithm>
+#include <atomic>
+
+#include "gemm.cuh"
+
+namespace dmrg {
+namespace {
+
+constexpr int kConsumers = 128;            // threads of the four consumer warps
+constexpr int kThreads = kConsumers + 32;  // and the producer warp
+constexpr int kMaxPolls = 1 << 22;         // of a wait, before it gives up
+
+constexpr int kCtasPerSm = 2;
+constexpr int kRegs = 168;                     // per thread: at most 3 of the 10 warps share a sub-core's registers
+// Operand ring.  A step takes only the space of its own blocks, so that narrow
+// tiles keep many steps in flight.
+constexpr int kSlots = 16;                     // steps in flight, at most
+constexpr int kRing = 106 * 1024;              // bytes
+constexpr int kPad = kImgSlice * kImgBlock * 8;  // a quarter with an odd unit reads one unit further
+
+struct Tile {  // a segment, as the consumers need it
+    int64_t c_off, aux_off;
+    int ldc, rows, cols, pm, pn, out_kb, steps, split;
+};
+struct StepMeta {  // of the step in a slot
+    double scale;
+    int kb;        // blocks of k
+    int off;       // its operands in the ring (bytes): A's blocks, then B's
+};
+constexpr int kTiles = kSlots + 1;  // every tile has a step
+struct Shared {
+    StepMeta meta[kSlots];
+    uint64_t full[kSlots], empty[kSlots];
+    Tile tiles[kTiles];
+    int last;
+};
+constexpr size_t kSmem = kRing + kPad + sizeof(Shared);
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned bar, int count) {
+    asm volatile("mbarrier.init.shared.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the barrier's phase `parity`; false when it gave up.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+    for (int n = 0; n < kMaxPolls; ++n) {
+        unsigned done;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_copy(unsigned dst, const double* src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// Programmatic dependent launch: wait_previous returns when the launch before this one
+// on the stream has completed and its writes are visible, so launch latency and the
+// first descriptor reads pass behind its last CTAs (D=300 matvec 30 -> 22.5 us).
+// launch_next lets the next launch in early: the pack kernel does; the GEMM kernel
+// leaves it to its CTAs' exits (the next launch's waiting CTAs would take the shared
+// memory of its own: Lanczos at D=512 1.27 -> 1.33 ms).
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory"); }
+
+__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+        : "+d"(d0), "+d"(d1)
+        : "d"(a), "d"(b));
+}
+
+struct GemmArgs {
+    const double *A, *B;
+    double *C, *aux;
+    const ImgTerm* terms;
+    const ImgSegment* segments;
+    int nsegments;
+    int units;        // 8-row units of a full panel
+    const GemmSplit* splits;
+    unsigned* tickets;  // of the split tiles, after the queue's two counters
+    int* status;
+    int accumulate;
+};
+
+// Where a tile's units go in an image output: the image's rows are the tile's
+// columns (B role) or rows (A role), its k indices the other side's.
+template <int OUT>
+struct ImageOut {
+    double* base;   // the panel's first block
+    int units, k0;  // row units of the panel; k unit of the tile's first unit
+    int kb_all;
+    __device__ __forceinline__ ImageOut(const GemmArgs& w, const Tile& g) {
+        units = ((OUT == kImgOutB ? g.cols : g.rows) + 7) >> 3;
+        k0 = (OUT == kImgOutB ? g.pm : g.pn) * w.units;
+        kb_all = g.out_kb;
+        base = w.C + (g.c_off + (int64_t)(OUT == kImgOutB ? g.pn : g.pm) * w.units * g.out_kb) * kImgBlock;
+    }
+    // Block of k unit `k` (of the tile) and row unit 0; `pitch`: to the next row unit.
+    __device__ __forceinline__ double* column(int k, int& pitch) const {
+        const int s = (k0 + k) / kImgSlice;
+        pitch = min(kImgSlice, kb_all - s * kImgSlice) * kImgBlock;
+        return base + (units * s * kImgSlice + (k0 + k) % kImgSlice) * kImgBlock;
+    }
+};
+// Element (r, c) of a unit in its block; c even: element (r, c + 1) is kPairStep further.
+template <int OUT>
+__device__ __forceinline__ int out_element(int r, int c) {
+    const int x = OUT == kImgOutB ? c : r, k = OUT == kImgOutB ? r : c;
+    return (4 * x + (k & 3)) * 2 + (k >> 2);
+}
+template <int OUT>
+constexpr int kPairStep = OUT == kImgOutB ? 8 : 2;
+
+// The consumer warps' work on one tile or part.  The unit counts are template
+// parameters of the whole loop (as run-time counts, or in a switch inside it, the
+// accumulators move between registers at every step).  SCALED: terms have scales
+// other than 1 (the products cost ~8% of the loop).
+template <int OUT, bool SCALED, int MI, int NJ>
+__device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const char* ring, Shared& sh, unsigned full,
+                                         unsigned empty, int& step, bool& ok) {
+    const StepMeta* meta = sh.meta;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int um0 = (warp >> 1) * MI, un0 = (warp & 1) * NJ, ua = (g.rows + 7) >> 3;
+    double acc[MI][NJ][2];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    auto block = [&](const double2* As, const double2* Bs, int stride, double scale) {
+        double2 a[MI], b[NJ];
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            a[i] = As[i * stride];
+            if (SCALED) {
+                a[i].x *= scale;
+                a[i].y *= scale;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) b[j] = Bs[j * stride];
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i].x, b[j].x);
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i].y, b[j].y);
+    };
+#pragma unroll 1
+    for (int n = max(g.steps, 1); n > 0; --n) {  // (one empty step without terms)
+        const int s = step % kSlots;
+        ok = ok && mbar_wait(full + 8 * s, (step / kSlots) & 1);
+        const double scale = SCALED ? meta[s].scale : 1.0;
+        const int kb = meta[s].kb;
+        const double2* As = reinterpret_cast<const double2*>(ring + meta[s].off) + lane;
+        const double2* Bs = As + ua * kb * 32;
+        if (kb == kImgSlice) {
+#pragma unroll
+            for (int q = 0; q < kImgSlice; ++q)
+                block(As + (um0 * kImgSlice + q) * 32, Bs + (un0 * kImgSlice + q) * 32, kImgSlice * 32, scale);
+        } else {
+#pragma unroll 1
+            for (int q = 0; q < kb; ++q) block(As + (um0 * kb + q) * 32, Bs + (un0 * kb + q) * 32, kb * 32, scale);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + 8 * s);
+        ++step;
+    }
+    if (g.split >= 0) {
+        // A part of a cut tile goes to the aux buffer as the threads hold it; the last CTA
+        // to finish one of the tile's parts sums them, in order, and resets the ticket.
+        const GemmSplit sp = w.splits[g.split];
+        constexpr int kPart = MI * NJ * kConsumers;  // double2 per part
+        double2* part = reinterpret_cast<double2*>(w.aux + g.aux_off) + threadIdx.x;
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) part[(i * NJ + j) * kConsumers] = make_double2(acc[i][j][0], acc[i][j][1]);
+        consumer_sync();  // every warp's part is written before the ticket is taken
+        if (threadIdx.x == 0) {
+            unsigned* tk = w.tickets + 2 + sp.ticket;
+            unsigned before;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(tk) : "memory");
+            sh.last = before == (unsigned)sp.chunks - 1;
+            if (sh.last) *tk = 0u;
+        }
+        consumer_sync();
+        if (!sh.last) return;
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        const double2* src = reinterpret_cast<const double2*>(w.aux + sp.aux_off) + threadIdx.x;
+#pragma unroll 1
+        for (int ch = 0; ch < sp.chunks; ++ch, src += kPart) {
+            double2 v[MI][NJ];
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) v[i][j] = __ldcg(src + (i * NJ + j) * kConsumers);
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    acc[i][j][0] += v[i][j].x;
+                    acc[i][j][1] += v[i][j].y;
+                }
+        }
+    }
+    const int fr = lane >> 2, fc = lane & 3;
+    if (OUT != kImgOutBlock) {  // whole units, zero outside the block
+        const ImageOut<OUT> image(w, g);
+        const int el = out_element<OUT>(fr, 2 * fc), rleft = g.rows - 8 * um0 - fr, cleft = g.cols - 8 * un0 - 2 * fc;
+        constexpr int KU = OUT == kImgOutB ? MI : NJ, XU = OUT == kImgOutB ? NJ : MI;  // k units, row units
+#pragma unroll
+        for (int k = 0; k < KU; ++k) {
+            int pitch;
+            double* col = image.column((OUT == kImgOutB ? um0 : un0) + k, pitch) + el;
+#pragma unroll
+            for (int x = 0; x < XU; ++x) {
+                const int i = OUT == kImgOutB ? k : x, j = OUT == kImgOutB ? x : k;
+                if (8 * (um0 + i) >= g.rows || 8 * (un0 + j) >= g.cols) continue;
+                double* o = col + ((OUT == kImgOutB ? un0 : um0) + x) * pitch;
+                o[0] = 8 * i < rleft && 8 * j < cleft ? acc[i][j][0] : 0.0;
+                o[kPairStep<OUT>] = 8 * i < rleft && 8 * j + 1 < cleft ? acc[i][j][1] : 0.0;
+            }
+        }
+        return;
+    }
+    const bool add = w.accumulate;
+    double* crow = w.C + g.c_off + (int64_t)(8 * um0 + fr) * g.ldc + 8 * un0 + 2 * fc;
+    const int rleft = g.rows - 8 * um0 - fr, cleft = g.cols - 8 * un0 - 2 * fc;
+#pragma unroll
+    for (int i = 0; i < MI; ++i, crow += 8 * (int64_t)g.ldc) {
+        if (8 * i >= rleft) break;
+        double old[NJ][2];
+        if (add) {
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) old[j][e] = 8 * j + e < cleft ? crow[8 * j + e] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (8 * j + e < cleft) crow[8 * j + e] = add ? old[j][e] + acc[i][j][e] : acc[i][j][e];
+    }
+}
+
+// The producer warp: takes segments from the queue (its first is its CTA's own) and
+// issues every step's copies in order.  The next segment's index, descriptor and
+// first terms are requested after this segment's first, second and third step, so
+// that each round trip passes behind a step (in one go, they held the first stage at
+// D=1024 at 75 us).  A segment's terms are read 32 at a time, one per lane.
+__device__ __forceinline__ void produce(const GemmArgs& w, char* ring, Shared& sh) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = smem_u32(sh.full), empty = smem_u32(sh.empty);
+    bool ok = true;
+    int n = 0, oldest = 0;   // steps issued; the oldest one not released yet
+    int head = 0, tail = 0;  // ring: end of the newest step, start of the oldest
+    // room for a step of `need` bytes: after the newest one, or at the ring's start; < 0: gave up
+    auto room = [&](int need) {
+        for (;;) {
+            int at;
+            if (oldest == n) at = 0;
+            else if (n - oldest == kSlots) at = -1;
+            else if (head > tail) at = head + need <= kRing ? head : need <= tail ? 0 : -1;
+            else at = head + need <= tail ? head : -1;
+            if (at >= 0) {
+                if (oldest == n) tail = at;
+                head = at + need;
+                return at;
+            }
+            if (!mbar_wait(empty + 8 * (oldest % kSlots), (oldest / kSlots) & 1)) return -1;
+            if (++oldest < n) tail = sh.meta[oldest % kSlots].off;
+        }
+    };
+    auto term_of = [&](const ImgSegment& g, int t) { return w.terms[min(g.t0 + t, g.t1)]; };  // entry t1 is readable
+    auto segment = [&](int i) { return w.segments[min(i, w.nsegments - 1)]; };
+    int idx = blockIdx.x, claim = 0, tiles = 0;
+    ImgSegment next = segment(idx);
+    ImgTerm first = term_of(next, lane);
+    wait_previous();  // the operands; before any step, so the consumers' writes are ordered as well
+    for (; idx < w.nsegments && ok; ++tiles) {
+        const ImgSegment g = next;
+        ImgTerm mine = first;
+        int ahead = 0;
+        auto look_ahead = [&]() {
+            if (ahead == 0) {
+                if (lane == 0) claim = (int)(gridDim.x + atomicAdd(w.tickets, 1u));
+            } else if (ahead == 1) {
+                idx = __shfl_sync(0xffffffffu, claim, 0);
+                next = segment(idx);
+            } else if (ahead == 2) {
+                first = term_of(next, lane);
+            }
+            ++ahead;
+        };
+        const int ua = (g.rows + 7) >> 3, ub = (g.cols + 7) >> 3;
+        int ti = 0, slice = g.k0;
+        for (int left = max(g.steps, 1); left > 0; --left) {  // a segment without terms: one empty step
+            int64_t ta = 0, tb = 0;
+            int tkb = 0;
+            double scale = 1.0;
+            if (g.steps > 0) {
+                for (;;) {
+                    tkb = __shfl_sync(0xffffffffu, mine.kb, ti & 31);
+                    if (slice * kImgSlice < tkb) break;
+                    slice = 0;
+                    if ((++ti & 31) == 0) mine = term_of(g, ti + lane);
+                }
+                ta = __shfl_sync(0xffffffffu, mine.a, ti & 31);
+                tb = __shfl_sync(0xffffffffu, mine.b, ti & 31);
+                scale = __shfl_sync(0xffffffffu, mine.scale, ti & 31);
+            }
+            const int kb = min(kImgSlice, tkb - slice * kImgSlice), bytes = kb * kImgBlock * 8, need = (ua + ub) * bytes;
+            const int at = room(need);
+            ok = at >= 0;
+            if (!ok) break;
+            const int s = n % kSlots;
+            if (lane == 0) {
+                if (left == max(g.steps, 1))
+                    sh.tiles[tiles % kTiles] = Tile{g.c_off, g.aux_off, g.ldc, g.rows, g.cols, g.pm, g.pn, g.out_kb, g.steps, g.split};
+                sh.meta[s].scale = scale;
+                sh.meta[s].kb = kb;
+                sh.meta[s].off = at;
+                const unsigned dst = smem_u32(ring) + at;
+                const int64_t panel = (int64_t)w.units * tkb;
+                mbar_expect(full + 8 * s, need);
+                if (need) {
+                    bulk_copy(dst, w.A + (ta + g.pm * panel + ua * slice * kImgSlice) * kImgBlock, ua * bytes, full + 8 * s);
+                    bulk_copy(dst + ua * bytes, w.B + (tb + g.pn * panel + ub * slice * kImgSlice) * kImgBlock, ub * bytes,
+                              full + 8 * s);
+                }
+            }
+            __syncwarp();
+            ++slice;
+            ++n;
+            look_ahead();
+        }
+        while (ahead < 3) look_ahead();
+    }
+    // the end: a step without a tile.  Then the queue's counters are reset by the last CTA out.
+    if (ok) ok = room(0) >= 0;
+    if (lane == 0) {
+        if (ok) {
+            sh.tiles[tiles % kTiles].steps = -1;
+            mbar_expect(full + 8 * (n % kSlots), 0);
+        } else {  // gave up: the copies in flight first (bounded), then leave; the consumers give up too
+            if (w.status) *w.status = DMRG_E_NUMERIC;
+            for (int i = oldest; i < n; ++i) mbar_wait(full + 8 * (i % kSlots), (i / kSlots) & 1);
+        }
+        if (atomicAdd(w.tickets + 1, 1u) == gridDim.x - 1) {
+            w.tickets[0] = 0u;
+            w.tickets[1] = 0u;
+        }
+    }
+}
+
+template <int OUT, bool SCALED>
+__global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
+    extern __shared__ __align__(128) char ring[];
+    Shared& sh = *reinterpret_cast<Shared*>(ring + kRing + kPad);
+    const unsigned full = smem_u32(sh.full), empty = smem_u32(sh.empty);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kSlots; ++s) {
+            mbar_init(full + 8 * s, 1);
+            mbar_init(empty + 8 * s, kConsumers / 32);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x >= kConsumers) {
+        produce(w, ring, sh);
+        return;
+    }
+    bool ok = true;
+    int step = 0;  // steps computed (slot = step % kSlots, its phase = step / kSlots)
+#pragma unroll 1
+    for (int tile = 0;; ++tile) {
+        // the tile's first step carries its descriptor
+        if (!mbar_wait(full + 8 * (step % kSlots), (step / kSlots) & 1)) {
+            if (w.status) *w.status = DMRG_E_NUMERIC;
+            return;
+        }
+        const Tile g = sh.tiles[tile % kTiles];
+        if (g.steps < 0) return;
+        switch (((g.rows + 15) >> 4) * 4 + ((g.cols + 15) >> 4) - 5) {  // units per warp
+#define DMRG_UNITS(MI, NJ)                                                                        \
+    case (MI - 1) * 4 + NJ - 1:                                                                   \
+        run_tile<OUT, SCALED, MI, NJ>(w, g, ring, sh, full, empty, step, ok);                \
+        break;
+#define DMRG_UNIT_ROW(MI) DMRG_UNITS(MI, 1) DMRG_UNITS(MI, 2) DMRG_UNITS(MI, 3) DMRG_UNITS(MI, 4)
+            DMRG_UNIT_ROW(1)
+            DMRG_UNIT_ROW(2)
+            DMRG_UNIT_ROW(3)
+            DMRG_UNIT_ROW(4)
+#undef DMRG_UNIT_ROW
+#undef DMRG_UNITS
+            default: break;
+        }
+        if (!ok) {
+            if (w.status) *w.status = DMRG_E_NUMERIC;
+            return;
+        }
+    }
+}
+
+// One (panel, slice) of a job per CTA; thread = lane of a block: two elements of the
+// source (k indices 4 apart) to one 16-byte store.  A warp reads 8 rows of 32 + 32
+// contiguous bytes (or, transposed, 4 + 4 rows of 64) and writes 512.
+constexpr int kPackThreads = 256;
+__global__ void __launch_bounds__(kPackThreads) img_pack_kernel(const ImgJob* __restrict__ jobs,
+                                                                const ImgChunk* __restrict__ chunks, int panel,
+                                                                const double* __restrict__ s0,
+                                                                const double* __restrict__ s1,
+                                                                const double* __restrict__ s2,
+                                                                double* __restrict__ img) {
+    const ImgChunk ch = chunks[blockIdx.x];
+    const ImgJob j = jobs[ch.job];
+    launch_next();
+    wait_previous();  // the sources are written, and the images' last readers are done
+    const double* src = (j.src == 0 ? s0 : j.src == 1 ? s1 : s2) + j.src_off;
+    const int kb_all = (j.k + 7) >> 3, kb = min(kImgSlice, kb_all - ch.slice * kImgSlice);
+    const int r0 = ch.panel * panel, units = (min(panel, j.rows - r0) + 7) >> 3, k0 = ch.slice * kImgSlice * 8;
+    double2* out = reinterpret_cast<double2*>(img) +
+                   (j.img + (int64_t)ch.panel * (panel / 8) * kb_all + (int64_t)units * ch.slice * kImgSlice) * 32;
+    const int lane = threadIdx.x & 31;
+    for (int b = threadIdx.x >> 5; b < units * kb; b += kPackThreads / 32) {
+        const int u = b / kb, q = b - u * kb;
+        const int r = r0 + 8 * u + (lane >> 2), c = k0 + 8 * q + (lane & 3);
+        double2 v = make_double2(0.0, 0.0);
+        if (r < j.rows) {
+            if (c < j.k) v.x = src[j.trans ? (int64_t)c * j.ld + r : (int64_t)r * j.ld + c];
+            if (c + 4 < j.k) v.y = src[j.trans ? (int64_t)(c + 4) * j.ld + r : (int64_t)r * j.ld + c + 4];
+        }
+        out[(int64_t)b * 32 + lane] = v;
+    }
+}
+
+// The kernel's dynamic shared memory is above the 48 KB default: raises its
+// allowance, once per device.
+template <class K>
+int allow_smem(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    DMRG_CUDA_TRY(cudaGetDevice(&dev));
+    const uint64_t bit = uint64_t(1) << (dev & 63);
+    if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return DMRG_OK;
+    DMRG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    done.fetch_or(bit, std::memory_order_release);
+    return DMRG_OK;
+}
+
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    count_launch();
+    DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return DMRG_OK;
+}
+
+template <int OUT, bool SCALED>
+int launch(int n, const GemmArgs& w, cudaStream_t st) {
+    static std::atomic<uint64_t> allowed{0};
+    DMRG_TRY(allow_smem(img_gemm_kernel<OUT, SCALED>, kSmem, allowed));
+    return launch_pdl(img_gemm_kernel<OUT, SCALED>, n, kThreads, kSmem, st, w);
+}
+
+// The schedule's cost model (cycles of a step and of a tile's own work) and cuts.
+constexpr int64_t kStepFixed = 400, kTileFixed = 2000;
+// k-steps of a part of a cut tile, at least: a part costs a round trip through the aux
+// buffer (D=300: 22.5 us; with parts of 4 steps 26.5, of 2 steps 40, uncut 28).
+constexpr int kMinPart = 8;
+// Products below use 32-wide tiles, see panel_for.
+constexpr double kSmallFlops = 4e8;
+
+// One k-step of a tile: 16 cycles per DMMA and sub-core.
+int64_t step_cost(int rows, int cols) {
+    return (int64_t)((rows + 15) / 16) * ((cols + 15) / 16) * kImgSlice * 2 * 16 + kStepFixed;
+}
+int steps_of(const ImgTerm& t) { return (t.kb + kImgSlice - 1) / kImgSlice; }
+
+}  // namespace
+
+int64_t ImgPack::add(int src, int64_t src_off, int rows, int k, int ld, bool trans) {
+    const int64_t img = blocks;
+    jobs.push_back(ImgJob{src_off, img, rows, k, ld, trans ? 1 : 0, src, 0});
+    blocks += img_blocks(rows, k);
+    return img;
+}
+
+int ImgPack::check_bounds(int64_t n0, int64_t n1, int64_t n2) const {
+    const int64_t sizes[3] = {n0, n1, n2};
+    for (const ImgJob& j : jobs) {
+        if (j.rows <= 0 || j.k <= 0) continue;
+        const int64_t end = j.src_off + (j.trans ? (int64_t)(j.k - 1) * j.ld + j.rows : (int64_t)(j.rows - 1) * j.ld + j.k);
+        if (j.src_off < 0 || end > sizes[j.src])
+            return set_error(DMRG_E_ARG, "packed operand %lld (%dx%d, ld %d) outside %lld", (long long)j.src_off, j.rows, j.k,
+                             j.ld, (long long)sizes[j.src]);
+    }
+    return DMRG_OK;
+}
+
+int ImgPack::finalize(int panel, cudaStream_t stream) {
+    chunks.clear();
+    first_chunk.assign(1, 0);
+    for (int j = 0; j < (int)jobs.size(); ++j) {
+        const int slices = (int)((img_units(jobs[j].k) + kImgSlice - 1) / kImgSlice);
+        for (int p = 0; p * panel < jobs[j].rows; ++p)
+            for (int s = 0; s < slices; ++s) chunks.push_back(ImgChunk{j, p, s, 0});
+        first_chunk.push_back((int)chunks.size());
+    }
+    DMRG_TRY(upload(d_jobs, jobs, stream));
+    return upload(d_chunks, chunks, stream);
+}
+
+int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
+                    double* img, cudaStream_t stream) {
+    if (c1 <= c0) return DMRG_OK;
+    return launch_pdl(img_pack_kernel, c1 - c0, kPackThreads, 0, stream, p.d_jobs.as<ImgJob>(),
+                      p.d_chunks.as<ImgChunk>() + c0, panel, s0, s1, s2, img);
+}
+
+// A 64x64 tile's k-step takes a CTA about a microsecond: with few of them, whole
+// blocks sit on few SMs.  Both widths measured: D=300 (0.1 GFLOP) 22.5 us in 32-wide
+// tiles, 28 us in 64-wide ones; D=512 (0.5 GFLOP) the same to 2%; D=1024 64-wide,
+// whose operand traffic is half.
+int ImgSchedule::panel_for(double flops) { return flops < kSmallFlops ? 32 : 64; }
+
+int ImgSchedule::check_bounds(int64_t a_blocks, int64_t b_blocks, int64_t out_size) const {
+    for (const ImgGroup& g : groups) {
+        if (g.m <= 0 || g.n <= 0) continue;
+        const int64_t end = out == kImgOutBlock ? g.c_off + (int64_t)(g.m - 1) * g.ldc + g.n : g.c_off + img_blocks(g.m, g.n);
+        if (g.c_off < 0 || end > out_size || (out == kImgOutBlock && g.n > g.ldc))
+            return set_error(DMRG_E_ARG, "packed GEMM output %lld (%dx%d) outside %lld", (long long)g.c_off, g.m, g.n,
+                             (long long)out_size);
+        for (int t = g.t0; t < g.t1; ++t) {
+            const ImgTerm& x = terms[t];
+            if (x.k <= 0) continue;
+            if (x.a < 0 || x.b < 0 || x.a + img_blocks(g.m, x.k) > a_blocks || x.b + img_blocks(g.n, x.k) > b_blocks)
+                return set_error(DMRG_E_ARG, "packed GEMM operand outside its images");
+        }
+    }
+    return DMRG_OK;
+}
+
+int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
+    segments.clear();
+    splits.clear();
+    aux_size = 0;
+    scaled = false;
+    if (num_sms <= 0) num_sms = 148;
+    std::vector<ImgTerm> live;  // terms with k-steps, by group
+    struct Tile {
+        int group, pm, pn, rows, cols;
+        int64_t steps, cost;  // k-steps; cycles of one
+    };
+    std::vector<Tile> tiles;
+    std::vector<ImgGroup> gr;
+    int64_t cost = 0;
+    for (const ImgGroup& g : groups) {
+        if (g.m <= 0 || g.n <= 0) continue;
+        ImgGroup x = g;
+        x.t0 = (int)live.size();
+        int64_t ks = 0;
+        for (int t = g.t0; t < g.t1; ++t)
+            if (terms[t].k > 0) {
+                live.push_back(terms[t]);
+                scaled = scaled || terms[t].scale != 1.0;
+                ks += steps_of(terms[t]);
+            }
+        x.t1 = (int)live.size();
+        for (int pm = 0; pm * panel < g.m; ++pm)
+            for (int pn = 0; pn * panel < g.n; ++pn) {
+                Tile t{(int)gr.size(), pm, pn, std::min(panel, g.m - pm * panel), std::min(panel, g.n - pn * panel), ks, 0};
+                t.cost = step_cost(t.rows, t.cols);
+                cost += ks * t.cost + kTileFixed;
+                tiles.push_back(t);
+            }
+        gr.push_back(x);
+    }
+    // a tile longer than a quarter of a CTA's share is cut into equal parts (a sixth or a
+    // tenth: no gain at D=1024)
+    const int64_t longest = std::max<int64_t>(1, cost / ((int64_t)num_sms * kCtasPerSm) / 4);
+    int ntickets = 0;
+    std::vector<std::pair<int64_t, int>> order;  // cost, segment
+    for (const Tile& t : tiles) {
+        const ImgGroup& g = gr[t.group];
+        const int64_t c_off = out == kImgOutBlock ? g.c_off + (int64_t)t.pm * panel * g.ldc + t.pn * panel : g.c_off;
+        int64_t parts = std::min((t.steps * t.cost + longest - 1) / longest, t.steps / kMinPart);
+        parts = std::max<int64_t>(parts, 1);
+        if (parts > 1) splits.push_back(GemmSplit{c_off, aux_size, g.ldc, t.rows, t.cols, (int)parts, ntickets++, 0});
+        for (int64_t k = 0; k < parts; ++k) {
+            const int64_t s0 = t.steps * k / parts, s1 = t.steps * (k + 1) / parts;
+            int64_t skip = s0;  // the part's first slice: its term, and the slice in it
+            ImgSegment s{};
+            s.c_off = c_off;
+            s.ldc = g.ldc;
+            s.rows = t.rows;
+            s.cols = t.cols;
+            s.pm = t.pm;
+            s.pn = t.pn;
+            s.steps = (int)(s1 - s0);
+            s.t0 = g.t0;
+            s.t1 = g.t1;
+            while (s.t0 < g.t1 && skip >= steps_of(live[s.t0])) skip -= steps_of(live[s.t0++]);
+            s.k0 = (int)skip;
+            s.split = -1;
+            s.out_kb = (int)img_units(out == kImgOutB ? g.m : g.n);
+            if (parts > 1) {
+                s.split = (int)splits.size() - 1;
+                s.aux_off = aux_size;
+                aux_size += (int64_t)((t.rows + 15) / 16) * ((t.cols + 15) / 16) * 2 * kConsumers;
+            }
+            order.push_back({s.steps * t.cost, (int)segments.size()});
+            segments.push_back(s);
+        }
+    }
+    // the queue: largest first
+    std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+    std::vector<ImgSegment> queue;
+    queue.reserve(segments.size());
+    for (const auto& o : order) queue.push_back(segments[o.second]);
+    segments.swap(queue);
+    ctas = (int)std::min<int64_t>((int64_t)num_sms * kCtasPerSm, (int64_t)segments.size());
+    live.push_back(ImgTerm{});  // a group's t1 is readable
+    DMRG_TRY(upload(d_terms, live, stream));
+    DMRG_TRY(upload(d_segments, segments, stream));
+    DMRG_TRY(upload(d_splits, splits, stream));
+    DMRG_TRY(upload(tickets, std::vector<unsigned>(2 + ntickets, 0u), stream));
+    return aux.alloc((size_t)std::max<int64_t>(aux_size, 1) * sizeof(double));
+}
+
+int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
+                    cudaStream_t stream) {
+    if (s.segments.empty()) return DMRG_OK;
+    const GemmArgs w{A, B, C, s.aux.as<double>(), s.d_terms.as<ImgTerm>(), s.d_segments.as<ImgSegment>(),
+                     (int)s.segments.size(), s.panel / 8, s.d_splits.as<GemmSplit>(), s.tickets.as<unsigned>(), status,
+                     accumulate ? 1 : 0};
+    switch (s.out * 2 + (s.scaled ? 1 : 0)) {
+        case kImgOutBlock * 2: return launch<kImgOutBlock, false>(s.ctas, w, stream);
+        case kImgOutBlock * 2 + 1: return launch<kImgOutBlock, true>(s.ctas, w, stream);
+        case kImgOutB * 2: return launch<kImgOutB, false>(s.ctas, w, stream);
+        case kImgOutA * 2: return launch<kImgOutA, false>(s.ctas, w, stream);
+        default: return set_error(DMRG_E_STATE, "image products take no scales");
+    }
+}
+
+}  // namespace dmrg

@@ -8,9 +8,10 @@
 //      -> out(i,j) += W * L[o1](i,k) T
 // issuing one MKL dgemm per product.  Here the same walk is done once per site,
 // on the host, to build two grouped launches:
-//   stage A: every T needed by at least one term, one group each (C = scratch);
+//   stage A: every T needed by at least one term, one group each;
 //   stage B: one group per output block (i, j) holding all of its
-//            (W, L block, T) terms, summed in registers by the tile owner.
+//            (W, L block, T) terms, summed in registers.
+// In FP64 both run on packed operand images (gemm_image.cu), T included.
 #include <algorithm>
 #include <cstdlib>
 #include <map>
@@ -104,32 +105,55 @@ int build_heff(dmrg_heff_s& h) {
         }
     }
 
-    // Stage A: one group per T.
-    h.sa.reset();
-    for (const TaskA& t : tasks) {
-        h.sa.add_group(t.t_off, t.b_j, t.a_k, t.b_j);
-        h.sa.add_term(ket.off[t.pos], t.b_l, t.r_off, t.b_j, t.b_l, 1.0);
-    }
-    // Stage B: one group per output block, terms in generation order.
-    h.sb.reset();
     std::vector<std::vector<int>> per_out(ket.count());
     for (int i = 0; i < (int)termsB.size(); ++i) per_out[termsB[i].out_pos].push_back(i);
-    for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
-        if (per_out[pos2].empty()) continue;
-        h.sb.add_group(ket.off[pos2], ket.cols[pos2], ket.rows[pos2], ket.cols[pos2]);
-        for (int i : per_out[pos2]) {
-            const TermB& t = termsB[i];
-            const TaskA& ta = tasks[t.t_index];
-            h.sb.add_term(t.l_off, t.lda, ta.t_off, ta.b_j, t.k, t.w);
-        }
-    }
     h.flops_alg = fa_alg + fb;
     h.flops_exec = fa_exec + fb;
-    DMRG_TRY(h.sa.check_bounds(ket.size, h.R.size, h.t_size));
-    DMRG_TRY(h.sb.check_bounds(h.L.size, h.t_size, ket.size));
     cudaStream_t st = h.ctx->stream;
-    DMRG_TRY(h.sa.finalize(64, 64, 16, st));
-    DMRG_TRY(h.sb.finalize(64, 64, 16, st, h.ctx->num_sms));
+    // FP64: operand images (psi first, so that a matvec on packed environments
+    // packs a prefix), stage A into T images, stage B into the output blocks.  Every
+    // output block is a group, so a launch that does not accumulate overwrites all.
+    {
+        h.img = ImgPack();
+        std::vector<int64_t> psi_img(ket.count());
+        for (int pos = 0; pos < ket.count(); ++pos)
+            psi_img[pos] = h.img.add(0, ket.off[pos], ket.rows[pos], ket.cols[pos], ket.cols[pos], false);
+        h.img_psi_jobs = (int)h.img.jobs.size();
+        std::map<int64_t, int64_t> r_img, l_img;
+        std::vector<int64_t> t_img(tasks.size());
+        int64_t t_blocks = 0;
+        h.ia = ImgSchedule();
+        h.ib = ImgSchedule();
+        h.ia.panel = h.ib.panel = ImgSchedule::panel_for(h.flops_exec);
+        h.ia.out = kImgOutB;
+        for (size_t i = 0; i < tasks.size(); ++i) {
+            const TaskA& t = tasks[i];
+            auto it = r_img.find(t.r_off);
+            if (it == r_img.end()) it = r_img.emplace(t.r_off, h.img.add(2, t.r_off, t.b_j, t.b_l, t.b_j, true)).first;
+            t_img[i] = t_blocks;
+            t_blocks += img_blocks(t.b_j, t.a_k);
+            h.ia.add_group(t_img[i], 0, t.a_k, t.b_j);
+            h.ia.add_term(psi_img[t.pos], it->second, t.b_l, 1.0);
+        }
+        for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
+            h.ib.add_group(ket.off[pos2], ket.cols[pos2], ket.rows[pos2], ket.cols[pos2]);
+            for (int i : per_out[pos2]) {
+                const TermB& t = termsB[i];
+                auto it = l_img.find(t.l_off);
+                if (it == l_img.end())
+                    it = l_img.emplace(t.l_off, h.img.add(1, t.l_off, ket.rows[pos2], t.k, t.lda, false)).first;
+                h.ib.add_term(it->second, t_img[t.t_index], t.k, t.w);
+            }
+        }
+        DMRG_TRY(h.img.check_bounds(ket.size, h.L.size, h.R.size));
+        DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
+        DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, ket.size));
+        DMRG_TRY(h.img.finalize(h.ia.panel, st));
+        DMRG_TRY(h.ia.finalize(st, h.ctx->num_sms));
+        DMRG_TRY(h.ib.finalize(st, h.ctx->num_sms));
+        DMRG_TRY(h.d_img.alloc((size_t)std::max<int64_t>(h.img.blocks, 1) * kImgBlock * sizeof(double)));
+        DMRG_TRY(h.d_t.alloc((size_t)std::max<int64_t>(t_blocks, 1) * kImgBlock * sizeof(double)));
+    }
     if (is_split(h.precision)) {
         const int fmt = split_fmt(h.precision);
         h.pk_psi.fmt = h.pk_L.fmt = h.pk_R.fmt = h.pa.fmt = h.pb.fmt = fmt;
@@ -194,25 +218,36 @@ int build_heff(dmrg_heff_s& h) {
         DMRG_TRY(h.img_R.alloc((size_t)std::max<int64_t>(h.pk_R.bytes, 16)));
         DMRG_TRY(h.img_T.alloc((size_t)std::max<int64_t>(h.t_img_bytes, 16)));
     }
-    DMRG_TRY(h.T.alloc((size_t)std::max<int64_t>(h.t_size, 1) * sizeof(double)));
     return DMRG_OK;
 }
 
 }  // namespace
 
-int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate) {
+// psi's images, and unless they are packed already the environments'; a launch.
+static int pack_operands(dmrg_heff_s& h, const double* psi, bool env_packed) {
+    const int psi_chunks = h.img.first_chunk[h.img_psi_jobs];
+    return launch_img_pack(h.img, h.ia.panel, 0, env_packed ? psi_chunks : (int)h.img.chunks.size(), psi, h.L_dev, h.R_dev,
+                           h.d_img.as<double>(), h.ctx->stream);
+}
+
+int dmrg::heff_pack_env(dmrg_heff_s& h) {
+    if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
+        return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
+    return launch_img_pack(h.img, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr, h.L_dev,
+                           h.R_dev, h.d_img.as<double>(), h.ctx->stream);
+}
+
+int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate, bool env_packed) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
-    if (!accumulate && h.site.ket.size)
-        DMRG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)h.site.ket.size * sizeof(double), st));
-    DMRG_TRY(launch_gemm_f64(h.sa, psi, h.R_dev, h.T.as<double>(), false, st));
-    DMRG_TRY(launch_gemm_f64(h.sb, h.L_dev, h.T.as<double>(), out, true, st));
-    return DMRG_OK;
+    DMRG_TRY(pack_operands(h, psi, env_packed));
+    DMRG_TRY(launch_img_gemm(h.ia, h.d_img.as<double>(), h.d_img.as<double>(), h.d_t.as<double>(), false, h.ctx->d_status, st));
+    return launch_img_gemm(h.ib, h.d_img.as<double>(), h.d_t.as<double>(), out, accumulate, h.ctx->d_status, st);
 }
 
 int dmrg::heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bool accumulate) {
-    if (!is_split(h.precision)) return heff_apply_fp64(h, psi, out, accumulate);
+    if (!is_split(h.precision)) return heff_apply_fp64(h, psi, out, accumulate, false);
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
@@ -312,19 +347,23 @@ int dmrg_heff_profile(dmrg_heff_t h, const double* psi, double* out, double* ms_
     const bool split = is_split(h->precision);
     DMRG_CUDA_TRY(cudaEventRecord(ev[0], st));
     int rc = DMRG_OK;
-    if (split) {  // stage A includes packing psi
+    if (split) {  // stage A includes packing its operands
         rc = launch_pack(h->pk_psi, psi, h->img_psi.as<unsigned char>(), st);
         if (rc == DMRG_OK)
             rc = launch_gemm_split(h->pa, h->img_psi.as<unsigned char>(), h->img_R.as<unsigned char>(), nullptr,
                                     h->img_T.as<unsigned char>(), false, h->ctx->d_status, st);
     } else {
-        rc = launch_gemm_f64(h->sa, psi, h->R_dev, h->T.as<double>(), false, st);
+        rc = pack_operands(*h, psi, false);
+        if (rc == DMRG_OK)
+            rc = launch_img_gemm(h->ia, h->d_img.as<double>(), h->d_img.as<double>(), h->d_t.as<double>(), false,
+                                 h->ctx->d_status, st);
     }
     cudaEventRecord(ev[1], st);
     if (rc == DMRG_OK)
         rc = split ? launch_gemm_split(h->pb, h->img_L.as<unsigned char>(), h->img_T.as<unsigned char>(), out,
                                         nullptr, true, h->ctx->d_status, st)
-                   : launch_gemm_f64(h->sb, h->L_dev, h->T.as<double>(), out, true, st);
+                   : launch_img_gemm(h->ib, h->d_img.as<double>(), h->d_t.as<double>(), out, true,
+                                     h->ctx->d_status, st);
     cudaEventRecord(ev[2], st);
     cudaError_t err = cudaEventSynchronize(ev[2]);
     float a = 0, b = 0;
@@ -350,9 +389,10 @@ int dmrg_heff_apply_host(dmrg_heff_t h, const double* psi_host, double* out_host
     }
     DMRG_TRY(dmrg_heff_apply(h, h->io_psi.as<double>(), h->io_out.as<double>(), accumulate));
     if (bytes) DMRG_CUDA_TRY(cudaMemcpyAsync(out_host, h->io_out.ptr, bytes, cudaMemcpyDeviceToHost, st));
+    int* status = h->ctx->h_pinned + 15;  // a bounded wait of the GEMM kernels that gave up
+    DMRG_CUDA_TRY(cudaMemcpyAsync(status, h->ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaStreamSynchronize(st));
-    if (is_split(h->precision)) return take_device_status(h->ctx);  // bounded tensor-core waits
-    return DMRG_OK;
+    return *status ? take_device_status(h->ctx) : DMRG_OK;
 }
 
 }  // extern "C"

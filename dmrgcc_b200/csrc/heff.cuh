@@ -16,14 +16,17 @@ struct dmrg_heff_s {
     bool use_graph = true;            // Lanczos loop as one captured CUDA graph (dmrg_heff_set_graph)
     dmrg::SiteDesc site;
     dmrg::EnvDesc L, R;
-    dmrg::GemmSchedule sa, sb;    // A: psi x R -> T ; B: L x T -> out (FP64 tiles)
+    // FP64: operand images (jobs psi, then L and R), A: psi x R -> T images, B: L x T -> out
+    dmrg::ImgPack img;
+    int img_psi_jobs = 0;
+    dmrg::ImgSchedule ia, ib;
+    dmrg::DeviceBuffer d_img, d_t;
     // split precisions (DMRG_PREC_TF32X3 / DMRG_PREC_BF16X3) only: operand images
     // and packed schedules
     dmrg::PackSchedule pk_psi, pk_L, pk_R;     // which blocks to pack, where
     dmrg::PackedSchedule pa, pb;               // A: psi x R -> T images ; B: L x T -> out
     dmrg::DeviceBuffer img_psi, img_L, img_R, img_T;
     int64_t t_img_bytes = 0;
-    dmrg::DeviceBuffer T;
     int64_t t_size = 0;
     const double* L_dev = nullptr;
     const double* R_dev = nullptr;
@@ -38,6 +41,9 @@ inline bool is_split(int precision) { return precision == DMRG_PREC_TF32X3 || pr
 inline int split_fmt(int precision) { return precision == DMRG_PREC_BF16X3 ? kFmtBF16 : kFmtTF32; }
 // out (+)= H_eff psi on the context stream, in the operator's precision.
 int heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bool accumulate);
-// out (+)= H_eff psi in FP64 whatever the operator's precision.
-int heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate);
+// out (+)= H_eff psi in FP64 whatever the operator's precision.  The environments are
+// packed anew unless env_packed: then heff_pack_env was called since they last changed
+// (a Lanczos run packs them once).
+int heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate, bool env_packed);
+int heff_pack_env(dmrg_heff_s& h);
 }  // namespace dmrg

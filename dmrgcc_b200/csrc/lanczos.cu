@@ -122,9 +122,10 @@ int run_exact(dmrg_heff_s& h, double* psi, double* energy) {
     double* Z = A + (size_t)n * n;
     double* ev = Z + (size_t)n * n;
     double* e = w.h.as<double>();
+    DMRG_TRY(heff_pack_env(h));
     for (int c = 0; c < n; ++c) {
         DMRG_LAUNCH unit_vector_kernel<<<1, 128, 0, st>>>(e, n, c);
-        DMRG_TRY(heff_apply_fp64(h, e, cols + (size_t)c * n, false));  // the dense branch stays FP64
+        DMRG_TRY(heff_apply_fp64(h, e, cols + (size_t)c * n, false, true));  // the dense branch stays FP64
     }
     DMRG_LAUNCH symmetrize_upper_kernel<<<std::max(1, (n * n + 255) / 256), 256, 0, st>>>(cols, A, n);
     DMRG_CUDA_TRY(cudaMemsetAsync(w.state.ptr, 0, 16 * sizeof(int), st));
@@ -159,7 +160,7 @@ int capture_iteration(dmrg_heff_s& h, int niter, double precision, double zero_t
     double* c = E + niter;
     double* tmp = c + niter;
     int* state = w.state.as<int>();
-    DMRG_TRY(split ? heff_apply_internal(h, x, hv, true) : heff_apply_fp64(h, x, hv, true));
+    DMRG_TRY(split ? heff_apply_internal(h, x, hv, true) : heff_apply_fp64(h, x, hv, true, true));
     DMRG_TRY(vec_dot_it(x, hv, n, alpha, state, w.rs, blocks, st));
     DMRG_TRY(vec_axpy_norm_it(alpha, x, hv, n, beta, state, w.rs, blocks, st));
     DMRG_TRY(launch_tridiag_lowest_it(alpha, beta, state + kIterSlot, E, state, precision, zero_tol, niter, st));
@@ -243,6 +244,7 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     DMRG_CUDA_TRY(cudaMemcpyAsync(V, psi, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     DMRG_CUDA_TRY(cudaMemsetAsync(hv, 0, n * sizeof(double), st));
     DMRG_CUDA_TRY(cudaMemsetAsync(state, 0, 16 * sizeof(int), st));
+    if (!split) DMRG_TRY(heff_pack_env(h));  // once per run: the environments cannot change during it
     int dim = 0;
     if (h.use_graph) {
         // the whole loop as one graph launch; the host reads the result once
@@ -262,7 +264,7 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     const int chunk = (int)std::min<int64_t>(8, std::max<int64_t>(2, 2000000 / (n + 100000)));
     for (int i = 0; i < niter && !h.use_graph; ++i) {
         double* vi = V + (int64_t)i * n;
-        DMRG_TRY(split ? heff_apply_internal(h, vi, hv, true) : heff_apply_fp64(h, vi, hv, true));
+        DMRG_TRY(split ? heff_apply_internal(h, vi, hv, true) : heff_apply_fp64(h, vi, hv, true, true));
         DMRG_TRY(vec_dot(vi, hv, n, alpha + i, w.rs, blocks, st));
         DMRG_TRY(vec_axpy_norm(alpha + i, vi, hv, n, beta + i, w.rs, blocks, st));
         DMRG_TRY(launch_tridiag_lowest(alpha, beta, i + 1, E, state, precision, zero_tol, niter, st));
@@ -289,9 +291,10 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     double e = 0.0;
     DMRG_CUDA_TRY(cudaMemcpyAsync(&e, E + dim - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, state, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state + 4, h.ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaStreamSynchronize(st));
+    if (w.h_state[4] != 0) DMRG_TRY(take_device_status(h.ctx));  // a bounded wait of a matvec gave up
     if (w.h_state[2] != 0) return set_error(DMRG_E_NUMERIC, "tridiagonal ground vector failed (m=%d)", dim);
-    if (split) DMRG_TRY(take_device_status(h.ctx));  // a tensor-core wait that gave up
     *energy = e;
     if (iters) *iters = dim;
     return DMRG_OK;
