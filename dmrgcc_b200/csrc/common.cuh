@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -138,6 +139,22 @@ int upload(DeviceBuffer& buf, const std::vector<T>& v, cudaStream_t stream) {
     DMRG_CUDA_TRY(cudaStreamSynchronize(stream));
     return DMRG_OK;
 }
+
+// Several host tables in one device allocation and one copy.
+class Tables {
+public:
+    template <class T>
+    size_t add(const std::vector<T>& v) {  // returns the table's offset
+        const size_t at = (host_.size() + 255) & ~size_t(255);
+        host_.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(host_.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+    int to(DeviceBuffer& buf, cudaStream_t stream) { return upload(buf, host_, stream); }
+
+private:
+    std::vector<unsigned char> host_;
+};
 
 }  // namespace dmrg
 

@@ -17,7 +17,6 @@
 
 #include "blocksparse.h"
 #include "gemm.cuh"
-#include "zgemm.cuh"
 
 using namespace dmrg;
 
@@ -31,11 +30,9 @@ struct dmrg_env_s {
     // FP64: images of the ket and of the input environment, stage 1 into images, stage 2 into blocks
     ImgPack img;
     ImgSchedule i1, i2;
-    DeviceBuffer d_img, d_mid;
+    ImgWork work;
     SplitPlan p1, p2;  // split precisions: the same two stages on the tcgen05 path
-    // the complex path (dmrg_zenv_create): the same stages on complex blocks
-    bool cplx = false;
-    ZGemmSchedule z1, z2;
+    bool cplx = false;  // the complex path (dmrg_zenv_create): the same stages on complex blocks
     DeviceBuffer scratch;
     int64_t scratch_size = 0;
     double flops_alg = 0, flops_exec = 0;
@@ -286,62 +283,95 @@ int build_right(dmrg_env_s& e) {
 
 namespace {
 
-// The FP64 execution of s1 and s2 on packed operands (gemm_image.cu).  The ket's
-// images serve stage 1 (its A operand) and stage 2 (its B operand): left, both read
-// K^T; right, both read K.
-int build_images(dmrg_env_s& e, cudaStream_t st) {
+// The FP64 execution of s1 and s2 on packed operands (gemm_image.cu).  Real: the
+// ket's images serve stage 1 (its A operand) and stage 2 (its B operand): left, both
+// read K^T; right, both read K.  Complex (W: the complex MPO, the schedules' stage 2
+// scales its 1-based positions): real forms of the blocks (gemm.cuh, ImgKind), the
+// bra conjugated (left: stage 1's A operand, right: stage 2's B operand); a term's
+// complex weight w G B is Re w (G B) + Im w (G (i B)).
+int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
     const BlockListDesc& ket = e.site.ket;
-    std::map<int64_t, int64_t> ket_img, env_img, mid_img;  // by offset
-    for (int k = 0; k < ket.count(); ++k) {
-        if (ket.rows[k] == 0 || ket.cols[k] == 0) continue;
-        ket_img[ket.off[k]] = e.side == 0 ? e.img.add(0, ket.off[k], ket.cols[k], ket.rows[k], ket.cols[k], true)
-                                          : e.img.add(0, ket.off[k], ket.rows[k], ket.cols[k], ket.cols[k], false);
-    }
-    e.i1.panel = e.i2.panel = ImgSchedule::panel_for(e.s1.flops + e.s2.flops);
+    const bool z = W != nullptr;
+    const int f = z ? 2 : 1;  // doubles per element
+    // images by offset: the ket as stage 1's A operand, as stage 2's B operand (and times i), ...
+    std::map<int64_t, int64_t> ket_a, ket_b[2], env_img, mid_img;
+    std::map<int64_t, int> ket_pos;
+    for (int k = 0; k < ket.count(); ++k)
+        if (ket.rows[k] > 0 && ket.cols[k] > 0) ket_pos[ket.off[k]] = k;
+    auto ket_image = [&](std::map<int64_t, int64_t>& at, int64_t off, ImgKind kind, bool conj, bool times_i) {
+        auto it = at.find(off);
+        if (it != at.end()) return it->second;
+        const int k = ket_pos.at(off), r = ket.rows[k], c = ket.cols[k];
+        const bool t = e.side == 0;
+        const int64_t img = z ? e.img.add_complex(0, off, t ? c : r, t ? r : c, c, t, kind, conj, times_i)
+                              : e.img.add(0, off, t ? c : r, t ? r : c, c, t);
+        at.emplace(off, img);
+        return img;
+    };
+    e.i1.panel = e.i2.panel = ImgSchedule::panel_for((z ? 4.0 : 1.0) * (e.s1.flops + e.s2.flops));
     e.i1.out = kImgOutA;
     int64_t mid = 0;
     for (const GemmGroup& g : e.s1.groups) {
         if (g.m <= 0 || g.n <= 0) continue;
         mid_img[g.c_off] = mid;
-        e.i1.add_group(mid, 0, g.m, g.n);
-        mid += img_blocks(g.m, g.n);
+        e.i1.add_group(mid, 0, g.m, f * g.n);
+        mid += img_blocks(g.m, f * g.n);
         for (int t = g.t0; t < g.t1; ++t) {
             const GemmTerm& x = e.s1.terms[t];
             if (x.k <= 0) continue;
             auto it = env_img.find(x.b_off);
-            if (it == env_img.end()) it = env_img.emplace(x.b_off, e.img.add(1, x.b_off, g.n, x.k, x.ldb, true)).first;
-            e.i1.add_term(ket_img.at(x.a_off), it->second, x.k, x.scale);
+            if (it == env_img.end())
+                it = env_img.emplace(x.b_off, z ? e.img.add_complex(1, x.b_off, g.n, x.k, x.ldb, true, kImgComplexB, false, false)
+                                                : e.img.add(1, x.b_off, g.n, x.k, x.ldb, true)).first;
+            e.i1.add_term(ket_image(ket_a, x.a_off, kImgComplexA, e.side == 0, false), it->second, f * x.k, 1.0);
         }
     }
+    std::map<int64_t, int> grouped;
     for (const GemmGroup& g : e.s2.groups) {
-        e.i2.add_group(g.c_off, g.ldc, g.m, g.n);
+        e.i2.add_group(f * g.c_off, f * g.ldc, g.m, f * g.n);
+        grouped[g.c_off] = 1;
         for (int t = g.t0; t < g.t1; ++t) {
             const GemmTerm& x = e.s2.terms[t];
-            if (x.k > 0 && g.m > 0 && g.n > 0) e.i2.add_term(mid_img.at(x.a_off), ket_img.at(x.b_off), x.k, x.scale);
+            if (x.k <= 0 || g.m <= 0 || g.n <= 0) continue;
+            if (!z) {
+                e.i2.add_term(mid_img.at(x.a_off), ket_image(ket_a, x.b_off, kImgReal, false, false), x.k, x.scale);
+                continue;
+            }
+            const size_t pos = (size_t)x.scale - 1;
+            for (int im = 0; im < 2; ++im)
+                if (W[2 * pos + im] != 0.0)
+                    e.i2.add_term(mid_img.at(x.a_off), ket_image(ket_b[im], x.b_off, kImgComplexB, e.side == 1, im != 0),
+                                  2 * x.k, W[2 * pos + im]);
         }
     }
     // output blocks that no term reaches are groups too, so that stage 2 overwrites everything
-    std::map<int64_t, int> grouped;
-    for (const GemmGroup& g : e.s2.groups) grouped[g.c_off] = 1;
     for (size_t o = 0; o < e.out.o.size(); ++o)
         for (int q = 0; q < e.out.o[o].count(); ++q) {
             const int64_t off = e.out.base[o] + e.out.o[o].off[q];
             const int m = e.out.o[o].rows[q], n = e.out.o[o].cols[q];
-            if (m > 0 && n > 0 && !grouped.count(off)) e.i2.add_group(off, n, m, n);
+            if (m > 0 && n > 0 && !grouped.count(off)) e.i2.add_group(f * off, f * n, m, f * n);
         }
-    DMRG_TRY(e.img.check_bounds(ket.size, e.in.size, 0));
+    DMRG_TRY(e.img.check_bounds(f * ket.size, f * e.in.size, 0));
     DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, mid));
-    DMRG_TRY(e.i2.check_bounds(mid, e.img.blocks, e.out.size));
+    DMRG_TRY(e.i2.check_bounds(mid, e.img.blocks, f * e.out.size));
     DMRG_TRY(e.img.finalize(e.i1.panel, st));
     DMRG_TRY(e.i1.finalize(st, e.ctx->num_sms));
     DMRG_TRY(e.i2.finalize(st, e.ctx->num_sms));
-    DMRG_TRY(e.d_img.alloc((size_t)std::max<int64_t>(e.img.blocks, 1) * kImgBlock * sizeof(double)));
-    return e.d_mid.alloc((size_t)std::max<int64_t>(mid, 1) * kImgBlock * sizeof(double));
+    return e.work.alloc(e.img.blocks, mid, e.i1, e.i2);
 }
 
-// The common part of both creators: the structure, and for a real update its execution.
+int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
+    cudaStream_t st = e.ctx->stream;
+    DMRG_TRY(launch_img_pack(e.img, e.i1.panel, 0, (int)e.img.chunks.size(), ket_dev, env_in_dev, nullptr,
+                             e.work.img, st));
+    DMRG_TRY(launch_img_gemm(e.i1, e.work.img, e.work.img, e.work.mid, false,
+                             e.ctx->d_status, st));
+    return launch_img_gemm(e.i2, e.work.mid, e.work.img, env_out_dev, false, e.ctx->d_status, st);
+}
+
+// The common part of both creators (Wc: a complex update's MPO).
 int create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg_blocks_t* ket, int d, int lb, int rb,
-           const double* W, const dmrg_blocks_t* env_in, int precision, bool cplx, dmrg_env_t* out) {
+           const double* W, const dmrg_blocks_t* env_in, int precision, const double* Wc, dmrg_env_t* out) {
     if (!ctx || !out || !env_in) return set_error(DMRG_E_ARG, "null argument");
     if (side != 0 && side != 1) return set_error(DMRG_E_ARG, "side must be 0 (left) or 1 (right)");
     if (precision != DMRG_PREC_FP64 && precision != DMRG_PREC_TF32X3 && precision != DMRG_PREC_BF16X3)
@@ -359,7 +389,7 @@ int create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg
     cudaStream_t st = ctx->stream;
     if (rc == DMRG_OK) rc = e->s1.check_bounds(e->site.ket.size, e->in.size, e->scratch_size);
     if (rc == DMRG_OK) rc = e->s2.check_bounds(e->scratch_size, e->site.ket.size, e->out.size);
-    if (rc == DMRG_OK && !cplx && precision == DMRG_PREC_FP64) rc = build_images(*e, st);
+    if (rc == DMRG_OK && precision == DMRG_PREC_FP64) rc = build_images(*e, st, Wc);
     if (rc == DMRG_OK && precision != DMRG_PREC_FP64) {
         const int fmt = precision == DMRG_PREC_BF16X3 ? kFmtBF16 : kFmtTF32;
         rc = e->scratch.alloc((size_t)std::max<int64_t>(e->scratch_size, 1) * sizeof(double));
@@ -380,7 +410,7 @@ extern "C" {
 
 int dmrg_env_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg_blocks_t* ket, int d,
                     int lb, int rb, const double* W, const dmrg_blocks_t* env_in, int precision, dmrg_env_t* out) {
-    return create(ctx, side, nl, nr, phys, ket, d, lb, rb, W, env_in, precision, false, out);
+    return create(ctx, side, nl, nr, phys, ket, d, lb, rb, W, env_in, precision, nullptr, out);
 }
 
 int dmrg_env_destroy(dmrg_env_t e) {
@@ -419,20 +449,16 @@ int dmrg_env_flops(dmrg_env_t e, double* alg, double* exec) {
 
 int dmrg_env_apply(dmrg_env_t e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
     if (!e) return set_error(DMRG_E_ARG, "null env");
-    cudaStream_t st = e->ctx->stream;
     // Both sides: stage 1 reads (ket, env_in), stage 2 its products and the ket.
     if (e->cplx) return set_error(DMRG_E_STATE, "a complex environment update runs through dmrg_zenv_apply");
     if (e->precision != DMRG_PREC_FP64) {  // tcgen05 split products, FP64 sums and FP64 storage
+        cudaStream_t st = e->ctx->stream;
         if (e->out.size) DMRG_CUDA_TRY(cudaMemsetAsync(env_out_dev, 0, (size_t)e->out.size * sizeof(double), st));
         DMRG_TRY(e->p1.run(ket_dev, env_in_dev, e->scratch.as<double>(), false, e->ctx->d_status, st));
         DMRG_TRY(e->p2.run(e->scratch.as<double>(), ket_dev, env_out_dev, true, e->ctx->d_status, st));
         return DMRG_OK;
     }
-    DMRG_TRY(launch_img_pack(e->img, e->i1.panel, 0, (int)e->img.chunks.size(), ket_dev, env_in_dev, nullptr,
-                             e->d_img.as<double>(), st));
-    DMRG_TRY(launch_img_gemm(e->i1, e->d_img.as<double>(), e->d_img.as<double>(), e->d_mid.as<double>(), false,
-                             e->ctx->d_status, st));
-    return launch_img_gemm(e->i2, e->d_mid.as<double>(), e->d_img.as<double>(), env_out_dev, false, e->ctx->d_status, st);
+    return run_images(*e, ket_dev, env_in_dev, env_out_dev);
 }
 
 }  // extern "C"
@@ -445,8 +471,8 @@ int dmrg_env_apply(dmrg_env_t e, const double* ket_dev, const double* env_in_dev
 // runs on a surrogate MPO whose nonzero entries are the (1-based) positions of
 // the complex entries that are nonzero (|w| != 0 exactly where the complex
 // reference takes the term), so the output block maps follow the same
-// zero_flag pass; its terms then become complex terms whose scale is the
-// complex entry at that position, with the conjugation on the bra operand.
+// zero_flag pass; build_images then takes the complex entry at each term's
+// position as its weight, with the conjugation on the bra operand.
 // ---------------------------------------------------------------------------
 extern "C" {
 
@@ -457,39 +483,8 @@ int dmrg_zenv_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, 
     std::vector<double> ids(nw, 0.0);
     for (size_t i = 0; i < nw; ++i)
         if (W[2 * i] != 0.0 || W[2 * i + 1] != 0.0) ids[i] = (double)(i + 1);
-    DMRG_TRY(create(ctx, side, nl, nr, phys, ket, d, lb, rb, ids.data(), env_in, DMRG_PREC_FP64, true, out));
+    DMRG_TRY(create(ctx, side, nl, nr, phys, ket, d, lb, rb, ids.data(), env_in, DMRG_PREC_FP64, W, out));
     dmrg_env_s* e = *out;
-    auto convert = [&](const GemmSchedule& s, ZGemmSchedule& z, bool stage2, int conj) {
-        z.reset();
-        z.ta = s.ta;
-        z.tb = s.tb;
-        for (const GemmGroup& g : s.groups) {
-            z.add_group(g.c_off, g.ldc, g.m, g.n);
-            for (int t = g.t0; t < g.t1; ++t) {
-                const GemmTerm& x = s.terms[t];
-                double re = x.scale, im = 0.0;
-                if (stage2) {
-                    const size_t pos = (size_t)x.scale - 1;
-                    re = W[2 * pos];
-                    im = W[2 * pos + 1];
-                }
-                z.add_term(x.a_off, x.lda, x.b_off, x.ldb, x.k, re, im, conj);
-            }
-        }
-    };
-    // left: stage 1 B^dagger L (conjugated A), stage 2 w F K;  right: stage 1 K R, stage 2 w G B^dagger
-    convert(e->s1, e->z1, false, side == 0 ? 1 : 0);
-    convert(e->s2, e->z2, true, side == 0 ? 0 : 2);
-    int rc = e->z1.check_bounds(e->site.ket.size, e->in.size, e->scratch_size);
-    if (rc == DMRG_OK) rc = e->z2.check_bounds(e->scratch_size, e->site.ket.size, e->out.size);
-    if (rc == DMRG_OK) rc = e->z1.finalize(ctx->stream);
-    if (rc == DMRG_OK) rc = e->z2.finalize(ctx->stream);
-    if (rc == DMRG_OK) rc = e->scratch.alloc((size_t)std::max<int64_t>(e->scratch_size, 1) * 2 * sizeof(double));
-    if (rc != DMRG_OK) {
-        delete e;
-        *out = nullptr;
-        return rc;
-    }
     e->cplx = true;
     e->flops_alg *= 4.0;  // a complex product is four real ones
     e->flops_exec *= 4.0;
@@ -498,11 +493,7 @@ int dmrg_zenv_create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, 
 
 int dmrg_zenv_apply(dmrg_env_t e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
     if (!e || !e->cplx) return set_error(DMRG_E_ARG, "not a complex environment update (dmrg_zenv_create)");
-    cudaStream_t st = e->ctx->stream;
-    if (e->out.size) DMRG_CUDA_TRY(cudaMemsetAsync(env_out_dev, 0, (size_t)e->out.size * 2 * sizeof(double), st));
-    DMRG_TRY(launch_zgemm(e->z1, ket_dev, env_in_dev, e->scratch.as<double>(), false, st));
-    DMRG_TRY(launch_zgemm(e->z2, e->scratch.as<double>(), ket_dev, env_out_dev, true, st));
-    return DMRG_OK;
+    return run_images(*e, ket_dev, env_in_dev, env_out_dev);
 }
 
 }  // extern "C"

@@ -124,13 +124,25 @@ constexpr int kImgSlice = 4;   // blocks of k (of 8) per slice
 inline int64_t img_units(int extent) { return (extent + 7) / 8; }
 inline int64_t img_blocks(int rows, int k) { return img_units(rows) * img_units(k); }
 
+// A complex product is the real product of real forms with interleaved parts, four
+// real products per complex one: C (m x n complex) as its own m x 2n doubles, A as
+// its m x 2k doubles, and B as the 2k x 2n matrix with the 2x2 block
+// [[re, im], [-im, re]] for every element.
+enum ImgKind {
+    kImgReal = 0,
+    kImgComplexA = 1,  // rows x 2k: (re, im) of z
+    kImgComplexB = 2   // 2 rows x 2k (rows: output columns): [[re, -im], [im, re]] of z
+};
 struct ImgJob {        // one operand block to pack
     int64_t src_off;   // doubles, into its source
     int64_t img;       // first block of its image
-    int rows, k, ld;   // X(r, c) = src[src_off + (trans ? c * ld + r : r * ld + c)]
+    int rows, k, ld;   // X(r, c) = src[src_off + (trans ? c * ld + r : r * ld + c)]; complex: elements
     int trans;
     int src;           // which of the launch's sources
-    int pad_;
+    int kind;          // ImgKind
+    int conj, times_i; // complex: z = x, conj(x), i x or i conj(x) of the source's x
+    __host__ __device__ int image_rows() const { return kind == kImgComplexB ? 2 * rows : rows; }
+    __host__ __device__ int image_k() const { return kind == kImgReal ? k : 2 * k; }
 };
 struct ImgChunk {      // one (panel, slice) of a job
     int job, panel, slice, pad_;
@@ -139,9 +151,14 @@ struct ImgPack {
     std::vector<ImgJob> jobs;
     std::vector<ImgChunk> chunks;
     int64_t blocks = 0;
-    DeviceBuffer d_jobs, d_chunks;
+    DeviceBuffer d_tables;  // jobs, chunks
+    size_t chunks_at = 0;
     // Appends an operand block; returns its image (first block).
     int64_t add(int src, int64_t src_off, int rows, int k, int ld, bool trans);
+    // The same for a complex block (src_off, rows, k and ld in elements).
+    int64_t add_complex(int src, int64_t src_off, int rows, int k, int ld, bool trans, ImgKind kind, bool conj,
+                        bool times_i);
+    bool complex = false;
     // Every read inside sources of the given sizes (doubles); DMRG_E_ARG otherwise.
     int check_bounds(int64_t n0, int64_t n1, int64_t n2) const;
     // Builds the chunk list for panels of `panel` rows and uploads.
@@ -182,7 +199,9 @@ struct ImgSegment {
 enum ImgOut {
     kImgOutBlock = 0,   // row-major FP64 blocks
     kImgOutB = 1,       // images of the transposed output: rows = columns n, k = rows m (a B operand)
-    kImgOutA = 2        // images of the output: rows = rows m, k = columns n (an A operand)
+    kImgOutA = 2,       // images of the output: rows = rows m, k = columns n (an A operand)
+    kImgOutZB = 3       // the output as a complex m x n/2 matrix, in the form of a complex B operand
+                        // (kImgComplexB): rows = columns n, k = 2 rows m
 };
 struct ImgSchedule {
     std::vector<ImgTerm> terms;
@@ -194,8 +213,11 @@ struct ImgSchedule {
     int ctas = 0;
     std::vector<GemmSplit> splits;
     int64_t aux_size = 0;
-    // tickets: the queue's two counters, then one per split tile; zero between launches
-    DeviceBuffer d_terms, d_segments, d_splits, tickets, aux;
+    // device tables: terms, segments, splits, tickets (the queue's two counters, then one
+    // per split tile; zero between launches)
+    DeviceBuffer d_tables;
+    size_t segments_at = 0, splits_at = 0, tickets_at = 0;
+    double* aux = nullptr;  // aux_size doubles, 16-byte aligned, set after finalize
 
     void add_group(int64_t c_off, int ldc, int m, int n) {
         groups.push_back(ImgGroup{c_off, ldc, m, n, (int)terms.size(), (int)terms.size(), 0});
@@ -213,6 +235,13 @@ struct ImgSchedule {
     // uploads.  Groups without terms are part of it: a launch that does not
     // accumulate writes zeros.
     int finalize(cudaStream_t stream, int num_sms);
+};
+// The device memory of a two-stage product in one allocation: the operand images,
+// the first stage's output images, the aux buffers of both schedules.
+struct ImgWork {
+    DeviceBuffer buf;
+    double *img = nullptr, *mid = nullptr;
+    int alloc(int64_t img_blocks, int64_t mid_blocks, ImgSchedule& a, ImgSchedule& b);
 };
 // C (+)= the products (block output), or the images of them into C (accumulate
 // is then ignored).  A wait that gives up sets *status = DMRG_E_NUMERIC.

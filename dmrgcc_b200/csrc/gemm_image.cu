@@ -13,6 +13,9 @@
 // the first product of a chain leaves its result as the next one's image with
 // fully coalesced 512-byte stores.
 //
+// Complex products run as real ones of twice the columns and k (ImgKind): same DMMAs
+// as four real products per complex one, and the same kernel.
+//
 // GEMM CTA: four consumer warps (2 x 2 quarters of the tile, MI x NJ units of 8x8
 // each) and a producer warp that issues the copies; steps are handed over by
 // mbarriers, so warps and tiles overlap.  All waits are bounded.
@@ -125,17 +128,20 @@ struct GemmArgs {
 };
 
 // Where a tile's units go in an image output: the image's rows are the tile's
-// columns (B role) or rows (A role), its k indices the other side's.
+// columns (B roles) or rows (A role), its k indices the other side's (twice, in the
+// complex B role).
 template <int OUT>
 struct ImageOut {
+    static constexpr bool kByColumn = OUT == kImgOutB || OUT == kImgOutZB;
+    static constexpr int kPer = OUT == kImgOutZB ? 2 : 1;  // k units per unit of the tile
     double* base;   // the panel's first block
     int units, k0;  // row units of the panel; k unit of the tile's first unit
     int kb_all;
     __device__ __forceinline__ ImageOut(const GemmArgs& w, const Tile& g) {
-        units = ((OUT == kImgOutB ? g.cols : g.rows) + 7) >> 3;
-        k0 = (OUT == kImgOutB ? g.pm : g.pn) * w.units;
+        units = ((kByColumn ? g.cols : g.rows) + 7) >> 3;
+        k0 = (kByColumn ? g.pm : g.pn) * w.units * kPer;
         kb_all = g.out_kb;
-        base = w.C + (g.c_off + (int64_t)(OUT == kImgOutB ? g.pn : g.pm) * w.units * g.out_kb) * kImgBlock;
+        base = w.C + (g.c_off + (int64_t)(kByColumn ? g.pn : g.pm) * w.units * g.out_kb) * kImgBlock;
     }
     // Block of k unit `k` (of the tile) and row unit 0; `pitch`: to the next row unit.
     __device__ __forceinline__ double* column(int k, int& pitch) const {
@@ -143,15 +149,16 @@ struct ImageOut {
         pitch = min(kImgSlice, kb_all - s * kImgSlice) * kImgBlock;
         return base + (units * s * kImgSlice + (k0 + k) % kImgSlice) * kImgBlock;
     }
+    // Offset in a block of the lane's pair (row fr, columns 2 fc and 2 fc + 1 of a
+    // unit; complex: in the block of k unit fr / 4 of the unit's two), and from the
+    // first element of the pair to the second.
+    static __device__ __forceinline__ int pair(int fr, int fc) {
+        if (OUT == kImgOutB) return (4 * (2 * fc) + (fr & 3)) * 2 + (fr >> 2);
+        if (OUT == kImgOutA) return (4 * fr + ((2 * fc) & 3)) * 2 + (fc >> 1);
+        return (4 * (2 * fc) + 2 * (fr & 1)) * 2 + ((fr & 3) >> 1);
+    }
+    static constexpr int kStep = OUT == kImgOutA ? 2 : 8;
 };
-// Element (r, c) of a unit in its block; c even: element (r, c + 1) is kPairStep further.
-template <int OUT>
-__device__ __forceinline__ int out_element(int r, int c) {
-    const int x = OUT == kImgOutB ? c : r, k = OUT == kImgOutB ? r : c;
-    return (4 * x + (k & 3)) * 2 + (k >> 2);
-}
-template <int OUT>
-constexpr int kPairStep = OUT == kImgOutB ? 8 : 2;
 
 // The consumer warps' work on one tile or part.  The unit counts are template
 // parameters of the whole loop (as run-time counts, or in a switch inside it, the
@@ -251,21 +258,31 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
         }
     }
     const int fr = lane >> 2, fc = lane & 3;
-    if (OUT != kImgOutBlock) {  // whole units, zero outside the block
-        const ImageOut<OUT> image(w, g);
-        const int el = out_element<OUT>(fr, 2 * fc), rleft = g.rows - 8 * um0 - fr, cleft = g.cols - 8 * un0 - 2 * fc;
-        constexpr int KU = OUT == kImgOutB ? MI : NJ, XU = OUT == kImgOutB ? NJ : MI;  // k units, row units
+    if constexpr (OUT != kImgOutBlock) {  // whole units, zero outside the block
+        using Image = ImageOut<OUT>;
+        const Image image(w, g);
+        const int el = Image::pair(fr, fc), rleft = g.rows - 8 * um0 - fr, cleft = g.cols - 8 * un0 - 2 * fc;
+        constexpr bool kCol = Image::kByColumn;
+        constexpr int KU = kCol ? MI : NJ, XU = kCol ? NJ : MI;  // k units, row units
 #pragma unroll
         for (int k = 0; k < KU; ++k) {
+            const int ku = ((kCol ? um0 : un0) + k) * Image::kPer + (OUT == kImgOutZB ? fr >> 2 : 0);
+            if (image.k0 + ku >= image.kb_all) continue;
             int pitch;
-            double* col = image.column((OUT == kImgOutB ? um0 : un0) + k, pitch) + el;
+            double* col = image.column(ku, pitch) + el;
 #pragma unroll
             for (int x = 0; x < XU; ++x) {
-                const int i = OUT == kImgOutB ? k : x, j = OUT == kImgOutB ? x : k;
+                const int i = kCol ? k : x, j = kCol ? x : k;
                 if (8 * (um0 + i) >= g.rows || 8 * (un0 + j) >= g.cols) continue;
-                double* o = col + ((OUT == kImgOutB ? un0 : um0) + x) * pitch;
-                o[0] = 8 * i < rleft && 8 * j < cleft ? acc[i][j][0] : 0.0;
-                o[kPairStep<OUT>] = 8 * i < rleft && 8 * j + 1 < cleft ? acc[i][j][1] : 0.0;
+                double* o = col + ((kCol ? un0 : um0) + x) * pitch;
+                const double v0 = 8 * i < rleft && 8 * j < cleft ? acc[i][j][0] : 0.0;
+                const double v1 = 8 * i < rleft && 8 * j + 1 < cleft ? acc[i][j][1] : 0.0;
+                o[0] = v0;
+                o[Image::kStep] = v1;
+                if (OUT == kImgOutZB) {  // v0 + i v1: [[v0, -v1], [v1, v0]]
+                    o[2] = -v1;
+                    o[Image::kStep + 2] = v0;
+                }
             }
         }
         return;
@@ -450,10 +467,29 @@ __global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
     }
 }
 
+// Element (r, c) of a job's image (zero outside it).
+template <bool COMPLEX>
+__device__ __forceinline__ double image_element(const ImgJob& j, const double* __restrict__ src, int r, int c) {
+    if (r >= j.image_rows() || c >= j.image_k()) return 0.0;
+    if (!COMPLEX || j.kind == kImgReal) return src[j.trans ? (int64_t)c * j.ld + r : (int64_t)r * j.ld + c];
+    const bool b = j.kind == kImgComplexB;
+    const int zr = b ? r >> 1 : r, zc = c >> 1;
+    // part 0: re z, 1: im z, with the B form's sign
+    int part = b ? (r ^ c) & 1 : c & 1;
+    double sign = b && (r & 1) == 0 && part ? -1.0 : 1.0;
+    if (j.times_i) {  // re (i x) = -im x, im (i x) = re x
+        if (part == 0) sign = -sign;
+        part ^= 1;
+    }
+    if (j.conj && part) sign = -sign;
+    return sign * src[2 * (j.trans ? (int64_t)zc * j.ld + zr : (int64_t)zr * j.ld + zc) + part];
+}
+
 // One (panel, slice) of a job per CTA; thread = lane of a block: two elements of the
-// source (k indices 4 apart) to one 16-byte store.  A warp reads 8 rows of 32 + 32
-// contiguous bytes (or, transposed, 4 + 4 rows of 64) and writes 512.
+// image (k indices 4 apart) to one 16-byte store.  Real: a warp reads 8 rows of 32 +
+// 32 contiguous bytes (or, transposed, 4 + 4 rows of 64) and writes 512.
 constexpr int kPackThreads = 256;
+template <bool COMPLEX>
 __global__ void __launch_bounds__(kPackThreads) img_pack_kernel(const ImgJob* __restrict__ jobs,
                                                                 const ImgChunk* __restrict__ chunks, int panel,
                                                                 const double* __restrict__ s0,
@@ -465,20 +501,16 @@ __global__ void __launch_bounds__(kPackThreads) img_pack_kernel(const ImgJob* __
     launch_next();
     wait_previous();  // the sources are written, and the images' last readers are done
     const double* src = (j.src == 0 ? s0 : j.src == 1 ? s1 : s2) + j.src_off;
-    const int kb_all = (j.k + 7) >> 3, kb = min(kImgSlice, kb_all - ch.slice * kImgSlice);
-    const int r0 = ch.panel * panel, units = (min(panel, j.rows - r0) + 7) >> 3, k0 = ch.slice * kImgSlice * 8;
+    const int kb_all = (j.image_k() + 7) >> 3, kb = min(kImgSlice, kb_all - ch.slice * kImgSlice);
+    const int r0 = ch.panel * panel, units = (min(panel, j.image_rows() - r0) + 7) >> 3, k0 = ch.slice * kImgSlice * 8;
     double2* out = reinterpret_cast<double2*>(img) +
                    (j.img + (int64_t)ch.panel * (panel / 8) * kb_all + (int64_t)units * ch.slice * kImgSlice) * 32;
     const int lane = threadIdx.x & 31;
     for (int b = threadIdx.x >> 5; b < units * kb; b += kPackThreads / 32) {
         const int u = b / kb, q = b - u * kb;
         const int r = r0 + 8 * u + (lane >> 2), c = k0 + 8 * q + (lane & 3);
-        double2 v = make_double2(0.0, 0.0);
-        if (r < j.rows) {
-            if (c < j.k) v.x = src[j.trans ? (int64_t)c * j.ld + r : (int64_t)r * j.ld + c];
-            if (c + 4 < j.k) v.y = src[j.trans ? (int64_t)(c + 4) * j.ld + r : (int64_t)r * j.ld + c + 4];
-        }
-        out[(int64_t)b * 32 + lane] = v;
+        out[(int64_t)b * 32 + lane] =
+            make_double2(image_element<COMPLEX>(j, src, r, c), image_element<COMPLEX>(j, src, r, c + 4));
     }
 }
 
@@ -537,8 +569,18 @@ int steps_of(const ImgTerm& t) { return (t.kb + kImgSlice - 1) / kImgSlice; }
 
 int64_t ImgPack::add(int src, int64_t src_off, int rows, int k, int ld, bool trans) {
     const int64_t img = blocks;
-    jobs.push_back(ImgJob{src_off, img, rows, k, ld, trans ? 1 : 0, src, 0});
+    jobs.push_back(ImgJob{src_off, img, rows, k, ld, trans ? 1 : 0, src, kImgReal, 0, 0});
     blocks += img_blocks(rows, k);
+    return img;
+}
+
+int64_t ImgPack::add_complex(int src, int64_t src_off, int rows, int k, int ld, bool trans, ImgKind kind, bool conj,
+                             bool times_i) {
+    const int64_t img = blocks;
+    const ImgJob j{2 * src_off, img, rows, k, ld, trans ? 1 : 0, src, kind, conj ? 1 : 0, times_i ? 1 : 0};
+    jobs.push_back(j);
+    blocks += img_blocks(j.image_rows(), j.image_k());
+    complex = true;
     return img;
 }
 
@@ -546,7 +588,8 @@ int ImgPack::check_bounds(int64_t n0, int64_t n1, int64_t n2) const {
     const int64_t sizes[3] = {n0, n1, n2};
     for (const ImgJob& j : jobs) {
         if (j.rows <= 0 || j.k <= 0) continue;
-        const int64_t end = j.src_off + (j.trans ? (int64_t)(j.k - 1) * j.ld + j.rows : (int64_t)(j.rows - 1) * j.ld + j.k);
+        const int64_t count = j.trans ? (int64_t)(j.k - 1) * j.ld + j.rows : (int64_t)(j.rows - 1) * j.ld + j.k;
+        const int64_t end = j.src_off + (j.kind == kImgReal ? count : 2 * count);
         if (j.src_off < 0 || end > sizes[j.src])
             return set_error(DMRG_E_ARG, "packed operand %lld (%dx%d, ld %d) outside %lld", (long long)j.src_off, j.rows, j.k,
                              j.ld, (long long)sizes[j.src]);
@@ -558,20 +601,22 @@ int ImgPack::finalize(int panel, cudaStream_t stream) {
     chunks.clear();
     first_chunk.assign(1, 0);
     for (int j = 0; j < (int)jobs.size(); ++j) {
-        const int slices = (int)((img_units(jobs[j].k) + kImgSlice - 1) / kImgSlice);
-        for (int p = 0; p * panel < jobs[j].rows; ++p)
+        const int slices = (int)((img_units(jobs[j].image_k()) + kImgSlice - 1) / kImgSlice);
+        for (int p = 0; p * panel < jobs[j].image_rows(); ++p)
             for (int s = 0; s < slices; ++s) chunks.push_back(ImgChunk{j, p, s, 0});
         first_chunk.push_back((int)chunks.size());
     }
-    DMRG_TRY(upload(d_jobs, jobs, stream));
-    return upload(d_chunks, chunks, stream);
+    Tables t;
+    t.add(jobs);
+    chunks_at = t.add(chunks);
+    return t.to(d_tables, stream);
 }
 
 int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
                     double* img, cudaStream_t stream) {
     if (c1 <= c0) return DMRG_OK;
-    return launch_pdl(img_pack_kernel, c1 - c0, kPackThreads, 0, stream, p.d_jobs.as<ImgJob>(),
-                      p.d_chunks.as<ImgChunk>() + c0, panel, s0, s1, s2, img);
+    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, c1 - c0, kPackThreads, 0, stream, p.d_tables.as<ImgJob>(),
+                      reinterpret_cast<const ImgChunk*>(p.d_tables.as<char>() + p.chunks_at) + c0, panel, s0, s1, s2, img);
 }
 
 // A 64x64 tile's k-step takes a CTA about a microsecond: with few of them, whole
@@ -583,7 +628,8 @@ int ImgSchedule::panel_for(double flops) { return flops < kSmallFlops ? 32 : 64;
 int ImgSchedule::check_bounds(int64_t a_blocks, int64_t b_blocks, int64_t out_size) const {
     for (const ImgGroup& g : groups) {
         if (g.m <= 0 || g.n <= 0) continue;
-        const int64_t end = out == kImgOutBlock ? g.c_off + (int64_t)(g.m - 1) * g.ldc + g.n : g.c_off + img_blocks(g.m, g.n);
+        const int64_t end = out == kImgOutBlock ? g.c_off + (int64_t)(g.m - 1) * g.ldc + g.n
+                            : g.c_off + img_blocks(out == kImgOutZB ? g.n : g.m, out == kImgOutZB ? 2 * g.m : g.n);
         if (g.c_off < 0 || end > out_size || (out == kImgOutBlock && g.n > g.ldc))
             return set_error(DMRG_E_ARG, "packed GEMM output %lld (%dx%d) outside %lld", (long long)g.c_off, g.m, g.n,
                              (long long)out_size);
@@ -659,7 +705,7 @@ int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
             while (s.t0 < g.t1 && skip >= steps_of(live[s.t0])) skip -= steps_of(live[s.t0++]);
             s.k0 = (int)skip;
             s.split = -1;
-            s.out_kb = (int)img_units(out == kImgOutB ? g.m : g.n);
+            s.out_kb = (int)img_units(out == kImgOutZB ? 2 * g.m : out == kImgOutB ? g.m : g.n);
             if (parts > 1) {
                 s.split = (int)splits.size() - 1;
                 s.aux_off = aux_size;
@@ -677,24 +723,38 @@ int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
     segments.swap(queue);
     ctas = (int)std::min<int64_t>((int64_t)num_sms * kCtasPerSm, (int64_t)segments.size());
     live.push_back(ImgTerm{});  // a group's t1 is readable
-    DMRG_TRY(upload(d_terms, live, stream));
-    DMRG_TRY(upload(d_segments, segments, stream));
-    DMRG_TRY(upload(d_splits, splits, stream));
-    DMRG_TRY(upload(tickets, std::vector<unsigned>(2 + ntickets, 0u), stream));
-    return aux.alloc((size_t)std::max<int64_t>(aux_size, 1) * sizeof(double));
+    Tables tab;
+    tab.add(live);
+    segments_at = tab.add(segments);
+    splits_at = tab.add(splits);
+    tickets_at = tab.add(std::vector<unsigned>(2 + ntickets, 0u));
+    return tab.to(d_tables, stream);
+}
+
+int ImgWork::alloc(int64_t img_blocks, int64_t mid_blocks, ImgSchedule& a, ImgSchedule& b) {
+    const int64_t n = (img_blocks + mid_blocks) * kImgBlock;
+    DMRG_TRY(buf.alloc((size_t)std::max<int64_t>(n + a.aux_size + b.aux_size, 1) * sizeof(double)));
+    img = buf.as<double>();
+    mid = img + img_blocks * kImgBlock;
+    a.aux = img + n;
+    b.aux = a.aux + a.aux_size;
+    return DMRG_OK;
 }
 
 int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
                     cudaStream_t stream) {
     if (s.segments.empty()) return DMRG_OK;
-    const GemmArgs w{A, B, C, s.aux.as<double>(), s.d_terms.as<ImgTerm>(), s.d_segments.as<ImgSegment>(),
-                     (int)s.segments.size(), s.panel / 8, s.d_splits.as<GemmSplit>(), s.tickets.as<unsigned>(), status,
-                     accumulate ? 1 : 0};
+    char* tab = s.d_tables.as<char>();
+    const GemmArgs w{A, B, C, s.aux, reinterpret_cast<const ImgTerm*>(tab),
+                     reinterpret_cast<const ImgSegment*>(tab + s.segments_at), (int)s.segments.size(), s.panel / 8,
+                     reinterpret_cast<const GemmSplit*>(tab + s.splits_at), reinterpret_cast<unsigned*>(tab + s.tickets_at),
+                     status, accumulate ? 1 : 0};
     switch (s.out * 2 + (s.scaled ? 1 : 0)) {
         case kImgOutBlock * 2: return launch<kImgOutBlock, false>(s.ctas, w, stream);
         case kImgOutBlock * 2 + 1: return launch<kImgOutBlock, true>(s.ctas, w, stream);
         case kImgOutB * 2: return launch<kImgOutB, false>(s.ctas, w, stream);
         case kImgOutA * 2: return launch<kImgOutA, false>(s.ctas, w, stream);
+        case kImgOutZB * 2: return launch<kImgOutZB, false>(s.ctas, w, stream);
         default: return set_error(DMRG_E_STATE, "image products take no scales");
     }
 }

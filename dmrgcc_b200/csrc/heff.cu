@@ -151,8 +151,7 @@ int build_heff(dmrg_heff_s& h) {
         DMRG_TRY(h.img.finalize(h.ia.panel, st));
         DMRG_TRY(h.ia.finalize(st, h.ctx->num_sms));
         DMRG_TRY(h.ib.finalize(st, h.ctx->num_sms));
-        DMRG_TRY(h.d_img.alloc((size_t)std::max<int64_t>(h.img.blocks, 1) * kImgBlock * sizeof(double)));
-        DMRG_TRY(h.d_t.alloc((size_t)std::max<int64_t>(t_blocks, 1) * kImgBlock * sizeof(double)));
+        DMRG_TRY(h.work.alloc(h.img.blocks, t_blocks, h.ia, h.ib));
     }
     if (is_split(h.precision)) {
         const int fmt = split_fmt(h.precision);
@@ -227,14 +226,14 @@ int build_heff(dmrg_heff_s& h) {
 static int pack_operands(dmrg_heff_s& h, const double* psi, bool env_packed) {
     const int psi_chunks = h.img.first_chunk[h.img_psi_jobs];
     return launch_img_pack(h.img, h.ia.panel, 0, env_packed ? psi_chunks : (int)h.img.chunks.size(), psi, h.L_dev, h.R_dev,
-                           h.d_img.as<double>(), h.ctx->stream);
+                           h.work.img, h.ctx->stream);
 }
 
 int dmrg::heff_pack_env(dmrg_heff_s& h) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     return launch_img_pack(h.img, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr, h.L_dev,
-                           h.R_dev, h.d_img.as<double>(), h.ctx->stream);
+                           h.R_dev, h.work.img, h.ctx->stream);
 }
 
 int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate, bool env_packed) {
@@ -242,8 +241,8 @@ int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool a
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
     DMRG_TRY(pack_operands(h, psi, env_packed));
-    DMRG_TRY(launch_img_gemm(h.ia, h.d_img.as<double>(), h.d_img.as<double>(), h.d_t.as<double>(), false, h.ctx->d_status, st));
-    return launch_img_gemm(h.ib, h.d_img.as<double>(), h.d_t.as<double>(), out, accumulate, h.ctx->d_status, st);
+    DMRG_TRY(launch_img_gemm(h.ia, h.work.img, h.work.img, h.work.mid, false, h.ctx->d_status, st));
+    return launch_img_gemm(h.ib, h.work.img, h.work.mid, out, accumulate, h.ctx->d_status, st);
 }
 
 int dmrg::heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bool accumulate) {
@@ -355,14 +354,14 @@ int dmrg_heff_profile(dmrg_heff_t h, const double* psi, double* out, double* ms_
     } else {
         rc = pack_operands(*h, psi, false);
         if (rc == DMRG_OK)
-            rc = launch_img_gemm(h->ia, h->d_img.as<double>(), h->d_img.as<double>(), h->d_t.as<double>(), false,
+            rc = launch_img_gemm(h->ia, h->work.img, h->work.img, h->work.mid, false,
                                  h->ctx->d_status, st);
     }
     cudaEventRecord(ev[1], st);
     if (rc == DMRG_OK)
         rc = split ? launch_gemm_split(h->pb, h->img_L.as<unsigned char>(), h->img_T.as<unsigned char>(), out,
                                         nullptr, true, h->ctx->d_status, st)
-                   : launch_img_gemm(h->ib, h->d_img.as<double>(), h->d_t.as<double>(), out, true,
+                   : launch_img_gemm(h->ib, h->work.img, h->work.mid, out, true,
                                      h->ctx->d_status, st);
     cudaEventRecord(ev[2], st);
     cudaError_t err = cudaEventSynchronize(ev[2]);

@@ -20,7 +20,7 @@ struct dmrg_heff_s {
     dmrg::ImgPack img;
     int img_psi_jobs = 0;
     dmrg::ImgSchedule ia, ib;
-    dmrg::DeviceBuffer d_img, d_t;
+    dmrg::ImgWork work;
     // split precisions (DMRG_PREC_TF32X3 / DMRG_PREC_BF16X3) only: operand images
     // and packed schedules
     dmrg::PackSchedule pk_psi, pk_L, pk_R;     // which blocks to pack, where

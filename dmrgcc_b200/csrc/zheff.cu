@@ -3,7 +3,9 @@
 // ComplexTensorContraction::MultiplyEffectHamilton (src/dmrg/complexdmrg/
 // complex_tensor_contraction.cc:1244-1312) is the real walk of heff.cu with
 // complex blocks and a complex MPO: stage A T = K R, stage B out += w L T, on
-// the complex grouped GEMM (zgemm.cu).  ComplexTensorLanczos::LanczosMethod
+// the packed real forms of the blocks (gemm_image.cu).  One complex grouped GEMM
+// (zgemm.cu) per stage, one CTA per 64x32 tile and no split k, took 175 us for the
+// 6x6 Hofstadter cylinder's middle site at D=256 (0.38 GFLOP); now 49 us.  ComplexTensorLanczos::LanczosMethod
 // (complex_tensor_lanczos.cc:14-160): alpha_i = <v_i|h> with the conjugated
 // product, h -= alpha_i v_i with the complex alpha, beta_i = sqrt(Re <h|h>), the
 // tridiagonal problem on Re alpha and beta (zheevd reads only the real diagonal
@@ -14,10 +16,11 @@
 // eigenvector (x, y) gives the complex ground state x + i y.
 #include <algorithm>
 #include <cmath>
+#include <map>
 
 #include "blocksparse.h"
 #include "eig.cuh"
-#include "zgemm.cuh"
+#include "gemm.cuh"
 #include "zvec.cuh"
 
 using namespace dmrg;
@@ -27,9 +30,11 @@ struct dmrg_zheff_s {
     SiteDesc site;              // structure; site.W holds the real parts
     std::vector<double> Wc;     // complex MPO [lb][rb][d][d] (re, im)
     EnvDesc L, R;
-    ZGemmSchedule sa, sb;
-    DeviceBuffer T;
-    int64_t t_size = 0;         // complex elements
+    // operand images (jobs psi, then L and R), A: psi x R -> T images, B: L x T -> out
+    ImgPack img;
+    int img_psi_jobs = 0;
+    ImgSchedule ia, ib;
+    ImgWork work;
     const double* L_dev = nullptr;
     const double* R_dev = nullptr;
     double flops_alg = 0;
@@ -80,11 +85,9 @@ int build_zheff(dmrg_zheff_s& h) {
         int pos;
         int64_t r_off;
         int b_l, b_j, a_k;
-        int64_t t_off;
     };
     std::vector<TermB> termsB;
     std::vector<TaskA> tasks;
-    h.t_size = 0;
     double fl = 0;
     for (int o2 = 0; o2 < s.rb; ++o2) {
         const BlockListDesc& Ro = h.R.o[o2];
@@ -121,47 +124,83 @@ int build_zheff(dmrg_zheff_s& h) {
                     }
                 }
                 if (used) {
-                    tasks.push_back(TaskA{pos, h.R.base[o2] + Ro.off[i], b_l, rc, a_k, h.t_size});
-                    h.t_size += (int64_t)a_k * rc;
+                    tasks.push_back(TaskA{pos, h.R.base[o2] + Ro.off[i], b_l, rc, a_k});
                 }
             }
         }
     }
-    h.sa.reset();
-    for (const TaskA& t : tasks) {
-        h.sa.add_group(t.t_off, t.b_j, t.a_k, t.b_j);
-        h.sa.add_term(ket.off[t.pos], t.b_l, t.r_off, t.b_j, t.b_l, 1.0, 0.0);
+    h.flops_alg = fl;
+    // As in heff.cu, on the real forms of the complex blocks (gemm.cuh, ImgKind).  A
+    // term's complex weight w L T is Re w (L T) + Im w ((i L) T).
+    h.img = ImgPack();
+    std::vector<int64_t> psi_img(ket.count());
+    for (int pos = 0; pos < ket.count(); ++pos)
+        psi_img[pos] = h.img.add_complex(0, ket.off[pos], ket.rows[pos], ket.cols[pos], ket.cols[pos], false, kImgComplexA,
+                                         false, false);
+    h.img_psi_jobs = (int)h.img.jobs.size();
+    std::map<int64_t, int64_t> r_img, l_img[2];  // [1]: i L
+    std::vector<int64_t> t_img(tasks.size());
+    int64_t t_blocks = 0;
+    h.ia = ImgSchedule();
+    h.ib = ImgSchedule();
+    h.ia.panel = h.ib.panel = ImgSchedule::panel_for(fl);
+    h.ia.out = kImgOutZB;
+    for (size_t i = 0; i < tasks.size(); ++i) {
+        const TaskA& t = tasks[i];
+        auto it = r_img.find(t.r_off);
+        if (it == r_img.end())
+            it = r_img.emplace(t.r_off, h.img.add_complex(2, t.r_off, t.b_j, t.b_l, t.b_j, true, kImgComplexB, false, false))
+                     .first;
+        t_img[i] = t_blocks;
+        t_blocks += img_blocks(2 * t.b_j, 2 * t.a_k);
+        h.ia.add_group(t_img[i], 0, t.a_k, 2 * t.b_j);
+        h.ia.add_term(psi_img[t.pos], it->second, 2 * t.b_l, 1.0);
     }
-    h.sb.reset();
     std::vector<std::vector<int>> per_out(ket.count());
     for (int i = 0; i < (int)termsB.size(); ++i) per_out[termsB[i].out_pos].push_back(i);
     for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
-        if (per_out[pos2].empty()) continue;
-        h.sb.add_group(ket.off[pos2], ket.cols[pos2], ket.rows[pos2], ket.cols[pos2]);
+        h.ib.add_group(2 * ket.off[pos2], 2 * ket.cols[pos2], ket.rows[pos2], 2 * ket.cols[pos2]);
         for (int i : per_out[pos2]) {
             const TermB& t = termsB[i];
-            const TaskA& ta = tasks[t.t_index];
-            h.sb.add_term(t.l_off, t.lda, ta.t_off, ta.b_j, t.k, t.wr, t.wi);
+            const double w[2] = {t.wr, t.wi};
+            for (int im = 0; im < 2; ++im) {
+                if (w[im] == 0.0) continue;
+                auto it = l_img[im].find(t.l_off);
+                if (it == l_img[im].end())
+                    it = l_img[im].emplace(t.l_off, h.img.add_complex(1, t.l_off, ket.rows[pos2], t.k, t.lda, false,
+                                                                      kImgComplexA, false, im != 0)).first;
+                h.ib.add_term(it->second, t_img[t.t_index], 2 * t.k, w[im]);
+            }
         }
     }
-    h.flops_alg = fl;
-    DMRG_TRY(h.sa.check_bounds(ket.size, h.R.size, h.t_size));
-    DMRG_TRY(h.sb.check_bounds(h.L.size, h.t_size, ket.size));
-    DMRG_TRY(h.sa.finalize(h.ctx->stream));
-    DMRG_TRY(h.sb.finalize(h.ctx->stream));
-    DMRG_TRY(h.T.alloc((size_t)std::max<int64_t>(h.t_size, 1) * 2 * sizeof(double)));
-    return DMRG_OK;
+    DMRG_TRY(h.img.check_bounds(2 * ket.size, 2 * h.L.size, 2 * h.R.size));
+    DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
+    DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, 2 * ket.size));
+    cudaStream_t st = h.ctx->stream;
+    DMRG_TRY(h.img.finalize(h.ia.panel, st));
+    DMRG_TRY(h.ia.finalize(st, h.ctx->num_sms));
+    DMRG_TRY(h.ib.finalize(st, h.ctx->num_sms));
+    return h.work.alloc(h.img.blocks, t_blocks, h.ia, h.ib);
 }
 
-int zapply(dmrg_zheff_s& h, const double* psi, double* out, bool accumulate) {
+// out (+)= H psi; the environments are packed anew unless env_packed (zpack_env was
+// called since they last changed: a Lanczos run packs them once).
+int zapply(dmrg_zheff_s& h, const double* psi, double* out, bool accumulate, bool env_packed) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_zheff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
-    if (!accumulate && h.site.ket.size)
-        DMRG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)h.site.ket.size * 2 * sizeof(double), st));
-    DMRG_TRY(launch_zgemm(h.sa, psi, h.R_dev, h.T.as<double>(), false, st));
-    DMRG_TRY(launch_zgemm(h.sb, h.L_dev, h.T.as<double>(), out, true, st));
-    return DMRG_OK;
+    double* img = h.work.img;
+    DMRG_TRY(launch_img_pack(h.img, h.ia.panel, 0, env_packed ? h.img.first_chunk[h.img_psi_jobs] : (int)h.img.chunks.size(),
+                             psi, h.L_dev, h.R_dev, img, st));
+    DMRG_TRY(launch_img_gemm(h.ia, img, img, h.work.mid, false, h.ctx->d_status, st));
+    return launch_img_gemm(h.ib, img, h.work.mid, out, accumulate, h.ctx->d_status, st);
+}
+
+int zpack_env(dmrg_zheff_s& h) {
+    if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
+        return set_error(DMRG_E_STATE, "dmrg_zheff_set_env was not called");
+    return launch_img_pack(h.img, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr, h.L_dev,
+                           h.R_dev, h.work.img, h.ctx->stream);
 }
 
 __global__ void zunit_kernel(double* x, int64_t n, int64_t c) {
@@ -223,9 +262,10 @@ int zexact(dmrg_zheff_s& h, double* psi, double* energy) {
     double* Z = A + (size_t)N * N;
     double* ev = Z + (size_t)N * N;
     double* e = h.h.as<double>();
+    DMRG_TRY(zpack_env(h));
     for (int c = 0; c < n; ++c) {
         DMRG_LAUNCH zunit_kernel<<<1, 128, 0, st>>>(e, n, c);
-        DMRG_TRY(zapply(h, e, cols + (size_t)2 * c * n, false));
+        DMRG_TRY(zapply(h, e, cols + (size_t)2 * c * n, false, true));
     }
     DMRG_LAUNCH realify_kernel<<<std::max(1, (n * n + 255) / 256), 256, 0, st>>>(reinterpret_cast<double2*>(cols), A, n);
     int* state = h.state.as<int>();
@@ -262,9 +302,10 @@ int zkrylov(dmrg_zheff_s& h, double* psi, int niter, double precision, double ze
     int host_state[4] = {0, 0, 0, 0};
     const int chunk = (int)std::min<int64_t>(8, std::max<int64_t>(2, 1000000 / (n + 50000)));
     int dim = 0;
+    DMRG_TRY(zpack_env(h));
     for (int i = 0; i < niter; ++i) {
         double* vi = V + (int64_t)i * ldv;
-        DMRG_TRY(zapply(h, vi, hv, true));
+        DMRG_TRY(zapply(h, vi, hv, true, true));
         DMRG_TRY(zvec_dot(vi, hv, n, alpha_c + 2 * i, h.zr, blocks, st));
         DMRG_TRY(zvec_axpy_norm(alpha_c + 2 * i, vi, hv, n, beta + i, h.zr, blocks, st));
         DMRG_LAUNCH real_part_kernel<<<1, 1, 0, st>>>(alpha_c + 2 * i, alpha + i);
@@ -294,7 +335,7 @@ int zkrylov(dmrg_zheff_s& h, double* psi, int niter, double precision, double ze
     double e = 0.0;
     DMRG_CUDA_TRY(cudaMemcpyAsync(&e, E + dim - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaMemcpyAsync(host_state, state, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    DMRG_CUDA_TRY(cudaStreamSynchronize(st));
+    DMRG_TRY(take_device_status(h.ctx));  // waits for the stream; a bounded wait of a matvec that gave up
     if (host_state[2] != 0) return set_error(DMRG_E_NUMERIC, "tridiagonal ground vector failed (m=%d)", dim);
     *energy = e;
     if (iters) *iters = dim;
@@ -352,7 +393,7 @@ int dmrg_zheff_set_env(dmrg_zheff_t h, const double* L_dev, const double* R_dev)
 
 int dmrg_zheff_apply(dmrg_zheff_t h, const double* psi, double* out, int accumulate) {
     if (!h) return set_error(DMRG_E_ARG, "null operator");
-    return zapply(*h, psi, out, accumulate != 0);
+    return zapply(*h, psi, out, accumulate != 0, false);
 }
 
 int dmrg_zlanczos(dmrg_zheff_t h, double* psi, int niter, double precision, double zero_tol, double* energy,
