@@ -37,7 +37,8 @@ __global__ void __launch_bounds__(kBisectThreads) tridiag_lowest_kernel(const do
     __shared__ double lo, hi, pivmin;
     __shared__ int first;
     if (state[0]) return;  // already converged: later speculative steps are no-ops
-    if (m_iter) m = *m_iter + 1;  // graph-captured loop: the dimension is the device's iteration + 1
+    if (m_iter) m = *m_iter;
+    if (m < 1 || m > niter) return;
     if (threadIdx.x == 0) {
         double l = DBL_MAX, h = -DBL_MAX, bmax = 0.0;
         for (int k = 0; k < m; ++k) {
@@ -350,8 +351,8 @@ int launch_tridiag_lowest(const double* alpha, const double* beta, int m, double
 
 int launch_tridiag_lowest_it(const double* alpha, const double* beta, const int* iter, double* E, int* state,
                              double precision, double zero_tol, int niter, cudaStream_t st) {
-    DMRG_LAUNCH tridiag_lowest_kernel<<<1, kBisectThreads, 0, st>>>(alpha, beta, 1, E, state, precision, zero_tol, niter,
-                                                                    iter);
+    DMRG_LAUNCH tridiag_lowest_kernel<<<1, kBisectThreads, 0, st>>>(alpha, beta, 0, E, state, precision, zero_tol,
+                                                                    niter, iter);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }

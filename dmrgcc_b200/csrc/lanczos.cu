@@ -8,9 +8,14 @@
 //   else v_{i+1} = h / beta_i, h = -beta_i v_i, v_{i+1} orthogonalised against
 //   v_0..v_i and normalised;  ground vector = sum_k y_k v_k.
 // Differences by design: the reorthogonalisation is classical Gram-Schmidt
-// applied twice (two multi-dot/update launch pairs) instead of one modified
-// Gram-Schmidt pass (2(i+1) dependent launches); the tridiagonal's lowest
-// eigenvalue comes from Sturm bisection on the device instead of dsyevd.
+// applied twice (with the rest of an iteration's vector work in one kernel,
+// vec_lanczos_step) instead of one modified Gram-Schmidt pass (2(i+1) dependent
+// steps); the tridiagonal's lowest eigenvalue comes from Sturm bisection on the
+// device instead of dsyevd.
+// One B200, us per call: 16-site chain D=64, 20 iterations 1279 -> 736 (vector work
+// in one kernel, the tridiagonal step beside the matvec, packed matvecs); cylinder
+// D=512, 12 iterations 1630 -> 1103.  Bound now by the chain of five dependent
+// kernels of an iteration (37 us at n = 2,037).
 // psi_dim < 100 takes the reference's exact-diagonalisation branch (:34-56):
 // the dense H_eff is assembled column by column from matvecs on unit vectors
 // and diagonalised by a device Jacobi solver.
@@ -30,8 +35,11 @@ namespace dmrg {
 struct LanczosWork {
     int niter = 0;
     int64_t n = 0;
-    DeviceBuffer V, h, scal, state, jac, y, dense, x;
+    DeviceBuffer V, h, scal, state, jac, y, dense, x, part;
     ReduceScratch rs;
+    // the captured loop's second branch (the tridiagonal problem beside the matvec)
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     int* h_state = nullptr;  // the context's pinned words: [done, dim, ...]
     int split_iters = 0;     // Krylov dimension of the last split-precision phase
     // the captured Krylov loop, one per matvec precision (0: FP64, 1: split),
@@ -45,6 +53,9 @@ struct LanczosWork {
     ~LanczosWork() {
         for (Graph& g : graph)
             if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
     }
 };
 
@@ -63,15 +74,6 @@ constexpr double kSplitPrecision = 1e-9;
 // Matvecs of the FP64 run that ends a mixed-precision Lanczos (<= 0: the full
 // run to the reference's convergence; dmrg_lanczos_set_polish).
 std::atomic<int> g_polish{4};
-
-// End of one captured Lanczos iteration: advance the device's iteration
-// counter and keep the loop going while the run has not converged.  The loop is
-// bounded: the tridiagonal step marks the run converged at dimension niter.
-__global__ void lanczos_advance_kernel(int* state, int niter, cudaGraphConditionalHandle loop) {
-    const int it = state[kIterSlot] + 1;
-    state[kIterSlot] = it;
-    cudaGraphSetConditional(loop, (state[0] == 0 && it < niter) ? 1u : 0u);
-}
 
 __global__ void unit_vector_kernel(double* x, int64_t n, int64_t c) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -96,9 +98,14 @@ int ensure_work(dmrg_heff_s& h, int niter) {
     LanczosWork& w = *h.lw;
     const int64_t n = h.site.ket.size;
     if (w.niter < niter || w.n != n) {
+        for (LanczosWork::Graph& g : w.graph) {  // captured on the buffers replaced below
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g.exec = nullptr;
+        }
         DMRG_TRY(w.V.alloc((size_t)std::max(niter, 1) * std::max<int64_t>(n, 1) * sizeof(double)));
         DMRG_TRY(w.h.alloc((size_t)std::max<int64_t>(n, 1) * sizeof(double)));
         DMRG_TRY(w.scal.alloc((size_t)(4 * std::max(niter, 1) + 16) * sizeof(double)));
+        DMRG_TRY(w.part.alloc((size_t)(2 * std::max(niter, 1) + 3) * lanczos_step_grid(n, h.ctx->num_sms) * sizeof(double)));
         DMRG_TRY(w.y.alloc((size_t)std::max(niter, 1) * sizeof(double)));
         const int m = std::max(niter, 128);
         DMRG_TRY(w.jac.alloc((size_t)(2 * m * m + 4 * m) * sizeof(double)));
@@ -107,7 +114,7 @@ int ensure_work(dmrg_heff_s& h, int niter) {
     }
     DMRG_TRY(w.x.alloc((size_t)std::max<int64_t>(n, 1) * sizeof(double)));
     DMRG_TRY(w.state.alloc(16 * sizeof(int)));
-    DMRG_TRY(w.rs.alloc(std::max(2 * h.ctx->num_sms, 64), std::max(niter, 1)));
+    DMRG_TRY(w.rs.alloc(std::max(2 * h.ctx->num_sms, 64), 1));
     w.h_state = h.ctx->h_pinned;
     return DMRG_OK;
 }
@@ -140,34 +147,42 @@ int run_exact(dmrg_heff_s& h, double* psi, double* energy) {
     return DMRG_OK;
 }
 
-// One Lanczos iteration i (i read on the device) for the captured loop:
-// h += H x;  alpha_i = <x|h>;  h -= alpha_i x;  beta_i = ||h||;  tridiagonal
-// step and convergence test;  unless converged: V_{i+1} = h / beta_i, h =
-// -beta_i x, reorthogonalised and normalised, x = V_{i+1};  i += 1.  x holds
-// V_i (the matvec input) so that the schedules' fixed operand pointers serve
-// every iteration.
+// A Lanczos iteration (its index i read and advanced on the device) is h += H x and
+// the vector work (vec_lanczos_step); x holds V_i, so that the schedules' fixed
+// operand pointers serve every iteration.
+int matvec(dmrg_heff_s& h, bool split) {
+    LanczosWork& w = *h.lw;
+    double *hv = w.h.as<double>(), *x = w.x.as<double>();
+    return split ? heff_apply_internal(h, x, hv, true) : heff_apply_fp64(h, x, hv, true, true);
+}
+int vector_step(dmrg_heff_s& h, int niter, cudaGraphConditionalHandle loop, cudaStream_t st) {
+    LanczosWork& w = *h.lw;
+    double* alpha = w.scal.as<double>();
+    return vec_lanczos_step(w.x.as<double>(), w.h.as<double>(), w.V.as<double>(), h.site.ket.size, niter, alpha,
+                            alpha + niter, w.part.as<double>(), w.state.as<int>(), loop, h.ctx->num_sms, st);
+}
+// The tridiagonal step and convergence test for the dimension reached.
+int tridiag_step(dmrg_heff_s& h, int niter, double precision, double zero_tol, cudaStream_t st) {
+    LanczosWork& w = *h.lw;
+    const double* alpha = w.scal.as<double>();
+    return launch_tridiag_lowest_it(alpha, alpha + niter, w.state.as<int>() + kIterSlot, w.scal.as<double>() + 2 * niter,
+                                    w.state.as<int>(), precision, zero_tol, niter, st);
+}
+
+// The captured loop's body: the tridiagonal step of the dimension reached beside the
+// matvec, then the vector work.  The step is a serial chain of ~10 us that only
+// decides whether the loop goes on, so it runs beside the next matvec instead of
+// ahead of it; an iteration past convergence writes only what nothing reads.
 int capture_iteration(dmrg_heff_s& h, int niter, double precision, double zero_tol, bool split,
                       cudaGraphConditionalHandle loop, cudaStream_t st) {
     LanczosWork& w = *h.lw;
-    const int64_t n = h.site.ket.size;
-    const int blocks = std::min<int64_t>((n + kVecThreads - 1) / kVecThreads, 2 * h.ctx->num_sms);
-    double* V = w.V.as<double>();
-    double* hv = w.h.as<double>();
-    double* x = w.x.as<double>();
-    double* alpha = w.scal.as<double>();
-    double* beta = alpha + niter;
-    double* E = beta + niter;
-    double* c = E + niter;
-    double* tmp = c + niter;
-    int* state = w.state.as<int>();
-    DMRG_TRY(split ? heff_apply_internal(h, x, hv, true) : heff_apply_fp64(h, x, hv, true, true));
-    DMRG_TRY(vec_dot_it(x, hv, n, alpha, state, w.rs, blocks, st));
-    DMRG_TRY(vec_axpy_norm_it(alpha, x, hv, n, beta, state, w.rs, blocks, st));
-    DMRG_TRY(launch_tridiag_lowest_it(alpha, beta, state + kIterSlot, E, state, precision, zero_tol, niter, st));
-    DMRG_TRY(vec_lanczos_step_it(beta, x, hv, V, n, niter, c, tmp, x, state, w.rs, blocks, st));
-    DMRG_LAUNCH lanczos_advance_kernel<<<1, 1, 0, st>>>(state, niter, loop);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
+    DMRG_CUDA_TRY(cudaEventRecord(w.fork, st));
+    DMRG_CUDA_TRY(cudaStreamWaitEvent(w.side, w.fork, 0));
+    DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, w.side));
+    DMRG_CUDA_TRY(cudaEventRecord(w.join, w.side));
+    DMRG_TRY(matvec(h, split));
+    DMRG_CUDA_TRY(cudaStreamWaitEvent(st, w.join, 0));
+    return vector_step(h, niter, loop, st);
 }
 
 // Captures the Krylov loop of one run as a CUDA graph: a conditional WHILE node
@@ -184,6 +199,9 @@ int build_loop_graph(dmrg_heff_s& h, int niter, double precision, double zero_to
         cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
     }
+    if (!w.side) DMRG_CUDA_TRY(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
+    if (!w.fork) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
+    if (!w.join) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
     cudaGraph_t graph = nullptr;
     DMRG_CUDA_TRY(cudaGraphCreate(&graph, 0));
     int rc = DMRG_OK;
@@ -238,10 +256,9 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     double* alpha = w.scal.as<double>();
     double* beta = alpha + niter;
     double* E = beta + niter;
-    double* c = E + niter;
-    double* tmp = c + niter;
     int* state = w.state.as<int>();
     DMRG_CUDA_TRY(cudaMemcpyAsync(V, psi, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    DMRG_CUDA_TRY(cudaMemcpyAsync(w.x.ptr, psi, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     DMRG_CUDA_TRY(cudaMemsetAsync(hv, 0, n * sizeof(double), st));
     DMRG_CUDA_TRY(cudaMemsetAsync(state, 0, 16 * sizeof(int), st));
     if (!split) DMRG_TRY(heff_pack_env(h));  // once per run: the environments cannot change during it
@@ -249,25 +266,23 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     if (h.use_graph) {
         // the whole loop as one graph launch; the host reads the result once
         DMRG_TRY(build_loop_graph(h, niter, precision, zero_tol, split));
-        DMRG_CUDA_TRY(cudaMemcpyAsync(w.x.ptr, psi, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
         DMRG_CUDA_TRY(cudaGraphLaunch(w.graph[split ? 1 : 0].exec, st));
+        DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, st));  // the last dimension's, if still open
         DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         DMRG_CUDA_TRY(cudaStreamSynchronize(st));
         dim = w.h_state[0] ? w.h_state[1] : 0;
     }
-    // The convergence test runs on the device (tridiag_lowest_kernel records the
-    // first dimension that meets it and ignores later calls).  The host reads it
-    // once per `chunk` iterations instead of after each one, so the GPU is not
-    // left idle between iterations; the few iterations enqueued past
-    // convergence write vectors and coefficients beyond `dim`, which nothing
-    // reads.  Cheap matvecs get longer chunks.
+    // Launch by launch: the convergence test runs on the device (tridiag_lowest_kernel
+    // records the first dimension that meets it and ignores later calls).  The host
+    // reads it once per `chunk` iterations instead of after each one, so the GPU is
+    // not left idle between iterations; the few iterations enqueued past convergence
+    // write vectors and coefficients beyond `dim`, which nothing reads.  Cheap
+    // matvecs get longer chunks.
     const int chunk = (int)std::min<int64_t>(8, std::max<int64_t>(2, 2000000 / (n + 100000)));
     for (int i = 0; i < niter && !h.use_graph; ++i) {
-        double* vi = V + (int64_t)i * n;
-        DMRG_TRY(split ? heff_apply_internal(h, vi, hv, true) : heff_apply_fp64(h, vi, hv, true, true));
-        DMRG_TRY(vec_dot(vi, hv, n, alpha + i, w.rs, blocks, st));
-        DMRG_TRY(vec_axpy_norm(alpha + i, vi, hv, n, beta + i, w.rs, blocks, st));
-        DMRG_TRY(launch_tridiag_lowest(alpha, beta, i + 1, E, state, precision, zero_tol, niter, st));
+        DMRG_TRY(matvec(h, split));
+        DMRG_TRY(vector_step(h, niter, 0, st));
+        DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, st));
         if ((i + 1) % chunk == 0 || i + 1 == niter) {
             DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             DMRG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -276,14 +291,6 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
                 break;
             }
         }
-        if (i + 1 == niter) break;  // the last vector slot is V[niter - 1]
-        double* vn = V + (int64_t)(i + 1) * n;
-        DMRG_TRY(vec_lanczos_shift(beta + i, vi, hv, vn, n, blocks, st));
-        // classical Gram-Schmidt twice; the second pass also normalises
-        DMRG_TRY(vec_multidot(V, n, i + 1, vn, n, c, w.rs, blocks, st));
-        DMRG_TRY(vec_combine(V, n, i + 1, c, -1.0, vn, 1.0, n, blocks, st));
-        DMRG_TRY(vec_multidot(V, n, i + 1, vn, n, c, w.rs, blocks, st));
-        DMRG_TRY(vec_combine_normalize(V, n, i + 1, c, -1.0, vn, n, tmp, w.rs, blocks, st));
     }
     if (dim <= 0) return set_error(DMRG_E_NUMERIC, "Lanczos ended without a converged dimension");
     DMRG_TRY(launch_tridiag_ground_vector(alpha, beta, E, state + 1, w.y.as<double>(), state + 2, st));

@@ -1,6 +1,9 @@
 // FP64 vector kernels (see vec.cuh).  These are HBM-bound: each reads its
 // operands once with coalesced grid-stride loops and reduces deterministically.
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <atomic>
 
 #include "vec.cuh"
 
@@ -58,73 +61,18 @@ __global__ void __launch_bounds__(kVecThreads) dot_kernel(const double* __restri
     last_block_finalize(partial, ticket, out, take_sqrt != 0);
 }
 
-__global__ void __launch_bounds__(kVecThreads) axpy_norm_kernel(const double* __restrict__ alpha,
-                                                                const double* __restrict__ x, double* __restrict__ y,
-                                                                int64_t n, double* partial, unsigned* ticket,
-                                                                double* out) {
-    const double a = *alpha;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = y[i] - a * x[i];
-        y[i] = v;
-        acc += v * v;
-    }
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-    last_block_finalize(partial, ticket, out, true);
-}
-
-// grid (nb, m): block (b, k) reduces its slice of <V_k, w> into partial[k * nb + b];
-// the last block of row k to finish sums the row in index order into c[k]
-// (tickets[k] counts the row's blocks and is reset).
-__global__ void __launch_bounds__(kVecThreads) multidot_kernel(const double* __restrict__ V, int64_t ldv,
-                                                               const double* __restrict__ w, int64_t n,
-                                                               double* partial, unsigned* tickets,
-                                                               double* __restrict__ c) {
-    const int k = blockIdx.y;
-    const double* v = V + (int64_t)k * ldv;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        acc += v[i] * w[i];
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[(int64_t)k * gridDim.x + blockIdx.x] = acc;
-    __shared__ bool is_last;
-    __threadfence();
-    if (threadIdx.x == 0) is_last = (atomicAdd(tickets + k, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    double r = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-        r += ((volatile double*)partial)[(int64_t)k * gridDim.x + b];
-    r = block_sum(r);
-    if (threadIdx.x == 0) {
-        c[k] = r;
-        tickets[k] = 0u;
-    }
-}
-
-// w = beta_w * w + sign * sum_k c[k] V_k; with `partial` non-null also the norm
-// of the new w into *out (the reduction of dot_kernel(w, w): same slices, same
-// order).
+// w = beta_w * w + sign * sum_k c[k] V_k
 __global__ void __launch_bounds__(kVecThreads) combine_kernel(const double* __restrict__ V, int64_t ldv, int m,
                                                               const double* __restrict__ c, double sign,
-                                                              double* __restrict__ w, double beta_w, int64_t n,
-                                                              double* partial, unsigned* ticket, double* out) {
+                                                              double* __restrict__ w, double beta_w, int64_t n) {
     __shared__ double cs[kMaxVec];
     for (int k = threadIdx.x; k < m; k += blockDim.x) cs[k] = sign * c[k];
     __syncthreads();
-    double nrm = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double acc = beta_w == 0.0 ? 0.0 : beta_w * w[i];
         for (int k = 0; k < m; ++k) acc += cs[k] * V[(int64_t)k * ldv + i];
         w[i] = acc;
-        nrm += acc * acc;
     }
-    if (partial == nullptr) return;  // uniform
-    nrm = block_sum(nrm);
-    if (threadIdx.x == 0) partial[blockIdx.x] = nrm;
-    last_block_finalize(partial, ticket, out, true);
 }
 
 __global__ void __launch_bounds__(kVecThreads) lanczos_shift_kernel(const double* __restrict__ beta,
@@ -147,158 +95,183 @@ __global__ void __launch_bounds__(kVecThreads) scale_inv_kernel(double* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Device-indexed forms for the graph-captured Lanczos loop: the iteration i is
-// read from state[kIterSlot] instead of being baked into launch arguments, so
-// one captured iteration body serves every i.  Each computes exactly what its
-// host-indexed twin above computes for that i (same slices, same reduction
-// order, same effective grid), so a graph run is bit-identical to a launch-by-
-// launch run.  Every kernel returns at once when state[0] (converged) is set.
+// One Lanczos iteration's vector work in one kernel (see vec_lanczos_step).
+//
+// The work is small (n doubles times a few passes over at most i + 1 vectors) and
+// chains five reductions, each needed by the whole next pass, so it is bound by
+// latency: as eight launches it took 45 us of an iteration at n = 2,037 and 60 us
+// at n = 140,000.  The CTAs keep one slice each of all vectors and meet at a
+// barrier per reduction instead: the hardware barrier of a cluster of 8 where the
+// slices are short, else the grid barrier of a cooperative launch of one CTA per SM.
+// The basis does not depend on the iteration's matvec, so its slices (as many as
+// fit) are copied to shared memory while the first two reductions run.
+// Reductions are deterministic (fixed slices, partials summed in a fixed order).
+constexpr int kStepThreads = 512, kStepWarps = kStepThreads / 32;
+constexpr int kStepCluster = 8;
+// Up to here one cluster: its barrier takes a fraction of the grid's, but eight SMs
+// read the basis.  Measured, us per iteration of a 20-iteration Lanczos run, cluster /
+// grid: n = 2,037 37 / 43, 7,760 42 / 45, 21,425 78 / 58 (before: 64, 77, 106).
+constexpr int64_t kClusterMax = 16384;
+constexpr int64_t kStepShared = 24 * 1024;  // doubles of shared memory: w's slice (if it fits), then the basis
 
-__global__ void __launch_bounds__(kVecThreads) dot_it_kernel(const double* __restrict__ x,
-                                                             const double* __restrict__ y, int64_t n,
-                                                             double* partial, unsigned* ticket,
-                                                             double* out_base, const int* state) {
-    if (state[0]) return;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        acc += x[i] * y[i];
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-    last_block_finalize(partial, ticket, out_base + state[kIterSlot], false);
+struct StepArgs {
+    double *x, *h, *V;
+    int64_t n;
+    int niter;
+    double *alpha, *beta;  // of every iteration
+    double* part;          // (2 niter + 3) * grid partials
+    int* state;
+    int slice_in_smem, basis_in_smem;  // w's slice; vectors of the basis
+    cudaGraphConditionalHandle loop;   // the captured loop's, or 0
+};
+
+__device__ __forceinline__ double warp_sum_all(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
 }
 
-__global__ void __launch_bounds__(kVecThreads) axpy_norm_it_kernel(const double* __restrict__ alpha_base,
-                                                                   const double* __restrict__ x,
-                                                                   double* __restrict__ y, int64_t n,
-                                                                   double* partial, unsigned* ticket,
-                                                                   double* out_base, const int* state) {
-    if (state[0]) return;
-    const int it = state[kIterSlot];
-    const double a = alpha_base[it];
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kStepThreads) lanczos_step_kernel(const StepArgs a) {
+    namespace cg = cooperative_groups;
+    extern __shared__ double sm[];
+    const int it = a.state[kIterSlot];
+    if (it >= a.niter) return;  // the same for every CTA
+    const int G = gridDim.x, rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto meet = [&]() {
+        if (CLUSTER) cg::this_cluster().sync();
+        else cg::this_grid().sync();
+    };
+    const int64_t chunk = (a.n + G - 1) / G, base = min((int64_t)rank * chunk, a.n);
+    const int len = (int)(min(base + chunk, a.n) - base);
+    // shared: warp partials, coefficients, CTA partials (cluster), w's slice, the basis
+    double* red = sm;                         // kStepWarps * niter
+    double* cs = red + kStepWarps * a.niter;  // niter
+    double* mine = cs + a.niter;              // 2 niter + 3
+    double* wsm = mine + 2 * a.niter + 3;
+    double* basis = wsm + (a.slice_in_smem ? chunk : 0);
+    double* x = a.x + base;
+    double* h = a.h + base;
+    const double* V = a.V + base;
+    const int m = it + 1, kept = it + 1 < a.niter ? min(m, a.basis_in_smem) : 0;
+    for (int k = 0; k < kept; ++k)
+        for (int j = tid; j < len; j += kStepThreads) cp_async8(basis + (int64_t)k * chunk + j, V + (int64_t)k * a.n + j);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    // Partial `slot` of this CTA, and the warp's sum of all CTAs' (in every lane).
+    auto put = [&](int slot, double v) {
+        if (CLUSTER) mine[slot] = v;
+        else a.part[(int64_t)slot * G + rank] = v;
+    };
+    auto get = [&](int slot) {
+        double v = 0.0;
+        if (CLUSTER) {
+            if (lane < kStepCluster) v = cg::this_cluster().map_shared_rank(mine, lane)[slot];
+        } else {
+            for (int r = lane; r < G; r += 32) v += __ldcg(a.part + (int64_t)slot * G + r);
+        }
+        return warp_sum_all(v);
+    };
+    // Sum of the threads' v over all CTAs, the same in every thread.
+    auto total = [&](double v, int slot) {
+        v = warp_sum_all(v);
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            v = warp_sum_all(lane < kStepWarps ? red[lane] : 0.0);
+            if (lane == 0) put(slot, v);
+        }
+        meet();
+        return get(slot);
+    };
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = y[i] - a * x[i];
-        y[i] = v;
+#pragma unroll 4
+    for (int j = tid; j < len; j += kStepThreads) acc += x[j] * h[j];
+    const double al = total(acc, 0);
+    acc = 0.0;
+#pragma unroll 4
+    for (int j = tid; j < len; j += kStepThreads) {
+        const double v = h[j] - al * x[j];
+        h[j] = v;
         acc += v * v;
     }
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-    last_block_finalize(partial, ticket, out_base + it, true);
-}
-
-// v_next = V + (i+1) ldv = h / beta_i ; h = -beta_i x
-__global__ void __launch_bounds__(kVecThreads) lanczos_shift_it_kernel(const double* __restrict__ beta_base,
-                                                                       const double* __restrict__ x,
-                                                                       double* __restrict__ h, double* V,
-                                                                       int64_t ldv, int64_t n, int niter,
-                                                                       const int* state) {
-    if (state[0]) return;
-    const int it = state[kIterSlot];
-    if (it + 1 >= niter) return;
-    double* __restrict__ v_next = V + (int64_t)(it + 1) * ldv;
-    const double b = beta_base[it];
-    const double inv = 1.0 / b;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        v_next[i] = h[i] * inv;
-        h[i] = -b * x[i];
+    const double be = sqrt(total(acc, 1));
+    const bool last = it + 1 >= a.niter;  // the last vector slot is V[niter - 1]
+    if (rank == 0 && tid == 0) {
+        a.alpha[it] = al;
+        a.beta[it] = be;
+        // the next iteration (every CTA has read the counter); the captured loop goes on
+        // while no converged dimension is known
+        a.state[kIterSlot] = it + 1;
+        if (a.loop) cudaGraphSetConditional(a.loop, !last && a.state[0] == 0 ? 1u : 0u);
     }
-}
-
-// Number of slices of each vector in the multidot of m vectors:
-// clamp(blocks / m, 8, max_blocks) (the host-indexed multidot's grid width).
-__host__ __device__ __forceinline__ int multidot_slices(int blocks, int max_blocks, int m) {
-    int nb = blocks / m;
-    if (nb < 8) nb = 8;
-    if (nb > max_blocks) nb = max_blocks;
-    return nb;
-}
-
-// c[k] = <V_k, w> for k < m = i+1, w = V_{i+1}.  The host-indexed multidot runs
-// an (nb, m) grid; here that grid is flattened into a 1-D grid sized for the
-// largest nb * m of any iteration (multidot_it_grid): block j takes slice
-// b = j % nb of vector k = j / nb, blocks with k >= m return.  Same slices,
-// partials, tickets and reduction order as there.
-__global__ void __launch_bounds__(kVecThreads) multidot_it_kernel(const double* __restrict__ V, int64_t ldv,
-                                                                  int64_t n, int blocks, int max_blocks,
-                                                                  double* partial, unsigned* tickets,
-                                                                  double* __restrict__ c, int niter,
-                                                                  const int* state) {
-    if (state[0]) return;
-    const int it = state[kIterSlot];
-    if (it + 1 >= niter) return;
-    const int m = it + 1;
-    const int nb = multidot_slices(blocks, max_blocks, m);
-    const int k = (int)blockIdx.x / nb, b = (int)blockIdx.x % nb;
-    if (k >= m) return;
-    const double* __restrict__ w = V + (int64_t)m * ldv;
-    const double* __restrict__ v = V + (int64_t)k * ldv;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)b * blockDim.x + threadIdx.x; i < n; i += (int64_t)nb * blockDim.x) acc += v[i] * w[i];
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[(int64_t)k * nb + b] = acc;
-    __shared__ bool is_last;
-    __threadfence();
-    if (threadIdx.x == 0) is_last = (atomicAdd(tickets + k, 1u) == (unsigned)nb - 1);
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    double r = 0.0;
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) r += ((volatile double*)partial)[(int64_t)k * nb + j];
-    r = block_sum(r);
-    if (threadIdx.x == 0) {
-        c[k] = r;
-        tickets[k] = 0u;
+    if (!last) {
+        // w = h / beta, h = -beta x
+        double* next = a.V + (int64_t)m * a.n + base;
+        double* w = a.slice_in_smem ? wsm : next;
+        const double inv = 1.0 / be;
+#pragma unroll 4
+        for (int j = tid; j < len; j += kStepThreads) {
+            w[j] = h[j] * inv;
+            h[j] = -be * x[j];
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        // classical Gram-Schmidt against V_0 .. V_it, twice.  The dot products: the slice in
+        // `segs` segments of at least 256 elements, a warp per segment and vector.
+        const int segs = len >= 4096 ? 16 : len >= 2048 ? 8 : len >= 1024 ? 4 : len >= 512 ? 2 : 1;
+        const int per = (len + segs - 1) / segs, seg = warp % segs, j0 = min(seg * per, len), j1 = min(j0 + per, len);
+        for (int pass = 0; pass < 2; ++pass) {
+            __syncthreads();  // w and the basis are complete
+            const int slot = 3 + pass * a.niter;
+            for (int k = warp / segs; k < m; k += kStepWarps / segs) {
+                double s = 0.0;
+                if (k < kept) {
+                    const double* vk = basis + (int64_t)k * chunk;
+#pragma unroll 4
+                    for (int j = j0 + lane; j < j1; j += 32) s += vk[j] * w[j];
+                } else {
+                    const double* vk = V + (int64_t)k * a.n;
+#pragma unroll 8
+                    for (int j = j0 + lane; j < j1; j += 32) s += vk[j] * w[j];
+                }
+                s = warp_sum_all(s);
+                if (lane == 0) red[k * segs + seg] = s;
+            }
+            __syncthreads();
+            for (int k = tid; k < m; k += kStepThreads) {
+                double s = 0.0;
+                for (int q = 0; q < segs; ++q) s += red[k * segs + q];
+                put(slot + k, s);
+            }
+            meet();
+            for (int k = warp; k < m; k += kStepWarps) {
+                const double s = get(slot + k);
+                if (lane == 0) cs[k] = s;
+            }
+            __syncthreads();
+            for (int j = tid; j < len; j += kStepThreads) {
+                double v = w[j];
+#pragma unroll 4
+                for (int k = 0; k < kept; ++k) v -= cs[k] * basis[(int64_t)k * chunk + j];
+#pragma unroll 8
+                for (int k = kept; k < m; ++k) v -= cs[k] * V[(int64_t)k * a.n + j];
+                w[j] = v;
+            }
+        }
+        acc = 0.0;
+        for (int j = tid; j < len; j += kStepThreads) acc += w[j] * w[j];  // its own elements
+        __syncthreads();  // red is free
+        const double scale = 1.0 / sqrt(total(acc, 2));
+        for (int j = tid; j < len; j += kStepThreads) {
+            const double v = w[j] * scale;
+            next[j] = v;
+            x[j] = v;
+        }
     }
-}
-
-// Grid of multidot_it_kernel: the largest nb * m over the iterations m < niter.
-int multidot_it_grid(int blocks, int max_blocks, int niter) {
-    int g = 1;
-    for (int m = 1; m < niter; ++m) g = std::max(g, multidot_slices(blocks, max_blocks, m) * m);
-    return g;
-}
-
-// w = V_{i+1} (+)= sign * sum_{k<=i} c[k] V_k; with `partial` also ||w|| into *out
-__global__ void __launch_bounds__(kVecThreads) combine_it_kernel(const double* __restrict__ V, int64_t ldv,
-                                                                 const double* __restrict__ c, double sign,
-                                                                 int64_t n, double* partial, unsigned* ticket,
-                                                                 double* out, int niter, const int* state) {
-    if (state[0]) return;
-    const int it = state[kIterSlot];
-    if (it + 1 >= niter) return;
-    const int m = it + 1;
-    double* __restrict__ w = const_cast<double*>(V) + (int64_t)m * ldv;
-    __shared__ double cs[kMaxVec];
-    for (int k = threadIdx.x; k < m; k += blockDim.x) cs[k] = sign * c[k];
-    __syncthreads();
-    double nrm = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 1.0 * w[i];
-        for (int k = 0; k < m; ++k) acc += cs[k] * V[(int64_t)k * ldv + i];
-        w[i] = acc;
-        nrm += acc * acc;
-    }
-    if (partial == nullptr) return;  // uniform
-    nrm = block_sum(nrm);
-    if (threadIdx.x == 0) partial[blockIdx.x] = nrm;
-    last_block_finalize(partial, ticket, out, true);
-}
-
-// V_{i+1} /= *s, and the normalised vector also into x (the next matvec input)
-__global__ void __launch_bounds__(kVecThreads) scale_inv_it_kernel(double* V, int64_t ldv,
-                                                                   const double* __restrict__ s,
-                                                                   double* __restrict__ x, int64_t n, int niter,
-                                                                   const int* state) {
-    if (state[0]) return;
-    const int it = state[kIterSlot];
-    if (it + 1 >= niter) return;
-    double* __restrict__ w = V + (int64_t)(it + 1) * ldv;
-    const double inv = 1.0 / *s;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = w[i] * inv;
-        w[i] = v;
-        x[i] = v;
-    }
+    if (CLUSTER) meet();  // no CTA leaves while another may read its partials
 }
 
 }  // namespace
@@ -307,45 +280,16 @@ int ReduceScratch::alloc(int blocks, int max_vectors) {
     max_blocks = blocks;
     DMRG_TRY(partial.alloc((size_t)blocks * (max_vectors > 0 ? max_vectors : 1) * sizeof(double)));
     if (!ticket.ptr) {
-        DMRG_TRY(ticket.alloc((kRowTickets + kMaxVec) * sizeof(unsigned)));
+        DMRG_TRY(ticket.alloc(kTickets * sizeof(unsigned)));
         DMRG_TRY(ticket.zero());
     }
-    return DMRG_OK;
-}
-
-int vec_dot(const double* x, const double* y, int64_t n, double* out, ReduceScratch& rs, int blocks,
-            cudaStream_t st) {
-    blocks = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    DMRG_LAUNCH dot_kernel<<<blocks, kVecThreads, 0, st>>>(x, y, n, rs.partial.as<double>(), rs.ticket.as<unsigned>(), out, 0);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
-}
-
-int vec_axpy_norm(const double* alpha, const double* x, double* y, int64_t n, double* out, ReduceScratch& rs,
-                  int blocks, cudaStream_t st) {
-    blocks = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    DMRG_LAUNCH axpy_norm_kernel<<<blocks, kVecThreads, 0, st>>>(alpha, x, y, n, rs.partial.as<double>(),
-                                                     rs.ticket.as<unsigned>() + 1, out);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
-}
-
-int vec_multidot(const double* V, int64_t ldv, int m, const double* w, int64_t n, double* c, ReduceScratch& rs,
-                 int blocks, cudaStream_t st) {
-    if (m <= 0) return DMRG_OK;
-    const int nb = multidot_slices(blocks, rs.max_blocks, m);
-    if ((size_t)nb * m * sizeof(double) > rs.partial.bytes)
-        return set_error(DMRG_E_ARG, "multidot scratch too small (%d x %d)", nb, m);
-    DMRG_LAUNCH multidot_kernel<<<dim3(nb, m), kVecThreads, 0, st>>>(V, ldv, w, n, rs.partial.as<double>(),
-                                                         rs.ticket.as<unsigned>() + kRowTickets, c);
-    DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
 
 int vec_combine(const double* V, int64_t ldv, int m, const double* c, double sign, double* w, double beta_w,
                 int64_t n, int blocks, cudaStream_t st) {
     if (m > kMaxVec) return set_error(DMRG_E_ARG, "combine of %d > %d vectors", m, kMaxVec);
-    DMRG_LAUNCH combine_kernel<<<blocks, kVecThreads, 0, st>>>(V, ldv, m, c, sign, w, beta_w, n, nullptr, nullptr, nullptr);
+    DMRG_LAUNCH combine_kernel<<<blocks, kVecThreads, 0, st>>>(V, ldv, m, c, sign, w, beta_w, n);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
@@ -353,17 +297,6 @@ int vec_combine(const double* V, int64_t ldv, int m, const double* c, double sig
 int vec_lanczos_shift(const double* beta, const double* v_cur, double* h, double* v_next, int64_t n, int blocks,
                       cudaStream_t st) {
     DMRG_LAUNCH lanczos_shift_kernel<<<blocks, kVecThreads, 0, st>>>(beta, v_cur, h, v_next, n);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
-}
-
-int vec_combine_normalize(const double* V, int64_t ldv, int m, const double* c, double sign, double* w, int64_t n,
-                          double* out, ReduceScratch& rs, int blocks, cudaStream_t st) {
-    if (m > kMaxVec) return set_error(DMRG_E_ARG, "combine of %d > %d vectors", m, kMaxVec);
-    blocks = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    DMRG_LAUNCH combine_kernel<<<blocks, kVecThreads, 0, st>>>(V, ldv, m, c, sign, w, 1.0, n, rs.partial.as<double>(),
-                                                   rs.ticket.as<unsigned>() + 2, out);
-    DMRG_LAUNCH scale_inv_kernel<<<blocks, kVecThreads, 0, st>>>(w, out, n);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
@@ -377,47 +310,55 @@ int vec_normalize(double* x, int64_t n, double* out, ReduceScratch& rs, int bloc
     return DMRG_OK;
 }
 
-int vec_dot_it(const double* x, const double* y, int64_t n, double* out_base, const int* state, ReduceScratch& rs,
-               int blocks, cudaStream_t st) {
-    blocks = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    DMRG_LAUNCH dot_it_kernel<<<blocks, kVecThreads, 0, st>>>(x, y, n, rs.partial.as<double>(),
-                                                              rs.ticket.as<unsigned>(), out_base, state);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
+int lanczos_step_grid(int64_t n, int num_sms) {
+    if (n <= kClusterMax) return kStepCluster;
+    return (int)std::min<int64_t>(num_sms, (n + 1023) / 1024);
 }
 
-int vec_axpy_norm_it(const double* alpha_base, const double* x, double* y, int64_t n, double* out_base,
-                     const int* state, ReduceScratch& rs, int blocks, cudaStream_t st) {
-    blocks = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    DMRG_LAUNCH axpy_norm_it_kernel<<<blocks, kVecThreads, 0, st>>>(alpha_base, x, y, n, rs.partial.as<double>(),
-                                                                    rs.ticket.as<unsigned>() + 1, out_base, state);
-    DMRG_CUDA_TRY(cudaGetLastError());
-    return DMRG_OK;
-}
-
-int vec_lanczos_step_it(const double* beta_base, const double* x, double* h, double* V, int64_t n, int niter,
-                        double* c, double* tmp, double* x_next, const int* state, ReduceScratch& rs, int blocks,
-                        cudaStream_t st) {
+int vec_lanczos_step(double* x, double* h, double* V, int64_t n, int niter, double* alpha, double* beta, double* part,
+                     int* state, cudaGraphConditionalHandle loop, int num_sms, cudaStream_t st) {
     if (niter > kMaxVec) return set_error(DMRG_E_ARG, "Lanczos dimension %d > %d", niter, kMaxVec);
-    if ((size_t)rs.max_blocks * niter * sizeof(double) > rs.partial.bytes)
-        return set_error(DMRG_E_ARG, "multidot scratch too small (%d x %d)", rs.max_blocks, niter);
-    const int cb = blocks < rs.max_blocks ? blocks : rs.max_blocks;
-    unsigned* rows = rs.ticket.as<unsigned>() + kRowTickets;
-    const int mg = multidot_it_grid(blocks, rs.max_blocks, niter);
-    DMRG_LAUNCH lanczos_shift_it_kernel<<<blocks, kVecThreads, 0, st>>>(beta_base, x, h, V, n, n, niter, state);
-    // classical Gram-Schmidt twice; the second pass also normalises
-    DMRG_LAUNCH multidot_it_kernel<<<mg, kVecThreads, 0, st>>>(V, n, n, blocks, rs.max_blocks,
-                                                                          rs.partial.as<double>(), rows, c, niter,
-                                                                          state);
-    DMRG_LAUNCH combine_it_kernel<<<blocks, kVecThreads, 0, st>>>(V, n, c, -1.0, n, nullptr, nullptr, nullptr, niter,
-                                                                  state);
-    DMRG_LAUNCH multidot_it_kernel<<<mg, kVecThreads, 0, st>>>(V, n, n, blocks, rs.max_blocks,
-                                                                          rs.partial.as<double>(), rows, c, niter,
-                                                                          state);
-    DMRG_LAUNCH combine_it_kernel<<<cb, kVecThreads, 0, st>>>(V, n, c, -1.0, n, rs.partial.as<double>(),
-                                                              rs.ticket.as<unsigned>() + 2, tmp, niter, state);
-    DMRG_LAUNCH scale_inv_it_kernel<<<cb, kVecThreads, 0, st>>>(V, n, tmp, x_next, n, niter, state);
-    DMRG_CUDA_TRY(cudaGetLastError());
+    const int grid = lanczos_step_grid(n, num_sms);
+    const int64_t slice = (n + grid - 1) / grid, tables = (kStepWarps + 3) * (int64_t)niter + 3;
+    StepArgs a{x, h, V, n, niter, alpha, beta, part, state, 0, 0, loop};
+    int64_t room = kStepShared - tables;
+    if (slice <= room) {
+        a.slice_in_smem = 1;
+        room -= slice;
+    }
+    a.basis_in_smem = (int)std::min<int64_t>(room / std::max<int64_t>(slice, 1), niter);
+    const bool cluster = n <= kClusterMax;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kStepThreads);
+    cfg.dynamicSmemBytes = (size_t)(tables + (a.slice_in_smem + a.basis_in_smem) * slice) * sizeof(double);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cluster) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kStepCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    auto kernel = cluster ? lanczos_step_kernel<true> : lanczos_step_kernel<false>;
+    static_assert(kStepShared * sizeof(double) <= 227 * 1024 && (kStepWarps + 3) * kMaxVec + 3 <= kStepShared,
+                  "shared memory of a Lanczos step");
+    static std::atomic<uint64_t> allowed[2] = {};
+    int dev = 0;
+    DMRG_CUDA_TRY(cudaGetDevice(&dev));
+    const uint64_t bit = uint64_t(1) << (dev & 63);
+    std::atomic<uint64_t>& done = allowed[cluster ? 1 : 0];
+    if (dev >= 64 || !(done.load(std::memory_order_acquire) & bit)) {
+        DMRG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kStepShared * sizeof(double))));
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    count_launch();
+    DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
     return DMRG_OK;
 }
 
