@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "svd.cuh"
 
@@ -596,13 +597,31 @@ __global__ void fro2_kernel(const double* __restrict__ part_ss, int np, double* 
     fro2[i] = s;
 }
 
-// Q <- I for every problem.  Grid (problems, kSlices).
-__global__ void __launch_bounds__(256) init_identity_kernel(const SvdProblem* __restrict__ probs, double* __restrict__ Q) {
+// H <- W with its columns in the given order.  Grid (problems, kSlices).
+__global__ void __launch_bounds__(256) order_columns_kernel(const SvdProblem* __restrict__ probs,
+                                                            const int* __restrict__ order,
+                                                            const double* __restrict__ W, double* __restrict__ H) {
     const SvdProblem p = probs[blockIdx.x];
-    double* q = Q + p.q_off;
+    int64_t b, e;
+    slice_range((int64_t)p.rows * p.cols, blockIdx.y, b, e);
+    for (int64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
+        const int64_t c = i / p.rows;
+        H[p.w_off + i] = W[p.w_off + (int64_t)order[p.perm_off + c] * p.rows + (i - c * p.rows)];
+    }
+}
+
+// Q <- P Qx: row i of the accumulated rotation belongs to column order[i] of W.
+// Grid (problems, kSlices).
+__global__ void __launch_bounds__(256) order_rows_kernel(const SvdProblem* __restrict__ probs,
+                                                         const int* __restrict__ order,
+                                                         const double* __restrict__ Qx, double* __restrict__ Q) {
+    const SvdProblem p = probs[blockIdx.x];
     int64_t b, e;
     slice_range((int64_t)p.cols * p.cols, blockIdx.y, b, e);
-    for (int64_t idx = b + threadIdx.x; idx < e; idx += blockDim.x) q[idx] = (idx / p.cols == idx % p.cols) ? 1.0 : 0.0;
+    for (int64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
+        const int64_t c = i / p.cols;
+        Q[p.q_off + c * p.cols + order[p.perm_off + (i - c * p.cols)]] = Qx[p.q_off + i];
+    }
 }
 
 // Column norms of every working matrix, one warp per column (fixed reduction order).
@@ -628,11 +647,12 @@ __global__ void __launch_bounds__(256) rank_kernel(const SvdProblem* __restrict_
     const SvdProblem p = probs[blockIdx.x];
     const double* t = norm + p.s_off;
     for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < p.cols; j += gridDim.y * blockDim.x) {
-        const double v = t[j];
+        // a NaN ranks as the largest, so that the order is a permutation for any input
+        const double v = t[j], kv = isnan(v) ? INFINITY : v;
         int rank = 0;
         for (int o = 0; o < p.cols; ++o) {
-            const double u = t[o];
-            rank += (u > v) || (u == v && o < j);
+            const double u = isnan(t[o]) ? INFINITY : t[o];
+            rank += (u > kv) || (u == kv && o < j);
         }
         order[p.perm_off + rank] = j;
         if (sig) sig[p.s_off + rank] = v;
@@ -775,6 +795,8 @@ const std::vector<uint32_t>* pair_schedule() {
 
 int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaStream_t st) {
     probs.clear();
+    xprobs.clear();
+    t_size = 0;
     tiles.clear();
     tile_first.clear();
     index.assign(m.size(), -1);
@@ -793,6 +815,8 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
         p.q_off = qoff;
         p.s_off = soff;
         p.perm_off = soff;
+        p.t_off = t_size;
+        t_size += (int64_t)((p.cols + kQrPanel - 1) / kQrPanel) * kQrPanel * kQrPanel;
         woff += (int64_t)p.rows * p.cols;
         qoff += (int64_t)p.cols * p.cols;
         soff += p.cols;
@@ -801,7 +825,12 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
         for (int bi = 0; bi < nb; ++bi)
             for (int bj = bi; bj < nb; ++bj) tiles.push_back(SvdTile{(int)probs.size(), bi, bj, 0});
         probs.push_back(p);
+        p.rows = p.cols;
+        p.w_off = p.q_off;
+        xprobs.push_back(p);
     }
+    w_size = woff;
+    q_size = qoff;
     tile_first.push_back((int)tiles.size());
     // Capacities.  A sweep holds at most every block pair of a problem plus one
     // pair per block for blocks unconverged only within themselves; a round at
@@ -809,13 +838,13 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
     // kGramMinRows rows each, fewer items than ~4 per SM in the widest round
     // (bounds the partial-Gram buffer).
     int64_t widest = 0, sweep_tasks = 0, sweep_gram = 0, sweep_rot = 0, round_tasks = 0;
-    for (const SvdProblem& p : probs) {
+    for (const SvdProblem& p : xprobs) {
         widest += (int64_t)p.rows * (p.nbe / 2);
         round_tasks += p.nbe / 2;
     }
     gram_rows = (int)std::max<int64_t>(kGramMinRows, ((widest / 600 + 31) / 32) * 32);
     int64_t round_gram = 0;
-    for (const SvdProblem& p : probs) {
+    for (const SvdProblem& p : xprobs) {
         const int64_t pairs = (int64_t)p.nbe * (p.nbe - 1) / 2 + p.nbe;
         const int64_t gi = (p.rows + gram_rows - 1) / gram_rows;
         const int64_t ri = (p.rows + kPair - 1) / kPair + (p.cols + kPair - 1) / kPair;
@@ -831,28 +860,54 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
     max_round_gram = (int)round_gram;
     DMRG_TRY(d_w.alloc((size_t)std::max<int64_t>(woff, 1) * sizeof(double)));
     DMRG_TRY(d_q.alloc((size_t)std::max<int64_t>(qoff, 1) * sizeof(double)));
-    DMRG_TRY(d_s.alloc((size_t)std::max<int64_t>(2 * soff, 1) * sizeof(double)));
-    DMRG_TRY(d_perm.alloc((size_t)std::max<int64_t>(soff, 1) * sizeof(int)));
-    DMRG_TRY(d_fro2.alloc(std::max<size_t>(probs.size(), 1) * sizeof(double)));
-    DMRG_TRY(d_expo.alloc(std::max<size_t>(probs.size(), 1) * sizeof(int)));
-    DMRG_TRY(d_part.alloc(std::max<size_t>(probs.size(), 1) * 2 * kSlices * sizeof(double)));
-    DMRG_TRY(d_sign.alloc((size_t)std::max<int64_t>(soff, 1) * sizeof(double)));
-    DMRG_TRY(d_colmap.alloc((size_t)std::max<int64_t>(soff, 1) * sizeof(int)));
-    DMRG_TRY(d_norm.alloc((size_t)std::max<int64_t>(soff, 1) * sizeof(double)));
-    DMRG_TRY(d_bm.alloc(std::max<size_t>(tiles.size(), 1) * sizeof(double)));
-    if (!d_sched.ptr) {
-        const std::vector<uint32_t>* sched = pair_schedule();
-        if (!sched) return set_error(DMRG_E_STATE, "no pair schedule");
-        DMRG_TRY(upload(d_sched, *sched, st));
+    const auto some = [](int64_t n) { return (size_t)std::max<int64_t>(n, 1); };
+    s_size = soff;
+    DMRG_TRY(d_w.alloc(some(w_size) * sizeof(double)));
+    DMRG_TRY(d_q.alloc(some(q_size) * sizeof(double)));
+    DMRG_TRY(d_s.alloc(some(2 * soff) * sizeof(double)));
+    DMRG_TRY(d_perm.alloc(some(soff) * sizeof(int)));
+    DMRG_TRY(d_sign.alloc(some(soff) * sizeof(double)));
+    const std::vector<uint32_t>* sched = pair_schedule();
+    if (!sched) return set_error(DMRG_E_STATE, "no pair schedule");
+    Tables tab;
+    tab.add(probs);  // at offset 0: d_probs is the problem table
+    const size_t at_x = tab.add(xprobs), at_tiles = tab.add(tiles), at_sched = tab.add(*sched);
+    DMRG_TRY(tab.to(d_probs, st));
+    const unsigned char* tb = d_probs.as<unsigned char>();
+    work.xprobs = reinterpret_cast<const SvdProblem*>(tb + at_x);
+    work.tiles = reinterpret_cast<const SvdTile*>(tb + at_tiles);
+    work.sched = reinterpret_cast<const uint32_t*>(tb + at_sched);
+    // the workspace: two passes over its pieces, sizes then addresses
+    const int64_t np = (int64_t)probs.size();
+    size_t bytes = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass) DMRG_TRY(d_work.alloc(some((int64_t)bytes)));
+        unsigned char* base = d_work.as<unsigned char>();
+        bytes = 0;
+        const auto piece = [&](auto*& p, int64_t n) {
+            if (pass) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + bytes);
+            bytes += (some(n) * sizeof(*p) + 255) & ~size_t(255);
+        };
+        piece(work.h, w_size);
+        piece(work.h2, 2 * q_size);  // h2, then x: cleared together
+        piece(work.qx, q_size);
+        piece(work.t1, t_size);
+        piece(work.t2, t_size);
+        piece(work.fro2, np);
+        piece(work.part, np * 2 * kSlices);
+        piece(work.norm, soff);
+        piece(work.bm, (int64_t)tiles.size());
+        piece(work.gpart, (int64_t)max_round_gram * kPair * kPair);
+        piece(work.rot, (int64_t)max_round_tasks * kPair * kPair);
+        piece(work.tasks, max_tasks);
+        piece(work.gram_items, max_gram);
+        piece(work.rot_items, max_rot);
+        piece(work.expo, np);
+        piece(work.order, soff);
+        piece(work.colmap, soff);
+        piece(work.skip, max_round_tasks);
     }
-    DMRG_TRY(upload(d_probs, probs, st));
-    DMRG_TRY(upload(d_tiles, tiles, st));
-    DMRG_TRY(d_tasks.alloc(std::max<size_t>(max_tasks, 1) * sizeof(SvdTask)));
-    DMRG_TRY(d_gram_items.alloc(std::max<size_t>(max_gram, 1) * sizeof(SvdItem)));
-    DMRG_TRY(d_rot_items.alloc(std::max<size_t>(max_rot, 1) * sizeof(SvdItem)));
-    DMRG_TRY(d_gpart.alloc((size_t)std::max(max_round_gram, 1) * kPair * kPair * sizeof(double)));
-    DMRG_TRY(d_rot.alloc((size_t)std::max(max_round_tasks, 1) * kPair * kPair * sizeof(double)));
-    DMRG_TRY(d_skip.alloc((size_t)std::max(max_round_tasks, 1) * sizeof(int)));
+    work.x = work.h2 + q_size;
     DMRG_CUDA_TRY(cudaFuncSetAttribute(solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(SvdSmem)));
     static_assert(sizeof(SvdSmem) <= 227 * 1024, "pair solve shared memory");
@@ -861,7 +916,7 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
 }
 
 void BatchedSvd::add_task(int problem, int bi, int bj) {
-    const SvdProblem& p = probs[problem];
+    const SvdProblem& p = xprobs[problem];
     const int t = (int)tasks.size();
     SvdTask task{problem, bi, bj, (int)gram_items.size() - round_gram_first.back(), 0};
     for (int r0 = 0; r0 < p.rows; r0 += gram_rows)
@@ -964,8 +1019,8 @@ int BatchedSvd::schedule(const std::vector<double>& bm) {
     std::vector<std::vector<std::vector<std::pair<int, int>>>> per(probs.size());
     size_t rounds = 0;
     for (size_t pi = 0; pi < probs.size(); ++pi) {
-        const double tol = 2.0 * DBL_EPSILON * std::sqrt((double)probs[pi].rows);
-        per[pi] = problem_rounds(probs[pi], bm.data() + tile_first[pi], tol);
+        const double tol = 2.0 * DBL_EPSILON * std::sqrt((double)xprobs[pi].rows);
+        per[pi] = problem_rounds(xprobs[pi], bm.data() + tile_first[pi], tol);
         rounds = std::max(rounds, per[pi].size());
     }
     for (size_t r = 0; r < rounds; ++r) {
@@ -990,11 +1045,11 @@ void BatchedSvd::dump_unconverged(const char* path, const DeviceBuffer& w_in, co
     std::FILE* f = std::fopen(path, "ab");
     if (!f) return;
     std::vector<double> fro2(probs.size());
-    cudaMemcpyAsync(fro2.data(), d_fro2.ptr, fro2.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(fro2.data(), work.fro2, fro2.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
     for (size_t i = 0; i < probs.size(); ++i) {
         const SvdProblem& p = probs[i];
-        if (worst[i] <= 2.0 * DBL_EPSILON * std::sqrt((double)p.rows)) continue;
+        if (worst[i] <= 2.0 * DBL_EPSILON * std::sqrt((double)p.cols)) continue;
         const size_t cnt = (size_t)p.rows * p.cols;
         std::vector<double> a(cnt), b(cnt);
         cudaMemcpyAsync(a.data(), w_in.as<double>() + p.w_off, cnt * sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -1026,34 +1081,41 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
         DMRG_CUDA_TRY(cudaMemcpyAsync(w_in.ptr, d_w.ptr, d_w.bytes, cudaMemcpyDeviceToDevice, st));
     }
     const dim3 sliced(np, kSlices);
-    DMRG_LAUNCH init_identity_kernel<<<sliced, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_q.as<double>());
-    DMRG_LAUNCH slice_max_kernel<<<sliced, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), d_part.as<double>());
-    DMRG_LAUNCH prescale_kernel<<<sliced, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), d_part.as<double>(),
-                                                        d_expo.as<int>(), d_part.as<double>() + (int64_t)np * kSlices);
-    DMRG_LAUNCH fro2_kernel<<<(np + 127) / 128, 128, 0, st>>>(d_part.as<double>() + (int64_t)np * kSlices, np,
-                                                              d_fro2.as<double>());
+    DMRG_LAUNCH slice_max_kernel<<<sliced, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), work.part);
+    DMRG_LAUNCH prescale_kernel<<<sliced, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), work.part,
+                                                        work.expo, work.part + (int64_t)np * kSlices);
+    DMRG_LAUNCH fro2_kernel<<<(np + 127) / 128, 128, 0, st>>>(work.part + (int64_t)np * kSlices, np, work.fro2);
     static const bool debug = std::getenv("DMRG_SVD_DEBUG") != nullptr;  // per-sweep convergence to stderr
     int max_cols = 0;
     for (const SvdProblem& p : probs) max_cols = std::max(max_cols, p.cols);
     const dim3 colgrid(np, (max_cols + 7) / 8);
     const dim3 rankgrid(np, (max_cols + 255) / 256);
+    // Preconditioner: W P = Q1 R, R^T = Q2 R2, sweeps on X = R2^T (X J = Y), so that
+    // U S = Q1 Y and V = P Q2 J.
+    const SvdProblem* wp = d_probs.as<SvdProblem>();
+    const SvdProblem* xp = work.xprobs;
+    double *h = work.h, *h2 = work.h2, *x = work.x, *qx = work.qx, *t1 = work.t1, *t2 = work.t2;
+    DMRG_CUDA_TRY(cudaMemsetAsync(h2, 0, 2 * q_size * sizeof(double), st));
+    DMRG_LAUNCH colnorm_kernel<<<colgrid, 256, 0, st>>>(wp, d_w.as<double>(), work.norm);
+    DMRG_LAUNCH rank_kernel<<<rankgrid, 256, 0, st>>>(wp, work.norm, work.order, nullptr);
+    DMRG_LAUNCH order_columns_kernel<<<sliced, 256, 0, st>>>(wp, work.order, d_w.as<double>(), h);
+    DMRG_TRY(qr_factor(wp, np, max_cols, h, h2, t1, st));
+    DMRG_TRY(qr_factor(xp, np, max_cols, h2, x, t2, st));
+    DMRG_TRY(qr_apply(xp, np, max_cols, h2, t2, nullptr, qx, st));
     std::vector<double> bm(tiles.size()), worst(np);
     const int max_sweeps = g_max_sweeps.load();
     auto t_sweep = std::chrono::steady_clock::now();
     int sweep = 0;
     bool converged = false;
     for (;; ++sweep) {
-        // the sweep visits columns in descending norm order: blocks hold columns of
-        // similar size, which keeps the many tiny singular values of a noise-expanded
-        // tensor from converging only linearly; then every block pair is measured
-        DMRG_LAUNCH colnorm_kernel<<<colgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), d_norm.as<double>());
-        DMRG_LAUNCH rank_kernel<<<rankgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_norm.as<double>(), d_colmap.as<int>(),
-                                                    nullptr);
+        // the sweep visits columns in descending norm order (blocks hold columns of
+        // similar size); then every block pair is measured
+        DMRG_LAUNCH colnorm_kernel<<<colgrid, 256, 0, st>>>(xp, x, work.norm);
+        DMRG_LAUNCH rank_kernel<<<rankgrid, 256, 0, st>>>(xp, work.norm, work.colmap, nullptr);
         DMRG_LAUNCH measure_kernel<<<(int)tiles.size(), 128, 0, st>>>(
-            d_probs.as<SvdProblem>(), d_tiles.as<SvdTile>(), d_colmap.as<int>(), d_w.as<double>(),
-            d_norm.as<double>(), d_fro2.as<double>(), d_bm.as<double>());
+            xp, work.tiles, work.colmap, x, work.norm, work.fro2, work.bm);
         DMRG_CUDA_TRY(cudaGetLastError());
-        DMRG_CUDA_TRY(cudaMemcpyAsync(bm.data(), d_bm.ptr, bm.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        DMRG_CUDA_TRY(cudaMemcpyAsync(bm.data(), work.bm, bm.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
         DMRG_CUDA_TRY(cudaStreamSynchronize(st));
         for (int i = 0; i < np; ++i) {
             worst[i] = 0.0;
@@ -1083,29 +1145,27 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
         if ((int)tasks.size() > max_tasks || (int)gram_items.size() > max_gram || (int)rot_items.size() > max_rot ||
             widest_round > max_round_tasks || widest_gram > max_round_gram)
             return set_error(DMRG_E_STATE, "Jacobi SVD schedule exceeds its plan");
-        DMRG_CUDA_TRY(cudaMemcpyAsync(d_tasks.ptr, tasks.data(), tasks.size() * sizeof(SvdTask), cudaMemcpyHostToDevice, st));
-        DMRG_CUDA_TRY(cudaMemcpyAsync(d_gram_items.ptr, gram_items.data(), gram_items.size() * sizeof(SvdItem),
+        DMRG_CUDA_TRY(cudaMemcpyAsync(work.tasks, tasks.data(), tasks.size() * sizeof(SvdTask), cudaMemcpyHostToDevice, st));
+        DMRG_CUDA_TRY(cudaMemcpyAsync(work.gram_items, gram_items.data(), gram_items.size() * sizeof(SvdItem),
                                       cudaMemcpyHostToDevice, st));
-        DMRG_CUDA_TRY(cudaMemcpyAsync(d_rot_items.ptr, rot_items.data(), rot_items.size() * sizeof(SvdItem),
+        DMRG_CUDA_TRY(cudaMemcpyAsync(work.rot_items, rot_items.data(), rot_items.size() * sizeof(SvdItem),
                                       cudaMemcpyHostToDevice, st));
         for (int r = 0; r < rounds; ++r) {
             const int nt = round_first[r + 1] - round_first[r];
             const int ng = round_gram_first[r + 1] - round_gram_first[r];
             const int nr = round_rot_first[r + 1] - round_rot_first[r];
             if (nt == 0) continue;
-            DMRG_LAUNCH gram_kernel<<<ng, 128, 0, st>>>(d_probs.as<SvdProblem>(), d_tasks.as<SvdTask>(),
-                                                        d_gram_items.as<SvdItem>() + round_gram_first[r],
-                                                        d_colmap.as<int>(), d_w.as<double>(), d_gpart.as<double>());
+            DMRG_LAUNCH gram_kernel<<<ng, 128, 0, st>>>(xp, work.tasks, work.gram_items + round_gram_first[r],
+                                                        work.colmap, x, work.gpart);
             DMRG_LAUNCH solve_kernel<<<nt, kThreads, sizeof(SvdSmem), st>>>(
-                d_probs.as<SvdProblem>(), d_tasks.as<SvdTask>(), round_first[r], d_gpart.as<double>(),
-                d_fro2.as<double>(), d_rot.as<double>(), d_skip.as<int>(), d_sched.as<uint32_t>(), kInnerSweeps);
-            DMRG_LAUNCH rotate_kernel<<<nr, 128, kRotSmem, st>>>(d_probs.as<SvdProblem>(), d_tasks.as<SvdTask>(),
-                                                                 d_rot_items.as<SvdItem>() + round_rot_first[r],
-                                                                 round_first[r], d_rot.as<double>(), d_skip.as<int>(),
-                                                                 d_colmap.as<int>(), d_w.as<double>(), d_q.as<double>());
+                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip, work.sched, kInnerSweeps);
+            DMRG_LAUNCH rotate_kernel<<<nr, 128, kRotSmem, st>>>(xp, work.tasks, work.rot_items + round_rot_first[r],
+                                                                 round_first[r], work.rot, work.skip, work.colmap, x,
+                                                                 qx);
         }
         DMRG_CUDA_TRY(cudaGetLastError());
     }
+    DMRG_TRY(qr_apply(wp, np, max_cols, h, t1, x, d_w.as<double>(), st));
     if (!converged) {
         if (fail_dump) dump_unconverged(fail_dump, w_in, worst, st);
         int wi = 0;
@@ -1114,12 +1174,13 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
         return set_error(DMRG_E_NUMERIC, "Jacobi SVD did not converge in %d sweeps (sector %d x %d: off-diagonal %.3e)",
                          max_sweeps, probs[wi].m, probs[wi].n, worst[wi]);
     }
+    DMRG_LAUNCH order_rows_kernel<<<sliced, 256, 0, st>>>(wp, work.order, qx, d_q.as<double>());
     // singular values = final column norms, sorted
-    DMRG_LAUNCH colnorm_kernel<<<colgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), d_norm.as<double>());
-    DMRG_LAUNCH rank_kernel<<<rankgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_norm.as<double>(), d_perm.as<int>(), d_s.as<double>());
+    DMRG_LAUNCH colnorm_kernel<<<colgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(), work.norm);
+    DMRG_LAUNCH rank_kernel<<<rankgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), work.norm, d_perm.as<int>(), d_s.as<double>());
     DMRG_LAUNCH sign_kernel<<<colgrid, 256, 0, st>>>(d_probs.as<SvdProblem>(), d_w.as<double>(),
                                                                d_q.as<double>(), d_perm.as<int>(), d_sign.as<double>());
-    DMRG_LAUNCH unscale_kernel<<<dim3(np, 32), 256, 0, st>>>(d_probs.as<SvdProblem>(), d_expo.as<int>(),
+    DMRG_LAUNCH unscale_kernel<<<dim3(np, 32), 256, 0, st>>>(d_probs.as<SvdProblem>(), work.expo,
                                                              d_w.as<double>(), d_s.as<double>());
     DMRG_CUDA_TRY(cudaGetLastError());
     if (sweeps_out) *sweeps_out = sweep;  // sweeps that rotated

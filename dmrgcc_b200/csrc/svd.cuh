@@ -1,27 +1,35 @@
 // Batched FP64 SVD of the sector matrices of one canonicalisation, on the device.
 //
-// Algorithm: one-sided (Hestenes) Jacobi with 32-column blocks.  Each sector
-// matrix A (m x n) is held as a column-major working matrix W with c <= r
-// columns: W = A when n <= m (right rotations accumulate V), W = A^T otherwise
-// (they accumulate U).  A sweep first orders the columns by descending norm
-// (de Rijk's pivoting, applied block-wise: blocks then hold columns of similar
-// size, which halves the sweeps on noise-expanded tensors whose spectra are
-// mostly tiny), then measures every pair of column blocks at once (the 32x32
-// cross-Gram blocks of W, DMMA) and visits only the block pairs found
-// unconverged, in as few rounds as a matching of them allows (the round-robin
+// Algorithm: one-sided (Hestenes) Jacobi with 32-column blocks, preconditioned by
+// two QR factorisations.  Each sector matrix A (m x n) is held as a column-major
+// working matrix W with c <= r columns: W = A when n <= m (right rotations
+// accumulate V), W = A^T otherwise (they accumulate U).  With W P = Q1 R (P: columns
+// by descending norm) and R^T = Q2 R2 (Householder, svd_qr.cu), the sweeps run on
+// the c x c matrix X = R2^T, X J = Y, and U S = Q1 Y, V = P Q2 J.  A QR factor of
+// a transposed QR factor is close to diagonal and graded, so few rotations remain:
+// the tensors of a subspace expansion (spectra over nine decades and more) take 5
+// sweeps instead of 19 at D = 1024 and 3 instead of 10 at D = 64, on r / c times
+// fewer rows.  Two unpivoted factorisations did better than one with column
+// pivoting (whose norms serialise the panels): 24 against 38 rounds on a
+// 400 x 250 matrix.  Whole canonicalisation, D = 1024 cylinder tensor (17 sectors to
+// 611 x 510): 47.2 ms without, 12.8 ms with; D = 64 chain tensor (33 columns):
+// 2.03 and 0.92 ms.  A sweep first orders the columns by descending norm
+// (de Rijk's pivoting, applied block-wise), then measures every pair of column
+// blocks at once (the 32x32 cross-Gram blocks, DMMA) and visits only the block
+// pairs found unconverged, in as few rounds as a matching of them allows (the round-robin
 // order restricted to them, or a greedy matching by measure if that needs
 // fewer rounds).  In a round all pairs of all sectors are independent and each
 // is split over CTAs by rows: (1) partial 64x64 Gram matrices of the pair over
 // row ranges (DMMA), (2) one CTA per pair sums them and runs a few cyclic
 // Jacobi sweeps on the Gram matrix in shared memory, (3) 64-row slices of the
-// pair's columns of W and of the accumulated rotation are multiplied by the
+// pair's columns of X and of the accumulated rotation are multiplied by the
 // resulting 64x64 rotation (DMMA).  Converged when no pair has
-// |g_ij| > tol ||A||_F max(|x_i|, |x_j|), tol = 2 eps sqrt(rows): the
+// |g_ij| > tol ||A||_F max(|x_i|, |x_j|), tol = 2 eps sqrt(c): the
 // remaining non-orthogonality is a backward perturbation of A below rounding
 // level, the accuracy of a backward-stable SVD such as the reference's dgesvd
 // (singular values to ~eps ||A||, enough for its canpre cut at 1e-12 of a
 // normalised state); columns of a rank-deficient matrix
-// whose norm falls to rounding level (4 eps sqrt(rows) ||A||_F) are left out of
+// whose norm falls to rounding level (4 eps sqrt(c) ||A||_F) are left out of
 // rotations and of that test.  A matrix whose entries are all below 1/2 is
 // first scaled by a power of two (exact) so that its largest entry lies in
 // [0.5, 1), and scaled back at the end: the thresholds are relative, but their
@@ -38,6 +46,8 @@
 
 namespace dmrg {
 
+constexpr int kQrPanel = 16;  // columns of a QR panel
+
 struct SvdProblem {
     int m, n;            // the sector matrix A is m x n
     int rows, cols;      // working matrix W: rows x cols, cols <= rows, column-major (ld = rows)
@@ -47,6 +57,7 @@ struct SvdProblem {
     int64_t q_off;       // offset of the accumulated rotation (cols x cols, column-major)
     int64_t s_off;       // offset of the sorted singular values (cols doubles)
     int64_t perm_off;    // offset of the sort permutation (cols ints)
+    int64_t t_off;       // offset of the QR panels' T (kQrPanel^2 doubles per panel)
 };
 
 struct SvdTask {
@@ -68,6 +79,15 @@ struct SvdItem {   // a row range of one pair task's columns
     int r0, r1;
 };
 
+// Householder QR of every problem's matrix m (rows x cols at w_off): reflectors
+// into m, R^T into rt (cols x cols at q_off, whose upper triangle must be zero),
+// the panels' T into t.
+int qr_factor(const SvdProblem* probs, int np, int max_cols, double* m, double* rt, double* t, cudaStream_t st);
+// c (rows x cols at w_off) <- Q [src; 0] (src cols x cols at q_off), or the first
+// cols columns of Q with src null, for the reflectors in m and t.
+int qr_apply(const SvdProblem* probs, int np, int max_cols, const double* m, const double* t, const double* src,
+             double* c, cudaStream_t st);
+
 class BatchedSvd {
 public:
     // Plans the batch for the given sector shapes (m[i] x n[i]; entries with
@@ -84,15 +104,13 @@ public:
     void dump_unconverged(const char* path, const DeviceBuffer& w_in, const std::vector<double>& worst,
                           cudaStream_t st);
 
-    DeviceBuffer d_w, d_q, d_s, d_perm, d_probs, d_tasks, d_fro2;
-    DeviceBuffer d_expo;  // per problem: the power of two W was scaled by (prescale_kernel)
-    DeviceBuffer d_part;  // per problem and slice: largest magnitude, then sum of squares
-    DeviceBuffer d_sign;  // +-1 per sorted singular triplet (sign convention, set by run())
-    DeviceBuffer d_gram_items, d_rot_items, d_gpart, d_rot, d_skip;
-    DeviceBuffer d_colmap, d_norm;  // per sweep: columns in descending norm order
-    DeviceBuffer d_tiles, d_bm;     // the convergence measure's tiles and their values
-    DeviceBuffer d_sched;           // lane order of the pair solve's rotations (uploaded once)
+    // results: U S (the working matrices), the accumulated rotations, the sorted
+    // singular values, their permutation, and +-1 per sorted triplet (sign convention)
+    DeviceBuffer d_w, d_q, d_s, d_perm, d_sign;
+    DeviceBuffer d_probs;               // probs, then the other tables (see Work)
     std::vector<SvdProblem> probs;
+    std::vector<SvdProblem> xprobs;     // the square matrices that the sweeps run on: rows = cols, w_off = q_off
+    int64_t w_size = 0, q_size = 0, s_size = 0, t_size = 0;
     std::vector<int> index;             // sector -> problem (-1 when empty)
     std::vector<SvdTile> tiles;         // all block pairs bi <= bj of every problem
     std::vector<int> tile_first;        // per problem: its first tile
@@ -106,6 +124,25 @@ public:
     int max_round_tasks = 0, max_round_gram = 0;   // capacities (per round)
 
 private:
+    // Device addresses in d_probs (tables) and d_work (one allocation: a plan is
+    // made for every site step, and an allocation costs more than a small kernel).
+    struct Work {
+        const SvdProblem* xprobs;
+        const SvdTile* tiles;       // the convergence measure's tiles
+        const uint32_t* sched;      // lane order of the pair solve's rotations
+        double *h, *t1;             // reflectors of W and their T
+        double *h2, *t2;            // R^T, then its reflectors; their T
+        double *x, *qx;             // the matrix of the sweeps and its accumulated rotation
+        double *fro2, *part;        // per problem; per problem and slice: largest magnitude, then sum of squares
+        double *norm, *bm;          // column norms; the tiles' measures
+        double *gpart, *rot;        // partial Gram matrices and rotations of a round
+        SvdTask* tasks;
+        SvdItem *gram_items, *rot_items;
+        int *expo;                  // per problem: the power of two W was scaled by (prescale_kernel)
+        int *order, *colmap, *skip; // the columns of W, of x in descending norm order
+    } work{};
+    DeviceBuffer d_work;
+
     // Builds the sweep's rounds from the block measures bm (tiles order);
     // returns the number of rounds (0: converged).
     int schedule(const std::vector<double>& bm);
