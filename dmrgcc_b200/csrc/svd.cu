@@ -23,10 +23,12 @@ constexpr int kChunk = 32;      // rows per streamed chunk
 #endif
 constexpr int kThreads = DMRG_SVD_SOLVE_THREADS;   // pair-solve CTA
 constexpr int kLd = kPair + 1;  // padded row of the shared 64x64 matrices
-#ifndef DMRG_SVD_INNER_SWEEPS
-#define DMRG_SVD_INNER_SWEEPS 2
-#endif
-constexpr int kInnerSweeps = DMRG_SVD_INNER_SWEEPS;
+// Sweeps of a pair solve: one where a sector has further pairs, whose rotations undo
+// a pair's diagonality again (D = 1024: 10.2 ms of sweeps with one, 11.6 with two,
+// 13.4 with three); two where the pair is the whole sector and a further outer sweep
+// costs its launches (D = 64: 0.94 ms of canonicalisation, 1.09 with one).
+constexpr int kInnerSweepsMany = 1, kInnerSweepsOnly = 2;
+constexpr int kInnerSweeps = kInnerSweepsOnly;  // the larger
 constexpr int kMaxSweeps = 40;
 // The sweep cap in force (dmrg_svd_set_max_sweeps lowers it to provoke the
 // did-not-converge path without touching the device).
@@ -267,8 +269,7 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __res
                                                          const SvdTask* __restrict__ tasks, int first,
                                                          const double* __restrict__ gpart,
                                                          const double* __restrict__ fro2, double* __restrict__ rot,
-                                                         int* __restrict__ skip, const uint32_t* __restrict__ sched,
-                                                         int inner_sweeps) {
+                                                         int* __restrict__ skip, const uint32_t* __restrict__ sched) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SvdSmem& S = *reinterpret_cast<SvdSmem*>(smem_raw);
     const int t = first + blockIdx.x;
@@ -327,6 +328,7 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __res
     static_assert(kThreads % 32 == 0 && kItems * kThreads == (kPair / 2) * (kPair / 2) && kQRows * kWarps == kPair,
                   "even split of the Gram blocks and of the rows of Q");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int inner_sweeps = p.nbe > 2 ? kInnerSweepsMany : kInnerSweepsOnly;
     int steps = 0;  // rotation log entries written
     int cur = 0;    // the copy of G holding the current matrix
     for (int sweep = 0; sweep < inner_sweeps; ++sweep) {
@@ -1158,7 +1160,7 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
             DMRG_LAUNCH gram_kernel<<<ng, 128, 0, st>>>(xp, work.tasks, work.gram_items + round_gram_first[r],
                                                         work.colmap, x, work.gpart);
             DMRG_LAUNCH solve_kernel<<<nt, kThreads, sizeof(SvdSmem), st>>>(
-                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip, work.sched, kInnerSweeps);
+                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip, work.sched);
             DMRG_LAUNCH rotate_kernel<<<nr, 128, kRotSmem, st>>>(xp, work.tasks, work.rot_items + round_rot_first[r],
                                                                  round_first[r], work.rot, work.skip, work.colmap, x,
                                                                  qx);
