@@ -140,6 +140,34 @@ int upload(DeviceBuffer& buf, const std::vector<T>& v, cudaStream_t stream) {
     return DMRG_OK;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may start while the
+// launch before it on the stream still runs; wait_previous returns when that launch has
+// completed and its writes are visible, so that launch latency and set-up pass behind
+// its last CTAs.  Every CTA of such a kernel calls it before it reads or writes
+// anything that an earlier launch writes or reads.  launch_next lets the next launch
+// in before this one's CTAs have exited.
+#ifdef __CUDACC__
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    count_launch();
+    DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return DMRG_OK;
+}
+#endif
+
 // Several host tables in one device allocation and one copy.
 class Tables {
 public:

@@ -97,15 +97,10 @@ __device__ __forceinline__ void bulk_copy(unsigned dst, const double* src, unsig
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
-// Programmatic dependent launch: wait_previous returns when the launch before this one
-// on the stream has completed and its writes are visible, so launch latency and the
-// first descriptor reads pass behind its last CTAs (D=300 matvec 30 -> 22.5 us).
-// launch_next lets the next launch in early: the pack kernel does; the GEMM kernel
-// leaves it to its CTAs' exits (the next launch's waiting CTAs would take the shared
-// memory of its own: Lanczos at D=512 1.27 -> 1.33 ms).
-__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
+// Launches are chained (launch_pdl): D=300 matvec 30 -> 22.5 us.  The pack kernel lets
+// the next launch in early (launch_next); the GEMM kernel leaves it to its CTAs' exits
+// (the next launch's waiting CTAs would take the shared memory of its own: Lanczos at
+// D=512 1.27 -> 1.33 ms).
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory"); }
 
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
@@ -527,28 +522,11 @@ int allow_smem(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
     return DMRG_OK;
 }
 
-template <class... P, class... A>
-int launch_pdl(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-    return DMRG_OK;
-}
-
 template <int OUT, bool SCALED>
 int launch(int n, const GemmArgs& w, cudaStream_t st) {
     static std::atomic<uint64_t> allowed{0};
     DMRG_TRY(allow_smem(img_gemm_kernel<OUT, SCALED>, kSmem, allowed));
-    return launch_pdl(img_gemm_kernel<OUT, SCALED>, n, kThreads, kSmem, st, w);
+    return launch_pdl(img_gemm_kernel<OUT, SCALED>, dim3(n), kThreads, kSmem, st, w);
 }
 
 // The schedule's cost model (cycles of a step and of a tile's own work) and cuts.
@@ -615,7 +593,7 @@ int ImgPack::finalize(int panel, cudaStream_t stream) {
 int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
                     double* img, cudaStream_t stream) {
     if (c1 <= c0) return DMRG_OK;
-    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, c1 - c0, kPackThreads, 0, stream, p.d_tables.as<ImgJob>(),
+    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, dim3(c1 - c0), kPackThreads, 0, stream, p.d_tables.as<ImgJob>(),
                       reinterpret_cast<const ImgChunk*>(p.d_tables.as<char>() + p.chunks_at) + c0, panel, s0, s1, s2, img);
 }
 

@@ -205,6 +205,9 @@ int build_heff(dmrg_heff_s& h) {
             g.t1 = (int)h.pb.terms.size();
             h.pb.groups.push_back(g);
         }
+        int64_t covered = 0;
+        for (const PackedGroup& g : h.pb.groups) covered += (int64_t)g.m * g.n;
+        h.pb_covers = covered == ket.size;
         DMRG_TRY(h.pa.check_bounds(h.pk_psi.bytes, h.pk_R.bytes, 0, h.t_img_bytes));
         DMRG_TRY(h.pb.check_bounds(h.pk_L.bytes, h.t_img_bytes, ket.size, 0));
         DMRG_TRY(h.pk_psi.finalize(st));
@@ -250,13 +253,16 @@ int dmrg::heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bo
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
-    if (!accumulate && h.site.ket.size)
+    // out blocks that no term reaches are zero; where there are none, stage B stores
+    // every element and out needs no clearing
+    const bool clear = !accumulate && !h.pb_covers;
+    if (clear && h.site.ket.size)
         DMRG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)h.site.ket.size * sizeof(double), st));
     DMRG_TRY(launch_pack(h.pk_psi, psi, h.img_psi.as<unsigned char>(), st));
     DMRG_TRY(launch_gemm_split(h.pa, h.img_psi.as<unsigned char>(), h.img_R.as<unsigned char>(), nullptr,
                                 h.img_T.as<unsigned char>(), false, h.ctx->d_status, st));
-    DMRG_TRY(launch_gemm_split(h.pb, h.img_L.as<unsigned char>(), h.img_T.as<unsigned char>(), out, nullptr, true,
-                                h.ctx->d_status, st));
+    DMRG_TRY(launch_gemm_split(h.pb, h.img_L.as<unsigned char>(), h.img_T.as<unsigned char>(), out, nullptr,
+                                accumulate || clear, h.ctx->d_status, st));
     return DMRG_OK;
 }
 

@@ -23,6 +23,7 @@ struct dmrg_heff_s {
     dmrg::ImgWork work;
     // split precisions (DMRG_PREC_TF32X3 / DMRG_PREC_BF16X3) only: operand images
     // and packed schedules
+    bool pb_covers = false;                    // stage B stores every element of the output
     dmrg::PackSchedule pk_psi, pk_L, pk_R;     // which blocks to pack, where
     dmrg::PackedSchedule pa, pb;               // A: psi x R -> T images ; B: L x T -> out
     dmrg::DeviceBuffer img_psi, img_L, img_R, img_T;
