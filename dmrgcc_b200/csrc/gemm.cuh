@@ -321,8 +321,8 @@ struct PackedGroup {
     int64_t c_off;         // output mode 0: FP64 block at C + c_off (ldc), or its split-K chunk in aux
     int ldc;
     int cbuf;              // 1: split-K chunk, written to aux
-    int64_t t_img;         // output mode 1: the output written as B-role images (rows = columns n,
-    int t_slices;          // k = rows m) for a following packed GEMM; t_slices = ceil(m / pack_k(fmt))
+    int64_t t_img;         // output mode 1: the output written as operand images (rows = rows m,
+    int t_slices;          // k = columns n) for a following packed GEMM; t_slices = ceil(n / pack_k(fmt))
     int pad_;
 };
 struct PackedTile {
@@ -332,7 +332,7 @@ struct PackedSchedule {
     int fmt = kFmtTF32;
     std::vector<PackedTerm> terms;
     std::vector<PackedGroup> groups;
-    int out_mode = 0;  // 0: FP64 output blocks, 1: B-role images
+    int out_mode = 0;  // 0: FP64 output blocks, 1: operand images (one term of weight 1 per group)
     std::vector<PackedGroup> exec_groups;
     std::vector<GemmSplit> splits;
     std::vector<PackedTile> tiles;  // grouped by persistent CTA

@@ -22,7 +22,7 @@
 // so narrow tiles leave the tensor pipe mostly idle; at N = 128 the three
 // products of a k step run at close to the pipe's rate.
 //
-// GEMM (persistent: one CTA per SM walks its own list of tiles, 576 threads,
+// GEMM (persistent: one CTA per SM walks its own list of tiles, 320 threads,
 // warp-specialised; stage counters and the accumulator pair run on across tiles):
 //   warp 0 lane 0   producer: per stage waits the stage's "empty" barrier, arms
 //                   the "full" barrier with the byte count, issues the copies;
@@ -30,11 +30,12 @@
 //                   MMAs into the term's accumulator (two 128-column accumulators
 //                   alternate between terms), commits to "empty"; after a term's
 //                   last stage commits to the accumulator's "full" barrier;
-//   warps 2..17     epilogue: warp w reads TMEM lanes 32(w%4).. and columns
-//                   32((w-2)/4)..+31: per term wait, tcgen05.ld, add w_t * value
+//   warps 2..9      epilogue: warp w reads TMEM lanes 32(w%4).. and columns
+//                   64((w-2)/4)..+63: per term wait, tcgen05.ld, add w_t * value
 //                   into FP64 registers, release the accumulator; finally store
-//                   FP64 rows (or write the result as B-role images for the next
-//                   GEMM) through a per-warp shared-memory staging buffer.
+//                   FP64 rows through a per-warp shared-memory staging buffer.
+// Output mode 1 (T = psi R of the effective Hamiltonian): the result as operand
+// images for the next GEMM, straight from the accumulator (see the epilogue).
 // Every wait is bounded: on a timeout a role records DMRG_E_NUMERIC in the
 // status word and stops; the CTA frees its tensor memory and returns.
 #include <algorithm>
@@ -168,8 +169,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 // the 13 bits below it (the sign bit is untouched, so it works on either sign).
 __device__ __forceinline__ uint32_t tf32_bits(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
 
-__device__ __forceinline__ void split(double v, uint32_t& hi, uint32_t& lo) {
-    const float f = (float)v;
+__device__ __forceinline__ void split(float f, uint32_t& hi, uint32_t& lo) {
     hi = tf32_bits(f);
     lo = tf32_bits(f - __uint_as_float(hi));
 }
@@ -180,8 +180,7 @@ __device__ __forceinline__ uint16_t bf16_bits(float x) {
     asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ void split_bf16(double v, uint16_t& hi, uint16_t& lo) {
-    const float f = (float)v;
+__device__ __forceinline__ void split_bf16(float f, uint16_t& hi, uint16_t& lo) {
     hi = bf16_bits(f);
     lo = bf16_bits(f - __uint_as_float((uint32_t)hi << 16));
 }
@@ -189,7 +188,7 @@ __device__ __forceinline__ void split_bf16(double v, uint16_t& hi, uint16_t& lo)
 // Splits the values of one 16-byte chunk (4 TF32 or 8 BF16 consecutive k of a row)
 // and stores its hi and lo parts, `plane` bytes apart.
 template <int FMT>
-__device__ __forceinline__ void store_chunk(unsigned char* dst, int plane, const double* v) {
+__device__ __forceinline__ void store_chunk(unsigned char* dst, int plane, const float* v) {
     uint32_t hw[4], lw[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -251,12 +250,12 @@ __global__ void __launch_bounds__(128) pack_kernel(const PackJob* __restrict__ j
             c = idx & 3;
         }
         if (r >= prow || c >= 4) continue;
-        double v[KC];
+        float v[KC];
         const int row = r0 + r, k = k0 + c * KC;
 #pragma unroll
         for (int q = 0; q < KC; ++q) {
             const bool in = row < j.rows && k + q < j.k;
-            v[q] = !in ? 0.0 : j.trans ? s[(int64_t)(k + q) * j.ld + row] : s[(int64_t)row * j.ld + (k + q)];
+            v[q] = !in ? 0.0f : (float)(j.trans ? s[(int64_t)(k + q) * j.ld + row] : s[(int64_t)row * j.ld + (k + q)]);
         }
         store_chunk<FMT>(out + (r >> 3) * SBO + c * LBO + (r & 7) * 16, plane, v);
     }
@@ -273,7 +272,7 @@ static_assert(sizeof(Bars) <= 256, "barrier block");
 // left in the block rounded up to 16, at most TN.
 __device__ __forceinline__ int mma_n(int n, int pn) { return min(TN, (n - pn * TN + 15) & ~15); }
 
-template <int FMT>
+template <int FMT, int MODE>
 __global__ void __launch_bounds__(NT, 1) gemm_split_kernel(const unsigned char* __restrict__ a_imgs,
                                                             const unsigned char* __restrict__ b_imgs,
                                                             double* __restrict__ C, double* __restrict__ Caux,
@@ -282,7 +281,7 @@ __global__ void __launch_bounds__(NT, 1) gemm_split_kernel(const unsigned char* 
                                                             const PackedGroup* __restrict__ groups,
                                                             const PackedTile* __restrict__ tiles,
                                                             const int* __restrict__ cta_first,
-                                                            int accumulate, int out_mode, int* __restrict__ status) {
+                                                            int accumulate, int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem[];
     Bars& B = *reinterpret_cast<Bars*>(smem + BAR_OFF);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -392,8 +391,9 @@ __global__ void __launch_bounds__(NT, 1) gemm_split_kernel(const unsigned char* 
                             const uint64_t bhi = make_smem_desc(b_base + 2 * ks * LBO, LBO, SBO);
                             const uint64_t blo = make_smem_desc(b_base + PLANE + 2 * ks * LBO, LBO, SBO);
                             mma_split<FMT>(d, ahi, bhi, id, (s > 0 || ks > 0) ? 1u : 0u);
-                            mma_split<FMT>(d, ahi, blo, id, 1u);
-                            mma_split<FMT>(d, alo, bhi, id, 1u);
+                            // (output as images: the transposed product, its terms in the same order)
+                            mma_split<FMT>(d, MODE ? alo : ahi, MODE ? bhi : blo, id, 1u);
+                            mma_split<FMT>(d, MODE ? ahi : alo, MODE ? blo : bhi, id, 1u);
                         }
                         mma_commit(&B.empty[st]);  // the stage's buffer is free once these MMAs are done
                     }
@@ -402,8 +402,65 @@ __global__ void __launch_bounds__(NT, 1) gemm_split_kernel(const unsigned char* 
                 }
             }
         }
+    } else if constexpr (MODE == 1) {
+        // ---- epilogue, the output as operand images ----
+        // The MMAs compute the transposed block, so that a thread's accumulator row is
+        // an image row and its columns are consecutive k: a group of 16 columns is one
+        // TF32 slice's (or half a BF16 slice's) chunks of that row, which go from
+        // registers to the image planes; a store of a warp covers four runs of 128
+        // bytes.  Every group has one term of weight 1, so that the accumulator's
+        // FP32 value is the value to split.  (Read out as rows of k, summed in FP64
+        // and transposed through shared memory, the tiles' epilogues were four fifths of
+        // the launch: 22 us at D = 600 in BF16, 44 at D = 1024 in TF32; 15 and 34 now.)
+        constexpr int tk = FMT == kFmtBF16 ? 32 : 16, kc = FMT == kFmtBF16 ? 8 : 4;
+        const int quarter = warp & 3, cq = (warp - 2) >> 2;
+        int ti = 0;
+        for (int tt = tile_begin; tt < tile_end && ok; ++tt, ++ti) {
+            const PackedTile tile = tiles[tt];
+            const PackedGroup g = groups[tile.group];
+            const int acc = ti & 1;
+            const int prow = panel_rows(g.m, tile.pm);           // image rows of this panel
+            const int jl = quarter * 32 + lane;                  // this thread's
+            const bool row_ok = tile.pm * TM + jl < g.m;
+            const int plane = prow * kPackRowBytes;
+            unsigned char* dst = t_out + g.t_img + (int64_t)tile.pm * g.t_slices * kImage + (jl >> 3) * SBO + (jl & 7) * 16;
+            const bool got = mbar_wait(&B.accf[acc], (ti >> 1) & 1);
+            if (!__all_sync(0xffffffffu, got)) {  // warp-uniform: tcgen05.ld below is .sync.aligned
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int n = g.n - tile.pn * TN;                    // columns (k) left in the block
+            const int nk = g.t_slices * tk - tile.pn * TN;       // the same with the last slice's padding
+#pragma unroll
+            for (int h = 0; h < ECOLS / 16; ++h) {
+                const int c = cq * ECOLS + h * 16;
+                if (c >= nk) continue;
+                uint32_t v[16];
+                if (c < n) {
+                    tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN + c), v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                }
+                if (jl < prow) {
+                    const int k = tile.pn * TN + c;
+                    unsigned char* img = dst + (int64_t)(k / tk) * 2 * plane + k % tk / kc * LBO;
+#pragma unroll
+                    for (int q = 0; q < 16 / kc; ++q) {
+                        float x[kc];
+#pragma unroll
+                        for (int e = 0; e < kc; ++e)
+                            x[e] = row_ok && c + q * kc + e < n ? __uint_as_float(v[q * kc + e]) : 0.0f;
+                        store_chunk<FMT>(img + q * LBO, plane, x);
+                    }
+                }
+                __syncwarp();
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&B.acce[acc]);
+        }
     } else {
-        // ---- epilogue: warps 2..17 ----
+        // ---- epilogue, FP64 output ----
         const int quarter = warp & 3;                // TMEM lanes 32*quarter.. (rows of the tile)
         const int cq = (warp - 2) >> 2;              // accumulator columns cq*ECOLS..
         unsigned char* stg = smem + EPI_OFF + (warp - 2) * EPI_WARP_BYTES;
@@ -444,101 +501,42 @@ __global__ void __launch_bounds__(NT, 1) gemm_split_kernel(const unsigned char* 
             // coalesced (a thread holds one output row; rows are written by the warp).
             const int r0 = tile.pm * TM + quarter * 32;      // first output row of this warp
             const int c0 = tile.pn * TN + cq * ECOLS;        // first output column of this warp
-            if (out_mode == 0) {
-                // staging: 32 rows x 16 doubles, element (r, c) at r*16 + (c ^ (r & 15))
-                double* sd = reinterpret_cast<double*>(stg);
-                double* Cb = g.cbuf ? Caux : C;
-                const bool acc_out = accumulate && g.cbuf == 0;
-                const int rows = min(32, g.m - r0);
-                const int sub = lane >> 4, cl = lane & 15;    // lanes 0-15: even rows, 16-31: odd rows
+            // staging: 32 rows x 16 doubles, element (r, c) at r*16 + (c ^ (r & 15))
+            double* sd = reinterpret_cast<double*>(stg);
+            double* Cb = g.cbuf ? Caux : C;
+            const bool acc_out = accumulate && g.cbuf == 0;
+            const int rows = min(32, g.m - r0);
+            const int sub = lane >> 4, cl = lane & 15;    // lanes 0-15: even rows, 16-31: odd rows
 #pragma unroll
-                for (int h = 0; h < ECOLS / 16; ++h) {
+            for (int h = 0; h < ECOLS / 16; ++h) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) sd[lane * 16 + (j ^ (lane & 15))] = sum[h * 16 + j];
-                    __syncwarp();
-                    const int col = c0 + h * 16 + cl;
-                    if (col < g.n) {
-                        double* cp = Cb + g.c_off + (int64_t)r0 * g.ldc + col;
-                        if (acc_out) {
-                            // the old values are loaded 8 rows at a time ahead of the
-                            // stores: a load after a store through the same pointer
-                            // would wait for it, one memory round trip per row
-                            for (int rb = 0; rb < rows; rb += 16) {
-                                double old[8];
+                for (int j = 0; j < 16; ++j) sd[lane * 16 + (j ^ (lane & 15))] = sum[h * 16 + j];
+                __syncwarp();
+                const int col = c0 + h * 16 + cl;
+                if (col < g.n) {
+                    double* cp = Cb + g.c_off + (int64_t)r0 * g.ldc + col;
+                    if (acc_out) {
+                        // the old values are loaded 8 rows at a time ahead of the
+                        // stores: a load after a store through the same pointer
+                        // would wait for it, one memory round trip per row
+                        for (int rb = 0; rb < rows; rb += 16) {
+                            double old[8];
 #pragma unroll
-                                for (int u = 0; u < 8; ++u) {
-                                    const int r = rb + sub + 2 * u;
-                                    old[u] = r < rows ? cp[(int64_t)r * g.ldc] : 0.0;
-                                }
-#pragma unroll
-                                for (int u = 0; u < 8; ++u) {
-                                    const int r = rb + sub + 2 * u;
-                                    if (r < rows) cp[(int64_t)r * g.ldc] = old[u] + sd[r * 16 + (cl ^ (r & 15))];
-                                }
+                            for (int u = 0; u < 8; ++u) {
+                                const int r = rb + sub + 2 * u;
+                                old[u] = r < rows ? cp[(int64_t)r * g.ldc] : 0.0;
                             }
-                        } else {
-                            for (int r = sub; r < rows; r += 2) cp[(int64_t)r * g.ldc] = sd[r * 16 + (cl ^ (r & 15))];
-                        }
-                    }
-                    __syncwarp();
-                }
-            } else {
-                // The output as B-role images of X = output^T (image rows = output
-                // columns, k = output rows), zeros in the padding.  The warp's 32
-                // output rows are 32 consecutive k: two TF32 slices or one BF16 slice.
-                // Per pass of 16 columns the rows go through the staging buffer
-                // (as above); each lane then reads one 16-byte chunk's worth of k
-                // (4 TF32 or 8 BF16 values) of one image row, splits them and
-                // stores the hi and lo chunks.  The 32 lanes of one store cover 8
-                // image rows x 4 chunks: 512 contiguous bytes of a plane.
-                constexpr int tk = FMT == kFmtBF16 ? 32 : 16;
-                constexpr int kc = FMT == kFmtBF16 ? 8 : 4;          // k per 16-byte chunk
-                constexpr int NIT = 32 / tk * 2;                     // (slice, 8-row group) pairs per pass
-                double* sd = reinterpret_cast<double*>(stg);         // 32 rows x 16, (r, c) at r*16 + (c ^ (r & 15))
-                const int prow = panel_rows(g.n, tile.pn);           // image rows of this panel
-                const int j8 = lane & 7, cs = lane >> 3;             // row in an 8-row group, chunk in a slice
 #pragma unroll
-                for (int h = 0; h < ECOLS / 16; ++h) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) sd[lane * 16 + (j ^ (lane & 15))] = sum[h * 16 + j];
-                    __syncwarp();
-#pragma unroll
-                    for (int it = 0; it < NIT; ++it) {
-                        const int sh = it >> 1, gj = it & 1;         // slice of the warp's two (TF32), row group
-                        const int jx = gj * 8 + j8;                  // column within the pass
-                        const int jl = cq * ECOLS + h * 16 + jx;     // image row within the panel
-                        const int slice = (r0 + sh * tk) / tk;
-                        const int rk0 = sh * tk + cs * kc;           // first of this chunk's k, within the warp's rows
-                        if (jl < prow && slice < g.t_slices) {
-                            const bool col_ok = c0 + h * 16 + jx < g.n;
-                            uint32_t hw[4], lw[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                if constexpr (FMT == kFmtBF16) {
-                                    uint16_t hb[2], lb[2];
-#pragma unroll
-                                    for (int e = 0; e < 2; ++e) {
-                                        const int rk = rk0 + 2 * q + e;
-                                        const double v = (col_ok && r0 + rk < g.m) ? sd[rk * 16 + (jx ^ (rk & 15))] : 0.0;
-                                        split_bf16(v, hb[e], lb[e]);
-                                    }
-                                    hw[q] = (uint32_t)hb[0] | ((uint32_t)hb[1] << 16);
-                                    lw[q] = (uint32_t)lb[0] | ((uint32_t)lb[1] << 16);
-                                } else {
-                                    const int rk = rk0 + q;
-                                    const double v = (col_ok && r0 + rk < g.m) ? sd[rk * 16 + (jx ^ (rk & 15))] : 0.0;
-                                    split(v, hw[q], lw[q]);
-                                }
+                            for (int u = 0; u < 8; ++u) {
+                                const int r = rb + sub + 2 * u;
+                                if (r < rows) cp[(int64_t)r * g.ldc] = old[u] + sd[r * 16 + (cl ^ (r & 15))];
                             }
-                            unsigned char* dst = t_out + g.t_img + (int64_t)tile.pn * g.t_slices * kImage +
-                                                 (int64_t)slice * 2 * prow * kPackRowBytes + (jl >> 3) * SBO + cs * LBO +
-                                                 j8 * 16;
-                            *reinterpret_cast<uint4*>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                            *reinterpret_cast<uint4*>(dst + prow * kPackRowBytes) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                         }
+                    } else {
+                        for (int r = sub; r < rows; r += 2) cp[(int64_t)r * g.ldc] = sd[r * 16 + (cl ^ (r & 15))];
                     }
-                    __syncwarp();
                 }
+                __syncwarp();
             }
         }
     }
@@ -705,9 +703,11 @@ int PackedSchedule::check_bounds(int64_t a_bytes, int64_t b_bytes, int64_t c_siz
             if (g.c_off < 0 || g.c_off + (int64_t)(g.m - 1) * g.ldc + g.n > c_size || g.n > g.ldc)
                 return set_error(DMRG_E_ARG, "packed GEMM output %lld outside %lld", (long long)g.c_off,
                                  (long long)c_size);
-        } else if (g.t_img < 0 || g.t_img + image_bytes(g.n, g.t_slices) > t_bytes ||
-                   (int64_t)g.t_slices * pack_k(fmt) < g.m || g.t_img % 16) {
+        } else if (g.t_img < 0 || g.t_img + image_bytes(g.m, g.t_slices) > t_bytes ||
+                   g.t_slices != (g.n + pack_k(fmt) - 1) / pack_k(fmt) || g.t_img % 16) {
             return set_error(DMRG_E_ARG, "packed GEMM output images outside their buffer");
+        } else if (g.t1 != g.t0 + 1 || terms[g.t0].w != 1.0) {
+            return set_error(DMRG_E_ARG, "packed GEMM output images of a weighted or several-term group");
         }
     }
     return DMRG_OK;
@@ -725,7 +725,9 @@ int ensure_smem_attr() {
     if (dev < 0 || dev >= 64) return set_error(DMRG_E_ARG, "device ordinal %d not supported", dev);
     if (!g_smem_attr[FMT][dev].load()) {
         DMRG_CUDA_TRY(
-            cudaFuncSetAttribute(gemm_split_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+            cudaFuncSetAttribute(gemm_split_kernel<FMT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        DMRG_CUDA_TRY(
+            cudaFuncSetAttribute(gemm_split_kernel<FMT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         g_smem_attr[FMT][dev].store(true);
     }
     return DMRG_OK;
@@ -735,9 +737,9 @@ template <int FMT>
 int launch_fmt(const PackedSchedule& s, const unsigned char* a_imgs, const unsigned char* b_imgs, double* C,
                unsigned char* t_out, bool accumulate, int* status, int grid, cudaStream_t stream) {
     DMRG_TRY(ensure_smem_attr<FMT>());
-    return launch_pdl(gemm_split_kernel<FMT>, dim3(grid), NT, SMEM_BYTES, stream, a_imgs, b_imgs, C, s.aux.as<double>(),
-                      t_out, s.d_terms.as<PackedTerm>(), s.d_groups.as<PackedGroup>(), s.d_tiles.as<PackedTile>(),
-                      s.d_cta_first.as<int>(), accumulate ? 1 : 0, s.out_mode, status);
+    return launch_pdl(s.out_mode ? gemm_split_kernel<FMT, 1> : gemm_split_kernel<FMT, 0>, dim3(grid), NT, SMEM_BYTES,
+                      stream, a_imgs, b_imgs, C, s.aux.as<double>(), t_out, s.d_terms.as<PackedTerm>(), s.d_groups.as<PackedGroup>(), s.d_tiles.as<PackedTile>(),
+                      s.d_cta_first.as<int>(), accumulate ? 1 : 0, status);
 }
 }  // namespace
 

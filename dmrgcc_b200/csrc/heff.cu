@@ -177,11 +177,11 @@ int build_heff(dmrg_heff_s& h) {
             h.t_img_bytes += image_bytes(t.b_j, slices(t.a_k));
             PackedGroup g{};
             g.t0 = (int)h.pa.terms.size();
-            g.m = t.a_k;
-            g.n = t.b_j;
+            g.m = t.b_j;  // transposed: rows are the image's rows
+            g.n = t.a_k;
             g.t_img = t_img[i];
             g.t_slices = slices(t.a_k);
-            h.pa.terms.push_back(PackedTerm{psi_img[t.pos], it->second, slices(t.b_l), 0, 1.0});
+            h.pa.terms.push_back(PackedTerm{it->second, psi_img[t.pos], slices(t.b_l), 0, 1.0});
             g.t1 = (int)h.pa.terms.size();
             h.pa.groups.push_back(g);
         }
@@ -208,7 +208,7 @@ int build_heff(dmrg_heff_s& h) {
         int64_t covered = 0;
         for (const PackedGroup& g : h.pb.groups) covered += (int64_t)g.m * g.n;
         h.pb_covers = covered == ket.size;
-        DMRG_TRY(h.pa.check_bounds(h.pk_psi.bytes, h.pk_R.bytes, 0, h.t_img_bytes));
+        DMRG_TRY(h.pa.check_bounds(h.pk_R.bytes, h.pk_psi.bytes, 0, h.t_img_bytes));
         DMRG_TRY(h.pb.check_bounds(h.pk_L.bytes, h.t_img_bytes, ket.size, 0));
         DMRG_TRY(h.pk_psi.finalize(st));
         DMRG_TRY(h.pk_L.finalize(st));
@@ -259,7 +259,7 @@ int dmrg::heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bo
     if (clear && h.site.ket.size)
         DMRG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)h.site.ket.size * sizeof(double), st));
     DMRG_TRY(launch_pack(h.pk_psi, psi, h.img_psi.as<unsigned char>(), st));
-    DMRG_TRY(launch_gemm_split(h.pa, h.img_psi.as<unsigned char>(), h.img_R.as<unsigned char>(), nullptr,
+    DMRG_TRY(launch_gemm_split(h.pa, h.img_R.as<unsigned char>(), h.img_psi.as<unsigned char>(), nullptr,
                                 h.img_T.as<unsigned char>(), false, h.ctx->d_status, st));
     DMRG_TRY(launch_gemm_split(h.pb, h.img_L.as<unsigned char>(), h.img_T.as<unsigned char>(), out, nullptr,
                                 accumulate || clear, h.ctx->d_status, st));
@@ -355,7 +355,7 @@ int dmrg_heff_profile(dmrg_heff_t h, const double* psi, double* out, double* ms_
     if (split) {  // stage A includes packing its operands
         rc = launch_pack(h->pk_psi, psi, h->img_psi.as<unsigned char>(), st);
         if (rc == DMRG_OK)
-            rc = launch_gemm_split(h->pa, h->img_psi.as<unsigned char>(), h->img_R.as<unsigned char>(), nullptr,
+            rc = launch_gemm_split(h->pa, h->img_R.as<unsigned char>(), h->img_psi.as<unsigned char>(), nullptr,
                                     h->img_T.as<unsigned char>(), false, h->ctx->d_status, st);
     } else {
         rc = pack_operands(*h, psi, false);
