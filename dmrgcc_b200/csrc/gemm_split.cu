@@ -40,6 +40,7 @@
 // status word and stops; the CTA frees its tensor memory and returns.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstdint>
 #include <map>
 #include <tuple>
@@ -608,19 +609,36 @@ int PackedSchedule::finalize(cudaStream_t stream, int num_sms) {
     splits.clear();
     tiles.clear();
     aux_size = 0;
+    // A tile's time in cycles.  The MMA side: a stage's six MMAs, or its copies at what
+    // an SM gets of L2 when all of them read.  The epilogue: a term's read-out (64
+    // conversions a thread are most of it), then the output store.  The two overlap.
+    // (Counted as 4 per stage + 1 per term + 6 per tile, a launch's longest CTA took
+    // twice the shortest: D = 600 BF16 matvec 39.8 us, 38.1 with this; D = 1024 TF32
+    // 86.3 and 83.8.  Three shares per SM instead of two: 38.5 and 89.7, smaller least
+    // shares cost up to 4 us.)
+    auto stage_cost = [&](const PackedGroup& g, int pm, int pn) {
+        return std::max<int64_t>(400, (int64_t)2 * (panel_rows(g.m, pm) + panel_rows(g.n, pn)) * kPackRowBytes / 60);
+    };
+    auto tile_cost = [&](const PackedGroup& g, int pm, int pn, int64_t slices, int64_t nterms) {
+        const int64_t area = (int64_t)panel_rows(g.m, pm) * panel_rows(g.n, pn);
+        const int64_t epilogue = out_mode ? 1500 : 1400 * nterms + 1000 + 3000 * area / (TM * TN);
+        return std::max(slices * stage_cost(g, pm, pn), epilogue) + 500;
+    };
     auto stages = [&](const PackedGroup& g) {
         int64_t s = 0;
         for (int t = g.t0; t < g.t1; ++t) s += terms[t].slices;
         return s;
     };
     int64_t total = 0;
-    for (const PackedGroup& g : groups)
-        total += stages(g) * ((g.m + TM - 1) / TM) * ((g.n + TN - 1) / TN);
-    const int64_t share = (num_sms > 0 && out_mode == 0) ? std::max<int64_t>(8, total / ((int64_t)num_sms * 2)) : 0;
     for (const PackedGroup& g : groups) {
         if (g.m <= 0 || g.n <= 0 || g.t1 <= g.t0) continue;
-        const int64_t st = stages(g);
-        if (share == 0 || st <= 2 * share || g.t1 - g.t0 < 2) {
+        for (int pm = 0; pm * TM < g.m; ++pm)
+            for (int pn = 0; pn * TN < g.n; ++pn) total += tile_cost(g, pm, pn, stages(g), g.t1 - g.t0);
+    }
+    const int64_t share = (num_sms > 0 && out_mode == 0) ? std::max<int64_t>(8000, total / ((int64_t)num_sms * 2)) : 0;
+    for (const PackedGroup& g : groups) {
+        if (g.m <= 0 || g.n <= 0 || g.t1 <= g.t0) continue;
+        if (share == 0 || tile_cost(g, 0, 0, stages(g), g.t1 - g.t0) <= 2 * share || g.t1 - g.t0 < 2) {
             exec_groups.push_back(g);
             continue;
         }
@@ -629,7 +647,7 @@ int PackedSchedule::finalize(cudaStream_t stream, int num_sms) {
         int64_t acc = 0;
         for (int t = g.t0; t < g.t1; ++t) {
             acc += terms[t].slices;
-            if (acc >= share || t + 1 == g.t1) {
+            if (tile_cost(g, 0, 0, acc, t + 1 - t0) >= share || t + 1 == g.t1) {
                 PackedGroup c = g;
                 c.t0 = t0;
                 c.t1 = t + 1;
@@ -645,14 +663,14 @@ int PackedSchedule::finalize(cudaStream_t stream, int num_sms) {
         aux_size += (int64_t)sp.chunks * g.m * g.n;
         splits.push_back(sp);
     }
-    // Tile cost in quarter stages: 4 per stage (its MMAs), 1 per term (the
-    // accumulator read-out), 6 per tile (pipeline fill and the output store).
     std::vector<PackedTile> all;
     for (int gi = 0; gi < (int)exec_groups.size(); ++gi) {
         const PackedGroup& g = exec_groups[gi];
-        const int cost = (int)(4 * stages(g) + (g.t1 - g.t0) + 6);
+        const int64_t st = stages(g);
         for (int pm = 0; pm * TM < g.m; ++pm)
-            for (int pn = 0; pn * TN < g.n; ++pn) all.push_back(PackedTile{gi, pm, pn, cost});
+            for (int pn = 0; pn * TN < g.n; ++pn)
+                all.push_back(PackedTile{gi, pm, pn,
+                                         (int)std::min<int64_t>(tile_cost(g, pm, pn, st, g.t1 - g.t0), INT_MAX)});
     }
     std::stable_sort(all.begin(), all.end(), [](const PackedTile& a, const PackedTile& b) { return a.cost > b.cost; });
     // Longest-processing-time-first assignment to the persistent CTAs: each
