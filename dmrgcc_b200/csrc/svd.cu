@@ -18,17 +18,14 @@ namespace {
 constexpr int kBlk = 32;        // columns per block
 constexpr int kPair = 64;       // columns per pair
 constexpr int kChunk = 32;      // rows per streamed chunk
-#ifndef DMRG_SVD_SOLVE_THREADS
-#define DMRG_SVD_SOLVE_THREADS 512
-#endif
-constexpr int kThreads = DMRG_SVD_SOLVE_THREADS;   // pair-solve CTA
-constexpr int kLd = kPair + 1;  // padded row of the shared 64x64 matrices
+constexpr int kThreads = 256;               // pair solve: one thread per 4x4 Gram block
+constexpr int kSolveThreads = kThreads + 32;  // and a warp that finds the rotations
 // Sweeps of a pair solve: one where a sector has further pairs, whose rotations undo
-// a pair's diagonality again (D = 1024: 10.2 ms of sweeps with one, 11.6 with two,
-// 13.4 with three); two where the pair is the whole sector and a further outer sweep
-// costs its launches (D = 64: 0.94 ms of canonicalisation, 1.09 with one).
+// a pair's diagonality again (D = 1024, with the solve's sweep at 63 us: 10.2 ms of
+// sweeps with one, 11.6 with two, 13.4 with three); two where the pair is the whole
+// sector and a further outer sweep costs its launches (D = 64: 0.94 ms of
+// canonicalisation, 1.09 with one).
 constexpr int kInnerSweepsMany = 1, kInnerSweepsOnly = 2;
-constexpr int kInnerSweeps = kInnerSweepsOnly;  // the larger
 constexpr int kMaxSweeps = 40;
 // The sweep cap in force (dmrg_svd_set_max_sweeps lowers it to provoke the
 // did-not-converge path without touching the device).
@@ -43,30 +40,46 @@ constexpr int kGramMinRows = DMRG_SVD_GRAM_MIN_ROWS;  // rows of a Gram item, at
 // meaningful in FP64; rotating them only stirs rounding noise).
 constexpr double kZeroRel = 4.0 * DBL_EPSILON;
 
-constexpr int kSteps = kPair - 1;                 // steps of one cyclic sweep of a pair
-constexpr int kMaxSteps = kInnerSweeps * kSteps;  // rotation log capacity
+constexpr int kQuads = kPair / 4;         // groups of four columns
+constexpr int kClasses = (kPair - 1) / 3;  // partitions into groups of a sweep
+constexpr int kSteps = kPair - 1;          // steps of the circle schedule (pair_schedule())
 
 struct SvdSmem {
-    // the Gram matrix, double-buffered: a step reads one copy and writes the
-    // other, so that one barrier per step orders every read before the writes
-    double G[2][kPair * kLd];
-    // rotation log: step t, seat lane j -> (c, s) of the rotation of the two
-    // columns seated at lane j (see seat_column), oriented (first, second)
-    double2 log[kMaxSteps * (kPair / 2)];
-    double2 cs[kPair / 2];   // (c, s) of the step's rotation k, oriented as schedule entry k addresses it
-    int active[2];           // by step parity: the step rotates something
-    double red[kThreads / 32];
-    double flag;
-    uint32_t sched[kSteps * (kPair / 2)];   // the pair schedule (pair_schedule())
+    double G[kPair * kPair], Q[kPair * kPair];  // Gram matrix, accumulated rotation
+    double J[2][16 * kQuads];  // by parity: entry (a, b) of group g's 4x4 rotation at (4 a + b) * 16 + g
+    int active[2];             // by parity: some group rotates
 };
 
-// Seating of the pair solve's columns (the circle method of a round-robin
+// The order of a pair solve's sweep.  The 64 columns are the points of the affine
+// space of dimension 3 over the field of four elements (two bits a coordinate;
+// addition is XOR): it has 84 lines of 4 points, any two points lie on exactly one,
+// and the lines fall into 21 classes of 16 parallel lines, which partition the
+// points.  A class's 16 groups of four columns are rotated at once, each through its
+// six pairs; the 21 classes meet every pair once.  Group g of class c holds the
+// columns base(g) ^ shift[a], a < 4.  The bases are chosen so that their low four
+// bits are g: the columns of 16 neighbouring threads lie in 16 different 8-byte
+// banks.
+struct QuadClass {
+    int shift[4];
+    int c;
+    __host__ __device__ explicit QuadClass(int c_) : c(c_) {
+        const int d = c < 16 ? c | 16 : c < 20 ? (c - 16) | 4 : 1;  // the lines' direction
+        const int wd = ((d >> 1) & 0x15) | (((d ^ (d >> 1)) & 0x15) << 1);  // times the field's generator
+        shift[0] = 0;
+        shift[1] = d;
+        shift[2] = wd;
+        shift[3] = d ^ wd;
+    }
+    __host__ __device__ int base(int g) const { return g | (c < 16 ? 0 : c < 20 ? g >> 2 : g & 3) << 4; }
+};
+
+// Seating of the columns in the circle schedule (the circle method of a round-robin
 // tournament): at step r, seat 0 holds column 0 and seat s >= 1 holds column
 // ((s - 1 - r) mod 63) + 1; seat lane j owns seats j and 63 - j, whose columns
 // are the pair rotated at that step.  From one step to the next the column in
 // seat s moves to seat s + 1 (seat 63 to seat 1; seat 0 stays), so a lane's two
 // columns reach their next seats by one shuffle each way.
-__host__ __device__ __forceinline__ int seat_column(int seat, int r) {
+inline int seat_column(int seat, int r) {
     return seat == 0 ? 0 : ((seat - 1 - r) % kSteps + kSteps) % kSteps + 1;
 }
 
@@ -83,22 +96,6 @@ __host__ __device__ __forceinline__ void rr_pair(int r, int i, int N, int& p, in
         p = q;
         q = t;
     }
-}
-
-__device__ double block_max(double v, SvdSmem& S) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) S.red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w) m = fmax(m, S.red[w]);
-        S.flag = m;
-    }
-    __syncthreads();
-    const double r = S.flag;
-    __syncthreads();
-    return r;
 }
 
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
@@ -261,15 +258,112 @@ __global__ void __launch_bounds__(128) measure_kernel(const SvdProblem* __restri
     if (threadIdx.x == 0) bm[blockIdx.x] = fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
 }
 
+// 1 / sqrt(x) for normal x: the approximate instruction (relative error below
+// 1e-6), then one third-order step y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2, whose
+// next term is below 1e-18: rounding level on a chain of five operations.
+__device__ __forceinline__ double rsqrt_step(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// The rotation (c, s) of columns p < q of a symmetric 4x4 matrix (upper triangle
+// used) that annihilates entry (p, q); the identity if its measure calls for none.
+// No branch, so that the chains of a step's two pairs overlap.
+template <int p, int q>
+__device__ __forceinline__ bool angle4(const double (&A)[4][4], double zero2, double tol2f, double& c, double& s) {
+    const double apq = A[p][q], daa = A[p][p], dbb = A[q][q];
+    const bool on = daa > zero2 && dbb > zero2 && apq * apq > tol2f * fmax(daa, dbb);
+    // The rotation with tan = sign(x) y / (|x| + sqrt(x^2 + y^2)),
+    // x = dbb - daa, y = 2 apq (the smaller root of the Jacobi
+    // equation), as c = u / sqrt(u^2 + y^2), s = sign(x) y / sqrt(u^2 + y^2)
+    // with u = |x| + sqrt(x^2 + y^2): no division.  (Where the pair is rotated,
+    // apq^2 > tol2f zero2 is far from underflow, and so are both sums.)
+    const double xd = dbb - daa, y = 2.0 * apq, h = fma(xd, xd, y * y);
+    const double u = fma(h, rsqrt_step(h), fabs(xd));
+    const double rn = rsqrt_step(fma(u, u, y * y));
+    c = on ? u * rn : 1.0;
+    s = on ? (xd >= 0.0 ? y : -y) * rn : 0.0;
+    return on;
+}
+
+// Applies it to A and to the columns of two rows of the accumulated 4x4 rotation.
+template <int p, int q>
+__device__ __forceinline__ void rotate4(double (&A)[4][4], double (&J)[2][4], double c, double s) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (k == p || k == q) continue;
+        double& ap = k < p ? A[k][p] : A[p][k];
+        double& aq = k < q ? A[k][q] : A[q][k];
+        const double f = c * ap - s * aq, g = s * ap + c * aq;
+        ap = f;
+        aq = g;
+    }
+    const double daa = A[p][p], apq = A[p][q], dbb = A[q][q];
+    const double pp = c * daa - s * apq, pq = c * apq - s * dbb, qp = s * daa + c * apq, qq = s * apq + c * dbb;
+    A[p][p] = c * pp - s * pq;
+    A[p][q] = s * pp + c * pq;
+    A[q][q] = s * qp + c * qq;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const double f = c * J[k][p] - s * J[k][q], g = s * J[k][p] + c * J[k][q];
+        J[k][p] = f;
+        J[k][q] = g;
+    }
+}
+
+template <int p, int q, int r, int t>
+__device__ __forceinline__ bool rotate_pairs(double (&A)[4][4], double (&J)[2][4], double zero2, double tol2f) {
+    double c1, s1, c2, s2;
+    const bool a = angle4<p, q>(A, zero2, tol2f, c1, s1), b = angle4<r, t>(A, zero2, tol2f, c2, s2);
+    rotate4<p, q>(A, J, c1, s1);
+    rotate4<r, t>(A, J, c2, s2);
+    return a || b;
+}
+
+// The class's 16 rotations, by one warp: lane g and lane g + 16 work on group g, each
+// on all of its 4x4 Gram block and on two rows of its rotation.
+__device__ void find_rotations(SvdSmem& S, int par, const QuadClass& qc, int lane, double zero2, double tol2f) {
+    const int g = lane & 15, h = lane >> 4, b0 = qc.base(g);
+    double A[4][4], J[2][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = a; b < 4; ++b) A[a][b] = S.G[(b0 ^ qc.shift[a]) * kPair + (b0 ^ qc.shift[b])];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) J[k][b] = 2 * h + k == b ? 1.0 : 0.0;
+    bool any = rotate_pairs<0, 1, 2, 3>(A, J, zero2, tol2f);
+    any |= rotate_pairs<0, 2, 1, 3>(A, J, zero2, tol2f);
+    any |= rotate_pairs<0, 3, 1, 2>(A, J, zero2, tol2f);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) S.J[par][((2 * h + k) * 4 + b) * kQuads + g] = J[k][b];
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) S.active[par] = any ? 1 : 0;
+}
+
 // Stage 2: one CTA per pair task.  Sums the task's partial Gram matrices (fixed
 // order), measures the pair's convergence, and (unless converged) runs a few
 // cyclic Jacobi sweeps on the 64x64 Gram matrix, writing the accumulated 64x64
 // rotation to rot[task - first] and skip[task - first] = 0.
-__global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __restrict__ probs,
-                                                         const SvdTask* __restrict__ tasks, int first,
-                                                         const double* __restrict__ gpart,
-                                                         const double* __restrict__ fro2, double* __restrict__ rot,
-                                                         int* __restrict__ skip, const uint32_t* __restrict__ sched) {
+//
+// A chain of dependent steps in one CTA, bound by their latency and by the
+// shared-memory passes over G.  A step rotates the 16 groups of four columns of a
+// class (QuadClass) through their six pairs each and applies the 4x4 rotations to G
+// and Q: 21 steps a sweep, each one
+// pass over G and two barriers.  (Rotating 32 disjoint pairs at a time, 63 passes over
+// G a sweep, took 76 us for one sweep and 133 for two; 41 and 68 so, and the same
+// number of outer sweeps or one fewer.)  The next class's rotations, a chain of three
+// pair rotations, are found beside the update of Q.
+__global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SvdProblem* __restrict__ probs,
+                                                              const SvdTask* __restrict__ tasks, int first,
+                                                              const double* __restrict__ gpart,
+                                                              const double* __restrict__ fro2,
+                                                              double* __restrict__ rot, int* __restrict__ skip) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SvdSmem& S = *reinterpret_cast<SvdSmem*>(smem_raw);
     const int t = first + blockIdx.x;
@@ -277,7 +371,9 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __res
     const SvdProblem p = probs[task.problem];
     const double tol = 2.0 * DBL_EPSILON * sqrt((double)p.rows);
     const double zero2 = kZeroRel * kZeroRel * (double)p.rows * fro2[task.problem];
-    {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool worker = tid < kThreads;
+    if (worker) {
         // the partials in a fixed order (c ascending) per entry; the entries of
         // a thread are independent, so all of a partial's loads are in flight
         constexpr int kElems = kPair * kPair / kThreads;
@@ -285,17 +381,18 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __res
         double v[kElems];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) v[u] = 0.0;
-        const double* gp = gpart + (int64_t)task.g_first * kPair * kPair + threadIdx.x;
+        const double* gp = gpart + (int64_t)task.g_first * kPair * kPair + tid;
+#pragma unroll 2
         for (int c = 0; c < task.g_count; ++c, gp += kPair * kPair)
 #pragma unroll
             for (int u = 0; u < kElems; ++u) v[u] += gp[u * kThreads];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) {
-            const int idx = threadIdx.x + u * kThreads;
-            S.G[0][(idx / kPair) * kLd + idx % kPair] = v[u];
+            const int idx = tid + u * kThreads;
+            S.G[idx] = v[u];
+            S.Q[idx] = idx / kPair == idx % kPair ? 1.0 : 0.0;
         }
     }
-    for (int idx = threadIdx.x; idx < kSteps * (kPair / 2); idx += kThreads) S.sched[idx] = sched[idx];
     __syncthreads();
 
     // ---- convergence measure over the pair: |g_ij| / (||A||_F max(|x_i|, |x_j|)),
@@ -303,145 +400,89 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(const SvdProblem* __res
     // unrotated amounts to.  Below tol the pair is as converged as a backward
     // stable SVD can tell (for two columns of norm ~||A|| this is the usual
     // relative test; a column far below ||A|| needs only an angle ~tol ||A|| / |x|).
-    const double fro = sqrt(fro2[task.problem]);
-    double worst = 0.0;
-    for (int idx = threadIdx.x; idx < kPair * kPair; idx += kThreads) {
-        const int a = idx / kPair, b = idx % kPair;
-        if (a >= b) continue;
-        const double ga = S.G[0][a * kLd + a], gb = S.G[0][b * kLd + b];
-        if (ga > zero2 && gb > zero2) worst = fmax(worst, fabs(S.G[0][a * kLd + b]) / (fro * sqrt(fmax(ga, gb))));
-    }
-    worst = block_max(worst, S);
-    if (threadIdx.x == 0) skip[blockIdx.x] = worst <= tol ? 1 : 0;
-    if (worst <= tol) return;  // pair already orthogonal: nothing to rotate
+    // Here and for the rotations the bound is half of tol, in squared form, so that
+    // every pair that measure_kernel calls unconverged is rotated whatever the
+    // rounding of either expression.  A step that rotates nothing skips the update,
+    // and the solve ends once a sweep leaves every measure at or below the bound.
+    const double tol2f = 0.25 * tol * tol * fro2[task.problem];
+    const auto unconverged = [&] {
+        bool off = false;
+#pragma unroll 5
+        for (int idx = tid; idx < kPair * kPair; idx += kSolveThreads) {
+            const int a = idx / kPair, b = idx % kPair;
+            const double ga = S.G[a * kPair + a], gb = S.G[b * kPair + b], g = S.G[idx];
+            off |= a < b && ga > zero2 && gb > zero2 && g * g > tol2f * fmax(ga, gb);
+        }
+        return __syncthreads_or(off) != 0;
+    };
+    const bool rotate = unconverged();
+    if (tid == 0) skip[blockIdx.x] = rotate ? 0 : 1;
+    if (!rotate) return;
 
-    // A pair whose off-diagonal measure is at or below tol needs no rotation (the
-    // same test decides convergence); a step that rotates nothing skips the
-    // update, and the solve ends once a sweep leaves every measure at or below tol.
-    // rotation test: |g_ab| above half the convergence threshold, so that every
-    // pair the measure above calls unconverged is rotated whatever the rounding
-    // of either expression
-    const double tol2f = 0.25 * tol * tol * fro * fro;
-    constexpr int kWarps = kThreads / 32;
-    constexpr int kItems = (kPair / 2) * (kPair / 2) / kThreads;  // 2x2 Gram blocks per thread
-    constexpr int kQRows = kPair / kWarps;                         // rows of Q per warp
-    static_assert(kThreads % 32 == 0 && kItems * kThreads == (kPair / 2) * (kPair / 2) && kQRows * kWarps == kPair,
-                  "even split of the Gram blocks and of the rows of Q");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int inner_sweeps = p.nbe > 2 ? kInnerSweepsMany : kInnerSweepsOnly;
-    int steps = 0;  // rotation log entries written
-    int cur = 0;    // the copy of G holding the current matrix
+    const int gi = tid >> 4, gj = tid & 15;  // a worker's Gram block; for Q: rows 4 gi .. 4 gi + 3, group gj
+    if (!worker) find_rotations(S, 0, QuadClass(0), lane, zero2, tol2f);
+    __syncthreads();
+    int par = 0;
     for (int sweep = 0; sweep < inner_sweeps; ++sweep) {
         bool rotated = false;
-        for (int r = 0; r < kSteps; ++r, ++steps) {
-            // Warp 0 computes the step's 32 rotations (lane k: the pair of schedule
-            // entry k) while the other warps load the entries they update (the
-            // addresses come from the static schedule); a barrier publishes the
-            // rotations, and a step that rotates nothing ends there.
-            const unsigned e = S.sched[r * (kPair / 2) + lane];
-            const int pc = (e >> 12) & 1 ? (e >> 6) & 63 : e & 63;  // the lane's columns in the order it addresses them
-            const int qc = (e >> 12) & 1 ? e & 63 : (e >> 6) & 63;
-            const double* Gc = S.G[cur];
-            int pi[kItems], qi[kItems];
-            double x[kItems][4];
+        for (int c = 0; c < kClasses; ++c, par ^= 1) {
+            const QuadClass qc(c);
+            const bool active = S.active[par];  // the same verdict for every thread
+            double jj[4][4];
+            int col[4];
+            if (worker && active) {
+                const double* J = S.J[par];
 #pragma unroll
-            for (int u = 0; u < kItems; ++u) {
-                const unsigned ei = S.sched[r * (kPair / 2) + warp + kWarps * u];  // the row pair's entry
-                pi[u] = (ei >> 12) & 1 ? (ei >> 6) & 63 : ei & 63;
-                qi[u] = (ei >> 12) & 1 ? ei & 63 : (ei >> 6) & 63;
-                x[u][0] = Gc[pi[u] * kLd + pc];
-                x[u][1] = Gc[pi[u] * kLd + qc];
-                x[u][2] = Gc[qi[u] * kLd + pc];
-                x[u][3] = Gc[qi[u] * kLd + qc];
-            }
-            if (warp == 0) {
-                const int a = e & 63, b = (e >> 6) & 63;  // a < b
-                const double apq = Gc[a * kLd + b];
-                const double daa = Gc[a * kLd + a], dbb = Gc[b * kLd + b];
-                double c = 1.0, s = 0.0;
-                if (daa > zero2 && dbb > zero2 && apq * apq > tol2f * fmax(daa, dbb)) {
-                    // The rotation with tan = sign(x) y / (|x| + sqrt(x^2 + y^2)),
-                    // x = dbb - daa, y = 2 apq (the smaller root of the Jacobi
-                    // equation), as c = u / sqrt(u^2 + y^2), s = sign(x) y / sqrt(u^2 + y^2)
-                    // with u = |x| + sqrt(x^2 + y^2): no division.
-                    const double xd = dbb - daa, y = 2.0 * apq;
-                    const double u = fabs(xd) + sqrt(xd * xd + y * y);
-                    const double rn = rsqrt(u * u + y * y);
-                    c = u * rn;
-                    s = (xd >= 0.0 ? y : -y) * rn;
+                for (int e = 0; e < 16; ++e) jj[e >> 2][e & 3] = J[e * kQuads + gj];
+                const int bi = qc.base(gi), bj = qc.base(gj);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) col[b] = bj ^ qc.shift[b];
+                // B <- J_i^T B J_j, row by row of B, in place: nobody else touches the block
+                double x[4][4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    double y[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) y[b] = S.G[(bi ^ qc.shift[a]) * kPair + col[b]];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        x[a][b] = y[0] * jj[0][b] + y[1] * jj[1][b] + y[2] * jj[2][b] + y[3] * jj[3][b];
                 }
-                // the lane addresses p first: rotating (b, a) by (c, -s) is rotating (a, b) by (c, s)
-                const double se = (e >> 12) & 1 ? -s : s;
-                S.cs[lane] = make_double2(c, se);
-                S.log[steps * (kPair / 2) + ((e >> 13) & 31)] = make_double2(c, ((e >> 18) & 1) ? -se : se);
-                const bool any = __any_sync(0xffffffffu, s != 0.0);
-                if (lane == 0) S.active[steps & 1] = any ? 1 : 0;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const double j0 = J[a * kQuads + gi], j1 = J[(4 + a) * kQuads + gi], j2 = J[(8 + a) * kQuads + gi],
+                                 j3 = J[(12 + a) * kQuads + gi];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        S.G[(bi ^ qc.shift[a]) * kPair + col[b]] =
+                            j0 * x[0][b] + j1 * x[1][b] + j2 * x[2][b] + j3 * x[3][b];
+                }
             }
             __syncthreads();
-            if (!S.active[steps & 1]) continue;  // the same verdict for every thread
-            rotated = true;
-            // G <- J^T G J into the other copy: thread (i, j = lane) takes the 2x2
-            // block of rows (p_i, q_i) and columns (p_j, q_j), both rotations at
-            // once (an untouched block is copied), for i = warp + kWarps u
-            double* Gn = S.G[cur ^ 1];
-            const double2 csj = S.cs[lane];
+            // the next class's rotations beside the update of Q
+            if (!worker) {
+                find_rotations(S, par ^ 1, QuadClass(c + 1 == kClasses ? 0 : c + 1), lane, zero2, tol2f);
+            } else if (active) {
 #pragma unroll
-            for (int u = 0; u < kItems; ++u) {
-                const double2 csi = S.cs[warp + kWarps * u];
-                const double ci = csi.x, si = csi.y, c = csj.x, se = csj.y;
-                const double y11 = ci * x[u][0] - si * x[u][2], y12 = ci * x[u][1] - si * x[u][3];
-                const double y21 = si * x[u][0] + ci * x[u][2], y22 = si * x[u][1] + ci * x[u][3];
-                Gn[pi[u] * kLd + pc] = c * y11 - se * y12;
-                Gn[pi[u] * kLd + qc] = se * y11 + c * y12;
-                Gn[qi[u] * kLd + pc] = c * y21 - se * y22;
-                Gn[qi[u] * kLd + qc] = se * y21 + c * y22;
+                for (int a = 0; a < 4; ++a) {
+                    double* q = S.Q + (4 * gi + a) * kPair;
+                    double y[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) y[b] = q[col[b]];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        q[col[b]] = y[0] * jj[0][b] + y[1] * jj[1][b] + y[2] * jj[2][b] + y[3] * jj[3][b];
+                }
             }
-            cur ^= 1;
+            rotated |= active;
             __syncthreads();
         }
         if (!rotated || sweep + 1 == inner_sweeps) break;  // uniform: every thread saw the same flags
-        // the pair's measure after this sweep: a further sweep only if some entry is above tol
-        double off = 0.0;
-        for (int idx = threadIdx.x; idx < kPair * kPair; idx += kThreads) {
-            const int a = idx / kPair, b = idx % kPair;
-            if (a >= b) continue;
-            const double ga = S.G[cur][a * kLd + a], gb = S.G[cur][b * kLd + b], g = S.G[cur][a * kLd + b];
-            if (ga > zero2 && gb > zero2 && g * g > tol2f * fmax(ga, gb)) off = 1.0;
-        }
-        if (block_max(off, S) == 0.0) break;
-    }
-    __syncthreads();  // the log is complete
-
-    // The accumulated rotation Q = J_0 J_1 ... from the log, in registers: warp w
-    // takes rows kQRows w ... of Q, lane j the two entries of each row in the
-    // columns seated at lane j.  After each step's rotation the entries move to their next
-    // seats (seat_column): seat s -> s + 1 for 1 <= s <= 62, seat 63 -> seat 1.
-    double q1[kQRows], q2[kQRows];
-#pragma unroll
-    for (int k = 0; k < kQRows; ++k) {
-        const int row = kQRows * warp + k;
-        q1[k] = row == lane ? 1.0 : 0.0;               // seat lane (column lane at step 0)
-        q2[k] = row == kPair - 1 - lane ? 1.0 : 0.0;   // seat 63 - lane
-    }
-    for (int t = 0; t < steps; ++t) {
-        const double2 cs = S.log[t * (kPair / 2) + lane];
-#pragma unroll
-        for (int k = 0; k < kQRows; ++k) {
-            const double f = cs.x * q1[k] - cs.y * q2[k], g = cs.y * q1[k] + cs.x * q2[k];
-            const double up = __shfl_up_sync(0xffffffffu, lane == 0 ? g : f, 1);  // seat j - 1 (lane 0: seat 63)
-            const double dn = __shfl_down_sync(0xffffffffu, g, 1);               // seat 62 - j
-            q1[k] = lane == 0 ? f : up;
-            q2[k] = lane == 31 ? f : dn;
-        }
+        if (!unconverged()) break;
     }
     double* R = rot + (int64_t)blockIdx.x * kPair * kPair;
-    const int c1 = seat_column(lane, steps), c2 = seat_column(kPair - 1 - lane, steps);
-#pragma unroll
-    for (int k = 0; k < kQRows; ++k) {
-        const int row = kQRows * warp + k;
-        R[row * kPair + c1] = q1[k];
-        R[row * kPair + c2] = q2[k];
-    }
+    for (int idx = tid; idx < kPair * kPair; idx += kSolveThreads) R[idx] = S.Q[idx];
 }
 
 // Stage 3: item = (pair task, segment, row range): the pair's 64 columns of W
@@ -690,7 +731,8 @@ __global__ void __launch_bounds__(256) sign_kernel(const SvdProblem* __restrict_
     if (lane == 0) sign[p.s_off + j] = (first < p.m && u[first] < 0.0) ? -1.0 : 1.0;
 }
 
-// Lane order of the pair solve's rotations.  Step r rotates the 32 column pairs
+// The circle schedule of a 64-column sweep, which dmrg_svd_pair_schedule reports (the
+// device's order is QuadClass's).  Step r rotates the 32 column pairs
 // seated at the 32 seat lanes (seat_column); chosen here is which lane of the
 // Gram update takes which pair and which of its two columns the lane addresses
 // first.  Entry (r, lane) = a | b << 6 | flip << 12 | j << 13 | jflip << 18:
@@ -869,16 +911,13 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
     DMRG_TRY(d_s.alloc(some(2 * soff) * sizeof(double)));
     DMRG_TRY(d_perm.alloc(some(soff) * sizeof(int)));
     DMRG_TRY(d_sign.alloc(some(soff) * sizeof(double)));
-    const std::vector<uint32_t>* sched = pair_schedule();
-    if (!sched) return set_error(DMRG_E_STATE, "no pair schedule");
     Tables tab;
     tab.add(probs);  // at offset 0: d_probs is the problem table
-    const size_t at_x = tab.add(xprobs), at_tiles = tab.add(tiles), at_sched = tab.add(*sched);
+    const size_t at_x = tab.add(xprobs), at_tiles = tab.add(tiles);
     DMRG_TRY(tab.to(d_probs, st));
     const unsigned char* tb = d_probs.as<unsigned char>();
     work.xprobs = reinterpret_cast<const SvdProblem*>(tb + at_x);
     work.tiles = reinterpret_cast<const SvdTile*>(tb + at_tiles);
-    work.sched = reinterpret_cast<const uint32_t*>(tb + at_sched);
     // the workspace: two passes over its pieces, sizes then addresses
     const int64_t np = (int64_t)probs.size();
     size_t bytes = 0;
@@ -1159,8 +1198,8 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
             if (nt == 0) continue;
             DMRG_LAUNCH gram_kernel<<<ng, 128, 0, st>>>(xp, work.tasks, work.gram_items + round_gram_first[r],
                                                         work.colmap, x, work.gpart);
-            DMRG_LAUNCH solve_kernel<<<nt, kThreads, sizeof(SvdSmem), st>>>(
-                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip, work.sched);
+            DMRG_LAUNCH solve_kernel<<<nt, kSolveThreads, sizeof(SvdSmem), st>>>(
+                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip);
             DMRG_LAUNCH rotate_kernel<<<nr, 128, kRotSmem, st>>>(xp, work.tasks, work.rot_items + round_rot_first[r],
                                                                  round_first[r], work.rot, work.skip, work.colmap, x,
                                                                  qx);
