@@ -6,9 +6,9 @@
 // other CTAs update the rest, and a column lives in the registers of one warp, so
 // that a column step has one barrier.  16 columns is the widest panel whose 1024
 // rows fit the registers of one CTA.  Both factorisations at 17 sectors to
-// 611 x 510 and 837 x 360: 64 launches, 1.96 ms (47 us while panels have more than
-// 512 rows, 28 us and less below); to 33 columns: 6 launches, 75 us.  Forming Q and
-// applying it: 145 and 258 us, bound by the DMMA rate of the SMs that hold the
+// 611 x 510 and 837 x 360: 64 launches, 1.68 ms (37 us while panels have more than
+// 512 rows, 25 us and less below); to 33 columns: 6 launches, 80 us.  Forming Q and
+// applying it: 136 and 239 us, bound by the DMMA rate of the SMs that hold the
 // largest sectors' tiles.
 #include <algorithm>
 
@@ -18,7 +18,8 @@ namespace dmrg {
 namespace {
 
 constexpr int kNb = kQrPanel;        // columns of a panel, and of a tile that it is applied to
-constexpr int kThreads = 32 * kNb;   // one warp per panel column
+constexpr int kStepWarps = 8;        // qr_step_kernel: two panel columns per warp
+constexpr int kApplyWarps = 16;      // qr_apply_kernel
 constexpr int kMaxReg = 32;          // rows a lane holds in registers, at most (1024-row panels)
 // Below this squared norm (columns under 1e-140 of a matrix whose largest entry is
 // at least 1/2) the part of a column under the diagonal counts as zero: its square
@@ -27,8 +28,8 @@ constexpr double kTiny2 = 1e-280;
 
 struct QrSmem {
     union {
-        double red[kNb][kNb * kNb];      // the warps' parts of V^T C
-        double v[2][32 * kMaxReg];       // the current reflector, double-buffered
+        double red[kApplyWarps][kNb * kNb];  // the warps' parts of V^T C
+        double v[2][32 * kMaxReg];           // the current reflector, double-buffered
     };
     double t[kNb * kNb];                 // the panel's T
     double z[kNb * kNb], tz[kNb * kNb];  // V^T C and -T^(T) V^T C
@@ -48,13 +49,13 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
 // major: 32- and 64-byte pieces, L2 hits), the two products splitting the rows
 // over the warps.  With `rt`, rows 0..15 of the result (finished rows of the
 // factor) go to rt transposed (entry (row, c) at rt[c + row * ldr]) instead of C.
-template <bool TRANSPOSED>
+template <bool TRANSPOSED, int WARPS>
 __device__ void apply_panel(const double* V, int ldv, int m, int nv, const double* __restrict__ T, double* C, int ldc,
                             int nc, double* rt, int ldr, QrSmem& S) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
     if (threadIdx.x < kNb * kNb) S.t[threadIdx.x] = T[threadIdx.x];
     double acc[2][2][2] = {};
-    for (int r0 = warp * 32; r0 < m; r0 += 32 * kNb) {
+    for (int r0 = warp * 32; r0 < m; r0 += 32 * WARPS) {
 #pragma unroll
         for (int kk = 0; kk < 32; kk += 4) {
             const int r = r0 + kk + fc;
@@ -70,7 +71,7 @@ __device__ void apply_panel(const double* V, int ldv, int m, int nv, const doubl
                 for (int n = 0; n < 2; ++n) dmma_8x8x4(acc[i][n][0], acc[i][n][1], a[i], b[n]);
         }
     }
-    const int parts = min(kNb, (m + 31) / 32);
+    const int parts = min(WARPS, (m + 31) / 32);
     if (warp < parts) {
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -99,8 +100,8 @@ __device__ void apply_panel(const double* V, int ldv, int m, int nv, const doubl
     for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int n = 0; n < 2; ++n) b[k][n] = S.tz[(4 * k + fc) * kNb + n * 8 + fr];
-#pragma unroll 2
-    for (int r0 = warp * 8; r0 < m; r0 += 8 * kNb) {
+#pragma unroll 4
+    for (int r0 = warp * 8; r0 < m; r0 += 8 * WARPS) {
         const int r = r0 + fr;
         double a[4], c[2][2];
 #pragma unroll
@@ -148,68 +149,92 @@ __device__ __forceinline__ void reflector(double alpha, double ss, double& beta,
     }
 }
 
-// Householder QR of a panel (m x nc, nc <= 16), one warp per column, the column
-// in R registers per lane (rows lane + 32 i).  Step j: its warp makes the
-// reflector and publishes it in shared memory; after the step's one barrier
-// every warp dots it with its own column - a later column is updated, an earlier
-// one (which holds its reflector by then) gives the entry v_i . v_j that T needs.
-// The warp of column j + 1 goes straight on to its reflector, so a step costs one
-// dot product, one update and one norm of a column.  R (transposed) goes to rt.
+// Householder QR of a panel (m x nc, nc <= 16).  Warp w holds columns w and w + 8 in
+// R registers a lane each (rows lane + 32 i).  Step j: the column's warp makes the
+// reflector and publishes it in shared memory; after the step's one barrier every
+// warp reads it once into registers and dots it with its two columns - a later
+// column is updated, an earlier one (which holds its reflector by then) gives the
+// entry v_i . v_j that T needs.  The warp of column j + 1 goes straight on to its
+// reflector, so a step costs one dot product, one update and one norm of a column.
+// (With one column a warp and the reflector read twice, the shared-memory wavefronts
+// of 16 warps bound it: 37 us for 837 rows, 26 so.)  R
+// (transposed) goes to rt.
 template <int R>
 __device__ void factor_panel(double* A, int lda, int m, int nc, double* rt, int ldr, QrSmem& S) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double x[R];
+    double x[2][R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) x[i] = w < nc && lane + 32 * i < m ? A[lane + 32 * i + (int64_t)w * lda] : 0.0;
-    for (int j = 0; j < nc; ++j) {
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int col = w + kStepWarps * c, r = lane + 32 * i;
+            x[c][i] = col < nc && r < m ? A[r + (int64_t)col * lda] : 0.0;
+        }
+    const auto reflect = [&](double (&y)[R], int j) {
+        double ss[4] = {lane > j ? y[0] * y[0] : 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 1; i < R; ++i) ss[i & 3] += y[i] * y[i];
+        const double s = warp_sum((ss[0] + ss[1]) + (ss[2] + ss[3]));
+        double beta, tau, scale;
+        reflector(__shfl_sync(0xffffffffu, y[0], j), s, beta, tau, scale);
+        if (lane <= j) rt[j + (int64_t)lane * ldr] = lane == j ? beta : y[0];
         double* v = S.v[j & 1];
-        if (w == j) {
-            double ss = lane > j ? x[0] * x[0] : 0.0;
+        y[0] = lane > j ? y[0] * scale : lane == j ? 1.0 : 0.0;
+        v[lane] = y[0];
 #pragma unroll
-            for (int i = 1; i < R; ++i) ss += x[i] * x[i];
-            ss = warp_sum(ss);
-            double beta, tau, scale;
-            reflector(__shfl_sync(0xffffffffu, x[0], j), ss, beta, tau, scale);
-            if (lane <= j) rt[j + (int64_t)lane * ldr] = lane == j ? beta : x[0];
-            x[0] = lane > j ? x[0] * scale : lane == j ? 1.0 : 0.0;
-            v[lane] = x[0];
-#pragma unroll
-            for (int i = 1; i < R; ++i) {
-                x[i] *= scale;
-                v[lane + 32 * i] = x[i];
-            }
-            if (lane == 0) S.tau[j] = tau;
+        for (int i = 1; i < R; ++i) {
+            y[i] *= scale;
+            v[lane + 32 * i] = y[i];
+        }
+        if (lane == 0) S.tau[j] = tau;
+    };
+    for (int j = 0; j < nc; ++j) {
+        if (w == (j & (kStepWarps - 1))) {
+            if (j < kStepWarps) reflect(x[0], j);
+            else reflect(x[1], j);
         }
         __syncthreads();
-        if (w != j && w < nc) {
-            double d0 = 0.0, d1 = 0.0;
+        double v[R];
 #pragma unroll
-            for (int i = 0; i < R; i += 2) {
-                d0 += x[i] * v[lane + 32 * i];
-                if (i + 1 < R) d1 += x[i + 1] * v[lane + 32 * (i + 1)];
-            }
-            const double d = warp_sum(d0 + d1);
-            if (w > j) {
-                const double f = S.tau[j] * d;
+        for (int i = 0; i < R; ++i) v[i] = S.v[j & 1][lane + 32 * i];
+        double d[2][2] = {};
 #pragma unroll
-                for (int i = 0; i < R; ++i) x[i] -= f * v[lane + 32 * i];
-            } else if (lane == 0) {
-                S.s[w * kNb + j] = d;
+        for (int i = 0; i < R; ++i) {
+            d[0][i & 1] += x[0][i] * v[i];
+            d[1][i & 1] += x[1][i] * v[i];
+        }
+        const double d0 = warp_sum(d[0][0] + d[0][1]), d1 = warp_sum(d[1][0] + d[1][1]);
+        const double tau = S.tau[j];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int col = w + kStepWarps * c;
+            const double dc = c ? d1 : d0;
+            if (col > j) {
+                const double f = tau * dc;
+#pragma unroll
+                for (int i = 0; i < R; ++i) x[c][i] -= f * v[i];
+            } else if (col < j && lane == 0) {
+                S.s[col * kNb + j] = dc;
             }
         }
     }
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-        if (w < nc && lane + 32 * i < m) A[lane + 32 * i + (int64_t)w * lda] = x[i];
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int col = w + kStepWarps * c, r = lane + 32 * i;
+            if (col < nc && r < m) A[r + (int64_t)col * lda] = x[c][i];
+        }
 }
 
 // The same for panels of more rows than the registers hold, on the columns in
 // global memory (the CTA's own writes, ordered by the steps' barriers).
 __device__ void factor_panel_long(double* A, int lda, int m, int nc, double* rt, int ldr, QrSmem& S) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* x = A + (int64_t)w * lda;
     for (int j = 0; j < nc; ++j) {
-        if (w == j) {
+        const double* v = A + (int64_t)j * lda;
+        if (w == (j & (kStepWarps - 1))) {
+            double* x = A + (int64_t)j * lda;
             double ss = 0.0;
             for (int r = lane; r < m; r += 32) ss += r > j ? x[r] * x[r] : 0.0;
             ss = warp_sum(ss);
@@ -221,18 +246,19 @@ __device__ void factor_panel_long(double* A, int lda, int m, int nc, double* rt,
             if (lane == 0) S.tau[j] = tau;
         }
         __syncthreads();
-        if (w != j && w < nc) {
-            const double* v = A + (int64_t)j * lda;
+        for (int col = w; col < nc; col += kStepWarps) {
+            if (col == j) continue;
+            double* x = A + (int64_t)col * lda;
             double d = 0.0;
 #pragma unroll 4
             for (int r = lane; r < m; r += 32) d += x[r] * v[r];
             d = warp_sum(d);
-            if (w > j) {
+            if (col > j) {
                 const double f = S.tau[j] * d;
 #pragma unroll 4
                 for (int r = lane; r < m; r += 32) x[r] -= f * v[r];
             } else if (lane == 0) {
-                S.s[w * kNb + j] = d;
+                S.s[col * kNb + j] = d;
             }
         }
         __syncwarp();
@@ -244,7 +270,7 @@ __device__ void factor_panel_long(double* A, int lda, int m, int nc, double* rt,
 // as it is): CTA (problem, y) applies the reflectors of panel s - 1 to the tile of
 // 16 columns s + y; the one of the next panel (y = 0) then factors it and forms its
 // T, while the others finish the update.
-__global__ void __launch_bounds__(kThreads) qr_step_kernel(const SvdProblem* __restrict__ probs, double* M, double* RT,
+__global__ void __launch_bounds__(32 * kStepWarps) qr_step_kernel(const SvdProblem* __restrict__ probs, double* M, double* RT,
                                                            double* T, int s) {
     __shared__ __align__(16) QrSmem S;
     const SvdProblem p = probs[blockIdx.x];
@@ -256,7 +282,7 @@ __global__ void __launch_bounds__(kThreads) qr_step_kernel(const SvdProblem* __r
     double* t = T + p.t_off;
     if (s > 0) {
         const int k0 = (s - 1) * kNb;
-        apply_panel<true>(M + p.w_off + k0 + (int64_t)k0 * p.rows, p.rows, p.rows - k0, kNb, t + (s - 1) * kNb * kNb,
+        apply_panel<true, kStepWarps>(M + p.w_off + k0 + (int64_t)k0 * p.rows, p.rows, p.rows - k0, kNb, t + (s - 1) * kNb * kNb,
                           A + k0, p.rows, nc, rt + c0 + (int64_t)k0 * p.cols, p.cols, S);
     }
     if (blockIdx.y) return;
@@ -293,7 +319,7 @@ __global__ void __launch_bounds__(kThreads) qr_step_kernel(const SvdProblem* __r
 // 16 columns, which nothing but its own reflector blocks touch.  C (rows x cols, at
 // w_off) starts as the identity (`src` null; the blocks whose rows lie below the
 // tile's columns leave it as it is) or as src (cols x cols, at q_off) above zeros.
-__global__ void __launch_bounds__(kThreads) qr_apply_kernel(const SvdProblem* __restrict__ probs, const double* M,
+__global__ void __launch_bounds__(32 * kApplyWarps) qr_apply_kernel(const SvdProblem* __restrict__ probs, const double* M,
                                                             const double* __restrict__ T,
                                                             const double* __restrict__ src, double* C) {
     __shared__ __align__(16) QrSmem S;
@@ -302,14 +328,14 @@ __global__ void __launch_bounds__(kThreads) qr_apply_kernel(const SvdProblem* __
     if (c0 >= p.cols) return;
     const int nc = min(kNb, p.cols - c0);
     double* c = C + p.w_off + (int64_t)c0 * p.rows;
-    for (int64_t e = threadIdx.x; e < (int64_t)nc * p.rows; e += kThreads) {
+    for (int64_t e = threadIdx.x; e < (int64_t)nc * p.rows; e += blockDim.x) {
         const int r = (int)(e % p.rows), j = (int)(e / p.rows);
         c[e] = src ? (r < p.cols ? src[p.q_off + r + (int64_t)(c0 + j) * p.cols] : 0.0) : (r == c0 + j ? 1.0 : 0.0);
     }
     __syncthreads();
     for (int k = src ? (p.cols - 1) / kNb : (int)blockIdx.y; k >= 0; --k) {
         const int k0 = k * kNb;
-        apply_panel<false>(M + p.w_off + k0 + (int64_t)k0 * p.rows, p.rows, p.rows - k0, min(kNb, p.cols - k0),
+        apply_panel<false, kApplyWarps>(M + p.w_off + k0 + (int64_t)k0 * p.rows, p.rows, p.rows - k0, min(kNb, p.cols - k0),
                            T + p.t_off + k * kNb * kNb, c + k0, p.rows, nc, nullptr, 0, S);
     }
 }
@@ -319,14 +345,14 @@ __global__ void __launch_bounds__(kThreads) qr_apply_kernel(const SvdProblem* __
 int qr_factor(const SvdProblem* probs, int np, int max_cols, double* m, double* rt, double* t, cudaStream_t st) {
     const int panels = (max_cols + kNb - 1) / kNb;
     for (int s = 0; s < panels; ++s)
-        DMRG_LAUNCH qr_step_kernel<<<dim3(np, panels - s), kThreads, 0, st>>>(probs, m, rt, t, s);
+        DMRG_LAUNCH qr_step_kernel<<<dim3(np, panels - s), 32 * kStepWarps, 0, st>>>(probs, m, rt, t, s);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
 
 int qr_apply(const SvdProblem* probs, int np, int max_cols, const double* m, const double* t, const double* src,
              double* c, cudaStream_t st) {
-    DMRG_LAUNCH qr_apply_kernel<<<dim3(np, (max_cols + kNb - 1) / kNb), kThreads, 0, st>>>(probs, m, t, src, c);
+    DMRG_LAUNCH qr_apply_kernel<<<dim3(np, (max_cols + kNb - 1) / kNb), 32 * kApplyWarps, 0, st>>>(probs, m, t, src, c);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
