@@ -54,8 +54,8 @@ def bench_config(psi_dim: int, gflop: float) -> dict:
 def profiled_traffic() -> dict | None:
     """DRAM bytes per matvec of the FP64 path (stage A + stage B launches), from
     the committed ncu summary of the same workload (a line
-    `traffic_bytes_per_matvec: <bytes>` in profiles/gemm_f64_heff_cyl8x4_D1024.md)."""
-    p = os.path.join(ROOT, "profiles", "gemm_f64_heff_cyl8x4_D1024.md")
+    `traffic_bytes_per_matvec: <bytes>` in profiles/gemm_image_heff_cyl8x4_D1024.md)."""
+    p = os.path.join(ROOT, "profiles", "gemm_image_heff_cyl8x4_D1024.md")
     try:
         with open(p) as f:
             for line in f:
@@ -563,19 +563,19 @@ def run_b200(args) -> None:
             "data": "synthetic (seeded splitmix64 values on the reference's own D=1024 block structure)",
             "config": bench_config(step.psi_dim, alg_flops * 1e-9),
             # exec_flops counts the products the schedule runs (each K*R product
-            # once), not the padding of the 64x64x16 DMMA tiles around them
+            # once), not the padding of the 8x8x4 DMMA units around them
             "detail": {"precision": args.precision, "gflop_per_step_scheduled": exec_flops * 1e-9,
                        "gflop_note": "scheduled products without the tile padding of the DMMA tiles",
                        "l2": "256 MiB write between timed steps (outside the per-step CUDA-event pair)",
                        "parallelism": f"replicas x{world}"},
             # counted by the library (dmrg_launch_count) around the timed loop: per
-            # matvec the stage A and stage B grouped GEMMs and the stage B split-K reduce
+            # matvec the operand packing and the stage A and stage B grouped GEMMs
             "gpu_launches": launches,
             "e2e": {"value": e2e_value, "unit": "TFLOP/s", "h2d_bytes_per_step": step.psi_dim * 8,
                     "d2h_bytes_per_step": step.psi_dim * 8,
                     "note": "dmrg_heff_apply_host: pinned psi in, matvec, result out, sync; environments resident"},
             "roofline": {
-                "bound": "tensor", "kernel": "gemm_f64_kernel (whole matvec: stage A + stage B)",
+                "bound": "tensor", "kernel": "img_gemm_kernel (whole matvec: packing, stage A, stage B)",
                 "achieved": alg_flops / (ms_per_step * 1e-3) * 1e-12, "peak": fp64_peak, "unit": "TFLOP/s",
                 "frac": alg_flops / (ms_per_step * 1e-3) * 1e-12 / fp64_peak,
                 "traffic": traffic["bytes"] if traffic else None,
