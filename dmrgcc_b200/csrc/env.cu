@@ -13,7 +13,8 @@
 // :974-1060): per output bond index, blocks in row-major (first, second) sector
 // order, present wherever some contribution has a nonzero W.
 #include <algorithm>
-#include <map>
+#include <unordered_map>
+#include <unordered_set>
 
 #include "blocksparse.h"
 #include "gemm.cuh"
@@ -294,11 +295,19 @@ int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
     const bool z = W != nullptr;
     const int f = z ? 2 : 1;  // doubles per element
     // images by offset: the ket as stage 1's A operand, as stage 2's B operand (and times i), ...
-    std::map<int64_t, int64_t> ket_a, ket_b[2], env_img, mid_img;
-    std::map<int64_t, int> ket_pos;
+    // (hashed: a sweep creates an update per site, and ordered maps were half of its planning)
+    using Images = std::unordered_map<int64_t, int64_t>;
+    Images ket_a, ket_b[2], env_img, mid_img;
+    std::unordered_map<int64_t, int> ket_pos;
+    mid_img.reserve(e.s1.groups.size());
+    env_img.reserve(e.s1.terms.size());
+    e.i1.terms.reserve(e.s1.terms.size());
+    e.i1.groups.reserve(e.s1.groups.size());
+    e.i2.terms.reserve((z ? 2 : 1) * e.s2.terms.size());
+    e.i2.groups.reserve(e.s2.groups.size());
     for (int k = 0; k < ket.count(); ++k)
         if (ket.rows[k] > 0 && ket.cols[k] > 0) ket_pos[ket.off[k]] = k;
-    auto ket_image = [&](std::map<int64_t, int64_t>& at, int64_t off, ImgKind kind, bool conj, bool times_i) {
+    auto ket_image = [&](Images& at, int64_t off, ImgKind kind, bool conj, bool times_i) {
         auto it = at.find(off);
         if (it != at.end()) return it->second;
         const int k = ket_pos.at(off), r = ket.rows[k], c = ket.cols[k];
@@ -326,10 +335,10 @@ int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
             e.i1.add_term(ket_image(ket_a, x.a_off, kImgComplexA, e.side == 0, false), it->second, f * x.k, 1.0);
         }
     }
-    std::map<int64_t, int> grouped;
+    std::unordered_set<int64_t> grouped(2 * e.s2.groups.size());
     for (const GemmGroup& g : e.s2.groups) {
         e.i2.add_group(f * g.c_off, f * g.ldc, g.m, f * g.n);
-        grouped[g.c_off] = 1;
+        grouped.insert(g.c_off);
         for (int t = g.t0; t < g.t1; ++t) {
             const GemmTerm& x = e.s2.terms[t];
             if (x.k <= 0 || g.m <= 0 || g.n <= 0) continue;

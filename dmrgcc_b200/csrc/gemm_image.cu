@@ -634,6 +634,9 @@ int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
     };
     std::vector<Tile> tiles;
     std::vector<ImgGroup> gr;
+    live.reserve(terms.size() + 1);
+    gr.reserve(groups.size());
+    tiles.reserve(groups.size());
     int64_t cost = 0;
     for (const ImgGroup& g : groups) {
         if (g.m <= 0 || g.n <= 0) continue;
@@ -661,6 +664,8 @@ int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
     const int64_t longest = std::max<int64_t>(1, cost / ((int64_t)num_sms * kCtasPerSm) / 4);
     int ntickets = 0;
     std::vector<std::pair<int64_t, int>> order;  // cost, segment
+    order.reserve(tiles.size());
+    segments.reserve(tiles.size());
     for (const Tile& t : tiles) {
         const ImgGroup& g = gr[t.group];
         const int64_t c_off = out == kImgOutBlock ? g.c_off + (int64_t)t.pm * panel * g.ldc + t.pn * panel : g.c_off;
