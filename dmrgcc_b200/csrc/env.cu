@@ -363,10 +363,7 @@ int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
     DMRG_TRY(e.img.check_bounds(f * ket.size, f * e.in.size, 0));
     DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, mid));
     DMRG_TRY(e.i2.check_bounds(mid, e.img.blocks, f * e.out.size));
-    DMRG_TRY(e.img.finalize(e.i1.panel, st));
-    DMRG_TRY(e.i1.finalize(st, e.ctx->num_sms));
-    DMRG_TRY(e.i2.finalize(st, e.ctx->num_sms));
-    return e.work.alloc(e.img.blocks, mid, e.i1, e.i2);
+    return e.work.finalize(e.img, e.i1, e.i2, mid, st, e.ctx->num_sms);
 }
 
 int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {

@@ -151,8 +151,8 @@ struct ImgPack {
     std::vector<ImgJob> jobs;
     std::vector<ImgChunk> chunks;
     int64_t blocks = 0;
-    DeviceBuffer d_tables;  // jobs, chunks
-    size_t chunks_at = 0;
+    char* tables = nullptr;  // in ImgWork
+    size_t jobs_at = 0, chunks_at = 0;
     // Appends an operand block; returns its image (first block).
     int64_t add(int src, int64_t src_off, int rows, int k, int ld, bool trans);
     // The same for a complex block (src_off, rows, k and ld in elements).
@@ -162,7 +162,7 @@ struct ImgPack {
     // Every read inside sources of the given sizes (doubles); DMRG_E_ARG otherwise.
     int check_bounds(int64_t n0, int64_t n1, int64_t n2) const;
     // Builds the chunk list for panels of `panel` rows and uploads.
-    int finalize(int panel, cudaStream_t stream);
+    void plan(int panel, Tables& tab);
     std::vector<int> first_chunk;  // chunks before each job, and in all
 };
 // Packs the jobs of chunks [c0, c1) from the three sources into img.
@@ -215,8 +215,8 @@ struct ImgSchedule {
     int64_t aux_size = 0;
     // device tables: terms, segments, splits, tickets (the queue's two counters, then one
     // per split tile; zero between launches)
-    DeviceBuffer d_tables;
-    size_t segments_at = 0, splits_at = 0, tickets_at = 0;
+    char* tables = nullptr;  // in ImgWork
+    size_t terms_at = 0, segments_at = 0, splits_at = 0, tickets_at = 0;
     double* aux = nullptr;  // aux_size doubles, 16-byte aligned, set after finalize
 
     void add_group(int64_t c_off, int ldc, int m, int n) {
@@ -231,17 +231,18 @@ struct ImgSchedule {
     // Every image read and output write inside buffers of the given sizes (blocks;
     // doubles for a block output); DMRG_E_ARG otherwise.
     int check_bounds(int64_t a_blocks, int64_t b_blocks, int64_t out_size) const;
-    // Cuts the groups into tiles and long tiles into parts, orders the queue and
-    // uploads.  Groups without terms are part of it: a launch that does not
+    // Cuts the groups into tiles and long tiles into parts, orders the queue and adds
+    // the tables.  Groups without terms are part of it: a launch that does not
     // accumulate writes zeros.
-    int finalize(cudaStream_t stream, int num_sms);
+    void plan(int num_sms, Tables& tab);
 };
-// The device memory of a two-stage product in one allocation: the operand images,
-// the first stage's output images, the aux buffers of both schedules.
+// The device memory of a two-stage product: the tables in one upload; in one
+// allocation the operand images, the first stage's output images, the aux buffers of
+// both schedules.
 struct ImgWork {
-    DeviceBuffer buf;
+    DeviceBuffer d_tables, buf;
     double *img = nullptr, *mid = nullptr;
-    int alloc(int64_t img_blocks, int64_t mid_blocks, ImgSchedule& a, ImgSchedule& b);
+    int finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms);
 };
 // C (+)= the products (block output), or the images of them into C (accumulate
 // is then ignored).  A wait that gives up sets *status = DMRG_E_NUMERIC.

@@ -575,7 +575,7 @@ int ImgPack::check_bounds(int64_t n0, int64_t n1, int64_t n2) const {
     return DMRG_OK;
 }
 
-int ImgPack::finalize(int panel, cudaStream_t stream) {
+void ImgPack::plan(int panel, Tables& tab) {
     chunks.clear();
     first_chunk.assign(1, 0);
     for (int j = 0; j < (int)jobs.size(); ++j) {
@@ -584,17 +584,16 @@ int ImgPack::finalize(int panel, cudaStream_t stream) {
             for (int s = 0; s < slices; ++s) chunks.push_back(ImgChunk{j, p, s, 0});
         first_chunk.push_back((int)chunks.size());
     }
-    Tables t;
-    t.add(jobs);
-    chunks_at = t.add(chunks);
-    return t.to(d_tables, stream);
+    jobs_at = tab.add(jobs);
+    chunks_at = tab.add(chunks);
 }
 
 int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
                     double* img, cudaStream_t stream) {
     if (c1 <= c0) return DMRG_OK;
-    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, dim3(c1 - c0), kPackThreads, 0, stream, p.d_tables.as<ImgJob>(),
-                      reinterpret_cast<const ImgChunk*>(p.d_tables.as<char>() + p.chunks_at) + c0, panel, s0, s1, s2, img);
+    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, dim3(c1 - c0), kPackThreads, 0, stream,
+                      reinterpret_cast<const ImgJob*>(p.tables + p.jobs_at),
+                      reinterpret_cast<const ImgChunk*>(p.tables + p.chunks_at) + c0, panel, s0, s1, s2, img);
 }
 
 // A 64x64 tile's k-step takes a CTA about a microsecond: with few of them, whole
@@ -621,7 +620,7 @@ int ImgSchedule::check_bounds(int64_t a_blocks, int64_t b_blocks, int64_t out_si
     return DMRG_OK;
 }
 
-int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
+void ImgSchedule::plan(int num_sms, Tables& tab) {
     segments.clear();
     splits.clear();
     aux_size = 0;
@@ -706,19 +705,23 @@ int ImgSchedule::finalize(cudaStream_t stream, int num_sms) {
     segments.swap(queue);
     ctas = (int)std::min<int64_t>((int64_t)num_sms * kCtasPerSm, (int64_t)segments.size());
     live.push_back(ImgTerm{});  // a group's t1 is readable
-    Tables tab;
-    tab.add(live);
+    terms_at = tab.add(live);
     segments_at = tab.add(segments);
     splits_at = tab.add(splits);
     tickets_at = tab.add(std::vector<unsigned>(2 + ntickets, 0u));
-    return tab.to(d_tables, stream);
 }
 
-int ImgWork::alloc(int64_t img_blocks, int64_t mid_blocks, ImgSchedule& a, ImgSchedule& b) {
-    const int64_t n = (img_blocks + mid_blocks) * kImgBlock;
+int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms) {
+    Tables tab;
+    p.plan(a.panel, tab);
+    a.plan(num_sms, tab);
+    b.plan(num_sms, tab);
+    DMRG_TRY(tab.to(d_tables, stream));
+    p.tables = a.tables = b.tables = d_tables.as<char>();
+    const int64_t n = (p.blocks + mid_blocks) * kImgBlock;
     DMRG_TRY(buf.alloc((size_t)std::max<int64_t>(n + a.aux_size + b.aux_size, 1) * sizeof(double)));
     img = buf.as<double>();
-    mid = img + img_blocks * kImgBlock;
+    mid = img + p.blocks * kImgBlock;
     a.aux = img + n;
     b.aux = a.aux + a.aux_size;
     return DMRG_OK;
@@ -727,8 +730,8 @@ int ImgWork::alloc(int64_t img_blocks, int64_t mid_blocks, ImgSchedule& a, ImgSc
 int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
                     cudaStream_t stream) {
     if (s.segments.empty()) return DMRG_OK;
-    char* tab = s.d_tables.as<char>();
-    const GemmArgs w{A, B, C, s.aux, reinterpret_cast<const ImgTerm*>(tab),
+    char* tab = s.tables;
+    const GemmArgs w{A, B, C, s.aux, reinterpret_cast<const ImgTerm*>(tab + s.terms_at),
                      reinterpret_cast<const ImgSegment*>(tab + s.segments_at), (int)s.segments.size(), s.panel / 8,
                      reinterpret_cast<const GemmSplit*>(tab + s.splits_at), reinterpret_cast<unsigned*>(tab + s.tickets_at),
                      status, accumulate ? 1 : 0};

@@ -148,10 +148,7 @@ int build_heff(dmrg_heff_s& h) {
         DMRG_TRY(h.img.check_bounds(ket.size, h.L.size, h.R.size));
         DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
         DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, ket.size));
-        DMRG_TRY(h.img.finalize(h.ia.panel, st));
-        DMRG_TRY(h.ia.finalize(st, h.ctx->num_sms));
-        DMRG_TRY(h.ib.finalize(st, h.ctx->num_sms));
-        DMRG_TRY(h.work.alloc(h.img.blocks, t_blocks, h.ia, h.ib));
+        DMRG_TRY(h.work.finalize(h.img, h.ia, h.ib, t_blocks, st, h.ctx->num_sms));
     }
     if (is_split(h.precision)) {
         const int fmt = split_fmt(h.precision);

@@ -177,10 +177,7 @@ int build_zheff(dmrg_zheff_s& h) {
     DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
     DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, 2 * ket.size));
     cudaStream_t st = h.ctx->stream;
-    DMRG_TRY(h.img.finalize(h.ia.panel, st));
-    DMRG_TRY(h.ia.finalize(st, h.ctx->num_sms));
-    DMRG_TRY(h.ib.finalize(st, h.ctx->num_sms));
-    return h.work.alloc(h.img.blocks, t_blocks, h.ia, h.ib);
+    return h.work.finalize(h.img, h.ia, h.ib, t_blocks, st, h.ctx->num_sms);
 }
 
 // out (+)= H psi; the environments are packed anew unless env_packed (zpack_env was
