@@ -52,6 +52,7 @@ _SIGS = {
     "dmrg_ctx_set_stream": (C.c_int, [_VP, _VP]),
     "dmrg_ctx_stream": (_VP, [_VP]),
     "dmrg_ctx_sync": (C.c_int, [_VP]),
+    "dmrg_ctx_set_wait_polls": (C.c_int, [_VP, C.c_int]),
     "dmrg_malloc": (C.c_int, [_VP, C.c_size_t, C.POINTER(_VP)]),
     "dmrg_free": (C.c_int, [_VP, _VP]),
     "dmrg_memcpy_h2d": (C.c_int, [_VP, _VP, _VP, C.c_size_t]),
@@ -222,6 +223,10 @@ class Context:
 
     def sync(self) -> None:
         check(lib().dmrg_ctx_sync(self.h), "dmrg_ctx_sync")
+
+    def set_wait_polls(self, polls: int) -> None:
+        """Tries of a bounded device wait before it gives up (< 0: the default)."""
+        check(lib().dmrg_ctx_set_wait_polls(self.h, polls), "dmrg_ctx_set_wait_polls")
 
     def fp64_peak(self, mode: int = 0, iters: int = 20000) -> float:
         """Measured FP64 TFLOP/s (mode 0: DMMA, 1: DFMA)."""

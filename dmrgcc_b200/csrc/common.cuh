@@ -184,6 +184,9 @@ private:
     std::vector<unsigned char> host_;
 };
 
+// Tries of a bounded wait in a packed FP64 GEMM before it gives up.
+constexpr int kWaitPolls = 1 << 22;
+
 }  // namespace dmrg
 
 struct dmrg_ctx_s {
@@ -193,6 +196,7 @@ struct dmrg_ctx_s {
     int num_sms = 148;
     // Device-side error word: kernels with iteration caps write a nonzero code.
     int* d_status = nullptr;
+    int wait_polls = dmrg::kWaitPolls;  // dmrg_ctx_set_wait_polls
     // Pinned host words for small per-iteration device->host reads (Lanczos
     // convergence flags); one context is used by one host thread at a time.
     int* h_pinned = nullptr;

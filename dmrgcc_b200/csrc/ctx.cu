@@ -195,6 +195,12 @@ int dmrg_ctx_sync(dmrg_ctx_t ctx) {
     return dmrg::take_device_status(ctx);
 }
 
+int dmrg_ctx_set_wait_polls(dmrg_ctx_t ctx, int polls) {
+    if (!ctx) return set_error(DMRG_E_ARG, "null context");
+    ctx->wait_polls = polls < 0 ? kWaitPolls : polls;
+    return DMRG_OK;
+}
+
 int dmrg_malloc(dmrg_ctx_t ctx, size_t bytes, void** dev) {
     if (!ctx || !dev) return set_error(DMRG_E_ARG, "null argument");
     cudaError_t e = cudaMalloc(dev, bytes ? bytes : 1);

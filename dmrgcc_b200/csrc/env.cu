@@ -370,9 +370,8 @@ int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, d
     cudaStream_t st = e.ctx->stream;
     DMRG_TRY(launch_img_pack(e.img, e.i1.panel, 0, (int)e.img.chunks.size(), ket_dev, env_in_dev, nullptr,
                              e.work.img, st));
-    DMRG_TRY(launch_img_gemm(e.i1, e.work.img, e.work.img, e.work.mid, false,
-                             e.ctx->d_status, st));
-    return launch_img_gemm(e.i2, e.work.mid, e.work.img, env_out_dev, false, e.ctx->d_status, st);
+    DMRG_TRY(launch_img_gemm(e.i1, e.work.img, e.work.img, e.work.mid, false, *e.ctx));
+    return launch_img_gemm(e.i2, e.work.mid, e.work.img, env_out_dev, false, *e.ctx);
 }
 
 // The common part of both creators (Wc: a complex update's MPO).

@@ -245,9 +245,10 @@ struct ImgWork {
     int finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms);
 };
 // C (+)= the products (block output), or the images of them into C (accumulate
-// is then ignored).  A wait that gives up sets *status = DMRG_E_NUMERIC.
-int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
-                    cudaStream_t stream);
+// is then ignored), on the context's stream.  A wait that gives up sets the context's
+// status word to DMRG_E_NUMERIC.
+int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate,
+                    const dmrg_ctx_s& ctx);
 
 // ---------------------------------------------------------------------------
 // Split-precision paths on the tcgen05 tensor cores (gemm_split.cu).

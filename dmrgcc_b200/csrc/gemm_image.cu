@@ -18,7 +18,9 @@
 //
 // GEMM CTA: four consumer warps (2 x 2 quarters of the tile, MI x NJ units of 8x8
 // each) and a producer warp that issues the copies; steps are handed over by
-// mbarriers, so warps and tiles overlap.  All waits are bounded.
+// mbarriers, so warps and tiles overlap.  All waits are bounded (kWaitPolls, or the
+// context's limit): a warp whose wait gives up sets the status word and leaves, before it
+// uses anything that the wait was for; the others' waits on it then run out too.
 //
 // Split of the work: two persistent CTAs per SM take tiles, largest first, from a
 // queue (equal shares dealt out beforehand left SMs idle for a fifth of a D=1024
@@ -41,7 +43,6 @@ namespace {
 
 constexpr int kConsumers = 128;            // threads of the four consumer warps
 constexpr int kThreads = kConsumers + 32;  // and the producer warp
-constexpr int kMaxPolls = 1 << 22;         // of a wait, before it gives up
 
 constexpr int kCtasPerSm = 2;
 constexpr int kRegs = 168;                     // per thread: at most 3 of the 10 warps share a sub-core's registers
@@ -63,9 +64,11 @@ struct StepMeta {  // of the step in a slot
 constexpr int kTiles = kSlots + 1;  // every tile has a step
 struct Shared {
     StepMeta meta[kSlots];
-    uint64_t full[kSlots], empty[kSlots];
+    uint64_t full[kSlots], empty[kSlots], met;
     Tile tiles[kTiles];
     int last;
+    int gave_up;  // a consumer has
+    int issued;   // steps, once the producer is through
 };
 constexpr size_t kSmem = kRing + kPad + sizeof(Shared);
 
@@ -79,9 +82,10 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar) {
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the barrier's phase `parity`; false when it gave up.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    for (int n = 0; n < kMaxPolls; ++n) {
+// Waits for the barrier's phase `parity`; false when it gave up after `polls` tries
+// (at least one).
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int polls) {
+    for (int n = 1;; ++n) {
         unsigned done;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -89,8 +93,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
+        if (n >= polls) return false;
     }
-    return false;
+}
+// The same for a whole warp, which agrees: false when any lane gave up.
+__device__ __forceinline__ bool warp_wait(unsigned bar, unsigned parity, int polls) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, polls));
 }
 __device__ __forceinline__ void bulk_copy(unsigned dst, const double* src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
@@ -101,7 +109,14 @@ __device__ __forceinline__ void bulk_copy(unsigned dst, const double* src, unsig
 // the next launch in early (launch_next); the GEMM kernel leaves it to its CTAs' exits
 // (the next launch's waiting CTAs would take the shared memory of its own: Lanczos at
 // D=512 1.27 -> 1.33 ms).
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory"); }
+
+// The four consumer warps meet; false when one of them did not come (it gave up).  An
+// mbarrier: bar.sync would wait for ever for a warp that has left.
+__device__ __forceinline__ bool consumers_meet(unsigned bar, int& meetings, int polls) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+    return warp_wait(bar, meetings++ & 1, polls);
+}
 
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -119,6 +134,7 @@ struct GemmArgs {
     const GemmSplit* splits;
     unsigned* tickets;  // of the split tiles, after the queue's two counters
     int* status;
+    int polls;          // of a bounded wait
     int accumulate;
 };
 
@@ -158,10 +174,10 @@ struct ImageOut {
 // The consumer warps' work on one tile or part.  The unit counts are template
 // parameters of the whole loop (as run-time counts, or in a switch inside it, the
 // accumulators move between registers at every step).  SCALED: terms have scales
-// other than 1 (the products cost ~8% of the loop).
+// other than 1 (the products cost ~8% of the loop).  False when a wait gave up.
 template <int OUT, bool SCALED, int MI, int NJ>
-__device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const char* ring, Shared& sh, unsigned full,
-                                         unsigned empty, int& step, bool& ok) {
+__device__ __forceinline__ bool run_tile(const GemmArgs& w, const Tile& g, const char* ring, Shared& sh, unsigned full,
+                                         unsigned empty, int& step, int& meetings) {
     const StepMeta* meta = sh.meta;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int um0 = (warp >> 1) * MI, un0 = (warp & 1) * NJ, ua = (g.rows + 7) >> 3;
@@ -194,16 +210,20 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
 #pragma unroll 1
     for (int n = max(g.steps, 1); n > 0; --n) {  // (one empty step without terms)
         const int s = step % kSlots;
-        ok = ok && mbar_wait(full + 8 * s, (step / kSlots) & 1);
+        const bool got = mbar_wait(full + 8 * s, (step / kSlots) & 1, w.polls);
+        // Read ahead of the vote, used only after it.  (The vote stands in both branches: ahead
+        // of them it costs an environment update at D=1024 3 us of 171.)
         const double scale = SCALED ? meta[s].scale : 1.0;
-        const int kb = meta[s].kb;
-        const double2* As = reinterpret_cast<const double2*>(ring + meta[s].off) + lane;
+        const int kb = meta[s].kb, off = meta[s].off;
+        const double2* As = reinterpret_cast<const double2*>(ring + off) + lane;
         const double2* Bs = As + ua * kb * 32;
         if (kb == kImgSlice) {
+            if (!__all_sync(0xffffffffu, got)) return false;
 #pragma unroll
             for (int q = 0; q < kImgSlice; ++q)
                 block(As + (um0 * kImgSlice + q) * 32, Bs + (un0 * kImgSlice + q) * 32, kImgSlice * 32, scale);
         } else {
+            if (!__all_sync(0xffffffffu, got)) return false;
 #pragma unroll 1
             for (int q = 0; q < kb; ++q) block(As + (um0 * kb + q) * 32, Bs + (un0 * kb + q) * 32, kb * 32, scale);
         }
@@ -221,7 +241,8 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
         for (int i = 0; i < MI; ++i)
 #pragma unroll
             for (int j = 0; j < NJ; ++j) part[(i * NJ + j) * kConsumers] = make_double2(acc[i][j][0], acc[i][j][1]);
-        consumer_sync();  // every warp's part is written before the ticket is taken
+        const unsigned met = smem_u32(&sh.met);
+        if (!consumers_meet(met, meetings, w.polls)) return false;  // every warp's part is written before the ticket is taken
         if (threadIdx.x == 0) {
             unsigned* tk = w.tickets + 2 + sp.ticket;
             unsigned before;
@@ -229,8 +250,8 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
             sh.last = before == (unsigned)sp.chunks - 1;
             if (sh.last) *tk = 0u;
         }
-        consumer_sync();
-        if (!sh.last) return;
+        if (!consumers_meet(met, meetings, w.polls)) return false;
+        if (!sh.last) return true;
 #pragma unroll
         for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -280,7 +301,7 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
                 }
             }
         }
-        return;
+        return true;
     }
     const bool add = w.accumulate;
     double* crow = w.C + g.c_off + (int64_t)(8 * um0 + fr) * g.ldc + 8 * un0 + 2 * fc;
@@ -301,6 +322,7 @@ __device__ __forceinline__ void run_tile(const GemmArgs& w, const Tile& g, const
             for (int e = 0; e < 2; ++e)
                 if (8 * j + e < cleft) crow[8 * j + e] = add ? old[j][e] + acc[i][j][e] : acc[i][j][e];
     }
+    return true;
 }
 
 // The producer warp: takes segments from the queue (its first is its CTA's own) and
@@ -327,7 +349,7 @@ __device__ __forceinline__ void produce(const GemmArgs& w, char* ring, Shared& s
                 head = at + need;
                 return at;
             }
-            if (!mbar_wait(empty + 8 * (oldest % kSlots), (oldest / kSlots) & 1)) return -1;
+            if (!warp_wait(empty + 8 * (oldest % kSlots), (oldest / kSlots) & 1, w.polls)) return -1;
             if (++oldest < n) tail = sh.meta[oldest % kSlots].off;
         }
     };
@@ -402,15 +424,20 @@ __device__ __forceinline__ void produce(const GemmArgs& w, char* ring, Shared& s
         if (ok) {
             sh.tiles[tiles % kTiles].steps = -1;
             mbar_expect(full + 8 * (n % kSlots), 0);
-        } else {  // gave up: the copies in flight first (bounded), then leave; the consumers give up too
+        } else {  // gave up: the consumers have, or will
             if (w.status) *w.status = DMRG_E_NUMERIC;
-            for (int i = oldest; i < n; ++i) mbar_wait(full + 8 * (i % kSlots), (i / kSlots) & 1);
         }
         if (atomicAdd(w.tickets + 1, 1u) == gridDim.x - 1) {
             w.tickets[0] = 0u;
             w.tickets[1] = 0u;
         }
     }
+    // No copy is in flight when the CTA leaves.  The consumers have waited for them all,
+    // unless one gave up: one that does so later than this finds `issued`.
+    if (lane == 0) *const_cast<volatile int*>(&sh.issued) = n;
+    __threadfence_block();
+    if (!ok || *const_cast<volatile int*>(&sh.gave_up))
+        for (int i = oldest; i < n; ++i) warp_wait(full + 8 * (i % kSlots), (i / kSlots) & 1, kWaitPolls);
 }
 
 template <int OUT, bool SCALED>
@@ -423,6 +450,8 @@ __global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
             mbar_init(full + 8 * s, 1);
             mbar_init(empty + 8 * s, kConsumers / 32);
         }
+        mbar_init(smem_u32(&sh.met), kConsumers / 32);
+        sh.gave_up = sh.issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
@@ -430,21 +459,27 @@ __global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
         produce(w, ring, sh);
         return;
     }
-    bool ok = true;
-    int step = 0;  // steps computed (slot = step % kSlots, its phase = step / kSlots)
+    // A warp that gives up says so, and waits (with the full limit) for the copies that the
+    // producer may have left in flight; one that is still issuing sees to them itself.
+    auto give_up = [&](int step) {
+        if (w.status) *w.status = DMRG_E_NUMERIC;
+        *const_cast<volatile int*>(&sh.gave_up) = 1;
+        __threadfence_block();
+        const int issued = *const_cast<volatile int*>(&sh.issued);
+        for (int i = step; i < issued; ++i) mbar_wait(full + 8 * (i % kSlots), (i / kSlots) & 1, kWaitPolls);
+    };
+    int step = 0, meetings = 0;  // steps computed (slot = step % kSlots, its phase = step / kSlots); of the warps
 #pragma unroll 1
     for (int tile = 0;; ++tile) {
         // the tile's first step carries its descriptor
-        if (!mbar_wait(full + 8 * (step % kSlots), (step / kSlots) & 1)) {
-            if (w.status) *w.status = DMRG_E_NUMERIC;
-            return;
-        }
+        bool ok = w.polls > 0 && warp_wait(full + 8 * (step % kSlots), (step / kSlots) & 1, w.polls);
+        if (!ok) return give_up(step);
         const Tile g = sh.tiles[tile % kTiles];
         if (g.steps < 0) return;
         switch (((g.rows + 15) >> 4) * 4 + ((g.cols + 15) >> 4) - 5) {  // units per warp
 #define DMRG_UNITS(MI, NJ)                                                                        \
     case (MI - 1) * 4 + NJ - 1:                                                                   \
-        run_tile<OUT, SCALED, MI, NJ>(w, g, ring, sh, full, empty, step, ok);                \
+        ok = run_tile<OUT, SCALED, MI, NJ>(w, g, ring, sh, full, empty, step, meetings);          \
         break;
 #define DMRG_UNIT_ROW(MI) DMRG_UNITS(MI, 1) DMRG_UNITS(MI, 2) DMRG_UNITS(MI, 3) DMRG_UNITS(MI, 4)
             DMRG_UNIT_ROW(1)
@@ -455,10 +490,7 @@ __global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
 #undef DMRG_UNITS
             default: break;
         }
-        if (!ok) {
-            if (w.status) *w.status = DMRG_E_NUMERIC;
-            return;
-        }
+        if (!ok) return give_up(step);
     }
 }
 
@@ -727,14 +759,15 @@ int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_bl
     return DMRG_OK;
 }
 
-int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate, int* status,
-                    cudaStream_t stream) {
+int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, double* C, bool accumulate,
+                    const dmrg_ctx_s& ctx) {
+    cudaStream_t stream = ctx.stream;
     if (s.segments.empty()) return DMRG_OK;
     char* tab = s.tables;
     const GemmArgs w{A, B, C, s.aux, reinterpret_cast<const ImgTerm*>(tab + s.terms_at),
                      reinterpret_cast<const ImgSegment*>(tab + s.segments_at), (int)s.segments.size(), s.panel / 8,
                      reinterpret_cast<const GemmSplit*>(tab + s.splits_at), reinterpret_cast<unsigned*>(tab + s.tickets_at),
-                     status, accumulate ? 1 : 0};
+                     ctx.d_status, ctx.wait_polls, accumulate ? 1 : 0};
     switch (s.out * 2 + (s.scaled ? 1 : 0)) {
         case kImgOutBlock * 2: return launch<kImgOutBlock, false>(s.ctas, w, stream);
         case kImgOutBlock * 2 + 1: return launch<kImgOutBlock, true>(s.ctas, w, stream);

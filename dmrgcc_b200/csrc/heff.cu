@@ -241,8 +241,8 @@ int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool a
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
     DMRG_TRY(pack_operands(h, psi, env_packed));
-    DMRG_TRY(launch_img_gemm(h.ia, h.work.img, h.work.img, h.work.mid, false, h.ctx->d_status, st));
-    return launch_img_gemm(h.ib, h.work.img, h.work.mid, out, accumulate, h.ctx->d_status, st);
+    DMRG_TRY(launch_img_gemm(h.ia, h.work.img, h.work.img, h.work.mid, false, *h.ctx));
+    return launch_img_gemm(h.ib, h.work.img, h.work.mid, out, accumulate, *h.ctx);
 }
 
 int dmrg::heff_apply_internal(dmrg_heff_s& h, const double* psi, double* out, bool accumulate) {
@@ -357,15 +357,13 @@ int dmrg_heff_profile(dmrg_heff_t h, const double* psi, double* out, double* ms_
     } else {
         rc = pack_operands(*h, psi, false);
         if (rc == DMRG_OK)
-            rc = launch_img_gemm(h->ia, h->work.img, h->work.img, h->work.mid, false,
-                                 h->ctx->d_status, st);
+            rc = launch_img_gemm(h->ia, h->work.img, h->work.img, h->work.mid, false, *h->ctx);
     }
     cudaEventRecord(ev[1], st);
     if (rc == DMRG_OK)
         rc = split ? launch_gemm_split(h->pb, h->img_L.as<unsigned char>(), h->img_T.as<unsigned char>(), out,
                                         nullptr, true, h->ctx->d_status, st)
-                   : launch_img_gemm(h->ib, h->work.img, h->work.mid, out, true,
-                                     h->ctx->d_status, st);
+                   : launch_img_gemm(h->ib, h->work.img, h->work.mid, out, true, *h->ctx);
     cudaEventRecord(ev[2], st);
     cudaError_t err = cudaEventSynchronize(ev[2]);
     float a = 0, b = 0;

@@ -189,8 +189,8 @@ int zapply(dmrg_zheff_s& h, const double* psi, double* out, bool accumulate, boo
     double* img = h.work.img;
     DMRG_TRY(launch_img_pack(h.img, h.ia.panel, 0, env_packed ? h.img.first_chunk[h.img_psi_jobs] : (int)h.img.chunks.size(),
                              psi, h.L_dev, h.R_dev, img, st));
-    DMRG_TRY(launch_img_gemm(h.ia, img, img, h.work.mid, false, h.ctx->d_status, st));
-    return launch_img_gemm(h.ib, img, h.work.mid, out, accumulate, h.ctx->d_status, st);
+    DMRG_TRY(launch_img_gemm(h.ia, img, img, h.work.mid, false, *h.ctx));
+    return launch_img_gemm(h.ib, img, h.work.mid, out, accumulate, *h.ctx);
 }
 
 int zpack_env(dmrg_zheff_s& h) {

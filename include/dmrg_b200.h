@@ -77,6 +77,13 @@ int dmrg_ctx_destroy(dmrg_ctx_t ctx);
 int dmrg_ctx_set_stream(dmrg_ctx_t ctx, void* stream);
 void* dmrg_ctx_stream(dmrg_ctx_t ctx);
 int dmrg_ctx_sync(dmrg_ctx_t ctx);
+/* Tries after which a wait inside the packed FP64 products (dmrg_heff_apply,
+ * dmrg_zheff_apply, dmrg_env_apply and what runs on them) gives up; polls < 0: the
+ * default.  The call that then reads the context's status (dmrg_ctx_sync, the Lanczos
+ * solvers, dmrg_heff_apply_host) returns DMRG_E_NUMERIC.  Holds for operators' later
+ * applications (a captured Lanczos loop keeps the limit it was captured with).  For
+ * fault-injection tests of that path; no reference counterpart. */
+int dmrg_ctx_set_wait_polls(dmrg_ctx_t ctx, int polls);
 /* Device memory helpers for callers without their own allocator. */
 int dmrg_malloc(dmrg_ctx_t ctx, size_t bytes, void** dev);
 int dmrg_free(dmrg_ctx_t ctx, void* dev);

@@ -1,0 +1,60 @@
+"""A bounded wait of the packed FP64 products that gives up: the kernels end, the status
+reaches the caller, and nothing of it is left for the next application.
+
+The limit is lowered on the host (Context.set_wait_polls); one sector, enough work for
+64-wide tiles that are cut into parts, and a small case of one tile."""
+import numpy as np
+import pytest
+
+from dmrgcc_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(9, 17, 1), (190, 185, 5), (70, 450, 14)]
+
+
+@pytest.fixture()
+def own_ctx():
+    c = capi.Context(0)
+    yield c
+    c.close()
+
+
+def _case(ctx, kind, m, n, bond):
+    """An operator and its buffers: apply() and the output's download()."""
+    rng = np.random.default_rng(11)
+    cplx = kind[0] == "z"
+
+    def values(*shape):
+        x = rng.standard_normal(shape)
+        return x + 1j * rng.standard_normal(shape) if cplx else x
+
+    def upload(x):
+        return capi.DeviceArray.from_host(ctx, np.ascontiguousarray(x).view(np.float64))
+
+    W = values(bond, bond, 1, 1)
+    site = capi.SiteProblem(1, 1, np.zeros((1, 1)), capi.BlockSpec([0], [0], [m], [n]), W.real)
+    L = [capi.BlockSpec([0], [0], [m], [m])] * bond
+    R = [capi.BlockSpec([0], [0], [n], [n])] * bond
+    dk, dl, dr = upload(values(m, n)), upload(values(bond, m, m)), upload(values(bond, n, n))
+    if kind.endswith("env"):
+        op, out = capi.Env(ctx, 0, site, L, Wc=W if cplx else None), upload(values(bond, n, n))
+        return op, (lambda: op.apply(dk, dl, out)), out.download
+    op = capi.ZHeff(ctx, site, L, R, W) if cplx else capi.Heff(ctx, site, L, R)
+    op.set_env(dl, dr)
+    out = upload(values(m, n))
+    return op, (lambda: op.apply(dk, out)), out.download
+
+
+@pytest.mark.parametrize("kind", ["heff", "zheff", "env", "zenv"])
+@pytest.mark.parametrize("m,n,bond", SHAPES)
+def test_give_up_reports(own_ctx, kind, m, n, bond):
+    op, apply, _ = _case(own_ctx, kind, m, n, bond)
+    own_ctx.set_wait_polls(0)
+    apply()
+    with pytest.raises(capi.DmrgError) as err:
+        own_ctx.sync()
+    assert err.value.code == capi.E_NUMERIC
+    own_ctx.sync()  # the status is read once
+    own_ctx.set_wait_polls(-1)
+    op.close()
