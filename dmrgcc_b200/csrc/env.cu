@@ -368,8 +368,7 @@ int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
 
 int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
     cudaStream_t st = e.ctx->stream;
-    DMRG_TRY(launch_img_pack(e.img, e.i1.panel, 0, (int)e.img.chunks.size(), ket_dev, env_in_dev, nullptr,
-                             e.work.img, st));
+    DMRG_TRY(launch_img_pack(e.img, e.work, e.i1.panel, 0, (int)e.img.chunks.size(), ket_dev, env_in_dev, nullptr, st));
     DMRG_TRY(launch_img_gemm(e.i1, e.work.img, e.work.img, e.work.mid, false, *e.ctx));
     return launch_img_gemm(e.i2, e.work.mid, e.work.img, env_out_dev, false, *e.ctx);
 }

@@ -165,10 +165,6 @@ struct ImgPack {
     void plan(int panel, Tables& tab);
     std::vector<int> first_chunk;  // chunks before each job, and in all
 };
-// Packs the jobs of chunks [c0, c1) from the three sources into img.
-int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
-                    double* img, cudaStream_t stream);
-
 struct ImgTerm {
     int64_t a, b;  // images (first blocks) of the two operands
     int k;
@@ -213,10 +209,12 @@ struct ImgSchedule {
     int ctas = 0;
     std::vector<GemmSplit> splits;
     int64_t aux_size = 0;
-    // device tables: terms, segments, splits, tickets (the queue's two counters, then one
-    // per split tile; zero between launches)
+    // device tables: terms, segments, splits
     char* tables = nullptr;  // in ImgWork
-    size_t terms_at = 0, segments_at = 0, splits_at = 0, tickets_at = 0;
+    size_t terms_at = 0, segments_at = 0, splits_at = 0;
+    // device counters, in ImgWork: the queue's, then one per split tile
+    unsigned* tickets = nullptr;
+    int ntickets = 0;  // split tiles
     double* aux = nullptr;  // aux_size doubles, 16-byte aligned, set after finalize
 
     void add_group(int64_t c_off, int ldc, int m, int n) {
@@ -242,8 +240,14 @@ struct ImgSchedule {
 struct ImgWork {
     DeviceBuffer d_tables, buf;
     double *img = nullptr, *mid = nullptr;
+    unsigned* tickets = nullptr;  // the counters of both schedules
+    int ntickets = 0;
     int finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms);
 };
+// Packs the jobs of chunks [c0, c1) from the three sources into the images, and zeroes
+// the counters: one such launch goes ahead of every application's products.
+int launch_img_pack(const ImgPack& p, const ImgWork& work, int panel, int c0, int c1, const double* s0, const double* s1,
+                    const double* s2, cudaStream_t stream);
 // C (+)= the products (block output), or the images of them into C (accumulate
 // is then ignored), on the context's stream.  A wait that gives up sets the context's
 // status word to DMRG_E_NUMERIC.

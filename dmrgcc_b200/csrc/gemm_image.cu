@@ -132,7 +132,7 @@ struct GemmArgs {
     int nsegments;
     int units;        // 8-row units of a full panel
     const GemmSplit* splits;
-    unsigned* tickets;  // of the split tiles, after the queue's two counters
+    unsigned* tickets;  // the queue's counter, then the split tiles'; zero at the start
     int* status;
     int polls;          // of a bounded wait
     int accumulate;
@@ -233,7 +233,7 @@ __device__ __forceinline__ bool run_tile(const GemmArgs& w, const Tile& g, const
     }
     if (g.split >= 0) {
         // A part of a cut tile goes to the aux buffer as the threads hold it; the last CTA
-        // to finish one of the tile's parts sums them, in order, and resets the ticket.
+        // to finish one of the tile's parts sums them, in order.
         const GemmSplit sp = w.splits[g.split];
         constexpr int kPart = MI * NJ * kConsumers;  // double2 per part
         double2* part = reinterpret_cast<double2*>(w.aux + g.aux_off) + threadIdx.x;
@@ -244,11 +244,12 @@ __device__ __forceinline__ bool run_tile(const GemmArgs& w, const Tile& g, const
         const unsigned met = smem_u32(&sh.met);
         if (!consumers_meet(met, meetings, w.polls)) return false;  // every warp's part is written before the ticket is taken
         if (threadIdx.x == 0) {
-            unsigned* tk = w.tickets + 2 + sp.ticket;
             unsigned before;
-            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(tk) : "memory");
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n"
+                         : "=r"(before)
+                         : "l"(w.tickets + 1 + sp.ticket)
+                         : "memory");
             sh.last = before == (unsigned)sp.chunks - 1;
-            if (sh.last) *tk = 0u;
         }
         if (!consumers_meet(met, meetings, w.polls)) return false;
         if (!sh.last) return true;
@@ -418,7 +419,7 @@ __device__ __forceinline__ void produce(const GemmArgs& w, char* ring, Shared& s
         }
         while (ahead < 3) look_ahead();
     }
-    // the end: a step without a tile.  Then the queue's counters are reset by the last CTA out.
+    // the end: a step without a tile
     if (ok) ok = room(0) >= 0;
     if (lane == 0) {
         if (ok) {
@@ -426,10 +427,6 @@ __device__ __forceinline__ void produce(const GemmArgs& w, char* ring, Shared& s
             mbar_expect(full + 8 * (n % kSlots), 0);
         } else {  // gave up: the consumers have, or will
             if (w.status) *w.status = DMRG_E_NUMERIC;
-        }
-        if (atomicAdd(w.tickets + 1, 1u) == gridDim.x - 1) {
-            w.tickets[0] = 0u;
-            w.tickets[1] = 0u;
         }
     }
     // No copy is in flight when the CTA leaves.  The consumers have waited for them all,
@@ -471,8 +468,9 @@ __global__ void __maxnreg__(kRegs) img_gemm_kernel(const GemmArgs w) {
     int step = 0, meetings = 0;  // steps computed (slot = step % kSlots, its phase = step / kSlots); of the warps
 #pragma unroll 1
     for (int tile = 0;; ++tile) {
-        // the tile's first step carries its descriptor
-        bool ok = w.polls > 0 && warp_wait(full + 8 * (step % kSlots), (step / kSlots) & 1, w.polls);
+        // the tile's first step carries its descriptor (a lowered limit also caps the tiles,
+        // so that a test can stop a launch part of the way)
+        bool ok = tile < w.polls && warp_wait(full + 8 * (step % kSlots), (step / kSlots) & 1, w.polls);
         if (!ok) return give_up(step);
         const Tile g = sh.tiles[tile % kTiles];
         if (g.steps < 0) return;
@@ -514,19 +512,26 @@ __device__ __forceinline__ double image_element(const ImgJob& j, const double* _
 
 // One (panel, slice) of a job per CTA; thread = lane of a block: two elements of the
 // image (k indices 4 apart) to one 16-byte store.  Real: a warp reads 8 rows of 32 +
-// 32 contiguous bytes (or, transposed, 4 + 4 rows of 64) and writes 512.
+// 32 contiguous bytes (or, transposed, 4 + 4 rows of 64) and writes 512.  The first CTA
+// also zeroes the counters of the products that follow: every application starts from
+// zero, whatever became of the one before.
 constexpr int kPackThreads = 256;
 template <bool COMPLEX>
 __global__ void __launch_bounds__(kPackThreads) img_pack_kernel(const ImgJob* __restrict__ jobs,
-                                                                const ImgChunk* __restrict__ chunks, int panel,
+                                                                const ImgChunk* __restrict__ chunks, int nchunks,
+                                                                unsigned* __restrict__ tickets, int ntickets, int panel,
                                                                 const double* __restrict__ s0,
                                                                 const double* __restrict__ s1,
                                                                 const double* __restrict__ s2,
                                                                 double* __restrict__ img) {
-    const ImgChunk ch = chunks[blockIdx.x];
-    const ImgJob j = jobs[ch.job];
+    const bool chunk = (int)blockIdx.x < nchunks;  // (a launch without chunks has one CTA)
+    const ImgChunk ch = chunk ? chunks[blockIdx.x] : ImgChunk{};
+    const ImgJob j = chunk ? jobs[ch.job] : ImgJob{};
     launch_next();
     wait_previous();  // the sources are written, and the images' last readers are done
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < ntickets; i += kPackThreads) tickets[i] = 0u;
+    if (!chunk) return;
     const double* src = (j.src == 0 ? s0 : j.src == 1 ? s1 : s2) + j.src_off;
     const int kb_all = (j.image_k() + 7) >> 3, kb = min(kImgSlice, kb_all - ch.slice * kImgSlice);
     const int r0 = ch.panel * panel, units = (min(panel, j.image_rows() - r0) + 7) >> 3, k0 = ch.slice * kImgSlice * 8;
@@ -620,12 +625,14 @@ void ImgPack::plan(int panel, Tables& tab) {
     chunks_at = tab.add(chunks);
 }
 
-int launch_img_pack(const ImgPack& p, int panel, int c0, int c1, const double* s0, const double* s1, const double* s2,
-                    double* img, cudaStream_t stream) {
-    if (c1 <= c0) return DMRG_OK;
-    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, dim3(c1 - c0), kPackThreads, 0, stream,
-                      reinterpret_cast<const ImgJob*>(p.tables + p.jobs_at),
-                      reinterpret_cast<const ImgChunk*>(p.tables + p.chunks_at) + c0, panel, s0, s1, s2, img);
+int launch_img_pack(const ImgPack& p, const ImgWork& work, int panel, int c0, int c1, const double* s0, const double* s1,
+                    const double* s2, cudaStream_t stream) {
+    const int n = std::max(c1 - c0, 0);
+    if (n == 0 && work.ntickets == 0) return DMRG_OK;
+    return launch_pdl(p.complex ? img_pack_kernel<true> : img_pack_kernel<false>, dim3(std::max(n, 1)), kPackThreads, 0,
+                      stream, reinterpret_cast<const ImgJob*>(p.tables + p.jobs_at),
+                      reinterpret_cast<const ImgChunk*>(p.tables + p.chunks_at) + c0, n, work.tickets, work.ntickets, panel,
+                      s0, s1, s2, work.img);
 }
 
 // A 64x64 tile's k-step takes a CTA about a microsecond: with few of them, whole
@@ -656,6 +663,7 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
     segments.clear();
     splits.clear();
     aux_size = 0;
+    ntickets = 0;
     scaled = false;
     if (num_sms <= 0) num_sms = 148;
     std::vector<ImgTerm> live;  // terms with k-steps, by group
@@ -693,7 +701,6 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
     // a tile longer than a quarter of a CTA's share is cut into equal parts (a sixth or a
     // tenth: no gain at D=1024)
     const int64_t longest = std::max<int64_t>(1, cost / ((int64_t)num_sms * kCtasPerSm) / 4);
-    int ntickets = 0;
     std::vector<std::pair<int64_t, int>> order;  // cost, segment
     order.reserve(tiles.size());
     segments.reserve(tiles.size());
@@ -740,7 +747,6 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
     terms_at = tab.add(live);
     segments_at = tab.add(segments);
     splits_at = tab.add(splits);
-    tickets_at = tab.add(std::vector<unsigned>(2 + ntickets, 0u));
 }
 
 int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms) {
@@ -748,8 +754,13 @@ int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_bl
     p.plan(a.panel, tab);
     a.plan(num_sms, tab);
     b.plan(num_sms, tab);
+    // the counters of both stages, one after the other (none where there is no product)
+    ntickets = a.segments.empty() && b.segments.empty() ? 0 : 2 + a.ntickets + b.ntickets;
+    const size_t tickets_at = tab.add(std::vector<unsigned>(ntickets, 0u));
     DMRG_TRY(tab.to(d_tables, stream));
     p.tables = a.tables = b.tables = d_tables.as<char>();
+    tickets = a.tickets = reinterpret_cast<unsigned*>(d_tables.as<char>() + tickets_at);
+    b.tickets = a.tickets + 1 + a.ntickets;
     const int64_t n = (p.blocks + mid_blocks) * kImgBlock;
     DMRG_TRY(buf.alloc((size_t)std::max<int64_t>(n + a.aux_size + b.aux_size, 1) * sizeof(double)));
     img = buf.as<double>();
@@ -763,10 +774,10 @@ int launch_img_gemm(const ImgSchedule& s, const double* A, const double* B, doub
                     const dmrg_ctx_s& ctx) {
     cudaStream_t stream = ctx.stream;
     if (s.segments.empty()) return DMRG_OK;
-    char* tab = s.tables;
+    const char* tab = s.tables;
     const GemmArgs w{A, B, C, s.aux, reinterpret_cast<const ImgTerm*>(tab + s.terms_at),
                      reinterpret_cast<const ImgSegment*>(tab + s.segments_at), (int)s.segments.size(), s.panel / 8,
-                     reinterpret_cast<const GemmSplit*>(tab + s.splits_at), reinterpret_cast<unsigned*>(tab + s.tickets_at),
+                     reinterpret_cast<const GemmSplit*>(tab + s.splits_at), s.tickets,
                      ctx.d_status, ctx.wait_polls, accumulate ? 1 : 0};
     switch (s.out * 2 + (s.scaled ? 1 : 0)) {
         case kImgOutBlock * 2: return launch<kImgOutBlock, false>(s.ctas, w, stream);

@@ -225,15 +225,15 @@ int build_heff(dmrg_heff_s& h) {
 // psi's images, and unless they are packed already the environments'; a launch.
 static int pack_operands(dmrg_heff_s& h, const double* psi, bool env_packed) {
     const int psi_chunks = h.img.first_chunk[h.img_psi_jobs];
-    return launch_img_pack(h.img, h.ia.panel, 0, env_packed ? psi_chunks : (int)h.img.chunks.size(), psi, h.L_dev, h.R_dev,
-                           h.work.img, h.ctx->stream);
+    return launch_img_pack(h.img, h.work, h.ia.panel, 0, env_packed ? psi_chunks : (int)h.img.chunks.size(), psi, h.L_dev,
+                           h.R_dev, h.ctx->stream);
 }
 
 int dmrg::heff_pack_env(dmrg_heff_s& h) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
-    return launch_img_pack(h.img, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr, h.L_dev,
-                           h.R_dev, h.work.img, h.ctx->stream);
+    return launch_img_pack(h.img, h.work, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr,
+                           h.L_dev, h.R_dev, h.ctx->stream);
 }
 
 int dmrg::heff_apply_fp64(dmrg_heff_s& h, const double* psi, double* out, bool accumulate, bool env_packed) {

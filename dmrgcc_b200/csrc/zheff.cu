@@ -187,8 +187,8 @@ int zapply(dmrg_zheff_s& h, const double* psi, double* out, bool accumulate, boo
         return set_error(DMRG_E_STATE, "dmrg_zheff_set_env was not called");
     cudaStream_t st = h.ctx->stream;
     double* img = h.work.img;
-    DMRG_TRY(launch_img_pack(h.img, h.ia.panel, 0, env_packed ? h.img.first_chunk[h.img_psi_jobs] : (int)h.img.chunks.size(),
-                             psi, h.L_dev, h.R_dev, img, st));
+    const int chunks = env_packed ? h.img.first_chunk[h.img_psi_jobs] : (int)h.img.chunks.size();
+    DMRG_TRY(launch_img_pack(h.img, h.work, h.ia.panel, 0, chunks, psi, h.L_dev, h.R_dev, st));
     DMRG_TRY(launch_img_gemm(h.ia, img, img, h.work.mid, false, *h.ctx));
     return launch_img_gemm(h.ib, img, h.work.mid, out, accumulate, *h.ctx);
 }
@@ -196,8 +196,8 @@ int zapply(dmrg_zheff_s& h, const double* psi, double* out, bool accumulate, boo
 int zpack_env(dmrg_zheff_s& h) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_zheff_set_env was not called");
-    return launch_img_pack(h.img, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr, h.L_dev,
-                           h.R_dev, h.work.img, h.ctx->stream);
+    return launch_img_pack(h.img, h.work, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr,
+                           h.L_dev, h.R_dev, h.ctx->stream);
 }
 
 __global__ void zunit_kernel(double* x, int64_t n, int64_t c) {

@@ -79,7 +79,7 @@ void* dmrg_ctx_stream(dmrg_ctx_t ctx);
 int dmrg_ctx_sync(dmrg_ctx_t ctx);
 /* Tries after which a wait inside the packed FP64 products (dmrg_heff_apply,
  * dmrg_zheff_apply, dmrg_env_apply and what runs on them) gives up; polls < 0: the
- * default.  The call that then reads the context's status (dmrg_ctx_sync, the Lanczos
+ * default.  A thread block also ends, in the same way, after `polls` tiles.  The call that then reads the context's status (dmrg_ctx_sync, the Lanczos
  * solvers, dmrg_heff_apply_host) returns DMRG_E_NUMERIC.  Holds for operators' later
  * applications (a captured Lanczos loop keeps the limit it was captured with).  For
  * fault-injection tests of that path; no reference counterpart. */

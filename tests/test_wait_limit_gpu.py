@@ -21,7 +21,7 @@ def own_ctx():
 
 
 def _case(ctx, kind, m, n, bond):
-    """An operator and its buffers: apply() and the output's download()."""
+    """An operator and its buffers: apply(which of two inputs) and the output's download()."""
     rng = np.random.default_rng(11)
     cplx = kind[0] == "z"
 
@@ -36,14 +36,14 @@ def _case(ctx, kind, m, n, bond):
     site = capi.SiteProblem(1, 1, np.zeros((1, 1)), capi.BlockSpec([0], [0], [m], [n]), W.real)
     L = [capi.BlockSpec([0], [0], [m], [m])] * bond
     R = [capi.BlockSpec([0], [0], [n], [n])] * bond
-    dk, dl, dr = upload(values(m, n)), upload(values(bond, m, m)), upload(values(bond, n, n))
+    dk, dl, dr = [upload(values(m, n)) for _ in range(2)], upload(values(bond, m, m)), upload(values(bond, n, n))
     if kind.endswith("env"):
         op, out = capi.Env(ctx, 0, site, L, Wc=W if cplx else None), upload(values(bond, n, n))
-        return op, (lambda: op.apply(dk, dl, out)), out.download
+        return op, (lambda i=0: op.apply(dk[i], dl, out)), out.download
     op = capi.ZHeff(ctx, site, L, R, W) if cplx else capi.Heff(ctx, site, L, R)
     op.set_env(dl, dr)
     out = upload(values(m, n))
-    return op, (lambda: op.apply(dk, out)), out.download
+    return op, (lambda i=0: op.apply(dk[i], out)), out.download
 
 
 @pytest.mark.parametrize("kind", ["heff", "zheff", "env", "zenv"])
@@ -57,4 +57,27 @@ def test_give_up_reports(own_ctx, kind, m, n, bond):
     assert err.value.code == capi.E_NUMERIC
     own_ctx.sync()  # the status is read once
     own_ctx.set_wait_polls(-1)
+    op.close()
+
+
+@pytest.mark.parametrize("kind", ["heff", "zheff", "env", "zenv"])
+@pytest.mark.parametrize("m,n,bond", SHAPES)
+def test_next_application_is_whole(own_ctx, kind, m, n, bond):
+    """However far a launch came before it gave up (some parts of a cut tile done, some
+    not), the operator's next application gives what it gave before, bit for bit."""
+    op, apply, download = _case(own_ctx, kind, m, n, bond)
+    apply()
+    own_ctx.sync()
+    want = download()
+    for polls in range(6):
+        own_ctx.set_wait_polls(polls)
+        apply(1)
+        try:
+            own_ctx.sync()
+        except capi.DmrgError as err:
+            assert err.code == capi.E_NUMERIC
+        own_ctx.set_wait_polls(-1)
+        apply()
+        own_ctx.sync()
+        assert np.array_equal(download(), want)
     op.close()
