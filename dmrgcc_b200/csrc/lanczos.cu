@@ -141,7 +141,9 @@ int run_exact(dmrg_heff_s& h, double* psi, double* energy) {
     double e0 = 0.0;
     DMRG_CUDA_TRY(cudaMemcpyAsync(&e0, ev, sizeof(double), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, w.state.ptr, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state + 4, h.ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaStreamSynchronize(st));
+    if (w.h_state[4] != 0) DMRG_TRY(take_device_status(h.ctx));  // a bounded wait of a matvec gave up
     if (w.h_state[2] != 0) return set_error(DMRG_E_NUMERIC, "Jacobi eigensolver did not converge (n=%d)", n);
     *energy = e0;
     return DMRG_OK;
@@ -292,7 +294,10 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
             }
         }
     }
-    if (dim <= 0) return set_error(DMRG_E_NUMERIC, "Lanczos ended without a converged dimension");
+    if (dim <= 0) {
+        DMRG_TRY(take_device_status(h.ctx));  // the cause, if a matvec gave up
+        return set_error(DMRG_E_NUMERIC, "Lanczos ended without a converged dimension");
+    }
     DMRG_TRY(launch_tridiag_ground_vector(alpha, beta, E, state + 1, w.y.as<double>(), state + 2, st));
     DMRG_TRY(vec_combine(V, n, dim, w.y.as<double>(), 1.0, psi, 0.0, n, blocks, st));
     double e = 0.0;

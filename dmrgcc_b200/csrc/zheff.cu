@@ -273,7 +273,7 @@ int zexact(dmrg_zheff_s& h, double* psi, double* energy) {
     int status[4] = {0, 0, 0, 0};
     DMRG_CUDA_TRY(cudaMemcpyAsync(&e0, ev, sizeof(double), cudaMemcpyDeviceToHost, st));
     DMRG_CUDA_TRY(cudaMemcpyAsync(status, state, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    DMRG_CUDA_TRY(cudaStreamSynchronize(st));
+    DMRG_TRY(take_device_status(h.ctx));  // waits for the stream; a bounded wait of a matvec that gave up
     if (status[2] != 0) return set_error(DMRG_E_NUMERIC, "Jacobi eigensolver did not converge (2n=%d)", N);
     *energy = e0;
     return DMRG_OK;
@@ -326,7 +326,10 @@ int zkrylov(dmrg_zheff_s& h, double* psi, int niter, double precision, double ze
         }
         DMRG_TRY(vec_normalize(vn, 2 * n, tmp, h.rs, blocks, st));
     }
-    if (dim <= 0) return set_error(DMRG_E_NUMERIC, "complex Lanczos ended without a converged dimension");
+    if (dim <= 0) {
+        DMRG_TRY(take_device_status(h.ctx));  // the cause, if a matvec gave up
+        return set_error(DMRG_E_NUMERIC, "complex Lanczos ended without a converged dimension");
+    }
     DMRG_TRY(launch_tridiag_ground_vector(alpha, beta, E, state + 1, h.y.as<double>(), state + 2, st));
     DMRG_TRY(vec_combine(V, ldv, dim, h.y.as<double>(), 1.0, psi, 0.0, 2 * n, blocks, st));
     double e = 0.0;

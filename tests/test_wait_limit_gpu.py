@@ -81,3 +81,20 @@ def test_next_application_is_whole(own_ctx, kind, m, n, bond):
         own_ctx.sync()
         assert np.array_equal(download(), want)
     op.close()
+
+
+@pytest.mark.parametrize("kind", ["heff", "zheff"])
+@pytest.mark.parametrize("m,n", [(5, 7), (13, 17)])
+def test_lanczos_reports(own_ctx, kind, m, n):
+    """The eigensolver, in its dense branch (below 100 components) and beyond: its own call
+    fails, and the next one is not blamed for it."""
+    op, _, _ = _case(own_ctx, kind, m, n, 1)
+    x = np.random.default_rng(5).standard_normal(m * n * (2 if kind == "zheff" else 1))
+    psi = capi.DeviceArray.from_host(own_ctx, x / np.linalg.norm(x))
+    own_ctx.set_wait_polls(0)
+    with pytest.raises(capi.DmrgError) as err:
+        op.lanczos(psi, 4)
+    assert err.value.code == capi.E_NUMERIC and "gave up waiting" in str(err.value)
+    own_ctx.sync()
+    own_ctx.set_wait_polls(-1)
+    op.close()
