@@ -546,23 +546,25 @@ __global__ void __launch_bounds__(kPackThreads) img_pack_kernel(const ImgJob* __
     }
 }
 
-// The kernel's dynamic shared memory is above the 48 KB default: raises its
-// allowance, once per device.
-template <class K>
-int allow_smem(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
+// The kernels' dynamic shared memory is above the 48 KB default: raises their
+// allowance, once per device.  Made when a product is planned, so that no launch inside
+// a stream capture has to make it.
+int allow_smem() {
+    static std::atomic<bool> done[64] = {};
     int dev = 0;
     DMRG_CUDA_TRY(cudaGetDevice(&dev));
-    const uint64_t bit = uint64_t(1) << (dev & 63);
-    if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return DMRG_OK;
-    DMRG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    done.fetch_or(bit, std::memory_order_release);
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return DMRG_OK;
+    using Kernel = void (*)(const GemmArgs);
+    for (Kernel k : {Kernel(img_gemm_kernel<kImgOutBlock, false>), Kernel(img_gemm_kernel<kImgOutBlock, true>),
+                     Kernel(img_gemm_kernel<kImgOutB, false>), Kernel(img_gemm_kernel<kImgOutA, false>),
+                     Kernel(img_gemm_kernel<kImgOutZB, false>)})
+        DMRG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return DMRG_OK;
 }
 
 template <int OUT, bool SCALED>
 int launch(int n, const GemmArgs& w, cudaStream_t st) {
-    static std::atomic<uint64_t> allowed{0};
-    DMRG_TRY(allow_smem(img_gemm_kernel<OUT, SCALED>, kSmem, allowed));
     return launch_pdl(img_gemm_kernel<OUT, SCALED>, dim3(n), kThreads, kSmem, st, w);
 }
 
@@ -750,6 +752,7 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
 }
 
 int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms) {
+    DMRG_TRY(allow_smem());
     Tables tab;
     p.plan(a.panel, tab);
     a.plan(num_sms, tab);

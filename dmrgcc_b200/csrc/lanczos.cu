@@ -97,6 +97,7 @@ int ensure_work(dmrg_heff_s& h, int niter) {
     if (!h.lw) h.lw = new LanczosWork();
     LanczosWork& w = *h.lw;
     const int64_t n = h.site.ket.size;
+    DMRG_TRY(lanczos_step_prepare());
     if (w.niter < niter || w.n != n) {
         for (LanczosWork::Graph& g : w.graph) {  // captured on the buffers replaced below
             if (g.exec) cudaGraphExecDestroy(g.exec);

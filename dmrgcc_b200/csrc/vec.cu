@@ -315,6 +315,20 @@ int lanczos_step_grid(int64_t n, int num_sms) {
     return (int)std::min<int64_t>(num_sms, (n + 1023) / 1024);
 }
 
+int lanczos_step_prepare() {
+    static_assert(kStepShared * sizeof(double) <= 227 * 1024 && (kStepWarps + 3) * kMaxVec + 3 <= kStepShared,
+                  "shared memory of a Lanczos step");
+    static std::atomic<bool> done[64] = {};
+    int dev = 0;
+    DMRG_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return DMRG_OK;
+    for (auto kernel : {lanczos_step_kernel<true>, lanczos_step_kernel<false>})
+        DMRG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kStepShared * sizeof(double))));
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    return DMRG_OK;
+}
+
 int vec_lanczos_step(double* x, double* h, double* V, int64_t n, int niter, double* alpha, double* beta, double* part,
                      int* state, cudaGraphConditionalHandle loop, int num_sms, cudaStream_t st) {
     if (niter > kMaxVec) return set_error(DMRG_E_ARG, "Lanczos dimension %d > %d", niter, kMaxVec);
@@ -345,18 +359,6 @@ int vec_lanczos_step(double* x, double* h, double* V, int64_t n, int niter, doub
         attr.val.cooperative = 1;
     }
     auto kernel = cluster ? lanczos_step_kernel<true> : lanczos_step_kernel<false>;
-    static_assert(kStepShared * sizeof(double) <= 227 * 1024 && (kStepWarps + 3) * kMaxVec + 3 <= kStepShared,
-                  "shared memory of a Lanczos step");
-    static std::atomic<uint64_t> allowed[2] = {};
-    int dev = 0;
-    DMRG_CUDA_TRY(cudaGetDevice(&dev));
-    const uint64_t bit = uint64_t(1) << (dev & 63);
-    std::atomic<uint64_t>& done = allowed[cluster ? 1 : 0];
-    if (dev >= 64 || !(done.load(std::memory_order_acquire) & bit)) {
-        DMRG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(kStepShared * sizeof(double))));
-        done.fetch_or(bit, std::memory_order_release);
-    }
     count_launch();
     DMRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
     return DMRG_OK;

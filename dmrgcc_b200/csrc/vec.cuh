@@ -39,6 +39,8 @@ constexpr int kTickets = 4;  // of a ReduceScratch
 // converged dimension) and iterations are left.
 constexpr int kIterSlot = 4;
 int lanczos_step_grid(int64_t n, int num_sms);  // CTAs of a step
+// The kernel's shared-memory allowance on this device; once, ahead of any capture.
+int lanczos_step_prepare();
 // part: (2 niter + 3) * lanczos_step_grid(n, num_sms) doubles of scratch.
 int vec_lanczos_step(double* x, double* h, double* V, int64_t n, int niter, double* alpha, double* beta, double* part,
                      int* state, cudaGraphConditionalHandle loop, int num_sms, cudaStream_t st);
