@@ -33,9 +33,11 @@ __global__ void __launch_bounds__(kBisectThreads) tridiag_lowest_kernel(const do
                                                                          const double* __restrict__ beta, int m,
                                                                          double* __restrict__ E, int* state,
                                                                          double precision, double zero_tol,
-                                                                         int niter, const int* m_iter) {
+                                                                         int niter, const int* m_iter,
+                                                                         cudaGraphConditionalHandle loop) {
     __shared__ double lo, hi, pivmin;
     __shared__ int first;
+    if (loop && threadIdx.x == 0) cudaGraphSetConditional(loop, 0u);
     if (state[0]) return;  // already converged: later speculative steps are no-ops
     if (m_iter) m = *m_iter;
     if (m < 1 || m > niter) return;
@@ -76,6 +78,8 @@ __global__ void __launch_bounds__(kBisectThreads) tridiag_lowest_kernel(const do
         if (beta[m - 1] < zero_tol || fabs(lam - prev) < precision || m == niter) {
             state[0] = 1;
             state[1] = m;
+        } else if (loop) {
+            cudaGraphSetConditional(loop, 1u);
         }
     }
 }
@@ -344,15 +348,16 @@ __global__ void __launch_bounds__(32) tridiag_vector_kernel(const double* __rest
 int launch_tridiag_lowest(const double* alpha, const double* beta, int m, double* E, int* state, double precision,
                           double zero_tol, int niter, cudaStream_t st) {
     DMRG_LAUNCH tridiag_lowest_kernel<<<1, kBisectThreads, 0, st>>>(alpha, beta, m, E, state, precision, zero_tol, niter,
-                                                                    nullptr);
+                                                                    nullptr, 0);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }
 
 int launch_tridiag_lowest_it(const double* alpha, const double* beta, const int* iter, double* E, int* state,
-                             double precision, double zero_tol, int niter, cudaStream_t st) {
+                             double precision, double zero_tol, int niter, cudaGraphConditionalHandle loop,
+                             cudaStream_t st) {
     DMRG_LAUNCH tridiag_lowest_kernel<<<1, kBisectThreads, 0, st>>>(alpha, beta, 0, E, state, precision, zero_tol,
-                                                                    niter, iter);
+                                                                    niter, iter, loop);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }

@@ -12,9 +12,11 @@ namespace dmrg {
 // E[m-1] receives the eigenvalue.  Skips all work when state[0] is already set.
 int launch_tridiag_lowest(const double* alpha, const double* beta, int m, double* E, int* state, double precision,
                           double zero_tol, int niter, cudaStream_t st);
-// The same with m = *iter read on the device; nothing for m < 1.
+// The same with m = *iter read on the device; nothing for m < 1.  `loop` (0: none): the
+// captured loop's condition, left true when the test fails.
 int launch_tridiag_lowest_it(const double* alpha, const double* beta, const int* iter, double* E, int* state,
-                             double precision, double zero_tol, int niter, cudaStream_t st);
+                             double precision, double zero_tol, int niter, cudaGraphConditionalHandle loop,
+                             cudaStream_t st);
 
 // Cyclic parallel (round-robin) Jacobi eigensolver for a symmetric n x n matrix A
 // (row-major, global memory, overwritten).  On return w[0..n) holds the

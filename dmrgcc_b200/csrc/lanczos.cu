@@ -37,7 +37,7 @@ struct LanczosWork {
     int64_t n = 0;
     DeviceBuffer V, h, scal, state, jac, y, dense, x, part;
     ReduceScratch rs;
-    // the captured loop's second branch (the tridiagonal problem beside the matvec)
+    // the captured loop's second branch (tridiag_beside)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     int* h_state = nullptr;  // the context's pinned words: [done, dim, ...]
@@ -70,6 +70,17 @@ namespace {
 // Convergence of the split-precision phase: |E_i - E_{i-1}| below this (the
 // matvec's relative error is ~1e-6, the Ritz value settles well before).
 constexpr double kSplitPrecision = 1e-9;
+
+// Where the captured loop's tridiagonal step stands: a serial chain of ~10 us that only
+// decides whether the loop goes on.  Beside the next matvec it costs no time, but a
+// solve that converges has then computed one iteration that nothing reads: it pays for
+// solves of more dimensions than an iteration takes tens of us.  Measured, us per
+// solve of 2 / 9 / 23 dimensions, beside / after the vector work: D = 300 (0.1 GFLOP)
+// 224 / 520 / 1455 and 188 / 536 / 1600; D = 512 (0.5) 341 / 922 / 2200 and 270 / 922 /
+// 2440; D = 800 (1.9) 588 / 1795 / 4775 and 432 / 1700 / 4910.  A run of the 8x4 cylinder
+// solves in 11 to 15 dimensions (median) up to 300,000 components, in 7 above: the line
+// lies where those sizes meet.
+constexpr double kBesideFlops = 1e9;
 
 // Matvecs of the FP64 run that ends a mixed-precision Lanczos (<= 0: the full
 // run to the reference's convergence; dmrg_lanczos_set_polish).
@@ -165,26 +176,33 @@ int vector_step(dmrg_heff_s& h, int niter, cudaGraphConditionalHandle loop, cuda
                             alpha + niter, w.part.as<double>(), w.state.as<int>(), loop, h.ctx->num_sms, st);
 }
 // The tridiagonal step and convergence test for the dimension reached.
-int tridiag_step(dmrg_heff_s& h, int niter, double precision, double zero_tol, cudaStream_t st) {
+int tridiag_step(dmrg_heff_s& h, int niter, double precision, double zero_tol, cudaGraphConditionalHandle loop,
+                 cudaStream_t st) {
     LanczosWork& w = *h.lw;
     const double* alpha = w.scal.as<double>();
     return launch_tridiag_lowest_it(alpha, alpha + niter, w.state.as<int>() + kIterSlot, w.scal.as<double>() + 2 * niter,
-                                    w.state.as<int>(), precision, zero_tol, niter, st);
+                                    w.state.as<int>(), precision, zero_tol, niter, loop, st);
 }
 
-// The captured loop's body: the tridiagonal step of the dimension reached beside the
-// matvec, then the vector work.  The step is a serial chain of ~10 us that only
-// decides whether the loop goes on, so it runs beside the next matvec instead of
-// ahead of it; an iteration past convergence writes only what nothing reads.
+bool tridiag_beside(const dmrg_heff_s& h) { return h.flops_exec < kBesideFlops; }
+
+// The captured loop's body: matvec, vector work, and the tridiagonal step, either of the
+// dimension just reached, at the end, or (tridiag_beside) of the one before, beside the
+// matvec; an iteration past convergence writes only what nothing reads.
 int capture_iteration(dmrg_heff_s& h, int niter, double precision, double zero_tol, bool split,
                       cudaGraphConditionalHandle loop, cudaStream_t st) {
-    LanczosWork& w = *h.lw;
-    DMRG_CUDA_TRY(cudaEventRecord(w.fork, st));
-    DMRG_CUDA_TRY(cudaStreamWaitEvent(w.side, w.fork, 0));
-    DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, w.side));
-    DMRG_CUDA_TRY(cudaEventRecord(w.join, w.side));
+    if (!tridiag_beside(h)) {
+        DMRG_TRY(matvec(h, split));
+        DMRG_TRY(vector_step(h, niter, 0, st));
+        return tridiag_step(h, niter, precision, zero_tol, loop, st);
+    }
+    LanczosWork& c = *h.lw;
+    DMRG_CUDA_TRY(cudaEventRecord(c.fork, st));
+    DMRG_CUDA_TRY(cudaStreamWaitEvent(c.side, c.fork, 0));
+    DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, 0, c.side));
+    DMRG_CUDA_TRY(cudaEventRecord(c.join, c.side));
     DMRG_TRY(matvec(h, split));
-    DMRG_CUDA_TRY(cudaStreamWaitEvent(st, w.join, 0));
+    DMRG_CUDA_TRY(cudaStreamWaitEvent(st, c.join, 0));
     return vector_step(h, niter, loop, st);
 }
 
@@ -202,9 +220,12 @@ int build_loop_graph(dmrg_heff_s& h, int niter, double precision, double zero_to
         cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
     }
-    if (!w.side) DMRG_CUDA_TRY(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
-    if (!w.fork) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
-    if (!w.join) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
+    if (tridiag_beside(h)) {
+        LanczosWork& c = *h.lw;
+        if (!c.side) DMRG_CUDA_TRY(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
+        if (!c.fork) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
+        if (!c.join) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
+    }
     cudaGraph_t graph = nullptr;
     DMRG_CUDA_TRY(cudaGraphCreate(&graph, 0));
     int rc = DMRG_OK;
@@ -270,7 +291,8 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
         // the whole loop as one graph launch; the host reads the result once
         DMRG_TRY(build_loop_graph(h, niter, precision, zero_tol, split));
         DMRG_CUDA_TRY(cudaGraphLaunch(w.graph[split ? 1 : 0].exec, st));
-        DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, st));  // the last dimension's, if still open
+        // the last dimension's, if still open
+        if (tridiag_beside(h)) DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, 0, st));
         DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         DMRG_CUDA_TRY(cudaStreamSynchronize(st));
         dim = w.h_state[0] ? w.h_state[1] : 0;
@@ -285,7 +307,7 @@ int krylov(dmrg_heff_s& h, double* psi, int niter, double precision, double zero
     for (int i = 0; i < niter && !h.use_graph; ++i) {
         DMRG_TRY(matvec(h, split));
         DMRG_TRY(vector_step(h, niter, 0, st));
-        DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, st));
+        DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, 0, st));
         if ((i + 1) % chunk == 0 || i + 1 == niter) {
             DMRG_CUDA_TRY(cudaMemcpyAsync(w.h_state, state, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             DMRG_CUDA_TRY(cudaStreamSynchronize(st));

@@ -55,3 +55,30 @@ def test_lanczos_step_forms(ctx, m, n, niter, graph):
     assert abs(e - _lowest(L, R, x, niter)) <= 1e-12 * norm
     assert abs(np.linalg.norm(v) - 1.0) <= 1e-12
     assert abs(v @ (L @ v.reshape(m, n) @ R).ravel() - e) <= 1e-12 * norm
+
+
+@pytest.mark.parametrize("m,n", [(13, 17), (113, 145), (150, 160), (640, 640)])
+@pytest.mark.parametrize("niter", [3, 100])
+def test_converged_loop(ctx, m, n, niter):
+    """A solve that converges before `niter`, and one that ends there, in both captured
+    forms (the convergence test beside the next matvec; after the vector work, above 1
+    GFLOP: the last shape) and both vector kernels: the captured loop launches the same
+    kernels as launch by launch, so dimension, energy and vector are the same bits."""
+    rng = np.random.default_rng(m)
+    u, v = (rng.standard_normal(k) for k in (m, n))
+    L, R = (np.eye(k) * 0.1 + np.outer(x, x) / (x @ x) for k, x in ((m, u), (n, v)))  # of -L (x) R: -1.21, -0.11, -0.01
+    site = capi.SiteProblem(1, 1, np.zeros((1, 1)), capi.BlockSpec([0], [0], [m], [n]), -np.ones((1, 1, 1, 1)))
+    start = rng.standard_normal(m * n)
+    got = []
+    for graph in (True, True, False):
+        h = capi.Heff(ctx, site, [capi.BlockSpec([0], [0], [m], [m])], [capi.BlockSpec([0], [0], [n], [n])])
+        h.set_graph(graph)
+        dl, dr, psi = (capi.DeviceArray.from_host(ctx, x) for x in (L, R, start / np.linalg.norm(start)))
+        h.set_env(dl, dr)
+        got.append((*h.lanczos(psi, niter, 1e-11, 1e-12), psi.download()))
+        h.close()
+    e, dim, vec = got[0]
+    assert dim == 3
+    for other in got[1:]:
+        assert other[:2] == (e, dim) and np.array_equal(other[2], vec)
+    assert abs(e + 1.21) <= 1e-10 and abs(abs(vec @ np.outer(u, v).ravel()) ** 2 / (u @ u) / (v @ v) - 1) <= 1e-9
