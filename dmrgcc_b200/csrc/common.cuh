@@ -200,4 +200,7 @@ struct dmrg_ctx_s {
     // Pinned host words for small per-iteration device->host reads (Lanczos
     // convergence flags); one context is used by one host thread at a time.
     int* h_pinned = nullptr;
+    // A captured Lanczos loop's second branch; made on first use.
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };

@@ -176,6 +176,9 @@ int dmrg_ctx_destroy(dmrg_ctx_t ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->d_status);
     cudaFreeHost(ctx->h_pinned);
+    if (ctx->fork) cudaEventDestroy(ctx->fork);
+    if (ctx->join) cudaEventDestroy(ctx->join);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return DMRG_OK;

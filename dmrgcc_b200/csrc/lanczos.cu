@@ -37,9 +37,6 @@ struct LanczosWork {
     int64_t n = 0;
     DeviceBuffer V, h, scal, state, jac, y, dense, x, part;
     ReduceScratch rs;
-    // the captured loop's second branch (tridiag_beside)
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
     int* h_state = nullptr;  // the context's pinned words: [done, dim, ...]
     int split_iters = 0;     // Krylov dimension of the last split-precision phase
     // the captured Krylov loop, one per matvec precision (0: FP64, 1: split),
@@ -53,9 +50,6 @@ struct LanczosWork {
     ~LanczosWork() {
         for (Graph& g : graph)
             if (g.exec) cudaGraphExecDestroy(g.exec);
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
-        if (side) cudaStreamDestroy(side);
     }
 };
 
@@ -196,7 +190,7 @@ int capture_iteration(dmrg_heff_s& h, int niter, double precision, double zero_t
         DMRG_TRY(vector_step(h, niter, 0, st));
         return tridiag_step(h, niter, precision, zero_tol, loop, st);
     }
-    LanczosWork& c = *h.lw;
+    const dmrg_ctx_s& c = *h.ctx;
     DMRG_CUDA_TRY(cudaEventRecord(c.fork, st));
     DMRG_CUDA_TRY(cudaStreamWaitEvent(c.side, c.fork, 0));
     DMRG_TRY(tridiag_step(h, niter, precision, zero_tol, 0, c.side));
@@ -220,8 +214,8 @@ int build_loop_graph(dmrg_heff_s& h, int niter, double precision, double zero_to
         cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
     }
-    if (tridiag_beside(h)) {
-        LanczosWork& c = *h.lw;
+    if (tridiag_beside(h)) {  // kept by the context: a sweep makes an operator per solve
+        dmrg_ctx_s& c = *h.ctx;
         if (!c.side) DMRG_CUDA_TRY(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
         if (!c.fork) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
         if (!c.join) DMRG_CUDA_TRY(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
