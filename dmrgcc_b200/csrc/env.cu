@@ -13,13 +13,36 @@
 // :974-1060): per output bond index, blocks in row-major (first, second) sector
 // order, present wherever some contribution has a nonzero W.
 #include <algorithm>
-#include <unordered_map>
-#include <unordered_set>
 
 #include "blocksparse.h"
 #include "gemm.cuh"
 
 using namespace dmrg;
+
+namespace {
+
+// The update's products, on either side.  Stage 1: a product of ket (or bra) block
+// `ket` and an input block, m x n with inner extent k, for every pair that some term
+// of stage 2 reads.  Stage 2: the terms of each output block, output blocks in order.
+struct Stage1Task {
+    int ket;
+    int o, blk;   // input block
+    int m, n, k;
+    int64_t off;  // in the scratch of the products
+};
+struct Stage2Term {
+    int task;
+    int ket;
+    double w;
+};
+struct EnvProducts {
+    std::vector<Stage1Task> tasks;
+    std::vector<Stage2Term> terms;  // by output block
+    std::vector<int> first;         // terms before each output block, and in all
+    int64_t scratch_size = 0;
+};
+
+}  // namespace
 
 struct dmrg_env_s {
     dmrg_ctx_t ctx = nullptr;
@@ -27,7 +50,7 @@ struct dmrg_env_s {
     int precision = DMRG_PREC_FP64;
     SiteDesc site;
     EnvDesc in, out;
-    GemmSchedule s1, s2;  // host description of both stages
+    EnvProducts products;  // of creation
     // FP64: images of the ket and of the input environment, stage 1 into images, stage 2 into blocks
     ImgPack img;
     ImgSchedule i1, i2;
@@ -35,335 +58,231 @@ struct dmrg_env_s {
     SplitPlan p1, p2;  // split precisions: the same two stages on the tcgen05 path
     bool cplx = false;  // the complex path (dmrg_zenv_create): the same stages on complex blocks
     DeviceBuffer scratch;
-    int64_t scratch_size = 0;
     double flops_alg = 0, flops_exec = 0;
 };
 
 namespace {
 
-struct Stage2Term {
-    int out_o, out_pos;
-    int scratch_index;  // which stage-1 product
-    int ket_pos;        // K block (left) or B block (right)
-    double w;
-};
-
-struct Stage1Task {
-    int ket_pos;
-    int o_in, blk_in;
-    int m, n, k;
-    int64_t off;
-};
-
-int build_left(dmrg_env_s& e) {
+// Output structure and products.  Left and right are mirror images: with (x, y) the
+// sectors of an input block of bond index `o`, block u of the ket list with sector x
+// (left: of its rows, right: of its columns) makes the stage 1 product, every block v
+// with sector y a term, per output index with a nonzero weight; the output block has the
+// other sectors of u and v.  One pass: the terms, in the order of the reference's loops,
+// flag the output blocks, and are then sorted into them.
+int build_products(dmrg_env_s& e) {
     const SiteDesc& s = e.site;
     const BlockListDesc& ket = s.ket;
-    auto same_left = ket.by_sector(0, s.nl);
-    // zero_flag pass -> output structure
-    std::vector<char> flag((size_t)s.rb * s.nr * s.nr, 0);
-    std::vector<int> dim_r(s.nr, -1);  // column count of the ket blocks with right sector r
+    const bool left = e.side == 0;
+    const char* name = left ? "L" : "R";
+    const int nx = left ? s.nl : s.nr, ny = left ? s.nr : s.nl;            // sectors of the input, of the output
+    const int in_bond = left ? s.lb : s.rb, out_bond = left ? s.rb : s.lb;
+    const std::vector<int>&inner = left ? ket.rows : ket.cols, &outer = left ? ket.cols : ket.rows;
+    const std::vector<int>& osec = left ? ket.right : ket.left;
+    const auto same = ket.by_sector(left ? 0 : 1, nx);
+    std::vector<int> dim(ny, -1);  // outer extent of the ket blocks by output sector
     for (int k = 0; k < ket.count(); ++k) {
-        int r = ket.right[k];
-        if (dim_r[r] == -1) dim_r[r] = ket.cols[k];
-        else if (dim_r[r] != ket.cols[k])
-            return set_error(DMRG_E_ARG, "ket blocks of right sector %d have different widths", r);
+        int& d = dim[osec[k]];
+        if (d == -1) d = outer[k];
+        else if (d != outer[k])
+            return left ? set_error(DMRG_E_ARG, "ket blocks of right sector %d have different widths", osec[k])
+                        : set_error(DMRG_E_ARG, "ket blocks of left sector %d have different heights", osec[k]);
     }
-    for (int o1 = 0; o1 < s.lb; ++o1) {
-        const BlockListDesc& Lo = e.in.o[o1];
-        for (int i = 0; i < Lo.count(); ++i) {
-            const int kdx = Lo.left[i], ldx = Lo.right[i];
-            if (kdx < 0 || kdx >= s.nl || ldx < 0 || ldx >= s.nl)
-                return set_error(DMRG_E_ARG, "L[%d] block %d sectors out of range", o1, i);
-            if (Lo.rows[i] == 0) continue;
-            for (int pk : same_left[kdx]) {
-                const int idx = ket.right[pk];
-                const int p1 = s.p(kdx, idx);
-                if (!s.left_nonzero(o1, p1)) continue;
-                for (int pl : same_left[ldx]) {
-                    const int jdx = ket.right[pl];
-                    const int p2 = s.p(ldx, jdx);
-                    for (int o2 = 0; o2 < s.rb; ++o2)
-                        if (s.w(o1, o2, p1, p2) != 0.0) flag[((size_t)o2 * s.nr + idx) * s.nr + jdx] = 1;
-                }
+    for (int o = 0; o < in_bond; ++o) {
+        const BlockListDesc& in = e.in.o[o];
+        for (int i = 0; i < in.count(); ++i)
+            if (in.left[i] < 0 || in.left[i] >= nx || in.right[i] < 0 || in.right[i] >= nx)
+                return set_error(DMRG_E_ARG, "%s[%d] block %d sectors out of range", name, o, i);
+    }
+    // by (o, pu): whether the reference takes the product; by (o, pu, pv): the output indexes
+    // with a nonzero weight, ascending
+    std::vector<char> taken((size_t)in_bond * s.d);
+    std::vector<int> outs, outs_first(1, 0);
+    for (int o = 0; o < in_bond; ++o)
+        for (int pu = 0; pu < s.d; ++pu) {
+            taken[(size_t)o * s.d + pu] = left ? s.left_nonzero(o, pu) : s.right_nonzero(o, pu);
+            for (int pv = 0; pv < s.d; ++pv) {
+                for (int q = 0; q < out_bond; ++q)
+                    if ((left ? s.w(o, q, pu, pv) : s.w(q, o, pv, pu)) != 0.0) outs.push_back(q);
+                outs_first.push_back((int)outs.size());
             }
         }
-    }
-    e.out.o.assign(s.rb, BlockListDesc());
-    for (int o2 = 0; o2 < s.rb; ++o2)
-        for (int i = 0; i < s.nr; ++i)
-            for (int j = 0; j < s.nr; ++j)
-                if (flag[((size_t)o2 * s.nr + i) * s.nr + j]) e.out.o[o2].push(i, j, dim_r[i], dim_r[j]);
-    e.out.rebase();
-
-    std::vector<Stage1Task> tasks;
-    std::vector<Stage2Term> terms;
+    struct Term {
+        int key;  // output index and sectors
+        Stage2Term t;
+    };
+    EnvProducts& pr = e.products;
+    std::vector<Term> terms;
+    std::vector<int> count((size_t)out_bond * ny * ny, 0);  // terms by key
     double f1_alg = 0, f2_alg = 0, f1_exec = 0, f2_exec = 0;
-    e.scratch_size = 0;
-    for (int o1 = 0; o1 < s.lb; ++o1) {
-        const BlockListDesc& Lo = e.in.o[o1];
-        for (int i = 0; i < Lo.count(); ++i) {
-            const int kdx = Lo.left[i], ldx = Lo.right[i];
-            const int lr = Lo.rows[i], lc = Lo.cols[i];
-            if (lr == 0) continue;
-            for (int pk : same_left[kdx]) {
-                const int idx = ket.right[pk];
-                const int p1 = s.p(kdx, idx);
-                if (!s.left_nonzero(o1, p1)) continue;
-                const int a_k = ket.rows[pk], b_i = ket.cols[pk];
-                if (a_k != lr) return set_error(DMRG_E_ARG, "ket block %d rows %d != L rows %d", pk, a_k, lr);
-                f1_alg += 2.0 * b_i * a_k * lc;
-                const int t_index = (int)tasks.size();
-                bool used = false;
-                for (int pl : same_left[ldx]) {
-                    const int jdx = ket.right[pl];
-                    const int p2 = s.p(ldx, jdx);
-                    if (ket.rows[pl] != lc) return set_error(DMRG_E_ARG, "ket block %d rows != L cols", pl);
-                    f2_alg += 2.0 * b_i * lc * ket.cols[pl];
-                    for (int o2 = 0; o2 < s.rb; ++o2) {
-                        const double w = s.w(o1, o2, p1, p2);
-                        if (w == 0.0) continue;
-                        const int q = e.out.o[o2].find(idx, jdx);
-                        terms.push_back(Stage2Term{o2, q, t_index, pl, w});
-                        f2_exec += 2.0 * b_i * lc * ket.cols[pl];
-                        used = true;
+    for (int o = 0; o < in_bond; ++o) {
+        const BlockListDesc& in = e.in.o[o];
+        for (int i = 0; i < in.count(); ++i) {
+            const int r = in.rows[i], c = in.cols[i];
+            if (r == 0) continue;
+            for (int u : same[in.left[i]]) {
+                const int pu = s.pb(u);
+                if (!taken[(size_t)o * s.d + pu]) continue;
+                if (inner[u] != r)
+                    return left ? set_error(DMRG_E_ARG, "ket block %d rows %d != L rows %d", u, inner[u], r)
+                                : set_error(DMRG_E_ARG, "ket block %d cols %d != R rows %d", u, inner[u], r);
+                f1_alg += 2.0 * outer[u] * r * c;
+                const size_t before = terms.size();
+                for (int v : same[in.right[i]]) {
+                    const int pv = s.pb(v);
+                    if (inner[v] != c)
+                        return left ? set_error(DMRG_E_ARG, "ket block %d rows != L cols", v)
+                                    : set_error(DMRG_E_ARG, "ket block %d cols != R cols", v);
+                    const double f = 2.0 * outer[u] * c * outer[v];
+                    f2_alg += f;
+                    const size_t at = ((size_t)o * s.d + pu) * s.d + pv;
+                    for (int x = outs_first[at]; x < outs_first[at + 1]; ++x) {
+                        const int q = outs[x], key = (q * ny + osec[u]) * ny + osec[v];
+                        const double w = left ? s.w(o, q, pu, pv) : s.w(q, o, pv, pu);
+                        terms.push_back(Term{key, Stage2Term{(int)pr.tasks.size(), v, w}});
+                        ++count[key];
+                        f2_exec += f;
                     }
                 }
-                if (used) {
-                    tasks.push_back(Stage1Task{pk, o1, i, b_i, lc, a_k, e.scratch_size});
-                    e.scratch_size += (int64_t)b_i * lc;
-                    f1_exec += 2.0 * b_i * a_k * lc;
+                if (terms.size() > before) {
+                    pr.tasks.push_back(Stage1Task{u, o, i, outer[u], c, r, pr.scratch_size});
+                    pr.scratch_size += (int64_t)outer[u] * c;
+                    f1_exec += 2.0 * outer[u] * r * c;
                 }
             }
         }
     }
-    // stage 1: F = B^T L  (A = ket block stored a_k x b_i -> transposed)
-    e.s1.reset();
-    e.s1.ta = true;
-    for (const Stage1Task& t : tasks) {
-        e.s1.add_group(t.off, t.n, t.m, t.n);
-        e.s1.add_term(ket.off[t.ket_pos], ket.cols[t.ket_pos], e.in.base[t.o_in] + e.in.o[t.o_in].off[t.blk_in],
-                      t.n, t.k, 1.0);
-    }
-    // stage 2: out += w F K, grouped per output block
-    e.s2.reset();
-    std::vector<int64_t> first(e.out.o.size() + 1, 0);
-    for (size_t o = 0; o < e.out.o.size(); ++o) first[o + 1] = first[o] + e.out.o[o].count();
-    std::vector<std::vector<int>> bucket(first.back());
-    for (int i = 0; i < (int)terms.size(); ++i) bucket[first[terms[i].out_o] + terms[i].out_pos].push_back(i);
-    for (size_t o = 0; o < e.out.o.size(); ++o) {
-        const BlockListDesc& Oo = e.out.o[o];
-        for (int q = 0; q < Oo.count(); ++q) {
-            const auto& b = bucket[first[o] + q];
-            if (b.empty()) continue;
-            e.s2.add_group(e.out.base[o] + Oo.off[q], Oo.cols[q], Oo.rows[q], Oo.cols[q]);
-            for (int ti : b) {
-                const Stage2Term& t = terms[ti];
-                const Stage1Task& st = tasks[t.scratch_index];
-                e.s2.add_term(st.off, st.n, ket.off[t.ket_pos], ket.cols[t.ket_pos], st.n, t.w);
+    e.out.o.assign(out_bond, BlockListDesc());
+    pr.first.assign(1, 0);
+    std::vector<int> next(count.size());  // where a key's next term goes
+    int n = 0;
+    for (int q = 0, key = 0; q < out_bond; ++q)
+        for (int i = 0; i < ny; ++i)
+            for (int j = 0; j < ny; ++j, ++key) {
+                if (!count[key]) continue;
+                e.out.o[q].push(i, j, dim[i], dim[j]);
+                next[key] = n;
+                pr.first.push_back(n += count[key]);
             }
-        }
-    }
+    e.out.rebase();
+    pr.terms.resize(terms.size());
+    for (const Term& t : terms) pr.terms[next[t.key]++] = t.t;
     e.flops_alg = f1_alg + f2_alg;
     e.flops_exec = f1_exec + f2_exec;
     return DMRG_OK;
 }
 
-int build_right(dmrg_env_s& e) {
-    const SiteDesc& s = e.site;
-    const BlockListDesc& ket = s.ket;
-    auto same_right = ket.by_sector(1, s.nr);
-    std::vector<char> flag((size_t)s.lb * s.nl * s.nl, 0);
-    std::vector<int> dim_l(s.nl, -1);
-    for (int k = 0; k < ket.count(); ++k) {
-        int l = ket.left[k];
-        if (dim_l[l] == -1) dim_l[l] = ket.rows[k];
-        else if (dim_l[l] != ket.rows[k])
-            return set_error(DMRG_E_ARG, "ket blocks of left sector %d have different heights", l);
-    }
-    for (int o2 = 0; o2 < s.rb; ++o2) {
-        const BlockListDesc& Ro = e.in.o[o2];
-        for (int i = 0; i < Ro.count(); ++i) {
-            const int ldx = Ro.left[i], kdx = Ro.right[i];
-            if (ldx < 0 || ldx >= s.nr || kdx < 0 || kdx >= s.nr)
-                return set_error(DMRG_E_ARG, "R[%d] block %d sectors out of range", o2, i);
-            if (Ro.rows[i] == 0) continue;
-            for (int pl : same_right[ldx]) {
-                const int jdx = ket.left[pl];
-                const int p2 = s.p(jdx, ldx);
-                if (!s.right_nonzero(o2, p2)) continue;
-                for (int pk : same_right[kdx]) {
-                    const int idx = ket.left[pk];
-                    const int p1 = s.p(idx, kdx);
-                    for (int o1 = 0; o1 < s.lb; ++o1)
-                        if (s.w(o1, o2, p1, p2) != 0.0) flag[((size_t)o1 * s.nl + jdx) * s.nl + idx] = 1;
-                }
-            }
-        }
-    }
-    e.out.o.assign(s.lb, BlockListDesc());
-    for (int o1 = 0; o1 < s.lb; ++o1)
-        for (int j = 0; j < s.nl; ++j)
-            for (int i = 0; i < s.nl; ++i)
-                if (flag[((size_t)o1 * s.nl + j) * s.nl + i]) e.out.o[o1].push(j, i, dim_l[j], dim_l[i]);
-    e.out.rebase();
-
-    std::vector<Stage1Task> tasks;
-    std::vector<Stage2Term> terms;
-    double f1_alg = 0, f2_alg = 0, f1_exec = 0, f2_exec = 0;
-    e.scratch_size = 0;
-    for (int o2 = 0; o2 < s.rb; ++o2) {
-        const BlockListDesc& Ro = e.in.o[o2];
-        for (int i = 0; i < Ro.count(); ++i) {
-            const int ldx = Ro.left[i], kdx = Ro.right[i];
-            const int rr = Ro.rows[i], rc = Ro.cols[i];
-            if (rr == 0) continue;
-            for (int pl : same_right[ldx]) {
-                const int jdx = ket.left[pl];
-                const int p2 = s.p(jdx, ldx);
-                if (!s.right_nonzero(o2, p2)) continue;
-                const int a_j = ket.rows[pl], b_l = ket.cols[pl];
-                if (b_l != rr) return set_error(DMRG_E_ARG, "ket block %d cols %d != R rows %d", pl, b_l, rr);
-                f1_alg += 2.0 * a_j * b_l * rc;
-                const int t_index = (int)tasks.size();
-                bool used = false;
-                for (int pk : same_right[kdx]) {
-                    const int idx = ket.left[pk];
-                    const int p1 = s.p(idx, kdx);
-                    if (ket.cols[pk] != rc) return set_error(DMRG_E_ARG, "ket block %d cols != R cols", pk);
-                    f2_alg += 2.0 * a_j * rc * ket.rows[pk];
-                    for (int o1 = 0; o1 < s.lb; ++o1) {
-                        const double w = s.w(o1, o2, p1, p2);
-                        if (w == 0.0) continue;
-                        const int q = e.out.o[o1].find(jdx, idx);
-                        terms.push_back(Stage2Term{o1, q, t_index, pk, w});
-                        f2_exec += 2.0 * a_j * rc * ket.rows[pk];
-                        used = true;
-                    }
-                }
-                if (used) {
-                    tasks.push_back(Stage1Task{pl, o2, i, a_j, rc, b_l, e.scratch_size});
-                    e.scratch_size += (int64_t)a_j * rc;
-                    f1_exec += 2.0 * a_j * b_l * rc;
-                }
-            }
-        }
-    }
-    // stage 1: G = K R
-    e.s1.reset();
-    for (const Stage1Task& t : tasks) {
-        e.s1.add_group(t.off, t.n, t.m, t.n);
-        e.s1.add_term(ket.off[t.ket_pos], ket.cols[t.ket_pos], e.in.base[t.o_in] + e.in.o[t.o_in].off[t.blk_in],
-                      t.n, t.k, 1.0);
-    }
-    // stage 2: out += w G B^T (B block stored a_i x b_k -> transposed)
-    e.s2.reset();
-    e.s2.tb = true;
-    std::vector<int64_t> first(e.out.o.size() + 1, 0);
-    for (size_t o = 0; o < e.out.o.size(); ++o) first[o + 1] = first[o] + e.out.o[o].count();
-    std::vector<std::vector<int>> bucket(first.back());
-    for (int i = 0; i < (int)terms.size(); ++i) bucket[first[terms[i].out_o] + terms[i].out_pos].push_back(i);
+// Calls f(offset, rows, cols, first term, end of its terms) for every output block.
+template <class F>
+void for_output(const dmrg_env_s& e, F f) {
+    int g = 0;
     for (size_t o = 0; o < e.out.o.size(); ++o) {
-        const BlockListDesc& Oo = e.out.o[o];
-        for (int q = 0; q < Oo.count(); ++q) {
-            const auto& b = bucket[first[o] + q];
-            if (b.empty()) continue;
-            e.s2.add_group(e.out.base[o] + Oo.off[q], Oo.cols[q], Oo.rows[q], Oo.cols[q]);
-            for (int ti : b) {
-                const Stage2Term& t = terms[ti];
-                const Stage1Task& st = tasks[t.scratch_index];
-                e.s2.add_term(st.off, st.n, ket.off[t.ket_pos], ket.cols[t.ket_pos], st.n, t.w);
-            }
-        }
+        const BlockListDesc& b = e.out.o[o];
+        for (int q = 0; q < b.count(); ++q, ++g)
+            f(e.out.base[o] + b.off[q], b.rows[q], b.cols[q], e.products.first[g], e.products.first[g + 1]);
     }
-    e.flops_alg = f1_alg + f2_alg;
-    e.flops_exec = f1_exec + f2_exec;
-    return DMRG_OK;
+}
+
+// The split precisions: the products on the operands where they lie.  Left: stage 1
+// F = B^T L (transposed A), stage 2 out += w F K; right: G = K R, out += w G B^T
+// (transposed B).
+int build_split(dmrg_env_s& e, cudaStream_t st) {
+    const BlockListDesc& ket = e.site.ket;
+    const EnvProducts& pr = e.products;
+    GemmSchedule s1, s2;
+    s1.ta = e.side == 0;
+    s2.tb = e.side == 1;
+    for (const Stage1Task& t : pr.tasks) {
+        s1.add_group(t.off, t.n, t.m, t.n);
+        s1.add_term(ket.off[t.ket], ket.cols[t.ket], e.in.base[t.o] + e.in.o[t.o].off[t.blk], t.n, t.k, 1.0);
+    }
+    for_output(e, [&](int64_t off, int m, int n, int t0, int t1) {
+        s2.add_group(off, n, m, n);
+        for (int i = t0; i < t1; ++i) {
+            const Stage2Term& t = pr.terms[i];
+            const Stage1Task& f = pr.tasks[t.task];
+            s2.add_term(f.off, f.n, ket.off[t.ket], ket.cols[t.ket], f.n, t.w);
+        }
+    });
+    DMRG_TRY(s1.check_bounds(ket.size, e.in.size, pr.scratch_size));
+    DMRG_TRY(s2.check_bounds(pr.scratch_size, ket.size, e.out.size));
+    const int fmt = e.precision == DMRG_PREC_BF16X3 ? kFmtBF16 : kFmtTF32;
+    DMRG_TRY(e.scratch.alloc((size_t)std::max<int64_t>(pr.scratch_size, 1) * sizeof(double)));
+    DMRG_TRY(e.p1.build(s1, fmt, ket.size, e.in.size, pr.scratch_size, st, e.ctx->num_sms));
+    return e.p2.build(s2, fmt, pr.scratch_size, ket.size, e.out.size, st, e.ctx->num_sms);
 }
 
 }  // namespace
 
 namespace {
 
-// The FP64 execution of s1 and s2 on packed operands (gemm_image.cu).  Real: the
+// FP64: the products on packed operands (gemm_image.cu).  Real: the
 // ket's images serve stage 1 (its A operand) and stage 2 (its B operand): left, both
-// read K^T; right, both read K.  Complex (W: the complex MPO, the schedules' stage 2
-// scales its 1-based positions): real forms of the blocks (gemm.cuh, ImgKind), the
+// read K^T; right, both read K.  Complex (W: the complex MPO, a term's weight is its
+// 1-based position): real forms of the blocks (gemm.cuh, ImgKind), the
 // bra conjugated (left: stage 1's A operand, right: stage 2's B operand); a term's
 // complex weight w G B is Re w (G B) + Im w (G (i B)).
 int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
     const BlockListDesc& ket = e.site.ket;
+    const EnvProducts& pr = e.products;
     const bool z = W != nullptr;
     const int f = z ? 2 : 1;  // doubles per element
-    // images by offset: the ket as stage 1's A operand, as stage 2's B operand (and times i), ...
-    // (hashed: a sweep creates an update per site, and ordered maps were half of its planning)
-    using Images = std::unordered_map<int64_t, int64_t>;
-    Images ket_a, ket_b[2], env_img, mid_img;
-    std::unordered_map<int64_t, int> ket_pos;
-    mid_img.reserve(e.s1.groups.size());
-    env_img.reserve(e.s1.terms.size());
-    e.i1.terms.reserve(e.s1.terms.size());
-    e.i1.groups.reserve(e.s1.groups.size());
-    e.i2.terms.reserve((z ? 2 : 1) * e.s2.terms.size());
-    e.i2.groups.reserve(e.s2.groups.size());
-    for (int k = 0; k < ket.count(); ++k)
-        if (ket.rows[k] > 0 && ket.cols[k] > 0) ket_pos[ket.off[k]] = k;
-    auto ket_image = [&](Images& at, int64_t off, ImgKind kind, bool conj, bool times_i) {
-        auto it = at.find(off);
-        if (it != at.end()) return it->second;
-        const int k = ket_pos.at(off), r = ket.rows[k], c = ket.cols[k];
+    // images (-1: not made yet): the ket as stage 1's A operand, as stage 2's B operand (and
+    // times i), the input environment, the products
+    std::vector<int64_t> ket_a(ket.count(), -1), ket_b[2], mid(pr.tasks.size());
+    for (auto& b : ket_b) b.assign(z ? ket.count() : 0, -1);
+    std::vector<std::vector<int64_t>> env(e.in.o.size());
+    for (size_t o = 0; o < env.size(); ++o) env[o].assign(e.in.o[o].count(), -1);
+    auto ket_image = [&](std::vector<int64_t>& at, int k, ImgKind kind, bool conj, bool times_i) {
+        if (at[k] >= 0) return at[k];
+        const int r = ket.rows[k], c = ket.cols[k];
         const bool t = e.side == 0;
-        const int64_t img = z ? e.img.add_complex(0, off, t ? c : r, t ? r : c, c, t, kind, conj, times_i)
-                              : e.img.add(0, off, t ? c : r, t ? r : c, c, t);
-        at.emplace(off, img);
-        return img;
+        return at[k] = z ? e.img.add_complex(0, ket.off[k], t ? c : r, t ? r : c, c, t, kind, conj, times_i)
+                         : e.img.add(0, ket.off[k], t ? c : r, t ? r : c, c, t);
     };
-    e.i1.panel = e.i2.panel = ImgSchedule::panel_for((z ? 4.0 : 1.0) * (e.s1.flops + e.s2.flops));
+    e.i1.panel = e.i2.panel = ImgSchedule::panel_for((z ? 4.0 : 1.0) * e.flops_exec);
     e.i1.out = kImgOutA;
-    int64_t mid = 0;
-    for (const GemmGroup& g : e.s1.groups) {
-        if (g.m <= 0 || g.n <= 0) continue;
-        mid_img[g.c_off] = mid;
-        e.i1.add_group(mid, 0, g.m, f * g.n);
-        mid += img_blocks(g.m, f * g.n);
-        for (int t = g.t0; t < g.t1; ++t) {
-            const GemmTerm& x = e.s1.terms[t];
-            if (x.k <= 0) continue;
-            auto it = env_img.find(x.b_off);
-            if (it == env_img.end())
-                it = env_img.emplace(x.b_off, z ? e.img.add_complex(1, x.b_off, g.n, x.k, x.ldb, true, kImgComplexB, false, false)
-                                                : e.img.add(1, x.b_off, g.n, x.k, x.ldb, true)).first;
-            e.i1.add_term(ket_image(ket_a, x.a_off, kImgComplexA, e.side == 0, false), it->second, f * x.k, 1.0);
-        }
+    e.i1.groups.reserve(pr.tasks.size());
+    e.i1.terms.reserve(pr.tasks.size());
+    e.i2.groups.reserve(pr.first.size());
+    e.i2.terms.reserve(f * pr.terms.size());
+    int64_t blocks = 0;
+    for (size_t i = 0; i < pr.tasks.size(); ++i) {
+        const Stage1Task& t = pr.tasks[i];
+        if (t.m <= 0 || t.n <= 0) continue;
+        mid[i] = blocks;
+        e.i1.add_group(blocks, 0, t.m, f * t.n);
+        blocks += img_blocks(t.m, f * t.n);
+        if (t.k <= 0) continue;
+        int64_t& b = env[t.o][t.blk];
+        const int64_t off = e.in.base[t.o] + e.in.o[t.o].off[t.blk];
+        if (b < 0)
+            b = z ? e.img.add_complex(1, off, t.n, t.k, t.n, true, kImgComplexB, false, false)
+                  : e.img.add(1, off, t.n, t.k, t.n, true);
+        e.i1.add_term(ket_image(ket_a, t.ket, kImgComplexA, e.side == 0, false), b, f * t.k, 1.0);
     }
-    std::unordered_set<int64_t> grouped(2 * e.s2.groups.size());
-    for (const GemmGroup& g : e.s2.groups) {
-        e.i2.add_group(f * g.c_off, f * g.ldc, g.m, f * g.n);
-        grouped.insert(g.c_off);
-        for (int t = g.t0; t < g.t1; ++t) {
-            const GemmTerm& x = e.s2.terms[t];
-            if (x.k <= 0 || g.m <= 0 || g.n <= 0) continue;
+    // (an output block without a live term is a group too: stage 2 overwrites everything)
+    for_output(e, [&](int64_t off, int m, int n, int t0, int t1) {
+        e.i2.add_group(f * off, f * n, m, f * n);
+        if (m <= 0 || n <= 0) return;
+        for (int i = t0; i < t1; ++i) {
+            const Stage2Term& t = pr.terms[i];
+            const int k = pr.tasks[t.task].n;
+            if (k <= 0) continue;
             if (!z) {
-                e.i2.add_term(mid_img.at(x.a_off), ket_image(ket_a, x.b_off, kImgReal, false, false), x.k, x.scale);
+                e.i2.add_term(mid[t.task], ket_image(ket_a, t.ket, kImgReal, false, false), k, t.w);
                 continue;
             }
-            const size_t pos = (size_t)x.scale - 1;
+            const size_t pos = (size_t)t.w - 1;
             for (int im = 0; im < 2; ++im)
                 if (W[2 * pos + im] != 0.0)
-                    e.i2.add_term(mid_img.at(x.a_off), ket_image(ket_b[im], x.b_off, kImgComplexB, e.side == 1, im != 0),
-                                  2 * x.k, W[2 * pos + im]);
+                    e.i2.add_term(mid[t.task], ket_image(ket_b[im], t.ket, kImgComplexB, e.side == 1, im != 0), 2 * k,
+                                  W[2 * pos + im]);
         }
-    }
-    // output blocks that no term reaches are groups too, so that stage 2 overwrites everything
-    for (size_t o = 0; o < e.out.o.size(); ++o)
-        for (int q = 0; q < e.out.o[o].count(); ++q) {
-            const int64_t off = e.out.base[o] + e.out.o[o].off[q];
-            const int m = e.out.o[o].rows[q], n = e.out.o[o].cols[q];
-            if (m > 0 && n > 0 && !grouped.count(off)) e.i2.add_group(f * off, f * n, m, f * n);
-        }
+    });
     DMRG_TRY(e.img.check_bounds(f * ket.size, f * e.in.size, 0));
-    DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, mid));
-    DMRG_TRY(e.i2.check_bounds(mid, e.img.blocks, f * e.out.size));
-    return e.work.finalize(e.img, e.i1, e.i2, mid, st, e.ctx->num_sms);
+    DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, blocks));
+    DMRG_TRY(e.i2.check_bounds(blocks, e.img.blocks, f * e.out.size));
+    return e.work.finalize(e.img, e.i1, e.i2, blocks, st, e.ctx->num_sms);
 }
 
 int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {
@@ -389,17 +308,10 @@ int create(dmrg_ctx_t ctx, int side, int nl, int nr, const int* phys, const dmrg
     int rc = build_site_desc(e->site, nl, nr, phys, ket, d, lb, rb, W);
     if (rc == DMRG_OK && !e->in.assign(env_in, side == 0 ? lb : rb))
         rc = set_error(DMRG_E_ARG, "invalid input environment");
-    if (rc == DMRG_OK) rc = side == 0 ? build_left(*e) : build_right(*e);
+    if (rc == DMRG_OK) rc = build_products(*e);
     cudaStream_t st = ctx->stream;
-    if (rc == DMRG_OK) rc = e->s1.check_bounds(e->site.ket.size, e->in.size, e->scratch_size);
-    if (rc == DMRG_OK) rc = e->s2.check_bounds(e->scratch_size, e->site.ket.size, e->out.size);
-    if (rc == DMRG_OK && precision == DMRG_PREC_FP64) rc = build_images(*e, st, Wc);
-    if (rc == DMRG_OK && precision != DMRG_PREC_FP64) {
-        const int fmt = precision == DMRG_PREC_BF16X3 ? kFmtBF16 : kFmtTF32;
-        rc = e->scratch.alloc((size_t)std::max<int64_t>(e->scratch_size, 1) * sizeof(double));
-        if (rc == DMRG_OK) rc = e->p1.build(e->s1, fmt, e->site.ket.size, e->in.size, e->scratch_size, st, ctx->num_sms);
-        if (rc == DMRG_OK) rc = e->p2.build(e->s2, fmt, e->scratch_size, e->site.ket.size, e->out.size, st, ctx->num_sms);
-    }
+    if (rc == DMRG_OK) rc = precision == DMRG_PREC_FP64 ? build_images(*e, st, Wc) : build_split(*e, st);
+    e->products = EnvProducts();
     if (rc != DMRG_OK) {
         delete e;
         return rc;

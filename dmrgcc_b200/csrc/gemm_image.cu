@@ -670,19 +670,19 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
     if (num_sms <= 0) num_sms = 148;
     std::vector<ImgTerm> live;  // terms with k-steps, by group
     struct Tile {
-        int group, pm, pn, rows, cols;
-        int64_t steps, cost;  // k-steps; cycles of one
+        int group, t0, t1;      // its group's live terms
+        int pm, pn, rows, cols;
+        int64_t steps, cost;    // k-steps; cycles of one
+        int64_t parts;
     };
     std::vector<Tile> tiles;
-    std::vector<ImgGroup> gr;
     live.reserve(terms.size() + 1);
-    gr.reserve(groups.size());
-    tiles.reserve(groups.size());
+    tiles.reserve(2 * groups.size());
     int64_t cost = 0;
-    for (const ImgGroup& g : groups) {
+    for (int gi = 0; gi < (int)groups.size(); ++gi) {
+        const ImgGroup& g = groups[gi];
         if (g.m <= 0 || g.n <= 0) continue;
-        ImgGroup x = g;
-        x.t0 = (int)live.size();
+        const int t0 = (int)live.size();
         int64_t ks = 0;
         for (int t = g.t0; t < g.t1; ++t)
             if (terms[t].k > 0) {
@@ -690,60 +690,63 @@ void ImgSchedule::plan(int num_sms, Tables& tab) {
                 scaled = scaled || terms[t].scale != 1.0;
                 ks += steps_of(terms[t]);
             }
-        x.t1 = (int)live.size();
         for (int pm = 0; pm * panel < g.m; ++pm)
             for (int pn = 0; pn * panel < g.n; ++pn) {
-                Tile t{(int)gr.size(), pm, pn, std::min(panel, g.m - pm * panel), std::min(panel, g.n - pn * panel), ks, 0};
+                Tile t{gi, t0, (int)live.size(), pm, pn, std::min(panel, g.m - pm * panel), std::min(panel, g.n - pn * panel),
+                       ks, 0, 1};
                 t.cost = step_cost(t.rows, t.cols);
                 cost += ks * t.cost + kTileFixed;
                 tiles.push_back(t);
             }
-        gr.push_back(x);
     }
     // a tile longer than a quarter of a CTA's share is cut into equal parts (a sixth or a
     // tenth: no gain at D=1024)
     const int64_t longest = std::max<int64_t>(1, cost / ((int64_t)num_sms * kCtasPerSm) / 4);
-    std::vector<std::pair<int64_t, int>> order;  // cost, segment
-    order.reserve(tiles.size());
-    segments.reserve(tiles.size());
+    // The queue: largest first, in classes of 1/1024 of the largest (as fast as exactly
+    // sorted; planning is on a sweep's path, and there a sort counts).
+    constexpr int kClasses = 1024;
+    int64_t most = 1;
+    for (Tile& t : tiles) {
+        t.parts = std::max<int64_t>(1, std::min((t.steps * t.cost + longest - 1) / longest, t.steps / kMinPart));
+        most = std::max(most, (t.steps + t.parts - 1) / t.parts * t.cost);
+    }
+    auto first_step = [](const Tile& t, int64_t part) { return t.steps * part / t.parts; };
+    auto class_of = [&](int64_t c) { return (int)((kClasses - 1) - c * (kClasses - 1) / most); };
+    std::vector<int> next(kClasses + 1, 0);  // where a class's next segment goes
+    for (const Tile& t : tiles)
+        for (int64_t k = 0; k < t.parts; ++k) ++next[class_of((first_step(t, k + 1) - first_step(t, k)) * t.cost) + 1];
+    for (int c = 0; c < kClasses; ++c) next[c + 1] += next[c];
+    segments.resize(next[kClasses]);
     for (const Tile& t : tiles) {
-        const ImgGroup& g = gr[t.group];
-        const int64_t c_off = out == kImgOutBlock ? g.c_off + (int64_t)t.pm * panel * g.ldc + t.pn * panel : g.c_off;
-        int64_t parts = std::min((t.steps * t.cost + longest - 1) / longest, t.steps / kMinPart);
-        parts = std::max<int64_t>(parts, 1);
-        if (parts > 1) splits.push_back(GemmSplit{c_off, aux_size, g.ldc, t.rows, t.cols, (int)parts, ntickets++, 0});
-        for (int64_t k = 0; k < parts; ++k) {
-            const int64_t s0 = t.steps * k / parts, s1 = t.steps * (k + 1) / parts;
-            int64_t skip = s0;  // the part's first slice: its term, and the slice in it
-            ImgSegment s{};
-            s.c_off = c_off;
-            s.ldc = g.ldc;
-            s.rows = t.rows;
-            s.cols = t.cols;
-            s.pm = t.pm;
-            s.pn = t.pn;
-            s.steps = (int)(s1 - s0);
-            s.t0 = g.t0;
-            s.t1 = g.t1;
-            while (s.t0 < g.t1 && skip >= steps_of(live[s.t0])) skip -= steps_of(live[s.t0++]);
-            s.k0 = (int)skip;
-            s.split = -1;
-            s.out_kb = (int)img_units(out == kImgOutZB ? 2 * g.m : out == kImgOutB ? g.m : g.n);
-            if (parts > 1) {
-                s.split = (int)splits.size() - 1;
+        const ImgGroup& g = groups[t.group];
+        ImgSegment s{};
+        s.c_off = out == kImgOutBlock ? g.c_off + (int64_t)t.pm * panel * g.ldc + t.pn * panel : g.c_off;
+        s.ldc = g.ldc;
+        s.rows = t.rows;
+        s.cols = t.cols;
+        s.pm = t.pm;
+        s.pn = t.pn;
+        s.t0 = t.t0;
+        s.t1 = t.t1;
+        s.split = -1;
+        s.out_kb = (int)img_units(out == kImgOutZB ? 2 * g.m : out == kImgOutB ? g.m : g.n);
+        if (t.parts > 1) {
+            s.split = (int)splits.size();
+            splits.push_back(GemmSplit{s.c_off, aux_size, g.ldc, t.rows, t.cols, (int)t.parts, ntickets++, 0});
+        }
+        for (int64_t k = 0; k < t.parts; ++k) {
+            s.steps = (int)(first_step(t, k + 1) - first_step(t, k));
+            if (t.parts > 1) {
                 s.aux_off = aux_size;
                 aux_size += (int64_t)((t.rows + 15) / 16) * ((t.cols + 15) / 16) * 2 * kConsumers;
             }
-            order.push_back({s.steps * t.cost, (int)segments.size()});
-            segments.push_back(s);
+            segments[next[class_of(s.steps * t.cost)]++] = s;
+            // the next part's first slice: its term, and the slice in it
+            int64_t skip = s.k0 + (int64_t)s.steps;
+            while (s.t0 < t.t1 && skip >= steps_of(live[s.t0])) skip -= steps_of(live[s.t0++]);
+            s.k0 = (int)skip;
         }
     }
-    // the queue: largest first
-    std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-    std::vector<ImgSegment> queue;
-    queue.reserve(segments.size());
-    for (const auto& o : order) queue.push_back(segments[o.second]);
-    segments.swap(queue);
     ctas = (int)std::min<int64_t>((int64_t)num_sms * kCtasPerSm, (int64_t)segments.size());
     live.push_back(ImgTerm{});  // a group's t1 is readable
     terms_at = tab.add(live);
