@@ -14,13 +14,10 @@
 // In FP64 both run on packed operand images (gemm_image.cu), T included.
 #include <algorithm>
 #include <cstdlib>
-#include <map>
 
 #include "heff.cuh"
 
 using namespace dmrg;
-
-
 
 namespace {
 
@@ -42,6 +39,7 @@ int build_heff(dmrg_heff_s& h) {
 
     struct TermB {
         int out_pos;
+        int l_blk;     // L block, counted over all bond indexes
         int64_t l_off;
         int lda;
         int t_index;
@@ -51,13 +49,31 @@ int build_heff(dmrg_heff_s& h) {
     std::vector<TermB> termsB;
     struct TaskA {
         int pos;       // ket block
-        int64_t r_off; // R block offset
+        int r_blk;     // R block, counted over all bond indexes
+        int64_t r_off;
         int b_l, b_j, a_k;
-        int64_t t_off;
     };
     std::vector<TaskA> tasks;
-    h.t_size = 0;
     double fa_alg = 0, fb = 0, fa_exec = 0;
+    // blocks before each bond index; L blocks by (bond index, sectors), first in list order;
+    // by (o2, p1, p2): the bond indexes o1 with a nonzero weight, ascending
+    std::vector<int> l_first(1, 0), r_first(1, 0), l_at((size_t)s.lb * s.nl * s.nl, -1), o1s, o1s_first(1, 0);
+    for (int o = 0; o < s.lb; ++o) {
+        for (int q = h.L.o[o].count() - 1; q >= 0; --q)
+            l_at[((size_t)o * s.nl + h.L.o[o].left[q]) * s.nl + h.L.o[o].right[q]] = q;
+        l_first.push_back(l_first.back() + h.L.o[o].count());
+    }
+    for (int o = 0; o < s.rb; ++o) r_first.push_back(r_first.back() + h.R.o[o].count());
+    for (int o2 = 0; o2 < s.rb; ++o2)
+        for (int p1 = 0; p1 < s.d; ++p1)
+            for (int p2 = 0; p2 < s.d; ++p2) {
+                for (int o1 = 0; o1 < s.lb; ++o1)
+                    if (s.w(o1, o2, p1, p2) != 0.0) o1s.push_back(o1);
+                o1s_first.push_back((int)o1s.size());
+            }
+    std::vector<char> taken((size_t)s.rb * s.d);
+    for (int o2 = 0; o2 < s.rb; ++o2)
+        for (int p2 = 0; p2 < s.d; ++p2) taken[(size_t)o2 * s.d + p2] = s.right_nonzero(o2, p2);
 
     for (int o2 = 0; o2 < s.rb; ++o2) {
         const BlockListDesc& Ro = h.R.o[o2];
@@ -68,7 +84,7 @@ int build_heff(dmrg_heff_s& h) {
             for (int pos : same_right[ldx]) {
                 const int kdx = ket.left[pos];
                 const int p2 = s.pb(pos);
-                if (!s.right_nonzero(o2, p2)) continue;
+                if (!taken[(size_t)o2 * s.d + p2]) continue;
                 const int a_k = ket.rows[pos], b_l = ket.cols[pos];
                 if (b_l != rr)
                     return set_error(DMRG_E_ARG, "ket block %d is %dx%d but R[%d] block %d is %dx%d", pos, a_k,
@@ -80,10 +96,11 @@ int build_heff(dmrg_heff_s& h) {
                 for (int pos2 : same_right[jdx]) {
                     const int idx = ket.left[pos2];
                     const int p1 = s.pb(pos2);
-                    for (int o1 = 0; o1 < s.lb; ++o1) {
+                    const size_t at = ((size_t)o2 * s.d + p1) * s.d + p2;
+                    for (int x = o1s_first[at]; x < o1s_first[at + 1]; ++x) {
+                        const int o1 = o1s[x];
                         const double w = s.w(o1, o2, p1, p2);
-                        if (w == 0.0) continue;
-                        const int q = h.L.o[o1].find(idx, kdx);
+                        const int q = l_at[((size_t)o1 * s.nl + idx) * s.nl + kdx];
                         if (q == -1) continue;
                         const int lr = h.L.o[o1].rows[q], lc = h.L.o[o1].cols[q];
                         if (lc != a_k || lr != ket.rows[pos2] || rc != ket.cols[pos2])
@@ -91,22 +108,27 @@ int build_heff(dmrg_heff_s& h) {
                                              "shape mismatch: L[%d] block %d %dx%d, K %dx%d, R %dx%d, out %dx%d", o1,
                                              q, lr, lc, a_k, b_l, rr, rc, ket.rows[pos2], ket.cols[pos2]);
                         if (lr == 0) continue;
-                        termsB.push_back(TermB{pos2, h.L.base[o1] + h.L.o[o1].off[q], lc, t_index, a_k, w});
+                        termsB.push_back(TermB{pos2, l_first[o1] + q, h.L.base[o1] + h.L.o[o1].off[q], lc, t_index, a_k, w});
                         fb += 2.0 * lr * lc * rc;
                         used = true;
                     }
                 }
                 if (used) {
-                    tasks.push_back(TaskA{pos, h.R.base[o2] + Ro.off[i], b_l, rc, a_k, h.t_size});
-                    h.t_size += (int64_t)a_k * rc;
+                    tasks.push_back(TaskA{pos, r_first[o2] + i, h.R.base[o2] + Ro.off[i], b_l, rc, a_k});
                     fa_exec += 2.0 * a_k * b_l * rc;
                 }
             }
         }
     }
 
-    std::vector<std::vector<int>> per_out(ket.count());
-    for (int i = 0; i < (int)termsB.size(); ++i) per_out[termsB[i].out_pos].push_back(i);
+    // the terms of output block `pos`: by_out[out_first[pos]] .. by_out[out_first[pos + 1] - 1]
+    std::vector<int> out_first(ket.count() + 1, 0), by_out(termsB.size());
+    for (const TermB& t : termsB) ++out_first[t.out_pos + 1];
+    for (int k = 0; k < ket.count(); ++k) out_first[k + 1] += out_first[k];
+    {
+        std::vector<int> next(out_first.begin(), out_first.end());
+        for (int i = 0; i < (int)termsB.size(); ++i) by_out[next[termsB[i].out_pos]++] = i;
+    }
     h.flops_alg = fa_alg + fb;
     h.flops_exec = fa_exec + fb;
     cudaStream_t st = h.ctx->stream;
@@ -119,8 +141,7 @@ int build_heff(dmrg_heff_s& h) {
         for (int pos = 0; pos < ket.count(); ++pos)
             psi_img[pos] = h.img.add(0, ket.off[pos], ket.rows[pos], ket.cols[pos], ket.cols[pos], false);
         h.img_psi_jobs = (int)h.img.jobs.size();
-        std::map<int64_t, int64_t> r_img, l_img;
-        std::vector<int64_t> t_img(tasks.size());
+        std::vector<int64_t> r_img(r_first.back(), -1), l_img(l_first.back(), -1), t_img(tasks.size());
         int64_t t_blocks = 0;
         h.ia = ImgSchedule();
         h.ib = ImgSchedule();
@@ -128,21 +149,20 @@ int build_heff(dmrg_heff_s& h) {
         h.ia.out = kImgOutB;
         for (size_t i = 0; i < tasks.size(); ++i) {
             const TaskA& t = tasks[i];
-            auto it = r_img.find(t.r_off);
-            if (it == r_img.end()) it = r_img.emplace(t.r_off, h.img.add(2, t.r_off, t.b_j, t.b_l, t.b_j, true)).first;
+            int64_t& r = r_img[t.r_blk];
+            if (r < 0) r = h.img.add(2, t.r_off, t.b_j, t.b_l, t.b_j, true);
             t_img[i] = t_blocks;
             t_blocks += img_blocks(t.b_j, t.a_k);
             h.ia.add_group(t_img[i], 0, t.a_k, t.b_j);
-            h.ia.add_term(psi_img[t.pos], it->second, t.b_l, 1.0);
+            h.ia.add_term(psi_img[t.pos], r, t.b_l, 1.0);
         }
         for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
             h.ib.add_group(ket.off[pos2], ket.cols[pos2], ket.rows[pos2], ket.cols[pos2]);
-            for (int i : per_out[pos2]) {
-                const TermB& t = termsB[i];
-                auto it = l_img.find(t.l_off);
-                if (it == l_img.end())
-                    it = l_img.emplace(t.l_off, h.img.add(1, t.l_off, ket.rows[pos2], t.k, t.lda, false)).first;
-                h.ib.add_term(it->second, t_img[t.t_index], t.k, t.w);
+            for (int i = out_first[pos2]; i < out_first[pos2 + 1]; ++i) {
+                const TermB& t = termsB[by_out[i]];
+                int64_t& l = l_img[t.l_blk];
+                if (l < 0) l = h.img.add(1, t.l_off, ket.rows[pos2], t.k, t.lda, false);
+                h.ib.add_term(l, t_img[t.t_index], t.k, t.w);
             }
         }
         DMRG_TRY(h.img.check_bounds(ket.size, h.L.size, h.R.size));
@@ -158,7 +178,7 @@ int build_heff(dmrg_heff_s& h) {
         std::vector<int64_t> psi_img(ket.count());
         for (int pos = 0; pos < ket.count(); ++pos)
             psi_img[pos] = h.pk_psi.add(ket.off[pos], ket.rows[pos], ket.cols[pos], ket.cols[pos], false);
-        std::map<int64_t, int64_t> r_img, l_img;
+        std::vector<int64_t> r_img(r_first.back(), -1), l_img(l_first.back(), -1);
         const int tk = pack_k(fmt);
         auto slices = [tk](int k) { return (k + tk - 1) / tk; };
         std::vector<int64_t> t_img(tasks.size());
@@ -167,9 +187,8 @@ int build_heff(dmrg_heff_s& h) {
         h.t_img_bytes = 0;
         for (size_t i = 0; i < tasks.size(); ++i) {
             const TaskA& t = tasks[i];
-            auto it = r_img.find(t.r_off);
-            if (it == r_img.end())
-                it = r_img.emplace(t.r_off, h.pk_R.add(t.r_off, t.b_j, t.b_l, t.b_j, true)).first;
+            int64_t& r = r_img[t.r_blk];
+            if (r < 0) r = h.pk_R.add(t.r_off, t.b_j, t.b_l, t.b_j, true);
             t_img[i] = h.t_img_bytes;
             h.t_img_bytes += image_bytes(t.b_j, slices(t.a_k));
             PackedGroup g{};
@@ -178,26 +197,25 @@ int build_heff(dmrg_heff_s& h) {
             g.n = t.a_k;
             g.t_img = t_img[i];
             g.t_slices = slices(t.a_k);
-            h.pa.terms.push_back(PackedTerm{it->second, psi_img[t.pos], slices(t.b_l), 0, 1.0});
+            h.pa.terms.push_back(PackedTerm{r, psi_img[t.pos], slices(t.b_l), 0, 1.0});
             g.t1 = (int)h.pa.terms.size();
             h.pa.groups.push_back(g);
         }
         h.pb.reset();
         h.pb.out_mode = 0;
         for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
-            if (per_out[pos2].empty()) continue;
+            if (out_first[pos2] == out_first[pos2 + 1]) continue;
             PackedGroup g{};
             g.t0 = (int)h.pb.terms.size();
             g.m = ket.rows[pos2];
             g.n = ket.cols[pos2];
             g.c_off = ket.off[pos2];
             g.ldc = ket.cols[pos2];
-            for (int i : per_out[pos2]) {
-                const TermB& t = termsB[i];
-                auto it = l_img.find(t.l_off);
-                if (it == l_img.end())
-                    it = l_img.emplace(t.l_off, h.pk_L.add(t.l_off, ket.rows[pos2], t.k, t.lda, false)).first;
-                h.pb.terms.push_back(PackedTerm{it->second, t_img[t.t_index], slices(t.k), 0, t.w});
+            for (int i = out_first[pos2]; i < out_first[pos2 + 1]; ++i) {
+                const TermB& t = termsB[by_out[i]];
+                int64_t& l = l_img[t.l_blk];
+                if (l < 0) l = h.pk_L.add(t.l_off, ket.rows[pos2], t.k, t.lda, false);
+                h.pb.terms.push_back(PackedTerm{l, t_img[t.t_index], slices(t.k), 0, t.w});
             }
             g.t1 = (int)h.pb.terms.size();
             h.pb.groups.push_back(g);

@@ -28,7 +28,6 @@ struct dmrg_heff_s {
     dmrg::PackedSchedule pa, pb;               // A: psi x R -> T images ; B: L x T -> out
     dmrg::DeviceBuffer img_psi, img_L, img_R, img_T;
     int64_t t_img_bytes = 0;
-    int64_t t_size = 0;
     const double* L_dev = nullptr;
     const double* R_dev = nullptr;
     double flops_alg = 0, flops_exec = 0;
