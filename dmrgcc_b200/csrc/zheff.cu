@@ -16,7 +16,6 @@
 // eigenvector (x, y) gives the complex ground state x + i y.
 #include <algorithm>
 #include <cmath>
-#include <map>
 
 #include "blocksparse.h"
 #include "eig.cuh"
@@ -77,18 +76,38 @@ int build_zheff(dmrg_zheff_s& h) {
     };
     struct TermB {
         int out_pos;
+        int l_blk;  // L block, counted over all bond indexes
         int64_t l_off;
         int lda, t_index, k;
         double wr, wi;
     };
     struct TaskA {
         int pos;
+        int r_blk;  // R block, counted over all bond indexes
         int64_t r_off;
         int b_l, b_j, a_k;
     };
     std::vector<TermB> termsB;
     std::vector<TaskA> tasks;
     double fl = 0;
+    // tables as in heff.cu
+    std::vector<int> l_first(1, 0), r_first(1, 0), l_at((size_t)s.lb * s.nl * s.nl, -1), o1s, o1s_first(1, 0);
+    for (int o = 0; o < s.lb; ++o) {
+        for (int q = h.L.o[o].count() - 1; q >= 0; --q)
+            l_at[((size_t)o * s.nl + h.L.o[o].left[q]) * s.nl + h.L.o[o].right[q]] = q;
+        l_first.push_back(l_first.back() + h.L.o[o].count());
+    }
+    for (int o = 0; o < s.rb; ++o) r_first.push_back(r_first.back() + h.R.o[o].count());
+    std::vector<char> taken((size_t)s.rb * s.d);
+    for (int o2 = 0; o2 < s.rb; ++o2) {
+        for (int p1 = 0; p1 < s.d; ++p1)
+            for (int p2 = 0; p2 < s.d; ++p2) {
+                for (int o1 = 0; o1 < s.lb; ++o1)
+                    if (wre(h.Wc, s, o1, o2, p1, p2) != 0.0 || wim(h.Wc, s, o1, o2, p1, p2) != 0.0) o1s.push_back(o1);
+                o1s_first.push_back((int)o1s.size());
+            }
+        for (int p2 = 0; p2 < s.d; ++p2) taken[(size_t)o2 * s.d + p2] = right_nonzero(o2, p2);
+    }
     for (int o2 = 0; o2 < s.rb; ++o2) {
         const BlockListDesc& Ro = h.R.o[o2];
         for (int i = 0; i < Ro.count(); ++i) {
@@ -97,7 +116,7 @@ int build_zheff(dmrg_zheff_s& h) {
             for (int pos : same_right[ldx]) {
                 const int kdx = ket.left[pos];
                 const int p2 = s.pb(pos);
-                if (!right_nonzero(o2, p2)) continue;
+                if (!taken[(size_t)o2 * s.d + p2]) continue;
                 const int a_k = ket.rows[pos], b_l = ket.cols[pos];
                 if (b_l != rr)
                     return set_error(DMRG_E_ARG, "ket block %d is %dx%d but R[%d] block %d is %dx%d", pos, a_k, b_l, o2,
@@ -109,22 +128,23 @@ int build_zheff(dmrg_zheff_s& h) {
                 for (int pos2 : same_right[jdx]) {
                     const int idx = ket.left[pos2];
                     const int p1 = s.pb(pos2);
-                    for (int o1 = 0; o1 < s.lb; ++o1) {
+                    const size_t at = ((size_t)o2 * s.d + p1) * s.d + p2;
+                    for (int x = o1s_first[at]; x < o1s_first[at + 1]; ++x) {
+                        const int o1 = o1s[x];
                         const double wr = wre(h.Wc, s, o1, o2, p1, p2), wi = wim(h.Wc, s, o1, o2, p1, p2);
-                        if (wr == 0.0 && wi == 0.0) continue;
-                        const int q = h.L.o[o1].find(idx, kdx);
+                        const int q = l_at[((size_t)o1 * s.nl + idx) * s.nl + kdx];
                         if (q == -1) continue;
                         const int lr = h.L.o[o1].rows[q], lc = h.L.o[o1].cols[q];
                         if (lc != a_k || lr != ket.rows[pos2] || rc != ket.cols[pos2])
                             return set_error(DMRG_E_ARG, "shape mismatch in the complex H_eff at L[%d] block %d", o1, q);
                         if (lr == 0) continue;
-                        termsB.push_back(TermB{pos2, h.L.base[o1] + h.L.o[o1].off[q], lc, t_index, a_k, wr, wi});
+                        termsB.push_back(TermB{pos2, l_first[o1] + q, h.L.base[o1] + h.L.o[o1].off[q], lc, t_index, a_k, wr, wi});
                         fl += 8.0 * lr * lc * rc;
                         used = true;
                     }
                 }
                 if (used) {
-                    tasks.push_back(TaskA{pos, h.R.base[o2] + Ro.off[i], b_l, rc, a_k});
+                    tasks.push_back(TaskA{pos, r_first[o2] + i, h.R.base[o2] + Ro.off[i], b_l, rc, a_k});
                 }
             }
         }
@@ -138,8 +158,8 @@ int build_zheff(dmrg_zheff_s& h) {
         psi_img[pos] = h.img.add_complex(0, ket.off[pos], ket.rows[pos], ket.cols[pos], ket.cols[pos], false, kImgComplexA,
                                          false, false);
     h.img_psi_jobs = (int)h.img.jobs.size();
-    std::map<int64_t, int64_t> r_img, l_img[2];  // [1]: i L
-    std::vector<int64_t> t_img(tasks.size());
+    std::vector<int64_t> r_img(r_first.back(), -1), l_img[2], t_img(tasks.size());  // l_img[1]: i L
+    for (auto& l : l_img) l.assign(l_first.back(), -1);
     int64_t t_blocks = 0;
     h.ia = ImgSchedule();
     h.ib = ImgSchedule();
@@ -147,29 +167,30 @@ int build_zheff(dmrg_zheff_s& h) {
     h.ia.out = kImgOutZB;
     for (size_t i = 0; i < tasks.size(); ++i) {
         const TaskA& t = tasks[i];
-        auto it = r_img.find(t.r_off);
-        if (it == r_img.end())
-            it = r_img.emplace(t.r_off, h.img.add_complex(2, t.r_off, t.b_j, t.b_l, t.b_j, true, kImgComplexB, false, false))
-                     .first;
+        int64_t& r = r_img[t.r_blk];
+        if (r < 0) r = h.img.add_complex(2, t.r_off, t.b_j, t.b_l, t.b_j, true, kImgComplexB, false, false);
         t_img[i] = t_blocks;
         t_blocks += img_blocks(2 * t.b_j, 2 * t.a_k);
         h.ia.add_group(t_img[i], 0, t.a_k, 2 * t.b_j);
-        h.ia.add_term(psi_img[t.pos], it->second, 2 * t.b_l, 1.0);
+        h.ia.add_term(psi_img[t.pos], r, 2 * t.b_l, 1.0);
     }
-    std::vector<std::vector<int>> per_out(ket.count());
-    for (int i = 0; i < (int)termsB.size(); ++i) per_out[termsB[i].out_pos].push_back(i);
+    std::vector<int> out_first(ket.count() + 1, 0), by_out(termsB.size());
+    for (const TermB& t : termsB) ++out_first[t.out_pos + 1];
+    for (int k = 0; k < ket.count(); ++k) out_first[k + 1] += out_first[k];
+    {
+        std::vector<int> next(out_first.begin(), out_first.end());
+        for (int i = 0; i < (int)termsB.size(); ++i) by_out[next[termsB[i].out_pos]++] = i;
+    }
     for (int pos2 = 0; pos2 < ket.count(); ++pos2) {
         h.ib.add_group(2 * ket.off[pos2], 2 * ket.cols[pos2], ket.rows[pos2], 2 * ket.cols[pos2]);
-        for (int i : per_out[pos2]) {
-            const TermB& t = termsB[i];
+        for (int i = out_first[pos2]; i < out_first[pos2 + 1]; ++i) {
+            const TermB& t = termsB[by_out[i]];
             const double w[2] = {t.wr, t.wi};
             for (int im = 0; im < 2; ++im) {
                 if (w[im] == 0.0) continue;
-                auto it = l_img[im].find(t.l_off);
-                if (it == l_img[im].end())
-                    it = l_img[im].emplace(t.l_off, h.img.add_complex(1, t.l_off, ket.rows[pos2], t.k, t.lda, false,
-                                                                      kImgComplexA, false, im != 0)).first;
-                h.ib.add_term(it->second, t_img[t.t_index], 2 * t.k, w[im]);
+                int64_t& l = l_img[im][t.l_blk];
+                if (l < 0) l = h.img.add_complex(1, t.l_off, ket.rows[pos2], t.k, t.lda, false, kImgComplexA, false, im != 0);
+                h.ib.add_term(l, t_img[t.t_index], 2 * t.k, w[im]);
             }
         }
     }
