@@ -282,7 +282,8 @@ int build_images(dmrg_env_s& e, cudaStream_t st, const double* W) {
     DMRG_TRY(e.img.check_bounds(f * ket.size, f * e.in.size, 0));
     DMRG_TRY(e.i1.check_bounds(e.img.blocks, e.img.blocks, blocks));
     DMRG_TRY(e.i2.check_bounds(blocks, e.img.blocks, f * e.out.size));
-    return e.work.finalize(e.img, e.i1, e.i2, blocks, st, e.ctx->num_sms);
+    DMRG_TRY(e.work.finalize(e.img, e.i1, e.i2, blocks, st, e.ctx->num_sms));
+    return e.work.allocate(e.i1, e.i2);
 }
 
 int run_images(dmrg_env_s& e, const double* ket_dev, const double* env_in_dev, double* env_out_dev) {

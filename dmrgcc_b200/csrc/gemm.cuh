@@ -234,15 +234,17 @@ struct ImgSchedule {
     // accumulate writes zeros.
     void plan(int num_sms, Tables& tab);
 };
-// The device memory of a two-stage product: the tables in one upload; in one
+// The device memory of a two-stage product: the tables in one upload (finalize); in one
 // allocation the operand images, the first stage's output images, the aux buffers of
-// both schedules.
+// both schedules (allocate, once).
 struct ImgWork {
     DeviceBuffer d_tables, buf;
     double *img = nullptr, *mid = nullptr;
+    int64_t img_size = 0, mid_size = 0;  // doubles
     unsigned* tickets = nullptr;  // the counters of both schedules
     int ntickets = 0;
     int finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_blocks, cudaStream_t stream, int num_sms);
+    int allocate(ImgSchedule& a, ImgSchedule& b);
 };
 // Packs the jobs of chunks [c0, c1) from the three sources into the images, and zeroes
 // the counters: one such launch goes ahead of every application's products.

@@ -767,10 +767,17 @@ int ImgWork::finalize(ImgPack& p, ImgSchedule& a, ImgSchedule& b, int64_t mid_bl
     p.tables = a.tables = b.tables = d_tables.as<char>();
     tickets = a.tickets = reinterpret_cast<unsigned*>(d_tables.as<char>() + tickets_at);
     b.tickets = a.tickets + 1 + a.ntickets;
-    const int64_t n = (p.blocks + mid_blocks) * kImgBlock;
+    img_size = p.blocks * kImgBlock;
+    mid_size = mid_blocks * kImgBlock;
+    return DMRG_OK;
+}
+
+int ImgWork::allocate(ImgSchedule& a, ImgSchedule& b) {
+    if (img) return DMRG_OK;
+    const int64_t n = img_size + mid_size;
     DMRG_TRY(buf.alloc((size_t)std::max<int64_t>(n + a.aux_size + b.aux_size, 1) * sizeof(double)));
     img = buf.as<double>();
-    mid = img + p.blocks * kImgBlock;
+    mid = img + img_size;
     a.aux = img + n;
     b.aux = a.aux + a.aux_size;
     return DMRG_OK;

@@ -169,6 +169,8 @@ int build_heff(dmrg_heff_s& h) {
         DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
         DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, ket.size));
         DMRG_TRY(h.work.finalize(h.img, h.ia, h.ib, t_blocks, st, h.ctx->num_sms));
+        // (a split operator's FP64 images: with its first FP64 solve, heff_pack_env)
+        if (!is_split(h.precision)) DMRG_TRY(h.work.allocate(h.ia, h.ib));
     }
     if (is_split(h.precision)) {
         const int fmt = split_fmt(h.precision);
@@ -250,6 +252,7 @@ static int pack_operands(dmrg_heff_s& h, const double* psi, bool env_packed) {
 int dmrg::heff_pack_env(dmrg_heff_s& h) {
     if ((!h.L_dev && h.L.size) || (!h.R_dev && h.R.size))
         return set_error(DMRG_E_STATE, "dmrg_heff_set_env was not called");
+    DMRG_TRY(h.work.allocate(h.ia, h.ib));
     return launch_img_pack(h.img, h.work, h.ia.panel, h.img.first_chunk[h.img_psi_jobs], (int)h.img.chunks.size(), nullptr,
                            h.L_dev, h.R_dev, h.ctx->stream);
 }

@@ -16,7 +16,7 @@ struct dmrg_heff_s {
     bool use_graph = true;            // Lanczos loop as one captured CUDA graph (dmrg_heff_set_graph)
     dmrg::SiteDesc site;
     dmrg::EnvDesc L, R;
-    // FP64: operand images (jobs psi, then L and R), A: psi x R -> T images, B: L x T -> out
+    // FP64 (a split operator's last phase too): operand images (jobs psi, then L and R), A: psi x R -> T images, B: L x T -> out
     dmrg::ImgPack img;
     int img_psi_jobs = 0;
     dmrg::ImgSchedule ia, ib;

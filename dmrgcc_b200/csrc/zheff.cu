@@ -198,7 +198,8 @@ int build_zheff(dmrg_zheff_s& h) {
     DMRG_TRY(h.ia.check_bounds(h.img.blocks, h.img.blocks, t_blocks));
     DMRG_TRY(h.ib.check_bounds(h.img.blocks, t_blocks, 2 * ket.size));
     cudaStream_t st = h.ctx->stream;
-    return h.work.finalize(h.img, h.ia, h.ib, t_blocks, st, h.ctx->num_sms);
+    DMRG_TRY(h.work.finalize(h.img, h.ia, h.ib, t_blocks, st, h.ctx->num_sms));
+    return h.work.allocate(h.ia, h.ib);
 }
 
 // out (+)= H psi; the environments are packed anew unless env_packed (zpack_env was

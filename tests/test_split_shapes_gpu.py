@@ -42,3 +42,21 @@ def test_split_heff_tiles(ctx, m, n, bond, accumulate, precision, bits):
     got = out.download().reshape(m, n) - (start if accumulate else 0.0)
     assert np.all(np.abs(got - want) <= rel * mag + 4 * np.finfo(float).eps * np.abs(start))
     h.close()
+
+
+def test_split_operator_memory(ctx):
+    """A split operator that only applies holds the split images (hi and lo, 8 bytes an
+    element in TF32X3) and no FP64 ones beside them; its dense or FP64 solve makes those."""
+    torch = pytest.importorskip("torch")
+    m, n, bond = 1500, 1400, 8
+    W = np.ones((bond, bond, 1, 1))
+    site = capi.SiteProblem(1, 1, np.zeros((1, 1)), capi.BlockSpec([0], [0], [m], [n]), W)
+    L, R = ([capi.BlockSpec([0], [0], [k], [k])] * bond for k in (m, n))
+    ctx.sync()
+    free = torch.cuda.mem_get_info()[0]
+    h = capi.Heff(ctx, site, L, R, capi.DMRG_PREC_TF32X3)
+    used = free - torch.cuda.mem_get_info()[0]
+    h.close()
+    elements = bond * (m * m + n * n) + (bond + 1) * m * n  # environments, products, psi
+    # rows in panels of 128 rounded to 8, k to 16; the sums of cut tiles; allocation granularity
+    assert used <= 1.5 * 8 * elements + (64 << 20), used
