@@ -103,6 +103,7 @@ _SIGS = {
     "dmrg_zcanon_out_blocks": (C.c_int, [_VP, _I, _I, _I, _I, _I]),
     "dmrg_zcanon_singular_values": (C.c_int, [_VP, C.c_int, C.c_int, _D, _I]),
     "dmrg_zcanon_write": (C.c_int, [_VP, _VP, _VP, _VP]),
+    "dmrg_svd_solve_groups": (C.c_int, [_I]),
     "dmrg_svd_pair_schedule": (C.c_int, [C.POINTER(C.c_uint)]),
     "dmrg_svd_plan_rounds": (C.c_int, [C.c_int, C.POINTER(C.c_double), C.c_double, C.c_int, C.POINTER(C.c_int),
                                        C.POINTER(C.c_int), C.POINTER(C.c_int)]),
@@ -575,8 +576,16 @@ def svd_plan_rounds(cols: int, bm, tol: float):
     return rounds
 
 
+def svd_solve_groups() -> np.ndarray:
+    """The Jacobi pair solve's order: the columns [21 steps, 16 groups, 4]."""
+    out = np.empty((21, 16, 4), np.int32)
+    check(lib().dmrg_svd_solve_groups(_iptr(out)), "dmrg_svd_solve_groups")
+    return out
+
+
 def svd_pair_schedule() -> np.ndarray:
-    """The Jacobi pair solve's rotation schedule, [63 steps, 32 lanes] of
+    """A circle schedule of 64 columns in pairs (the pair solve's own order is
+    svd_solve_groups), [63 steps, 32 lanes] of
     a | b << 6 | flip << 12 | seat lane << 13 | seat flip << 18 (host data; no
     GPU needed)."""
     out = np.zeros(63 * 32, dtype=np.uint32)

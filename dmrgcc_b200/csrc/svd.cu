@@ -73,8 +73,8 @@ struct QuadClass {
     __host__ __device__ int base(int g) const { return g | (c < 16 ? 0 : c < 20 ? g >> 2 : g & 3) << 4; }
 };
 
-// Seating of the columns in the circle schedule (the circle method of a round-robin
-// tournament): at step r, seat 0 holds column 0 and seat s >= 1 holds column
+// Seating of the columns in the circle schedule that dmrg_svd_pair_schedule reports and
+// no kernel reads (the circle method of a round-robin tournament): at step r, seat 0 holds column 0 and seat s >= 1 holds column
 // ((s - 1 - r) mod 63) + 1; seat lane j owns seats j and 63 - j, whose columns
 // are the pair rotated at that step.  From one step to the next the column in
 // seat s moves to seat s + 1 (seat 63 to seat 1; seat 0 stays), so a lane's two
@@ -1261,6 +1261,16 @@ extern "C" int dmrg_svd_plan_rounds(int cols, const double* bm, double tol, int 
     *n_pairs = k;
     *n_rounds = (int)rounds.size();
     return k <= cap ? DMRG_OK : dmrg::set_error(DMRG_E_ARG, "%d pairs, room for %d", k, cap);
+}
+
+extern "C" int dmrg_svd_solve_groups(int* out) {
+    if (!out) return dmrg::set_error(DMRG_E_ARG, "null argument");
+    for (int c = 0; c < dmrg::kClasses; ++c) {
+        const dmrg::QuadClass qc(c);
+        for (int g = 0; g < dmrg::kQuads; ++g)
+            for (int a = 0; a < 4; ++a) *out++ = qc.base(g) ^ qc.shift[a];
+    }
+    return DMRG_OK;
 }
 
 extern "C" int dmrg_svd_pair_schedule(unsigned int* out) {

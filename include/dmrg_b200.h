@@ -320,7 +320,14 @@ int dmrg_canon_out_blocks(dmrg_canon_t c, int* ket_rows, int* ket_cols, int* can
                           int* canon_cols, int* match_dim);
 int dmrg_canon_singular_values(dmrg_canon_t c, int sector, int cap, double* values, int* count);
 int dmrg_canon_write(dmrg_canon_t c, const double* ket_dev, double* new_ket_dev, double* canonical_dev);
-/* The Jacobi pair solve's rotation schedule (diagnostic; no reference
+/* The order in which the Jacobi pair solve rotates a pair's 64 columns (diagnostic;
+ * no reference counterpart): out[21 * 16 * 4], the four columns of group g of step c
+ * at out[(16 c + g) * 4].  A step's 16 groups partition the columns and are rotated at
+ * once, each through its six pairs; every two columns share one group; the columns at
+ * the same place of the 16 groups are distinct mod 16 (shared-memory banks). */
+int dmrg_svd_solve_groups(int* out);
+/* A circle schedule of 64 columns in pairs, 63 steps (diagnostic; the pair solve's
+ * order before dmrg_svd_solve_groups', which no kernel reads now; no reference
  * counterpart): out[63 * 32], entry (step r, lane) = a | b << 6 | flip << 12 |
  * j << 13 | jflip << 18 with (a, b), a < b, the pair of the pair's 64 columns
  * that the lane rotates in step r, flip = the lane addresses b first, j = the
