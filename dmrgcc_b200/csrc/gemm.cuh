@@ -1,5 +1,6 @@
-// Grouped multi-term block GEMM: the one contraction engine behind H_eff*psi,
-// the environment updates and the merge.
+// Grouped multi-term block GEMMs: on packed operand images (H_eff*psi, environment
+// updates), in split precision on the tensor cores, and, first, on the operands where
+// they lie (merges, expansion, orthonormalisation).
 //
 // A launch processes a list of output blocks ("groups").  Group g owns a
 // row-major m x n block C_g at C + c_off (leading dimension ldc) and a range of
@@ -296,10 +297,7 @@ struct PackJob {
     int64_t img_off;  // bytes, into the image buffer
     int rows, k, ld;  // logical X: rows x k; X(r, c) = src[src_off + (trans ? c*ld + r : r*ld + c)]
     int trans;
-    int prow_;
     int slices;       // ceil(k / pack_k(fmt))
-    int fmt;          // kFmtTF32 or kFmtBF16
-    int pad_;
 };
 struct PackImage {
     int job, panel, slice, pad_;

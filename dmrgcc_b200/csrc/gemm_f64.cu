@@ -39,18 +39,16 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
                  : "d"(a), "d"(b));
 }
 
-template <bool TA, bool TB>
+template <bool TB>
 __device__ __forceinline__ void load_stage(double* As, double* Bs, const double* __restrict__ A,
                                            const double* __restrict__ B, const GemmTerm& t, int k0,
                                            int m0, int n0, int m, int n, int tid) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int idx = tid + NT * i;
-        const int r = TA ? (idx & 63) : (idx >> 4);
-        const int c = TA ? (idx >> 6) : (idx & 15);
+        const int r = idx >> 4, c = idx & 15;
         const bool v = (m0 + r < m) && (k0 + c < t.k);
-        const int64_t off = TA ? (int64_t)(k0 + c) * t.lda + (m0 + r) : (int64_t)(m0 + r) * t.lda + (k0 + c);
-        cp_async8(TA ? (As + c * SB + r) : (As + r * SA + c), v ? (A + t.a_off + off) : A, v);
+        cp_async8(As + r * SA + c, v ? (A + t.a_off + (int64_t)(m0 + r) * t.lda + (k0 + c)) : A, v);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -63,7 +61,7 @@ __device__ __forceinline__ void load_stage(double* As, double* Bs, const double*
     }
 }
 
-template <bool TA, bool TB>
+template <bool TB>
 __device__ __forceinline__ void compute_stage(const double* As, const double* Bs, double (&acc)[4][4][2],
                                               double scale, int wm, int wn, int lane) {
     const int fr = lane >> 2, fc = lane & 3;
@@ -73,7 +71,7 @@ __device__ __forceinline__ void compute_stage(const double* As, const double* Bs
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = wm * 32 + i * 8 + fr, col = kk + fc;
-            a[i] = (TA ? As[col * SB + row] : As[row * SA + col]) * scale;
+            a[i] = As[row * SA + col] * scale;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -87,7 +85,7 @@ __device__ __forceinline__ void compute_stage(const double* As, const double* Bs
     }
 }
 
-template <bool TA, bool TB>
+template <bool TB>
 __global__ void __launch_bounds__(NT) gemm_f64_kernel(const double* __restrict__ A, const double* __restrict__ B,
                                                       double* __restrict__ C, double* __restrict__ Caux,
                                                       const GemmTerm* __restrict__ terms,
@@ -110,7 +108,7 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const double* __restrict__
         GemmTerm cur = terms[t];
         int k0 = 0, stage = 0;
         double sc_cur = cur.scale;
-        load_stage<TA, TB>(smA[0], smB[0], A, B, cur, 0, tile.m0, tile.n0, g.m, g.n, tid);
+        load_stage<TB>(smA[0], smB[0], A, B, cur, 0, tile.m0, tile.n0, g.m, g.n, tid);
         cp_async_commit();
         for (;;) {
             int nk0 = k0 + BK, nt = t;
@@ -123,7 +121,7 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const double* __restrict__
             const bool has_next = nt < g.t1;
             double sc_nxt = nxt.scale;
             if (has_next) {
-                load_stage<TA, TB>(smA[stage ^ 1], smB[stage ^ 1], A, B, nxt, nk0, tile.m0, tile.n0, g.m, g.n,
+                load_stage<TB>(smA[stage ^ 1], smB[stage ^ 1], A, B, nxt, nk0, tile.m0, tile.n0, g.m, g.n,
                                    tid);
                 cp_async_commit();
                 cp_async_wait<1>();
@@ -131,7 +129,7 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const double* __restrict__
                 cp_async_wait<0>();
             }
             __syncthreads();
-            compute_stage<TA, TB>(smA[stage], smB[stage], acc, sc_cur, wm, wn, lane);
+            compute_stage<TB>(smA[stage], smB[stage], acc, sc_cur, wm, wn, lane);
             __syncthreads();
             if (!has_next) break;
             stage ^= 1;
@@ -268,10 +266,9 @@ int launch_gemm_f64(const GemmSchedule& s, const double* A, const double* B, dou
     const auto* tl = s.d_tiles.as<GemmTile>();
     const int acc = accumulate ? 1 : 0;
     double* X = s.aux.as<double>();
-    if (!s.ta && !s.tb) DMRG_LAUNCH gemm_f64_kernel<false, false><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
-    else if (s.ta && !s.tb) DMRG_LAUNCH gemm_f64_kernel<true, false><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
-    else if (!s.ta && s.tb) DMRG_LAUNCH gemm_f64_kernel<false, true><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
-    else DMRG_LAUNCH gemm_f64_kernel<true, true><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
+    if (s.ta) return set_error(DMRG_E_STATE, "raw-operand products take no transposed A");
+    if (s.tb) DMRG_LAUNCH gemm_f64_kernel<true><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
+    else DMRG_LAUNCH gemm_f64_kernel<false><<<n, NT, 0, stream>>>(A, B, C, X, tr, gr, tl, acc);
     if (!s.splits.empty()) {
         int64_t biggest = 0;
         for (const GemmSplit& sp : s.splits) biggest = std::max<int64_t>(biggest, (int64_t)sp.m * sp.n);
@@ -284,16 +281,11 @@ int launch_gemm_f64(const GemmSchedule& s, const double* A, const double* B, dou
 }
 
 int launch_gemm_f64_tables(const GemmTerm* terms, const GemmGroup* groups, const GemmTile* tiles, int ntiles,
-                           bool ta, bool tb, const double* A, const double* B, double* C, bool accumulate,
-                           cudaStream_t stream) {
+                           const double* A, const double* B, double* C, bool accumulate, cudaStream_t stream) {
     // Same kernel as launch_gemm_f64, with device tables supplied by the caller
     // (no split-K groups: every group writes C directly).
     if (ntiles <= 0) return DMRG_OK;
-    const int acc = accumulate ? 1 : 0;
-    if (!ta && !tb) DMRG_LAUNCH gemm_f64_kernel<false, false><<<ntiles, NT, 0, stream>>>(A, B, C, nullptr, terms, groups, tiles, acc);
-    else if (ta && !tb) DMRG_LAUNCH gemm_f64_kernel<true, false><<<ntiles, NT, 0, stream>>>(A, B, C, nullptr, terms, groups, tiles, acc);
-    else if (!ta && tb) DMRG_LAUNCH gemm_f64_kernel<false, true><<<ntiles, NT, 0, stream>>>(A, B, C, nullptr, terms, groups, tiles, acc);
-    else DMRG_LAUNCH gemm_f64_kernel<true, true><<<ntiles, NT, 0, stream>>>(A, B, C, nullptr, terms, groups, tiles, acc);
+    DMRG_LAUNCH gemm_f64_kernel<false><<<ntiles, NT, 0, stream>>>(A, B, C, nullptr, terms, groups, tiles, accumulate ? 1 : 0);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }

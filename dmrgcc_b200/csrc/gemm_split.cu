@@ -67,14 +67,13 @@ constexpr int NEPI = DMRG_SPLIT_EPILOGUE_WARPS;              // epilogue warps: 
 constexpr int NT = 32 * (2 + NEPI);
 constexpr int ECOLS = TN * 4 / NEPI;                         // accumulator columns per epilogue warp
 // Epilogue staging per epilogue warp, 4 KB: 32 output rows x 16 doubles (16
-// columns at a time), or one plane of the warp's share of one slice of an output
-// image (ECOLS image rows x 64 bytes of k).
+// columns at a time); not used where the output is images.
 constexpr int EPI_OFF = NSTAGE * STAGE_BYTES;
 constexpr int EPI_WARP_BYTES = 4096;
 constexpr int BAR_OFF = EPI_OFF + NEPI * EPI_WARP_BYTES;
 constexpr int SMEM_BYTES = BAR_OFF + 256;
 static_assert(NEPI % 4 == 0 && ECOLS % 16 == 0 && ECOLS * NEPI == 4 * TN && TM == 128, "epilogue geometry");
-static_assert(EPI_WARP_BYTES >= 32 * 16 * 8 && EPI_WARP_BYTES >= ECOLS * kPackRowBytes, "staging sizes");
+static_assert(EPI_WARP_BYTES >= 32 * 16 * 8, "staging size");
 constexpr uint32_t TMEM_COLS = 2 * TN;                       // two 128-column accumulators
 constexpr long long kWaitLimit = 4000000;                    // try_wait polls before a wait gives up
 
@@ -572,7 +571,6 @@ __global__ void __launch_bounds__(256) split_reduce_tf32_kernel(double* __restri
 int64_t PackSchedule::add(int64_t src_off, int rows, int k, int ld, bool trans) {
     const int tk = pack_k(fmt);
     PackJob j{};
-    j.fmt = fmt;
     j.src_off = src_off;
     j.img_off = bytes;
     j.rows = rows;

@@ -35,8 +35,7 @@
 
 namespace dmrg {
 int launch_gemm_f64_tables(const GemmTerm* terms, const GemmGroup* groups, const GemmTile* tiles, int ntiles,
-                           bool ta, bool tb, const double* A, const double* B, double* C, bool accumulate,
-                           cudaStream_t st);
+                           const double* A, const double* B, double* C, bool accumulate, cudaStream_t st);
 }
 
 using namespace dmrg;
@@ -360,12 +359,12 @@ extern "C" int dmrg_heff_apply_noalloc(int nl, int nr, const int* phys, const dm
     double* T = reinterpret_cast<double*>(scratch + offT);
     DMRG_TRY(launch_gemm_f64_tables(reinterpret_cast<const GemmTerm*>(scratch + offTA),
                                     reinterpret_cast<const GemmGroup*>(scratch + offGA),
-                                    reinterpret_cast<const GemmTile*>(scratch + offLA), (int)ntA, false, false,
-                                    psi_dev, R_dev, T, false, st));
+                                    reinterpret_cast<const GemmTile*>(scratch + offLA), (int)ntA, psi_dev, R_dev, T,
+                                    false, st));
     DMRG_TRY(launch_gemm_f64_tables(reinterpret_cast<const GemmTerm*>(scratch + offTB),
                                     reinterpret_cast<const GemmGroup*>(scratch + offGB),
-                                    reinterpret_cast<const GemmTile*>(scratch + offLB), (int)ntB, false, false, L_dev,
-                                    T, out_dev, true, st));
+                                    reinterpret_cast<const GemmTile*>(scratch + offLB), (int)ntB, L_dev, T, out_dev,
+                                    true, st));
     // the staging image is reused by the next call: wait until the copy has read it
     DMRG_CUDA_TRY(cudaStreamSynchronize(st));
     return DMRG_OK;

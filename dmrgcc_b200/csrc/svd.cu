@@ -894,8 +894,6 @@ int BatchedSvd::plan(const std::vector<int>& m, const std::vector<int>& n, cudaS
     max_rot = (int)sweep_rot;
     max_round_tasks = (int)round_tasks;
     max_round_gram = (int)round_gram;
-    DMRG_TRY(d_w.alloc((size_t)std::max<int64_t>(woff, 1) * sizeof(double)));
-    DMRG_TRY(d_q.alloc((size_t)std::max<int64_t>(qoff, 1) * sizeof(double)));
     const auto some = [](int64_t n) { return (size_t)std::max<int64_t>(n, 1); };
     s_size = soff;
     DMRG_TRY(d_w.alloc(some(w_size) * sizeof(double)));

@@ -2,8 +2,7 @@
 //
 // A complex product is four real DMMA products (mma.sync.m8n8k4.f64):
 //   C_re += A_re B_re - A_im B_im,   C_im += A_re B_im + A_im B_re,
-// with the term's complex scale folded into the A fragments and conjugation
-// into the sign of the imaginary parts.  CTA: 128 threads (2 x 2 warps), a
+// with the term's complex scale folded into the A fragments.  CTA: 128 threads (2 x 2 warps), a
 // 64 x 32 complex output tile (each warp 32 x 16 = 4 x 2 DMMA tiles, a real and
 // an imaginary accumulator pair per tile: 32 FP64 registers per thread), k-step
 // 8, two shared-memory stages filled by 16-byte cp.async (one complex element
@@ -17,11 +16,8 @@ namespace {
 
 constexpr int ZM = 64, ZN = 32, ZK = 8, ZT = 128;
 constexpr int APAD = ZK + 1;   // row stride (complex) of a [64][8] A tile
-constexpr int ATPAD = ZM + 1;  // row stride of a [8][64] (transposed) A tile
 constexpr int BPAD = ZN + 1;   // row stride of a [8][32] B tile
-constexpr int BTPAD = ZK + 1;  // row stride of a [32][8] (transposed) B tile
-constexpr int ASTAGE = ZM * APAD > ZK * ATPAD ? ZM * APAD : ZK * ATPAD;
-constexpr int BSTAGE = ZK * BPAD > ZN * BTPAD ? ZK * BPAD : ZN * BTPAD;
+constexpr int ASTAGE = ZM * APAD, BSTAGE = ZK * BPAD;
 
 __device__ __forceinline__ void cp_async16(double2* smem, const double2* gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -39,54 +35,45 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-template <bool TA, bool TB>
 __device__ __forceinline__ void zload(double2* As, double2* Bs, const double2* __restrict__ A,
                                       const double2* __restrict__ B, const ZGemmTerm& t, int k0, int m0, int n0,
                                       int m, int n, int tid) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int idx = tid + ZT * i;
-        const int r = TA ? (idx & 63) : (idx >> 3);
-        const int c = TA ? (idx >> 6) : (idx & 7);
+        const int r = idx >> 3, c = idx & 7;
         const bool v = (m0 + r < m) && (k0 + c < t.k);
-        const int64_t off = TA ? (int64_t)(k0 + c) * t.lda + (m0 + r) : (int64_t)(m0 + r) * t.lda + (k0 + c);
-        cp_async16(TA ? (As + c * ATPAD + r) : (As + r * APAD + c), v ? (A + t.a_off + off) : A, v);
+        cp_async16(As + r * APAD + c, v ? (A + t.a_off + (int64_t)(m0 + r) * t.lda + (k0 + c)) : A, v);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int idx = tid + ZT * i;
-        const int nn = TB ? (idx >> 3) : (idx & 31);
-        const int c = TB ? (idx & 7) : (idx >> 5);
+        const int nn = idx & 31, c = idx >> 5;
         const bool v = (n0 + nn < n) && (k0 + c < t.k);
-        const int64_t off = TB ? (int64_t)(n0 + nn) * t.ldb + (k0 + c) : (int64_t)(k0 + c) * t.ldb + (n0 + nn);
-        cp_async16(TB ? (Bs + nn * BTPAD + c) : (Bs + c * BPAD + nn), v ? (B + t.b_off + off) : B, v);
+        cp_async16(Bs + c * BPAD + nn, v ? (B + t.b_off + (int64_t)(k0 + c) * t.ldb + (n0 + nn)) : B, v);
     }
 }
 
-template <bool TA, bool TB>
 __device__ __forceinline__ void zcompute(const double2* As, const double2* Bs, double (&re)[4][2][2],
-                                         double (&im)[4][2][2], double s_re, double s_im, int conj, int wm, int wn,
-                                         int lane) {
+                                         double (&im)[4][2][2], double s_re, double s_im, int wm, int wn, int lane) {
     const int fr = lane >> 2, fc = lane & 3;
-    const double ca = (conj & 1) ? -1.0 : 1.0, cb = (conj & 2) ? -1.0 : 1.0;
 #pragma unroll
     for (int kk = 0; kk < ZK; kk += 4) {
         double ar[4], ai[4], nai[4], br[2], bi[2];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = wm * 32 + i * 8 + fr, col = kk + fc;
-            const double2 x = TA ? As[col * ATPAD + row] : As[row * APAD + col];
-            const double xr = x.x, xi = ca * x.y;
-            ar[i] = xr * s_re - xi * s_im;  // scale folded into A
-            ai[i] = xr * s_im + xi * s_re;
+            const double2 x = As[row * APAD + col];
+            ar[i] = x.x * s_re - x.y * s_im;  // scale folded into A
+            ai[i] = x.x * s_im + x.y * s_re;
             nai[i] = -ai[i];
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int kr = kk + fc, nc = wn * 16 + j * 8 + fr;
-            const double2 y = TB ? Bs[nc * BTPAD + kr] : Bs[kr * BPAD + nc];
+            const double2 y = Bs[kr * BPAD + nc];
             br[j] = y.x;
-            bi[j] = cb * y.y;
+            bi[j] = y.y;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -100,7 +87,6 @@ __device__ __forceinline__ void zcompute(const double2* As, const double2* Bs, d
     }
 }
 
-template <bool TA, bool TB>
 __global__ void __launch_bounds__(ZT) zgemm_kernel(const double2* __restrict__ A, const double2* __restrict__ B,
                                                    double2* __restrict__ C, const ZGemmTerm* __restrict__ terms,
                                                    const GemmGroup* __restrict__ groups,
@@ -120,7 +106,7 @@ __global__ void __launch_bounds__(ZT) zgemm_kernel(const double2* __restrict__ A
     if (t < g.t1) {
         ZGemmTerm cur = terms[t];
         int k0 = 0, stage = 0;
-        zload<TA, TB>(smA[0], smB[0], A, B, cur, 0, tile.m0, tile.n0, g.m, g.n, tid);
+        zload(smA[0], smB[0], A, B, cur, 0, tile.m0, tile.n0, g.m, g.n, tid);
         cp_commit();
         for (;;) {
             int nk0 = k0 + ZK, nt = t;
@@ -132,14 +118,14 @@ __global__ void __launch_bounds__(ZT) zgemm_kernel(const double2* __restrict__ A
             }
             const bool has_next = nt < g.t1;
             if (has_next) {
-                zload<TA, TB>(smA[stage ^ 1], smB[stage ^ 1], A, B, nxt, nk0, tile.m0, tile.n0, g.m, g.n, tid);
+                zload(smA[stage ^ 1], smB[stage ^ 1], A, B, nxt, nk0, tile.m0, tile.n0, g.m, g.n, tid);
                 cp_commit();
                 cp_wait<1>();
             } else {
                 cp_wait<0>();
             }
             __syncthreads();
-            zcompute<TA, TB>(smA[stage], smB[stage], re, im, cur.s_re, cur.s_im, cur.conj, wm, wn, lane);
+            zcompute(smA[stage], smB[stage], re, im, cur.s_re, cur.s_im, wm, wn, lane);
             __syncthreads();
             if (!has_next) break;
             stage ^= 1;
@@ -182,8 +168,8 @@ int ZGemmSchedule::check_bounds(int64_t a_size, int64_t b_size, int64_t c_size) 
         for (int ti = g.t0; ti < g.t1; ++ti) {
             const ZGemmTerm& t = terms[ti];
             if (t.k <= 0) continue;
-            const int64_t ae = ta ? t.a_off + (int64_t)(t.k - 1) * t.lda + g.m : t.a_off + (int64_t)(g.m - 1) * t.lda + t.k;
-            const int64_t be = tb ? t.b_off + (int64_t)(g.n - 1) * t.ldb + t.k : t.b_off + (int64_t)(t.k - 1) * t.ldb + g.n;
+            const int64_t ae = t.a_off + (int64_t)(g.m - 1) * t.lda + t.k;
+            const int64_t be = t.b_off + (int64_t)(t.k - 1) * t.ldb + g.n;
             if (t.a_off < 0 || ae > a_size || t.b_off < 0 || be > b_size)
                 return set_error(DMRG_E_ARG, "complex GEMM operand outside its buffer");
         }
@@ -219,10 +205,7 @@ int launch_zgemm(const ZGemmSchedule& s, const double* A, const double* B, doubl
     const auto* gr = s.d_groups.as<GemmGroup>();
     const auto* tl = s.d_tiles.as<GemmTile>();
     const int acc = accumulate ? 1 : 0;
-    if (!s.ta && !s.tb) DMRG_LAUNCH zgemm_kernel<false, false><<<n, ZT, 0, stream>>>(a, b, c, tr, gr, tl, acc);
-    else if (s.ta && !s.tb) DMRG_LAUNCH zgemm_kernel<true, false><<<n, ZT, 0, stream>>>(a, b, c, tr, gr, tl, acc);
-    else if (!s.ta && s.tb) DMRG_LAUNCH zgemm_kernel<false, true><<<n, ZT, 0, stream>>>(a, b, c, tr, gr, tl, acc);
-    else DMRG_LAUNCH zgemm_kernel<true, true><<<n, ZT, 0, stream>>>(a, b, c, tr, gr, tl, acc);
+    DMRG_LAUNCH zgemm_kernel<<<n, ZT, 0, stream>>>(a, b, c, tr, gr, tl, acc);
     DMRG_CUDA_TRY(cudaGetLastError());
     return DMRG_OK;
 }

@@ -4,10 +4,8 @@
 // cblas_zgemm, src/tensor/complex_matrix.cc:294-318).
 //
 // Same shape as the real engine (gemm.cuh): a launch processes output blocks
-// ("groups"), each summing its terms  s_t * op(A_t) @ op(B_t)  in registers, with
-// a complex scale s_t; op() may transpose (schedule-wide TA / TB) and conjugate
-// (per term: bit 0 conjugates A, bit 1 conjugates B).  Offsets and leading
-// dimensions count complex elements.
+// ("groups"), each summing its terms  s_t * A_t @ B_t  in registers, with
+// a complex scale s_t.  Offsets and leading dimensions count complex elements.
 #pragma once
 
 #include <cstdint>
@@ -24,7 +22,7 @@ struct ZGemmTerm {
     int lda;
     int ldb;
     int k;
-    int conj;  // bit 0: conj(A), bit 1: conj(B)
+    int pad_;
     double s_re, s_im;
 };
 
@@ -32,7 +30,6 @@ struct ZGemmSchedule {
     std::vector<ZGemmTerm> terms;
     std::vector<GemmGroup> groups;  // GemmGroup::cbuf unused (no split-K)
     std::vector<GemmTile> tiles;
-    bool ta = false, tb = false;
     double flops = 0.0;  // real FLOPs: 8 m n k per term
     DeviceBuffer d_terms, d_groups, d_tiles;
 
@@ -40,16 +37,15 @@ struct ZGemmSchedule {
         terms.clear();
         groups.clear();
         tiles.clear();
-        ta = tb = false;
         flops = 0.0;
     }
     int add_group(int64_t c_off, int ldc, int m, int n) {
         groups.push_back(GemmGroup{c_off, ldc, m, n, (int)terms.size(), (int)terms.size(), 0});
         return (int)groups.size() - 1;
     }
-    void add_term(int64_t a_off, int lda, int64_t b_off, int ldb, int k, double s_re, double s_im, int conj = 0) {
+    void add_term(int64_t a_off, int lda, int64_t b_off, int ldb, int k, double s_re, double s_im) {
         GemmGroup& g = groups.back();
-        terms.push_back(ZGemmTerm{a_off, b_off, lda, ldb, k, conj, s_re, s_im});
+        terms.push_back(ZGemmTerm{a_off, b_off, lda, ldb, k, 0, s_re, s_im});
         g.t1 = (int)terms.size();
         flops += 8.0 * g.m * g.n * (double)k;
     }
