@@ -20,12 +20,12 @@ constexpr int kPair = 64;       // columns per pair
 constexpr int kChunk = 32;      // rows per streamed chunk
 constexpr int kThreads = 256;               // pair solve: one thread per 4x4 Gram block
 constexpr int kSolveThreads = kThreads + 32;  // and a warp that finds the rotations
-// Sweeps of a pair solve: one where a sector has further pairs, whose rotations undo
-// a pair's diagonality again (D = 1024, with the solve's sweep at 63 us: 10.2 ms of
-// sweeps with one, 11.6 with two, 13.4 with three); two where the pair is the whole
-// sector and a further outer sweep costs its launches (D = 64: 0.94 ms of
-// canonicalisation, 1.09 with one).
-constexpr int kInnerSweepsMany = 1, kInnerSweepsOnly = 2;
+// Sweeps of a pair solve, at most: one where a sector has further pairs, whose rotations
+// undo a pair's diagonality again (canonicalisation at D = 1024: 8.7 ms with one, 9.5
+// with two, 10.2 with three); three where the pair is the whole sector and a further outer
+// sweep costs its launches and a host round trip (D = 64: 0.94 ms with one, 0.80 with two,
+// 0.74 with three; two outer sweeps are then left).
+constexpr int kInnerSweepsMany = 1, kInnerSweepsOnly = 3;
 constexpr int kMaxSweeps = 40;
 // The sweep cap in force (dmrg_svd_set_max_sweeps lowers it to provoke the
 // did-not-converge path without touching the device).
