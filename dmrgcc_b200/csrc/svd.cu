@@ -20,12 +20,14 @@ constexpr int kPair = 64;       // columns per pair
 constexpr int kChunk = 32;      // rows per streamed chunk
 constexpr int kThreads = 256;               // pair solve: one thread per 4x4 Gram block
 constexpr int kSolveThreads = kThreads + 32;  // and a warp that finds the rotations
-// Sweeps of a pair solve, at most: one where a sector has further pairs, whose rotations
-// undo a pair's diagonality again (canonicalisation at D = 1024: 8.7 ms with one, 9.5
-// with two, 10.2 with three); three where the pair is the whole sector and a further outer
-// sweep costs its launches and a host round trip (D = 64: 0.94 ms with one, 0.80 with two,
-// 0.74 with three; two outer sweeps are then left).
-constexpr int kInnerSweepsMany = 1, kInnerSweepsOnly = 3;
+// Sweeps of a pair solve, at most, by the column blocks of the batch's largest sector
+// (a round's solves run side by side, so the batch has one number).  More than four
+// blocks: one, as a pair's other rounds undo its diagonality again (canonicalisation at
+// D = 1024, 8 blocks: 8.7 ms with one, 9.5 with two, 10.2 with three).  Up to four: two,
+// for three outer sweeps instead of five (D = 400 widened by half: 1.94 ms with one, 1.68
+// with two).  Where the pair is the whole sector: three, for two outer sweeps, each a
+// host round trip (D = 64: 0.94 ms with one, 0.80 with two, 0.74 with three).
+int inner_sweeps(int blocks) { return blocks > 4 ? 1 : blocks > 2 ? 2 : 3; }
 constexpr int kMaxSweeps = 40;
 // The sweep cap in force (dmrg_svd_set_max_sweeps lowers it to provoke the
 // did-not-converge path without touching the device).
@@ -353,7 +355,7 @@ __device__ void find_rotations(SvdSmem& S, int par, const QuadClass& qc, int lan
 // pair rotations, are found beside the update of Q.
 __global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SvdProblem* __restrict__ probs,
                                                               const SvdTask* __restrict__ tasks, int first,
-                                                              const double* __restrict__ gpart,
+                                                              int inner_sweeps, const double* __restrict__ gpart,
                                                               const double* __restrict__ fro2,
                                                               double* __restrict__ rot, int* __restrict__ skip) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -411,7 +413,6 @@ __global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SvdProblem* 
     if (tid == 0) skip[blockIdx.x] = rotate ? 0 : 1;
     if (!rotate) return;
 
-    const int inner_sweeps = p.nbe > 2 ? kInnerSweepsMany : kInnerSweepsOnly;
     const int gi = tid >> 4, gj = tid & 15;  // a worker's Gram block; for Q: rows 4 gi .. 4 gi + 3, group gj
     if (!worker) find_rotations(S, 0, QuadClass(0), lane, zero2, tol2f);
     __syncthreads();
@@ -1117,8 +1118,12 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
                                                         work.expo, work.part + (int64_t)np * kSlices);
     DMRG_LAUNCH fro2_kernel<<<(np + 127) / 128, 128, 0, st>>>(work.part + (int64_t)np * kSlices, np, work.fro2);
     static const bool debug = std::getenv("DMRG_SVD_DEBUG") != nullptr;  // per-sweep convergence to stderr
-    int max_cols = 0;
-    for (const SvdProblem& p : probs) max_cols = std::max(max_cols, p.cols);
+    int max_cols = 0, max_blocks = 0;
+    for (const SvdProblem& p : probs) {
+        max_cols = std::max(max_cols, p.cols);
+        max_blocks = std::max(max_blocks, p.nbe);
+    }
+    const int sweeps = inner_sweeps(max_blocks);
     const dim3 colgrid(np, (max_cols + 7) / 8);
     const dim3 rankgrid(np, (max_cols + 255) / 256);
     // Preconditioner: W P = Q1 R, R^T = Q2 R2, sweeps on X = R2^T (X J = Y), so that
@@ -1189,7 +1194,7 @@ int BatchedSvd::run(cudaStream_t st, int* sweeps_out) {
             DMRG_LAUNCH gram_kernel<<<ng, 128, 0, st>>>(xp, work.tasks, work.gram_items + round_gram_first[r],
                                                         work.colmap, x, work.gpart);
             DMRG_LAUNCH solve_kernel<<<nt, kSolveThreads, sizeof(SvdSmem), st>>>(
-                xp, work.tasks, round_first[r], work.gpart, work.fro2, work.rot, work.skip);
+                xp, work.tasks, round_first[r], sweeps, work.gpart, work.fro2, work.rot, work.skip);
             DMRG_LAUNCH rotate_kernel<<<nr, 128, kRotSmem, st>>>(xp, work.tasks, work.rot_items + round_rot_first[r],
                                                                  round_first[r], work.rot, work.skip, work.colmap, x,
                                                                  qx);
