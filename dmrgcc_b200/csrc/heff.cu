@@ -395,7 +395,7 @@ int dmrg_heff_profile(dmrg_heff_t h, const double* psi, double* out, double* ms_
     if (err != cudaSuccess) return set_error(DMRG_E_CUDA, "profile: %s", cudaGetErrorString(err));
     *ms_stage_a = a;
     *ms_stage_b = b;
-    return DMRG_OK;
+    return take_device_status(h->ctx);  // a bounded wait that gave up
 }
 
 int dmrg_heff_apply_host(dmrg_heff_t h, const double* psi_host, double* out_host, int accumulate) {

@@ -350,8 +350,8 @@ __device__ void find_rotations(SvdSmem& S, int par, const QuadClass& qc, int lan
 // class (QuadClass) through their six pairs each and applies the 4x4 rotations to G
 // and Q: 21 steps a sweep, each one
 // pass over G and two barriers.  (Rotating 32 disjoint pairs at a time, 63 passes over
-// G a sweep, took 76 us for one sweep and 133 for two; 41 and 68 so, and the same
-// number of outer sweeps or one fewer.)  The next class's rotations, a chain of three
+// G a sweep, took 76 us for one sweep at D = 1024, 47 so, and the same number of outer
+// sweeps or one fewer.)  The next class's rotations, a chain of three
 // pair rotations, are found beside the update of Q.
 __global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SvdProblem* __restrict__ probs,
                                                               const SvdTask* __restrict__ tasks, int first,

@@ -98,3 +98,16 @@ def test_lanczos_reports(own_ctx, kind, m, n):
     own_ctx.sync()
     own_ctx.set_wait_polls(-1)
     op.close()
+
+
+def test_profile_reports(own_ctx):
+    op, _, _ = _case(own_ctx, "heff", 9, 17, 1)
+    psi, out = capi.DeviceArray(own_ctx, 9 * 17), capi.DeviceArray(own_ctx, 9 * 17)
+    psi.zero()
+    out.zero()
+    own_ctx.set_wait_polls(0)
+    with pytest.raises(capi.DmrgError) as err:
+        op.profile(psi, out)
+    assert err.value.code == capi.E_NUMERIC
+    own_ctx.sync()
+    op.close()
