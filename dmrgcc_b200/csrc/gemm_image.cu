@@ -27,9 +27,9 @@
 // launch: the time of a step depends on what the SM's other CTA runs).  A long tile
 // is cut into parts, summed in order by the last CTA to finish one.
 //
-// Measured, one H_eff*psi of the 8x4 cylinder's middle site: D=1024 216 -> 184 us
+// Measured, one H_eff*psi of the 8x4 cylinder's middle site: D=1024 216 -> 186 us
 // (pack 10, first stage 70, second 105; its DMMAs alone 104 us at the 37 TFLOP/s of
-// a register-only loop), D=300 59 -> 22.5 us, 16-site chain at D=64 21.5 -> 15.5 us.
+// a register-only loop), D=300 59 -> 22.5 us, 16-site chain at D=64 21.5 -> 14.8 us.
 // What bounds it now: at D=1024 the DMMA pipe (75% busy; the rest is the tiles'
 // epilogues with one other CTA to cover them, and the last tiles); below D~300 three
 // launches' latency and the k-step chain of one tile.

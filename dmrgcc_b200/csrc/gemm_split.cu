@@ -607,8 +607,9 @@ int PackedSchedule::finalize(cudaStream_t stream, int num_sms) {
     splits.clear();
     tiles.clear();
     aux_size = 0;
-    // A tile's time in cycles.  The MMA side: a stage's six MMAs, or its copies at what
-    // an SM gets of L2 when all of them read.  The epilogue: a term's read-out (64
+    // A tile's time in cycles.  The MMA side: a stage's six MMAs, or its copies, counted at
+    // 60 bytes a cycle (a weight that balances the tiles, not a measured limit: L2 runs at
+    // a fifth of its peak).  The epilogue: a term's read-out (64
     // conversions a thread are most of it), then the output store.  The two overlap.
     // (Counted as 4 per stage + 1 per term + 6 per tile, a launch's longest CTA took
     // twice the shortest: D = 600 BF16 matvec 39.8 us, 38.1 with this; D = 1024 TF32

@@ -12,9 +12,9 @@
 // vec_lanczos_step) instead of one modified Gram-Schmidt pass (2(i+1) dependent
 // steps); the tridiagonal's lowest eigenvalue comes from Sturm bisection on the
 // device instead of dsyevd.
-// One B200, us per call: 16-site chain D=64, 20 iterations 1279 -> 736 (vector work
+// One B200, us per call: 16-site chain D=64, 20 iterations 1279 -> 749 (vector work
 // in one kernel, the tridiagonal step beside the matvec, packed matvecs); cylinder
-// D=512, 12 iterations 1630 -> 1103.  Bound now by the chain of five dependent
+// D=512, 12 iterations 1630 -> 1110.  Bound now by the chain of five dependent
 // kernels of an iteration (37 us at n = 2,037).
 // psi_dim < 100 takes the reference's exact-diagonalisation branch (:34-56):
 // the dense H_eff is assembled column by column from matvecs on unit vectors

@@ -13,7 +13,7 @@
 // pivoting (whose norms serialise the panels): 24 against 38 rounds on a
 // 400 x 250 matrix.  Whole canonicalisation, D = 1024 cylinder tensor (17 sectors to
 // 611 x 510): 47.2 ms without, 12.8 ms with; D = 64 chain tensor (33 columns):
-// 2.03 and 0.92 ms (8.5 and 0.77 with the later pair solve and panels).  A sweep first orders the columns by descending norm
+// 2.03 and 0.92 ms (8.7 and 0.75 with the later pair solve and panels).  A sweep first orders the columns by descending norm
 // (de Rijk's pivoting, applied block-wise), then measures every pair of column
 // blocks at once (the 32x32 cross-Gram blocks, DMMA) and visits only the block
 // pairs found unconverged, in as few rounds as a matching of them allows (the round-robin

@@ -5,7 +5,8 @@
 // complex blocks and a complex MPO: stage A T = K R, stage B out += w L T, on
 // the packed real forms of the blocks (gemm_image.cu).  One complex grouped GEMM
 // (zgemm.cu) per stage, one CTA per 64x32 tile and no split k, took 175 us for the
-// 6x6 Hofstadter cylinder's middle site at D=256 (0.38 GFLOP); now 49 us.  ComplexTensorLanczos::LanczosMethod
+// 6x6 Hofstadter cylinder's middle site at D=256 (0.38 GFLOP); now 53 us (49 with its
+// buffers warm in L2).  ComplexTensorLanczos::LanczosMethod
 // (complex_tensor_lanczos.cc:14-160): alpha_i = <v_i|h> with the conjugated
 // product, h -= alpha_i v_i with the complex alpha, beta_i = sqrt(Re <h|h>), the
 // tridiagonal problem on Re alpha and beta (zheevd reads only the real diagonal
