@@ -67,8 +67,8 @@ namespace {
 // sectors of an input block of bond index `o`, block u of the ket list with sector x
 // (left: of its rows, right: of its columns) makes the stage 1 product, every block v
 // with sector y a term, per output index with a nonzero weight; the output block has the
-// other sectors of u and v.  One pass: the terms, in the order of the reference's loops,
-// flag the output blocks, and are then sorted into them.
+// other sectors of u and v.  One pass collects the terms, in the order of the reference's
+// loops; they are then sorted, stably, by output block, and the blocks are those that occur.
 int build_products(dmrg_env_s& e) {
     const SiteDesc& s = e.site;
     const BlockListDesc& ket = s.ket;
@@ -107,12 +107,12 @@ int build_products(dmrg_env_s& e) {
             }
         }
     struct Term {
-        int key;  // output index and sectors
+        int row, j;  // output index and first sector, index * ny + sector; second sector
         Stage2Term t;
     };
     EnvProducts& pr = e.products;
     std::vector<Term> terms;
-    std::vector<int> count((size_t)out_bond * ny * ny, 0);  // terms by key
+    std::vector<int> row_first((size_t)out_bond * ny + 1, 0);  // terms by row: counts, then first
     double f1_alg = 0, f2_alg = 0, f1_exec = 0, f2_exec = 0;
     for (int o = 0; o < in_bond; ++o) {
         const BlockListDesc& in = e.in.o[o];
@@ -136,10 +136,10 @@ int build_products(dmrg_env_s& e) {
                     f2_alg += f;
                     const size_t at = ((size_t)o * s.d + pu) * s.d + pv;
                     for (int x = outs_first[at]; x < outs_first[at + 1]; ++x) {
-                        const int q = outs[x], key = (q * ny + osec[u]) * ny + osec[v];
+                        const int q = outs[x], row = q * ny + osec[u];
                         const double w = left ? s.w(o, q, pu, pv) : s.w(q, o, pv, pu);
-                        terms.push_back(Term{key, Stage2Term{(int)pr.tasks.size(), v, w}});
-                        ++count[key];
+                        terms.push_back(Term{row, osec[v], Stage2Term{(int)pr.tasks.size(), v, w}});
+                        ++row_first[row + 1];
                         f2_exec += f;
                     }
                 }
@@ -151,21 +151,27 @@ int build_products(dmrg_env_s& e) {
             }
         }
     }
+    for (size_t r = 1; r < row_first.size(); ++r) row_first[r] += row_first[r - 1];
+    std::vector<int> order(terms.size()), next(row_first.begin(), row_first.end() - 1);
+    for (int i = 0; i < (int)terms.size(); ++i) order[next[terms[i].row]++] = i;
     e.out.o.assign(out_bond, BlockListDesc());
     pr.first.assign(1, 0);
-    std::vector<int> next(count.size());  // where a key's next term goes
-    int n = 0;
-    for (int q = 0, key = 0; q < out_bond; ++q)
-        for (int i = 0; i < ny; ++i)
-            for (int j = 0; j < ny; ++j, ++key) {
-                if (!count[key]) continue;
-                e.out.o[q].push(i, j, dim[i], dim[j]);
-                next[key] = n;
-                pr.first.push_back(n += count[key]);
+    pr.terms.reserve(terms.size());
+    for (int r = 0; r + 1 < (int)row_first.size(); ++r) {
+        const auto b = order.begin() + row_first[r], end = order.begin() + row_first[r + 1];
+        auto second = [&](int x, int y) { return terms[x].j < terms[y].j; };
+        if (!std::is_sorted(b, end, second)) std::stable_sort(b, end, second);  // (one second sector, mostly)
+        for (auto x = b; x != end; ++x) {
+            const Term& t = terms[*x];
+            if (x == b || t.j != terms[x[-1]].j) {
+                if (x != b) pr.first.push_back((int)pr.terms.size());
+                e.out.o[r / ny].push(r % ny, t.j, dim[r % ny], dim[t.j]);
             }
+            pr.terms.push_back(t.t);
+        }
+        if (b != end) pr.first.push_back((int)pr.terms.size());
+    }
     e.out.rebase();
-    pr.terms.resize(terms.size());
-    for (const Term& t : terms) pr.terms[next[t.key]++] = t.t;
     e.flops_alg = f1_alg + f2_alg;
     e.flops_exec = f1_exec + f2_exec;
     return DMRG_OK;

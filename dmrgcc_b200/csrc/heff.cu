@@ -55,13 +55,18 @@ int build_heff(dmrg_heff_s& h) {
     };
     std::vector<TaskA> tasks;
     double fa_alg = 0, fb = 0, fa_exec = 0;
-    // blocks before each bond index; L blocks by (bond index, sectors), first in list order;
-    // by (o2, p1, p2): the bond indexes o1 with a nonzero weight, ascending
-    std::vector<int> l_first(1, 0), r_first(1, 0), l_at((size_t)s.lb * s.nl * s.nl, -1), o1s, o1s_first(1, 0);
+    // blocks before each bond index; the L blocks of a bond index and left sector, chained in
+    // list order; by (o2, p1, p2): the bond indexes o1 with a nonzero weight, ascending
+    std::vector<int> l_first(1, 0), r_first(1, 0), l_head((size_t)s.lb * s.nl, -1), l_next, o1s, o1s_first(1, 0);
     for (int o = 0; o < s.lb; ++o) {
-        for (int q = h.L.o[o].count() - 1; q >= 0; --q)
-            l_at[((size_t)o * s.nl + h.L.o[o].left[q]) * s.nl + h.L.o[o].right[q]] = q;
-        l_first.push_back(l_first.back() + h.L.o[o].count());
+        const int first = l_first.back();
+        l_next.resize(first + h.L.o[o].count());
+        for (int q = h.L.o[o].count() - 1; q >= 0; --q) {
+            int& head = l_head[(size_t)o * s.nl + h.L.o[o].left[q]];
+            l_next[first + q] = head;
+            head = q;
+        }
+        l_first.push_back((int)l_next.size());
     }
     for (int o = 0; o < s.rb; ++o) r_first.push_back(r_first.back() + h.R.o[o].count());
     for (int o2 = 0; o2 < s.rb; ++o2)
@@ -100,7 +105,8 @@ int build_heff(dmrg_heff_s& h) {
                     for (int x = o1s_first[at]; x < o1s_first[at + 1]; ++x) {
                         const int o1 = o1s[x];
                         const double w = s.w(o1, o2, p1, p2);
-                        const int q = l_at[((size_t)o1 * s.nl + idx) * s.nl + kdx];
+                        int q = l_head[(size_t)o1 * s.nl + idx];
+                        while (q != -1 && h.L.o[o1].right[q] != kdx) q = l_next[l_first[o1] + q];
                         if (q == -1) continue;
                         const int lr = h.L.o[o1].rows[q], lc = h.L.o[o1].cols[q];
                         if (lc != a_k || lr != ket.rows[pos2] || rc != ket.cols[pos2])
